@@ -2,8 +2,8 @@
 //
 // The full path (dsss_pd_sort) is laid out for one GPU holding every PE:
 //   1. one string sort of all n strings (K3, LCP as by-product);
-//   2. distinguishing-prefix rounds over that global order (K1/K2) — the
-//      result per string does not depend on the PE split;
+//   2. distinguishing prefixes from that order's LCPs (K1) — the result per
+//      string does not depend on the PE split;
 //   3. stable multisplit by PE of the global order gives each PE's local sorted
 //      order (a subsequence of a sorted sequence is sorted), i.e. exactly what
 //      radixsort_CI3 produces per PE (prefix_doubling.hpp:228);
@@ -247,9 +247,8 @@ struct PdLayout {
     uint64_t *pb, *bounds, *recv_begin;
     void* ms;
     SortLayout sort;
-    DpLayout dp;
     PartitionLayout part;
-    unsigned long long* rdig;  // prefix hashes at the first schedule depths, from the sort's first pass
+    uint32_t* minlen;
 };
 
 // n strings in nsets sets of p PEs each.
@@ -274,11 +273,8 @@ static void layout_pd(Carve& c, PdLayout& L, uint64_t n, uint32_t nsets, uint32_
     L.recv_begin = c.take<uint64_t>(npe + 1);
     L.ms = c.take<unsigned char>(multisplit_scratch_bytes(N, (uint32_t)npe));
     layout_sort(c, L.sort, N, nsets, small_max);
-    layout_dp(c, L.dp, N, nsets);
     layout_partition(c, L.part, N, p, factor, nsets);
-    // decided by a value both carving passes see (the sizing pass hands out
-    // null pointers)
-    L.rdig = L.dp.digest_share ? c.take<unsigned long long>(ROOT_DIGESTS * N) : nullptr;
+    L.minlen = c.take<uint32_t>(1);
 }
 
 // The fused path over nsets independent string sets of p PEs each (PE q of
@@ -329,11 +325,9 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
     a.h = L.handles;
     DSSS_CUDA(cudaMemsetAsync(L.err, 0, sizeof(uint32_t), st));
     // 1. one sort per set, all sets in one segmented sort
-    uint32_t rdig_mask = 0;
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, L.ord, L.lcp, smax, pin, st,
-                              p > 1 ? L.rdig : nullptr, &rdig_mask));
+        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, L.ord, L.lcp, smax, pin, st));
     }
     if (p == 1) {  // prefix_doubling.hpp:236: one PE sorts locally and returns no permutation
         DSSS_CUDA(cudaMemcpyAsync(out->local_order, L.ord, n * 4, cudaMemcpyDeviceToDevice, st));
@@ -344,8 +338,7 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
     // 2. distinguishing prefixes over each set's sorted order
     {
         StageTimer t("stage:dp", st);
-        DSSS_TRY(dp_rounds(L.dp, a, n, L.ord, L.lcp, L.dpg, nullptr, 0, nullptr, pin, st, nsets, set_begin.data(),
-                           rdig_mask ? L.rdig : nullptr, rdig_mask));
+        DSSS_TRY(dp_from_lcps(a, n, L.ord, L.lcp, L.minlen, L.dpg, st));
     }
     // 3. local orders per PE
     StageTimer t_local("stage:local", st);

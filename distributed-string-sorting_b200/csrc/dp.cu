@@ -18,6 +18,16 @@
 // prefix hash is shared with another candidate does not depend on which PE
 // holds either string, so one table over all PEs gives the same survivors.
 // The hash table is sized by the number of strings hashed in the round.
+//
+// Where one GPU holds every PE, the global sorted order and its LCPs decide
+// the rounds without a hash (dp_from_lcps): the strings that share a string's
+// d-byte prefix are its neighbours with LCPs of at least d, all of them still
+// candidates, since they share every shorter prefix too.  So a string stays in
+// the round at depth d exactly while m = max(LCP with its predecessor, LCP
+// with its successor) >= d, and its distinguishing prefix is the schedule's
+// first depth above m, or its length if that is smaller.  (The rounds differ
+// from this only if two different prefixes have the same 64-bit hash.)  The
+// hash rounds are for orders that are sorted per PE only.
 #include "internal.cuh"
 #include "dp.cuh"
 #include "util.cuh"
@@ -109,15 +119,36 @@ __global__ void __launch_bounds__(256) k_min_nbr_lcp(const uint32_t* lcp, uint64
     if ((threadIdx.x & 31) == 0 && m != 0xFFFFFFFFu) atomicMin(out, m);
 }
 
-// Index of the string set holding sorted position i (set_begin: nsets+1 bounds).
-__device__ __forceinline__ uint32_t set_of(const uint64_t* set_begin, uint32_t nsets, uint64_t i) {
-    uint32_t lo = 0, hi = nsets;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (set_begin[mid] <= i) lo = mid;
-        else hi = mid;
-    }
-    return lo;
+// The first depth above m of the schedule 8, 24, 40, 72, ..., 8 + 8 * 2^k.
+__device__ __forceinline__ uint64_t dp_depth_above(uint32_t m) {
+    if (m < 8) return 8;
+    const uint32_t k = 32 - __clz((m - 8) >> 3);  // the smallest k with 8 * 2^k > m - 8
+    return 8 + (8ull << max(k, 1u));
+}
+
+// One thread per sorted position.  Bound by HBM: 4 bytes of LCP read and 4
+// written per string; the length (a random read through the order) only where
+// the depth exceeds the shortest string.
+__global__ void __launch_bounds__(256) k_dp_from_lcps(ArenaDev a, const uint32_t* order, const uint32_t* lcp,
+                                                      uint64_t n, const uint32_t* minlen, uint32_t* dp) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint64_t d = dp_depth_above(max(i ? lcp[i] : 0u, i + 1 < n ? lcp[i + 1] : 0u));
+    if (d > *minlen) d = min(d, (uint64_t)a.len[order[i]]);
+    dp[i] = (uint32_t)d;
+}
+
+int dp_from_lcps(const ArenaDev& a, uint64_t n, const uint32_t* order, const uint32_t* lcp, uint32_t* minlen,
+                 uint32_t* dp, cudaStream_t st) {
+    if (n == 0) return DSSS_OK;
+    DSSS_CUDA(cudaMemsetAsync(minlen, 0xFF, sizeof(uint32_t), st));
+    DSSS_LAUNCH("k_min_len", st,
+                k_min_len<<<(unsigned)std::min<uint64_t>(grid_for(a.n, 256), 148 * 8), 256, 0, st>>>(a.len, a.h, a.n,
+                                                                                                   minlen));
+    DSSS_LAUNCH("k_dp_from_lcps", st,
+                k_dp_from_lcps<<<grid_for(n, 256), 256, 0, st>>>(a, order, lcp, n, minlen, dp));
+    DSSS_CUDA(cudaGetLastError());
+    return DSSS_OK;
 }
 
 // Adds the block's number of true flags to *ctr with one atomic per block
@@ -169,16 +200,11 @@ __global__ void __launch_bounds__(256) k_dp_mark(const uint8_t* kind, const uint
 }
 
 // Grid-stride over positions (grid a few blocks per SM): one pair of counter
-// atomics per block instead of per 256 positions.  hmask (with order): every
-// hashed string is marked for the arena-order form of the round (an atomic
-// OR into a bitmap of n bits, which stays in L2; random byte stores into a
-// byte per string measured slower).  lens (the
-// lengths in sorted order) may be null when every string reaches depth.
+// atomics per block instead of per 256 positions.  lens (the lengths in
+// sorted order) may be null when every string reaches depth.
 __global__ void __launch_bounds__(256) k_dp_classify(const uint8_t* st, int all, const uint32_t* lens,
                                                      const uint32_t* lcp, uint64_t n, uint32_t depth, uint32_t* dp,
-                                                     uint8_t* st_next, uint8_t* kind, uint32_t* counters,
-                                                     const uint64_t* set_begin, uint32_t nsets, uint32_t* set_cnt,
-                                                     const uint32_t* order = nullptr, uint32_t* hmask = nullptr) {
+                                                     uint8_t* st_next, uint8_t* kind, uint32_t* counters) {
     uint32_t nhashed = 0, nstays = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i - threadIdx.x % 32 < n; i += stride) {
@@ -206,26 +232,18 @@ __global__ void __launch_bounds__(256) k_dp_classify(const uint8_t* st, int all,
             st_next[i] = nx;
             nstays += nx;
             nhashed += hashed;
-            if (hashed && hmask) mark_string(hmask, order[i]);
-        }
-        if (nsets > 1) {  // hashed strings per set size the per-set table regions
-            const int lane = threadIdx.x & 31;
-            const uint32_t sid = hashed ? set_of(set_begin, nsets, i) : 0xFFFFFFFFu - lane;
-            const uint32_t peers = __match_any_sync(FULLM, sid);
-            if (hashed && lane == __ffs(peers) - 1) atomicAdd(&set_cnt[sid], (uint32_t)__popc(peers));
         }
     }
     block_add(counters + 0, nhashed);
     block_add(counters + 1, nstays);
 }
 
-// k_dp_classify for one string set over 16-byte-aligned arrays: four
+// k_dp_classify over 16-byte-aligned arrays: four
 // consecutive positions per thread, read and written as vectors (the same
 // per-position rule; st of the neighbours i - 1 and i + 4 read singly).
 __global__ void __launch_bounds__(256) k_dp_classify4(const uint8_t* st, int all, const uint32_t* lens,
                                                       const uint32_t* lcp, uint64_t n, uint32_t depth, uint32_t* dp,
-                                                      uint8_t* st_next, uint8_t* kind, uint32_t* counters,
-                                                      const uint32_t* order = nullptr, uint32_t* hmask = nullptr) {
+                                                      uint8_t* st_next, uint8_t* kind, uint32_t* counters) {
     uint32_t nhashed = 0, nstays = 0;
     const uint64_t groups = n >> 2;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -275,7 +293,6 @@ __global__ void __launch_bounds__(256) k_dp_classify4(const uint8_t* st, int all
             K[q] = k;
             X[q] = nx;
             nstays += nx;
-            if (k >= 2 && hmask) mark_string(hmask, order[i]);
         }
         if (all) {
             reinterpret_cast<uint4*>(dp)[t] = make_uint4(D[0], D[1], D[2], D[3]);
@@ -307,7 +324,6 @@ __global__ void __launch_bounds__(256) k_dp_classify4(const uint8_t* st, int all
                     k = root ? 3 : 2;
                     nx = root ? 1 : 0;
                     ++nhashed;
-                    if (hmask) mark_string(hmask, order[i]);
                 }
             }
         }
@@ -321,10 +337,10 @@ __global__ void __launch_bounds__(256) k_dp_classify4(const uint8_t* st, int all
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// Inserts h into the table region (base, mask) by linear probing; returns its
-// slot, NO_SLOT when the region is full.  The table always has free slots, so
+// Inserts h into the table of mask + 1 slots by linear probing; returns its
+// slot, NO_SLOT when the table is full.  The table always has free slots, so
 // a free or matching slot is reached within mask + 1 probes.
-__device__ __forceinline__ uint32_t table_insert(unsigned long long* tkeys, uint8_t* tdup, uint64_t base, uint32_t mask,
+__device__ __forceinline__ uint32_t table_insert(unsigned long long* tkeys, uint8_t* tdup, uint32_t mask,
                                                  unsigned long long h, uint32_t* err, uint32_t* ndup) {
     uint32_t sl = (uint32_t)(h ^ (h >> 32)) & mask;
     for (uint32_t probe = 0;; ++probe) {
@@ -332,35 +348,25 @@ __device__ __forceinline__ uint32_t table_insert(unsigned long long* tkeys, uint
             atomicExch(err, 1u);
             return NO_SLOT;
         }
-        const unsigned long long prev = atomicCAS(&tkeys[base + sl], EMPTY_KEY, h);
+        const unsigned long long prev = atomicCAS(&tkeys[sl], EMPTY_KEY, h);
         if (prev == EMPTY_KEY) break;
         if (prev == h) {
-            tdup[base + sl] = 1;
+            tdup[sl] = 1;
             atomicAdd(ndup, 1u);
             break;
         }
         sl = (sl + 1) & mask;
     }
-    return (uint32_t)(base + sl);
+    return sl;
 }
 
-// Each string set owns a power-of-two region of the table (base, mask): equal
-// prefixes in different sets are not duplicates of each other.
 __global__ void __launch_bounds__(256, 5) k_dp_hash(ArenaDev a, const uint64_t* soff, const uint8_t* kind, uint64_t n, uint32_t depth,
-                          unsigned long long* tkeys, uint8_t* tdup, uint32_t mask1, const uint64_t* set_begin,
-                          uint32_t nsets, const uint64_t* set_base, const uint32_t* set_mask, uint32_t* slot,
-                          uint32_t* err, uint32_t* ndup) {
+                          unsigned long long* tkeys, uint8_t* tdup, uint32_t mask, uint32_t* slot, uint32_t* err,
+                          uint32_t* ndup) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || kind[i] < 2) return;
-    uint64_t base = 0;
-    uint32_t mask = mask1;
-    if (nsets > 1) {
-        const uint32_t sid = set_of(set_begin, nsets, i);
-        base = set_base[sid];
-        mask = set_mask[sid];
-    }
     const unsigned long long h = filter_hash(xxh64_dev(a.chars + soff[i], depth));
-    slot[i] = table_insert(tkeys, tdup, base, mask, h, err, ndup);
+    slot[i] = table_insert(tkeys, tdup, mask, h, err, ndup);
 }
 
 // k_dp_hash for rounds that hash few positions (e.g. only the roots of long
@@ -371,9 +377,8 @@ __global__ void __launch_bounds__(256, 5) k_dp_hash(ArenaDev a, const uint64_t* 
 __global__ void __launch_bounds__(256) k_dp_hash_sparse(ArenaDev a, const uint64_t* soff, const uint32_t* order,
                                                         const uint8_t* kind, uint64_t n,
                                                         uint32_t depth, unsigned long long* tkeys, uint8_t* tdup,
-                                                        uint32_t mask1, const uint64_t* set_begin, uint32_t nsets,
-                                                        const uint64_t* set_base, const uint32_t* set_mask,
-                                                        uint32_t* slot, uint32_t* err, uint32_t* ndup) {
+                                                        uint32_t mask, uint32_t* slot, uint32_t* err,
+                                                        uint32_t* ndup) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t groups = (n + 15) / 16;
     for (uint64_t g = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += stride) {
@@ -399,13 +404,6 @@ __global__ void __launch_bounds__(256) k_dp_hash_sparse(ArenaDev a, const uint64
         for (int b = 0; b < 16; ++b) {
             if (!((w[b >> 2] >> (8 * (b & 3))) & 2u)) continue;
             const uint64_t i = g * 16 + b;
-            uint64_t base = 0;
-            uint32_t mask = mask1;
-            if (nsets > 1) {
-                const uint32_t sid = set_of(set_begin, nsets, i);
-                base = set_base[sid];
-                mask = set_mask[sid];
-            }
             uint64_t off;
             if (soff) {
                 off = soff[i];
@@ -414,7 +412,7 @@ __global__ void __launch_bounds__(256) k_dp_hash_sparse(ArenaDev a, const uint64
                 str_of(a, order[i], off, len);
             }
             const unsigned long long h = filter_hash(xxh64_dev(a.chars + off, depth));
-            slot[i] = table_insert(tkeys, tdup, base, mask, h, err, ndup);
+            slot[i] = table_insert(tkeys, tdup, mask, h, err, ndup);
         }
     }
 }
@@ -426,20 +424,16 @@ static bool sparse_round(uint64_t hashed, uint64_t n) { return hashed * 8 < n; }
 
 static int launch_dp_hash(const ArenaDev& a, const uint64_t* soff, const uint32_t* order, const uint8_t* kind,
                           uint64_t n, uint32_t depth,
-                          uint64_t hashed, unsigned long long* tkeys, uint8_t* tdup, uint32_t mask1,
-                          const uint64_t* set_begin, uint32_t nsets, const uint64_t* set_base,
-                          const uint32_t* set_mask, uint32_t* slot, uint32_t* err, uint32_t* ndup,
-                          cudaStream_t st) {
+                          uint64_t hashed, unsigned long long* tkeys, uint8_t* tdup, uint32_t mask, uint32_t* slot,
+                          uint32_t* err, uint32_t* ndup, cudaStream_t st) {
     if (sparse_round(hashed, n)) {
         DSSS_LAUNCH("k_dp_hash", st,
                     k_dp_hash_sparse<<<stride_grid((n + 15) / 16), 256, 0, st>>>(a, soff, order, kind, n, depth, tkeys,
-                                                                     tdup, mask1,
-                                                                     set_begin, nsets, set_base, set_mask, slot, err,
-                                                                     ndup));
+                                                                                 tdup, mask, slot, err, ndup));
     } else {
         DSSS_LAUNCH("k_dp_hash", st,
-                    k_dp_hash<<<grid_for(n, 256), 256, 0, st>>>(a, soff, kind, n, depth, tkeys, tdup, mask1, set_begin,
-                                                               nsets, set_base, set_mask, slot, err, ndup));
+                    k_dp_hash<<<grid_for(n, 256), 256, 0, st>>>(a, soff, kind, n, depth, tkeys, tdup, mask, slot, err,
+                                                               ndup));
     }
     return DSSS_OK;
 }
@@ -455,28 +449,18 @@ __global__ void __launch_bounds__(256, 5) k_dp_hash_store(ArenaDev a, const uint
 }
 
 __global__ void __launch_bounds__(256) k_dp_insert(const uint8_t* kind, uint64_t n, const unsigned long long* hbuf,
-                                                   unsigned long long* tkeys, uint8_t* tdup, uint32_t mask1,
-                                                   const uint64_t* set_begin, uint32_t nsets, const uint64_t* set_base,
-                                                   const uint32_t* set_mask, uint32_t* slot, uint32_t* err,
-                                                   uint32_t* ndup) {
+                                                   unsigned long long* tkeys, uint8_t* tdup, uint32_t mask,
+                                                   uint32_t* slot, uint32_t* err, uint32_t* ndup) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || kind[i] < 2) return;
-    uint64_t base = 0;
-    uint32_t mask = mask1;
-    if (nsets > 1) {
-        const uint32_t sid = set_of(set_begin, nsets, i);
-        base = set_base[sid];
-        mask = set_mask[sid];
-    }
-    slot[i] = table_insert(tkeys, tdup, base, mask, hbuf[i], err, ndup);
+    slot[i] = table_insert(tkeys, tdup, mask, hbuf[i], err, ndup);
 }
 
 // Dense hash rounds (at least 1/dp_digest of the positions hash) run in arena
 // order.  The classification marks every hashed string (kinds 2 and 3) in the
 // arena-order bitmap hmask; k_dp_arena_insert walks the strings front to
-// back, so the d-byte prefixes are read in address order (at the first
-// schedule depths it reads the hashes the string sort's first pass stored
-// instead), and inserts the hash of every marked string into the table.  The first insert of a hash
+// back, so the d-byte prefixes are read in address order, and inserts the
+// hash of every marked string into the table.  The first insert of a hash
 // owns its slot (tid); an equal later insert marks the slot shared and its
 // own string in the arena-order bitmap dmask.  k_dp_owner_dups then adds the
 // owners of shared slots to dmask, and k_dp_query_mask keeps every kind-2
@@ -486,50 +470,29 @@ __global__ void __launch_bounds__(256) k_dp_insert(const uint8_t* kind, uint64_t
 // back by the query.
 __device__ __forceinline__ bool bit_of(const uint32_t* m, uint64_t s) { return (m[s >> 5] >> (s & 31)) & 1u; }
 
-__global__ void __launch_bounds__(256) k_dp_arena_insert(ArenaDev a, uint32_t depth, const unsigned long long* dig,
-                                                         const uint32_t* hmask,
+__global__ void __launch_bounds__(256) k_dp_arena_insert(ArenaDev a, uint32_t depth, const uint32_t* hmask,
                                                          unsigned long long* tkeys, uint8_t* tdup, uint32_t* tid,
-                                                         uint32_t mask1, const uint64_t* set_begin, uint32_t nsets,
-                                                         const uint64_t* set_base, const uint32_t* set_mask,
-                                                         uint32_t* dmask, uint32_t* err, uint32_t* ndup,
-                                                         uint32_t check, uint32_t* bad) {
+                                                         uint32_t mask, uint32_t* dmask, uint32_t* err,
+                                                         uint32_t* ndup) {
     const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.n || (hmask && !bit_of(hmask, s))) return;
-    unsigned long long h;
-    if (dig) {  // stored by the string sort's first pass
-        h = dig[s];
-        if (check) {
-            uint64_t off;
-            uint32_t L;
-            str_of(a, (uint32_t)s, off, L);
-            if (h != filter_hash(xxh64_dev(a.chars + off, depth))) atomicExch(bad, 1u);
-        }
-    } else {
-        uint64_t off;
-        uint32_t L;
-        str_of(a, (uint32_t)s, off, L);
-        h = filter_hash(xxh64_dev(a.chars + off, depth));
-    }
-    uint64_t base = 0;
-    uint32_t mask = mask1;
-    if (nsets > 1) {  // a set's strings occupy the same index range in the arena and in the order
-        const uint32_t sid = set_of(set_begin, nsets, s);
-        base = set_base[sid];
-        mask = set_mask[sid];
-    }
+    uint64_t off;
+    uint32_t L;
+    str_of(a, (uint32_t)s, off, L);
+    const unsigned long long h = filter_hash(xxh64_dev(a.chars + off, depth));
     uint32_t sl = (uint32_t)(h ^ (h >> 32)) & mask;
     for (uint32_t probe = 0;; ++probe) {
         if (probe > mask) {
             atomicExch(err, 1u);
             return;
         }
-        const unsigned long long prev = atomicCAS(&tkeys[base + sl], EMPTY_KEY, h);
+        const unsigned long long prev = atomicCAS(&tkeys[sl], EMPTY_KEY, h);
         if (prev == EMPTY_KEY) {
-            tid[base + sl] = (uint32_t)s;
+            tid[sl] = (uint32_t)s;
             return;
         }
         if (prev == h) {
-            tdup[base + sl] = 1;
+            tdup[sl] = 1;
             atomicAdd(ndup, 1u);
             atomicOr(&dmask[s >> 5], 1u << (s & 31));
             return;
@@ -563,18 +526,15 @@ static uint32_t pd_buckets(uint64_t hashed) {
     return nb;
 }
 
-// The round's hashes of the hashed strings, in arena order, when the string
-// sort's first pass did not store them (or, check, to compare with them).
-__global__ void __launch_bounds__(256) k_dp_arena_hash(ArenaDev a, uint32_t depth, const unsigned long long* dig,
-                                                       const uint32_t* hmask, unsigned long long* out, uint32_t* bad) {
+// The round's hashes of the hashed strings, in arena order.
+__global__ void __launch_bounds__(256) k_dp_arena_hash(ArenaDev a, uint32_t depth, const uint32_t* hmask,
+                                                       unsigned long long* out) {
     const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.n || (hmask && !bit_of(hmask, s))) return;
     uint64_t off;
     uint32_t L;
     str_of(a, (uint32_t)s, off, L);
-    const unsigned long long h = filter_hash(xxh64_dev(a.chars + off, depth));
-    if (dig && h != dig[s]) atomicExch(bad, 1u);
-    out[s] = h;
+    out[s] = filter_hash(xxh64_dev(a.chars + off, depth));
 }
 
 // Pass 1 counts: per tile of PP_TILE arena positions, the hashed strings per
@@ -812,11 +772,10 @@ __global__ void k_pp_starts(const uint32_t* off1, uint32_t ntiles1, const uint32
     }
 }
 
-// One block per bucket: every pair whose hash occurs again in the bucket
-// (in the same string set) has its string marked in dmask.
+// One block per bucket: every pair whose hash occurs again in the bucket has
+// its string marked in dmask.
 __global__ void __launch_bounds__(PD_NT) k_dp_bucket_dups(const uint32_t* fstart, const unsigned long long* ph,
                                                           const uint32_t* ps, uint32_t* dmask, uint32_t* ndup,
-                                                          const uint64_t* set_begin, uint32_t nsets,
                                                           uint32_t* overflow) {
     extern __shared__ __align__(16) unsigned char pd_sm[];
     unsigned long long* key = (unsigned long long*)pd_sm;
@@ -842,8 +801,7 @@ __global__ void __launch_bounds__(PD_NT) k_dp_bucket_dups(const uint32_t* fstart
         for (uint32_t probe = 0; probe < PD_TAB; ++probe) {
             const uint32_t prev = atomicCAS(&tab[sl], 0xFFFFFFFFu, j);
             if (prev == 0xFFFFFFFFu) break;
-            if (key[prev] == h &&
-                (nsets <= 1 || set_of(set_begin, nsets, bs[prev]) == set_of(set_begin, nsets, bs[j]))) {
+            if (key[prev] == h) {
                 dup[j] = 1;
                 dup[prev] = 1;
                 break;
@@ -938,60 +896,6 @@ static uint64_t table_slots(uint64_t n) {
     return t;
 }
 
-// Per-set table regions, the same rule with 64 slots at least (none for a set
-// that hashes nothing).  Total <= 3 * hashed + 68 * nsets.
-__device__ __forceinline__ uint64_t set_slots(uint32_t c) {
-    if (c == 0) return 0;
-    uint64_t t = 64;
-    while (t < (uint64_t)c + c / 2 + 2) t <<= 1;
-    return t;
-}
-
-// Per-set filter regions in 32-bit words: a power of two >= bpk bits per
-// hashed string, 1024 bits at least.
-__device__ __forceinline__ uint64_t set_filter_bits(uint32_t c, uint32_t bpk) {
-    if (c == 0) return 0;
-    uint64_t t = 1024;
-    while (t < (uint64_t)c * bpk) t <<= 1;
-    return t;
-}
-
-constexpr int SET_NT = 1024;
-
-// One block: region base and mask per set from the per-set counts, total into
-// out[0..1] (lo, hi), *err set if it exceeds cap.  bpk == 0: hash-table
-// regions (slots); bpk > 0: filter regions (base in words, mask in bits).
-__global__ void __launch_bounds__(SET_NT) k_set_tables(const uint32_t* cnt, uint32_t nsets, uint64_t cap, uint32_t bpk,
-                                                       uint64_t* base, uint32_t* mask, uint32_t* out, uint32_t* err) {
-    __shared__ uint64_t part[SET_NT];
-    const uint32_t per = (nsets + SET_NT - 1) / SET_NT;
-    const uint32_t b = min(nsets, threadIdx.x * per), e = min(nsets, b + per);
-    auto size_of = [&](uint32_t c) -> uint64_t { return bpk ? set_filter_bits(c, bpk) / 32 : set_slots(c); };
-    uint64_t sum = 0;
-    for (uint32_t s = b; s < e; ++s) sum += size_of(cnt[s]);
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (int off = 1; off < SET_NT; off <<= 1) {
-        const uint64_t v = threadIdx.x >= (unsigned)off ? part[threadIdx.x - off] : 0;
-        __syncthreads();
-        part[threadIdx.x] += v;
-        __syncthreads();
-    }
-    uint64_t run = part[threadIdx.x] - sum;
-    for (uint32_t s = b; s < e; ++s) {
-        const uint64_t sl = size_of(cnt[s]);
-        base[s] = run;
-        mask[s] = sl ? (uint32_t)((bpk ? sl * 32 : sl) - 1) : 0;
-        run += sl;
-    }
-    if (threadIdx.x == SET_NT - 1) {
-        const uint64_t total = part[SET_NT - 1];
-        if (total > cap) *err = 1;
-        out[0] = (uint32_t)total;
-        out[1] = (uint32_t)(total >> 32);
-    }
-}
-
 // ---------------------------------------------------- fingerprint filter ----
 // Rounds that hash many strings find duplicate hashes without a table entry
 // per string: each hashed string sets one bit, chosen by its hash, of a
@@ -1002,25 +906,16 @@ __global__ void __launch_bounds__(SET_NT) k_set_tables(const uint32_t* cnt, uint
 // per duplicated hash; a string whose hash is not in that table is unique.
 // The outcome is exactly that of one table over all hashes.
 __global__ void k_dp_filter(ArenaDev a, const uint64_t* soff, const uint8_t* kind, uint64_t n, uint32_t depth,
-                            uint32_t* bits, uint32_t bmask1, const uint64_t* set_begin, uint32_t nsets,
-                            const uint64_t* set_wbase, const uint32_t* set_bmask, unsigned long long* hbuf,
-                            uint32_t* cand, uint32_t* ncand, uint32_t* set_ccnt) {
+                            uint32_t* bits, uint32_t bmask, unsigned long long* hbuf, uint32_t* cand,
+                            uint32_t* ncand) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     bool c = false;
-    uint32_t sid = 0;
     if (i < n && kind[i] >= 2) {
         const unsigned long long h = filter_hash(xxh64_dev(a.chars + soff[i], depth));
         hbuf[i] = h;
-        uint64_t wbase = 0;
-        uint32_t bm = bmask1;
-        if (nsets > 1) {
-            sid = set_of(set_begin, nsets, i);
-            wbase = set_wbase[sid];
-            bm = set_bmask[sid];
-        }
-        const uint32_t b = (uint32_t)(h >> 32) & bm;
+        const uint32_t b = (uint32_t)(h >> 32) & bmask;
         const uint32_t bit = 1u << (b & 31);
-        c = (atomicOr(&bits[wbase + (b >> 5)], bit) & bit) != 0;
+        c = (atomicOr(&bits[b >> 5], bit) & bit) != 0;
     }
     const int lane = threadIdx.x & 31;
     const uint32_t m = __ballot_sync(FULLM, c);
@@ -1029,45 +924,23 @@ __global__ void k_dp_filter(ArenaDev a, const uint64_t* soff, const uint8_t* kin
         if (lane == __ffs(m) - 1) base = atomicAdd(ncand, (uint32_t)__popc(m));
         base = __shfl_sync(FULLM, base, __ffs(m) - 1);
         if (c) cand[base + __popc(m & ((1u << lane) - 1u))] = (uint32_t)i;
-        if (nsets > 1) {
-            const uint32_t key = c ? sid : 0xFFFFFFFFu - lane;
-            const uint32_t peers = __match_any_sync(FULLM, key);
-            if (c && lane == __ffs(peers) - 1) atomicAdd(&set_ccnt[sid], (uint32_t)__popc(peers));
-        }
-    }
-}
-
-// Table region of position i: (base, mask).
-__device__ __forceinline__ void table_region(const uint64_t* set_begin, uint32_t nsets, const uint64_t* set_base,
-                                             const uint32_t* set_mask, uint32_t mask1, uint64_t i, uint64_t& base,
-                                             uint32_t& mask) {
-    base = 0;
-    mask = mask1;
-    if (nsets > 1) {
-        const uint32_t sid = set_of(set_begin, nsets, i);
-        base = set_base[sid];
-        mask = set_mask[sid];
     }
 }
 
 // Inserts the candidates' hashes (each distinct hash once).
 __global__ void k_cand_insert(const uint32_t* cand, uint32_t ncand, const unsigned long long* hbuf,
-                              unsigned long long* tkeys, uint32_t mask1, const uint64_t* set_begin, uint32_t nsets,
-                              const uint64_t* set_base, const uint32_t* set_mask, uint32_t* err) {
+                              unsigned long long* tkeys, uint32_t mask, uint32_t* err) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= ncand) return;
     const uint32_t i = cand[j];
     const unsigned long long h = hbuf[i];
-    uint64_t base;
-    uint32_t mask;
-    table_region(set_begin, nsets, set_base, set_mask, mask1, i, base, mask);
     uint32_t sl = (uint32_t)(h ^ (h >> 32)) & mask;
     for (uint32_t probe = 0;; ++probe) {
         if (probe > mask) {
             atomicExch(err, 1u);
             return;
         }
-        const unsigned long long prev = atomicCAS(&tkeys[base + sl], EMPTY_KEY, h);
+        const unsigned long long prev = atomicCAS(&tkeys[sl], EMPTY_KEY, h);
         if (prev == EMPTY_KEY || prev == h) return;
         sl = (sl + 1) & mask;
     }
@@ -1076,26 +949,21 @@ __global__ void k_cand_insert(const uint32_t* cand, uint32_t ncand, const unsign
 // Every hashed string whose hash is in the candidate table counts itself
 // there: tcnt byte bit 0 = seen, bit 1 = seen twice or more.
 __global__ void k_dp_count(const uint8_t* kind, uint64_t n, const unsigned long long* hbuf,
-                           const unsigned long long* tkeys, uint32_t* tcnt_words, uint32_t mask1,
-                           const uint64_t* set_begin, uint32_t nsets, const uint64_t* set_base,
-                           const uint32_t* set_mask, uint32_t* slot, uint32_t* err) {
+                           const unsigned long long* tkeys, uint32_t* tcnt_words, uint32_t mask, uint32_t* slot,
+                           uint32_t* err) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n || kind[i] < 2) return;
     const unsigned long long h = hbuf[i];
-    uint64_t base;
-    uint32_t mask;
-    table_region(set_begin, nsets, set_base, set_mask, mask1, i, base, mask);
     uint32_t sl = (uint32_t)(h ^ (h >> 32)) & mask;
     uint32_t found = NO_SLOT;
-    // a set without candidates has no region (mask 0): nothing to find
-    for (uint32_t probe = 0; mask != 0; ++probe) {
+    for (uint32_t probe = 0;; ++probe) {
         if (probe > mask) {
             atomicExch(err, 1u);
             break;
         }
-        const unsigned long long k = tkeys[base + sl];
+        const unsigned long long k = tkeys[sl];
         if (k == h) {
-            found = (uint32_t)(base + sl);
+            found = sl;
             break;
         }
         if (k == EMPTY_KEY) break;
@@ -1127,14 +995,8 @@ static uint64_t pow2_at_least(uint64_t x, uint64_t lo) {
     return t;
 }
 
-void layout_dp(Carve& c, DpLayout& L, uint64_t n, uint32_t nsets) {
+void layout_dp(Carve& c, DpLayout& L, uint64_t n) {
     uint64_t N = n ? n : 1;
-    if (nsets == 0) nsets = 1;
-    L.nsets_cap = nsets;
-    L.set_begin = c.take<uint64_t>(nsets + 1);
-    L.set_base = c.take<uint64_t>(nsets + 1);
-    L.set_mask = c.take<uint32_t>(nsets);
-    L.set_cnt = c.take<uint32_t>(nsets);
     L.st[0] = c.take<uint8_t>(N);
     L.st[1] = c.take<uint8_t>(N);
     L.kind = c.take<uint8_t>(N);
@@ -1142,15 +1004,10 @@ void layout_dp(Carve& c, DpLayout& L, uint64_t n, uint32_t nsets) {
     L.soff = c.take<uint64_t>(N);
     L.minlen = c.take<uint32_t>(2);  // shortest string, smallest neighbour LCP
     L.slot = c.take<uint32_t>(N);
-    // one set: the table for n keys; several: room for every set's own
-    // power-of-two region (at most 3 slots per key plus 68 per set)
-    L.slots = nsets == 1 ? table_slots(N) : 3 * N + 128ull * (nsets + 1);
+    L.slots = table_slots(N);
     L.tkeys = c.take<unsigned long long>(L.slots);
     L.tdup = c.take<uint8_t>(L.slots + 4);
     L.counters = c.take<uint32_t>(16);
-    L.set_bbase = c.take<uint64_t>(nsets);
-    L.set_bmask = c.take<uint32_t>(nsets);
-    L.set_ccnt = c.take<uint32_t>(nsets);
     // fingerprint filter: planned when a round may hash dp_filter_min strings
     L.filter_min = (uint64_t)tune(TUNE_DP_FILTER_MIN);
     L.filter_bpk = (uint32_t)tune(TUNE_DP_FILTER_BITS);
@@ -1195,7 +1052,7 @@ void layout_dp(Carve& c, DpLayout& L, uint64_t n, uint32_t nsets) {
     const bool filter = N >= L.filter_min;
     L.hbuf = (filter || L.split) ? c.take<unsigned long long>(N) : nullptr;
     if (filter) {
-        L.bm_words = (nsets == 1 ? pow2_at_least(N * L.filter_bpk, 1024) : 2 * N * L.filter_bpk + 1024ull * nsets) / 32;
+        L.bm_words = pow2_at_least(N * L.filter_bpk, 1024) / 32;
         L.bits = c.take<uint32_t>(L.bm_words);
         L.cand = c.take<uint32_t>(N);
     } else {
@@ -1207,18 +1064,11 @@ void layout_dp(Carve& c, DpLayout& L, uint64_t n, uint32_t nsets) {
 
 int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* order, const uint32_t* lcp,
               uint32_t* dp, uint64_t* round_counts, uint32_t max_rounds, uint32_t* rounds, uint32_t* pin,
-              cudaStream_t st, uint32_t nsets, const uint64_t* set_begin_host, const unsigned long long* rdig,
-              uint32_t rdig_mask) {
+              cudaStream_t st) {
     uint32_t r = 0;
     if (n == 0) {
         if (rounds) *rounds = 0;
         return DSSS_OK;
-    }
-    if (nsets == 0) nsets = 1;
-    if (nsets > 1) {
-        if (!set_begin_host || nsets > L.nsets_cap) return fail(DSSS_EINVAL, "string sets not planned");
-        DSSS_CUDA(cudaMemcpyAsync(L.set_begin, set_begin_host, (nsets + 1) * sizeof(uint64_t),
-                                  cudaMemcpyHostToDevice, st));
     }
     const unsigned grid = grid_for(n, 256);
     // lengths and offsets in sorted order are gathered (k_dp_lens, one random
@@ -1259,75 +1109,50 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
             continue;
         }
         DSSS_CUDA(cudaMemsetAsync(L.counters, 0, 16 * sizeof(uint32_t), st));
-        if (nsets > 1) DSSS_CUDA(cudaMemsetAsync(L.set_cnt, 0, nsets * sizeof(uint32_t), st));
         // a round that may turn out dense marks its hashed strings for the
         // arena-order form (every string of the arena must be in the order)
         const bool mark = L.hmask && a.n <= n && cands * L.digest_share >= n;
-        // the hashed strings are marked after the count, only when not every
-        // string of the arena is hashed (a null mask then stands for all)
-        uint32_t* hm = nullptr;
         if (depth > min_len) DSSS_TRY(need_lens());
         const uint32_t* lens = lens_ready ? L.lens : nullptr;  // nullptr: every string reaches the depth
-        if (nsets == 1 && aligned16(lcp) && aligned16(dp) && aligned16(L.lens) && aligned16(L.st[cur]) &&
+        if (aligned16(lcp) && aligned16(dp) && aligned16(L.lens) && aligned16(L.st[cur]) &&
             aligned16(L.st[cur ^ 1]) && aligned16(L.kind)) {
             DSSS_LAUNCH("k_dp_classify", st,
                         k_dp_classify4<<<stride_grid((n + 3) / 4), 256, 0, st>>>(L.st[cur], all_cands, lens, lcp, n,
                                                                                 (uint32_t)depth, dp, L.st[cur ^ 1],
-                                                                                L.kind, L.counters, order, hm));
+                                                                                L.kind, L.counters));
         } else {
             DSSS_LAUNCH("k_dp_classify", st,
                         k_dp_classify<<<stride_grid(n), 256, 0, st>>>(L.st[cur], all_cands, lens, lcp, n, (uint32_t)depth,
-                                                                     dp, L.st[cur ^ 1], L.kind, L.counters,
-                                                                     L.set_begin, nsets, L.set_cnt, order, hm));
-        }
-        if (nsets > 1) {
-            DSSS_LAUNCH("k_set_tables", st,
-                        k_set_tables<<<1, SET_NT, 0, st>>>(L.set_cnt, nsets, L.slots, 0, L.set_base, L.set_mask,
-                                                           L.counters + 4, L.counters + 2));
-            if (L.bits)
-                DSSS_LAUNCH("k_set_tables", st,
-                            k_set_tables<<<1, SET_NT, 0, st>>>(L.set_cnt, nsets, L.bm_words, L.filter_bpk,
-                                                               L.set_bbase, L.set_bmask, L.counters + 6,
-                                                               L.counters + 2));
+                                                                     dp, L.st[cur ^ 1], L.kind, L.counters));
         }
         DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         DSSS_CUDA(cudaStreamSynchronize(st));
         const uint32_t hashed = pin[0];
-        if (pin[2]) return fail(DSSS_EDEVICE, "distinguishing-prefix hash table regions exceed the plan");
         if (hashed && L.bits && hashed >= L.filter_min) {
             // fingerprint filter, then an exact table over the candidates only
             DSSS_TRY(need_lens());
-            const uint64_t words = nsets > 1 ? ((uint64_t)pin[7] << 32 | pin[6])
-                                             : pow2_at_least((uint64_t)hashed * L.filter_bpk, 1024) / 32;
+            const uint64_t words = pow2_at_least((uint64_t)hashed * L.filter_bpk, 1024) / 32;
             if (words > L.bm_words) return fail(DSSS_EDEVICE, "distinguishing-prefix filter exceeds the plan");
             DSSS_CUDA(cudaMemsetAsync(L.bits, 0, words * 4, st));
-            if (nsets > 1) DSSS_CUDA(cudaMemsetAsync(L.set_ccnt, 0, nsets * sizeof(uint32_t), st));
             DSSS_LAUNCH("k_dp_filter", st,
                         k_dp_filter<<<grid, 256, 0, st>>>(a, L.soff, L.kind, n, (uint32_t)depth, L.bits,
-                                                         (uint32_t)(words * 32 - 1), L.set_begin, nsets, L.set_bbase,
-                                                         L.set_bmask, L.hbuf, L.cand, L.counters + 3, L.set_ccnt));
-            if (nsets > 1)
-                DSSS_LAUNCH("k_set_tables", st,
-                            k_set_tables<<<1, SET_NT, 0, st>>>(L.set_ccnt, nsets, L.slots, 0, L.set_base, L.set_mask,
-                                                               L.counters + 4, L.counters + 2));
+                                                         (uint32_t)(words * 32 - 1), L.hbuf, L.cand,
+                                                         L.counters + 3));
             DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
             DSSS_CUDA(cudaStreamSynchronize(st));
-            if (pin[2]) return fail(DSSS_EDEVICE, "distinguishing-prefix hash table regions exceed the plan");
             const uint32_t ncand = pin[3];
             if (ncand) {  // else every hash is unique: no kind-2 string stays
-                const uint64_t slots = nsets > 1 ? ((uint64_t)pin[5] << 32 | pin[4]) : table_slots(ncand);
+                const uint64_t slots = table_slots(ncand);
                 if (slots > L.slots) return fail(DSSS_EDEVICE, "distinguishing-prefix hash table exceeds the plan");
                 DSSS_CUDA(cudaMemsetAsync(L.tkeys, 0xFF, slots * sizeof(unsigned long long), st));
                 DSSS_CUDA(cudaMemsetAsync(L.tdup, 0, (slots + 3) & ~3ull, st));
                 DSSS_LAUNCH("k_cand_insert", st,
                             k_cand_insert<<<grid_for(ncand, 256), 256, 0, st>>>(L.cand, ncand, L.hbuf, L.tkeys,
-                                                                                 (uint32_t)(slots - 1), L.set_begin,
-                                                                                 nsets, L.set_base, L.set_mask,
+                                                                                 (uint32_t)(slots - 1),
                                                                                  L.counters + 2));
                 DSSS_LAUNCH("k_dp_count", st,
                             k_dp_count<<<grid, 256, 0, st>>>(L.kind, n, L.hbuf, L.tkeys, (uint32_t*)L.tdup,
-                                                            (uint32_t)(slots - 1), L.set_begin, nsets, L.set_base,
-                                                            L.set_mask, L.slot, L.counters + 2));
+                                                            (uint32_t)(slots - 1), L.slot, L.counters + 2));
                 DSSS_LAUNCH("k_dp_query", st,
                             k_dp_query_cnt<<<grid, 256, 0, st>>>(L.kind, L.slot, L.tdup, n, L.st[cur ^ 1],
                                                                 L.counters));
@@ -1337,10 +1162,9 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                 if (pin[2]) return fail(DSSS_EDEVICE, "distinguishing-prefix hash table overflow");
             }
         } else if (hashed) {
-            const uint64_t slots = nsets > 1 ? ((uint64_t)pin[5] << 32 | pin[4]) : table_slots(hashed);
+            const uint64_t slots = table_slots(hashed);
             if (slots > L.slots) return fail(DSSS_EDEVICE, "distinguishing-prefix hash table exceeds the plan");
             const bool arena = mark && (uint64_t)hashed * L.digest_share >= n;
-            const uint32_t check = (uint32_t)tune(TUNE_DP_CHECK);
             const uint32_t* hmask = nullptr;  // every string of the arena hashed
             if (arena && hashed < a.n) {
                 DSSS_CUDA(cudaMemsetAsync(L.hmask, 0, L.mask_words * sizeof(uint32_t), st));
@@ -1349,9 +1173,6 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                 hmask = L.hmask;
             }
             if (arena) {
-                const int dj = root_digest_index(depth);
-                const unsigned long long* dig =
-                    rdig && dj >= 0 && ((rdig_mask >> dj) & 1u) ? rdig + (uint64_t)dj * a.n : nullptr;
                 // buckets in shared memory first; the table only if a bucket overflows
                 bool done = false;
                 uint32_t bbits = 1;  // at least two buckets (both radix shifts stay below 64)
@@ -1361,18 +1182,15 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                     static std::atomic<uint64_t> pd_configured{0};
                     DSSS_TRY(set_smem_once(pd_configured, k_dp_bucket_dups, (int)PD_SMEM));
                     DSSS_CUDA(cudaMemsetAsync(L.dmask, 0, L.mask_words * sizeof(uint32_t), st));
-                    const unsigned long long* hd = dig;
-                    if (!dig || check) {  // this round's hashes, in arena order
-                        DSSS_LAUNCH("k_dp_arena_hash", st,
-                                    k_dp_arena_hash<<<grid_for(a.n, 256), 256, 0, st>>>(
-                                        a, (uint32_t)depth, check ? dig : nullptr, hmask, L.pp_dig, L.counters + 9));
-                        hd = L.pp_dig;
-                    }
+                    // this round's hashes, in arena order
+                    DSSS_LAUNCH("k_dp_arena_hash", st,
+                                k_dp_arena_hash<<<grid_for(a.n, 256), 256, 0, st>>>(a, (uint32_t)depth, hmask,
+                                                                                   L.pp_dig));
                     // two radix passes: top b1 bits, then the next b2 inside each coarse bucket
                     const uint32_t b1 = std::min<uint32_t>(bbits, 8), b2 = bbits - b1;
                     const uint32_t nt1 = (uint32_t)((a.n + PP_TILE - 1) / PP_TILE);
                     DSSS_LAUNCH("k_pp_hist1", st,
-                                k_pp_hist1<<<nt1, PP_NT, 0, st>>>(a.n, hd, hmask, b1, nt1, L.pp_hist));
+                                k_pp_hist1<<<nt1, PP_NT, 0, st>>>(a.n, L.pp_dig, hmask, b1, nt1, L.pp_hist));
                     DSSS_TRY(exclusive_scan_u32(L.pp_hist, L.pp_off, 256ull * nt1, L.pp_total, L.pp_scan, st));
                     const unsigned long long* ph = L.pp_h1;
                     const uint32_t* ps = L.pp_s1;
@@ -1380,7 +1198,7 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                     DSSS_TRY(set_smem_once(pp1_configured, k_pp_scatter1, (int)PP_SMEM));
                     DSSS_TRY(set_smem_once(pp2_configured, k_pp_scatter2, (int)PP_SMEM));
                     DSSS_LAUNCH("k_pp_scatter1", st,
-                                k_pp_scatter1<<<nt1, PP_NT, PP_SMEM, st>>>(a.n, hd, hmask, b1, nt1, L.pp_off, L.pp_h1,
+                                k_pp_scatter1<<<nt1, PP_NT, PP_SMEM, st>>>(a.n, L.pp_dig, hmask, b1, nt1, L.pp_off, L.pp_h1,
                                                                            L.pp_s1));
                     uint32_t* off2 = nullptr;
                     if (b2) {
@@ -1406,8 +1224,7 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                                                                                   off2, b2, nb, L.pd_start));
                     DSSS_LAUNCH("k_dp_bucket_dups", st,
                                 k_dp_bucket_dups<<<nb, PD_NT, PD_SMEM, st>>>(L.pd_start, ph, ps, L.dmask,
-                                                                            L.counters + 8, L.set_begin, nsets,
-                                                                            L.counters + 10));
+                                                                            L.counters + 8, L.counters + 10));
                     DSSS_CUDA(cudaGetLastError());
                     DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 12 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
                     DSSS_CUDA(cudaStreamSynchronize(st));
@@ -1420,9 +1237,8 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                     DSSS_CUDA(cudaMemsetAsync(L.dmask, 0, L.mask_words * sizeof(uint32_t), st));
                     DSSS_LAUNCH("k_dp_arena_insert", st,
                                 k_dp_arena_insert<<<grid_for(a.n, 256), 256, 0, st>>>(
-                                    a, (uint32_t)depth, dig, hmask, L.tkeys, L.tdup, L.tid, (uint32_t)(slots - 1),
-                                    L.set_begin, nsets, L.set_base, L.set_mask, L.dmask, L.counters + 2,
-                                    L.counters + 8, check, L.counters + 9));
+                                    a, (uint32_t)depth, hmask, L.tkeys, L.tdup, L.tid, (uint32_t)(slots - 1), L.dmask,
+                                    L.counters + 2, L.counters + 8));
                     DSSS_LAUNCH("k_dp_owner_dups", st,
                                 k_dp_owner_dups<<<stride_grid(slots / 4), 256, 0, st>>>(
                                     (const uint32_t*)L.tdup, L.tid, slots / 4, L.dmask, L.counters + 8));
@@ -1441,13 +1257,12 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
                                 k_dp_hash_store<<<grid, 256, 0, st>>>(a, L.soff, L.kind, n, (uint32_t)depth, L.hbuf));
                     DSSS_LAUNCH("k_dp_insert", st,
                                 k_dp_insert<<<grid, 256, 0, st>>>(L.kind, n, L.hbuf, L.tkeys, L.tdup,
-                                                                 (uint32_t)(slots - 1), L.set_begin, nsets, L.set_base,
-                                                                 L.set_mask, L.slot, L.counters + 2, L.counters + 8));
+                                                                 (uint32_t)(slots - 1), L.slot, L.counters + 2,
+                                                                 L.counters + 8));
                 } else {
                     DSSS_TRY(launch_dp_hash(a, lens_ready ? L.soff : nullptr, order, L.kind, n, (uint32_t)depth, hashed,
-                                            L.tkeys, L.tdup,
-                                            (uint32_t)(slots - 1), L.set_begin, nsets, L.set_base, L.set_mask, L.slot,
-                                            L.counters + 2, L.counters + 8, st));
+                                            L.tkeys, L.tdup, (uint32_t)(slots - 1), L.slot, L.counters + 2,
+                                            L.counters + 8, st));
                 }
                 DSSS_LAUNCH("k_dp_query", st,
                             k_dp_query<<<stride_grid(n), 256, 0, st>>>(L.kind, L.slot, L.tdup, n, L.st[cur ^ 1],
@@ -1457,7 +1272,6 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
             DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 10 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
             DSSS_CUDA(cudaStreamSynchronize(st));
             if (pin[2]) return fail(DSSS_EDEVICE, "distinguishing-prefix hash table overflow");
-            if (pin[9]) return fail(DSSS_EDEVICE, "a stored prefix hash differs from the string's (dp_check)");
         }
         const uint32_t m = pin[1];
         if (round_counts && r < max_rounds) round_counts[r] = m;
@@ -1519,7 +1333,7 @@ int dp_one_round(const DpRoundLayout& R, const ArenaDev& a, uint64_t n, const ui
     }
     DSSS_LAUNCH("k_dp_classify", st,
                 k_dp_classify<<<stride_grid(n), 256, 0, st>>>(L.st[0], all, L.lens, lcp, n, depth, dp, L.st[1], L.kind,
-                                                   L.counters, nullptr, 1, nullptr));
+                                                   L.counters));
     DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));
     if (pin[3]) return fail(DSSS_EINVAL, "candidates must be ascending positions below n");
@@ -1527,8 +1341,8 @@ int dp_one_round(const DpRoundLayout& R, const ArenaDev& a, uint64_t n, const ui
         const uint64_t slots = table_slots(pin[0]);
         DSSS_CUDA(cudaMemsetAsync(L.tkeys, 0xFF, slots * sizeof(unsigned long long), st));
         DSSS_CUDA(cudaMemsetAsync(L.tdup, 0, slots, st));
-        DSSS_TRY(launch_dp_hash(a, L.soff, order, L.kind, n, depth, pin[0], L.tkeys, L.tdup, (uint32_t)(slots - 1), nullptr,
-                                1, nullptr, nullptr, L.slot, L.counters + 2, L.counters + 8, st));
+        DSSS_TRY(launch_dp_hash(a, L.soff, order, L.kind, n, depth, pin[0], L.tkeys, L.tdup, (uint32_t)(slots - 1),
+                                L.slot, L.counters + 2, L.counters + 8, st));
         DSSS_LAUNCH("k_dp_query", st,
                     k_dp_query<<<stride_grid(n), 256, 0, st>>>(L.kind, L.slot, L.tdup, n, L.st[1], L.counters,
                                                               L.counters + 8));
@@ -1594,7 +1408,7 @@ int dp_classify_hash(const DpSplitLayout& L, const ArenaDev& a, uint64_t n, cons
     DSSS_LAUNCH("k_dp_lens", st, k_dp_lens<<<lens_grid(n), 256, 0, st>>>(a, order, n, L.lens, L.soff));
     DSSS_LAUNCH("k_dp_classify", st,
                 k_dp_classify<<<stride_grid(n), 256, 0, st>>>(state_in, state_in == nullptr, L.lens, lcp, n, depth, dp, state_out,
-                                                   L.kind, L.counters, nullptr, 1, nullptr));
+                                                   L.kind, L.counters));
     DSSS_LAUNCH("k_hash_flags", st, k_hash_flags<<<grid, 256, 0, st>>>(L.kind, n, L.flag));
     DSSS_TRY(exclusive_scan_u32(L.flag, L.pos, n, L.counters + 4, L.scan, st));
     DSSS_LAUNCH("k_hash_compact", st,

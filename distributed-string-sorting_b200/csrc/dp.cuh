@@ -15,16 +15,8 @@ struct DpLayout {
     uint8_t* tdup;
     uint64_t slots;
     uint32_t* counters;
-    // independent string sets (batched sorts): sorted positions
-    // [set_begin[s], set_begin[s+1]) belong to set s; each set hashes into its
-    // own region [set_base[s], set_base[s] + set_mask[s] + 1) of the table
-    uint32_t nsets_cap;
-    uint64_t* set_begin;
-    uint64_t* set_base;
-    uint32_t* set_mask;
-    uint32_t* set_cnt;
     // fingerprint filter (planned when n >= filter_min): bitmap words,
-    // per-position hashes, candidate positions, per-set filter regions
+    // per-position hashes, candidate positions
     uint64_t filter_min;
     uint32_t filter_bpk;
     uint64_t bm_words;
@@ -45,8 +37,8 @@ struct DpLayout {
     // the hash's top bits in two radix passes into at most pd_nb buckets,
     // each deduplicated in shared memory: the pairs after the first pass
     // (pp_h1 / pp_s1) and after the second (pd_h / pd_s), the buckets' starts
-    // (pd_start, pd_nb + 1), the round's hashes in arena order when the sort
-    // did not store them (pp_dig), per-tile counts and their scan (pp_hist,
+    // (pd_start, pd_nb + 1), the round's hashes in arena order (pp_dig),
+    // per-tile counts and their scan (pp_hist,
     // pp_off: pp_hcap and 2 pp_hcap entries), the coarse buckets' layout
     // (pp_mid) and the passes' totals (pp_total)
     uint32_t pd_nb;
@@ -62,25 +54,21 @@ struct DpLayout {
     uint32_t* pp_mid;
     uint32_t* pp_total;
     unsigned char* pp_scan;
-    uint64_t* set_bbase;
-    uint32_t* set_bmask;
-    uint32_t* set_ccnt;
 };
 
-void layout_dp(Carve& c, DpLayout& L, uint64_t n, uint32_t nsets = 1);
+void layout_dp(Carve& c, DpLayout& L, uint64_t n);
 
 // order/lcp: strings in sorted order per PE (lcp 0 at every PE start); dp[i]
 // receives the distinguishing-prefix length of the string at position i.
-// set_begin_host (nsets + 1 bounds, NULL for one set): prefixes are only
-// duplicates of prefixes in the same set.
-// rdig (optional): the string sort's prefix hashes at the first schedule
-// depths (ROOT_DIGESTS arrays of a.n entries, array j for depth
-// root_digest_depth(j), valid where bit j of rdig_mask is set), read by the
-// arena-order rounds at those depths.
 int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* order, const uint32_t* lcp,
               uint32_t* dp, uint64_t* round_counts, uint32_t max_rounds, uint32_t* rounds, uint32_t* pin,
-              cudaStream_t st, uint32_t nsets = 1, const uint64_t* set_begin_host = nullptr,
-              const unsigned long long* rdig = nullptr, uint32_t rdig_mask = 0);
+              cudaStream_t st);
+
+// Distinguishing prefixes of strings in their global sorted order (every PE's
+// strings in one order, lcp its LCP array with 0 at every set's first string):
+// dp[i] of the string at position i.  minlen: one word of scratch.
+int dp_from_lcps(const ArenaDev& a, uint64_t n, const uint32_t* order, const uint32_t* lcp, uint32_t* minlen,
+                 uint32_t* dp, cudaStream_t st);
 
 struct DpRoundLayout {
     DpLayout dp;

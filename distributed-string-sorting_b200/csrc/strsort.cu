@@ -113,10 +113,6 @@ struct SortState {
     uint32_t seg_bits;  // the same inside the segment sorter
     uint32_t first;     // the first pass over the arena (host-driven passes)
     uint64_t cap_large, cap_small, cap_tiles, cap_chunks;
-    // first pass only: every string's prefix hashes at the first schedule
-    // depths (root_digests), ROOT_DIGESTS arrays of dig_n entries
-    unsigned long long* dig;
-    uint64_t dig_n;
     // sampled splitters: segments of at least split_min strings (0: never);
     // cap_spl tables of SPL_STRIDE keys per pass; the fix list holds
     // (position, depth) pairs of bucket starts whose LCP k_lcp_fix writes
@@ -318,18 +314,6 @@ __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uin
     const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
     const uint32_t d0 = sg.depth, cap = d0 + PREFIX_CAP;
     const uint32_t s0 = ord[sg.start];
-    // prefix hashes (first pass only) at the schedule depths past the common
-    // prefix this segment is expected to have: at or below it every string of
-    // the segment shares its prefix with the others, so a round there hashes
-    // one root per segment and never reads stored hashes; a depth skipped
-    // here is marked so that the rounds hash it from the strings
-    uint32_t dmask = 0;
-    if (S.dig) {
-        const uint32_t shared = sg.spec ? sg.spec - 1 : d0 + SPEC_MAX;
-        for (int j = 0; j < ROOT_DIGESTS; ++j)
-            if (root_digest_depth(j) > shared) dmask |= 1u << j;
-        if (dmask != (1u << ROOT_DIGESTS) - 1 && threadIdx.x == 0) atomicOr(&S.counters[15], ~dmask & 15u);
-    }
     uint64_t off0;
     uint32_t len0;
     str_of(S.a, s0, off0, len0);
@@ -357,7 +341,6 @@ __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uin
             uint32_t len;
             const uint32_t s = ord[i];
             str_of(S.a, s, off, len);
-            if (dmask) root_digests(S.a.chars + off, len, S.dig + s, S.dig_n, dmask);
             uint64_t x[PF_W];
             key_words<PF_W>(S.a.chars, off, len, d0, want, x);
             uint32_t l = D;
@@ -396,7 +379,6 @@ __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uin
         uint32_t len;
         const uint32_t s = ord[i];
         str_of(S.a, s, off, len);
-        if (dmask) root_digests(S.a.chars + off, len, S.dig + s, S.dig_n, dmask);
         // no need to compare past this thread's minimum so far
         const uint32_t lim = min(cap, mn);
         uint32_t l = 0;
@@ -2203,9 +2185,7 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
 
 int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
                  const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t small_max,
-                 uint32_t* pin, cudaStream_t st, unsigned long long* dig, uint32_t* dig_mask,
-                 const uint32_t* seg_depth) {
-    if (dig_mask) *dig_mask = 0;
+                 uint32_t* pin, cudaStream_t st, const uint32_t* seg_depth) {
     if (n == 0) return DSSS_OK;
     SortState S;
     S.a = a;
@@ -2244,14 +2224,6 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     S.fix = L.fix;
     S.cap_spl = L.cap_spl;
     S.cap_fix = L.cap_fix;
-    S.dig = nullptr;
-    S.dig_n = n;
-    // the first pass reads every string when every initial segment is large
-    // (none goes straight to the small sorts) and the ids are the arena's
-    bool dig_all = dig && !ids_in && n <= a.n;
-    for (uint32_t q = 0; dig_all && q < p; ++q)
-        if (pb_host[q + 1] - pb_host[q] <= (uint64_t)clamp_small_max(small_max)) dig_all = false;
-
     static std::atomic<uint64_t> scatter_configured{0};
     DSSS_TRY(set_smem_once(scatter_configured, k_scatter, (int)SCATTER_SMEM));
     DSSS_CUDA(cudaMemcpyAsync(L.pb, pb_host, (p + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
@@ -2276,8 +2248,6 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     uint32_t nlarge = pin[0];
     int cur = 0;
     uint32_t guard = 0;
-    S.dig = dig_all ? dig : nullptr;
-    bool first_pass = true;
     S.first = 1;
     // whether the list holds a segment without keys folded by the previous
     // scatter (no keys, a pivot pass, or the first pass): only then the
@@ -2321,10 +2291,7 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
         if (pin[10]) return fail(DSSS_EDEVICE, "string sort: internal consistency guard tripped");
         if (nlarge > L.cap_large) return fail(DSSS_EDEVICE, "string sort: large-segment list overflow");
         cur ^= 1;
-        if (first_pass && S.dig && dig_mask) *dig_mask = 15u & ~pin[15];  // depths no segment skipped
-        first_pass = false;
         S.first = 0;
-        S.dig = nullptr;
     }
     for (int b = 0; b < NBINS; ++b)
         if (pin[1 + b] > L.cap_small) return fail(DSSS_EDEVICE, "string sort: small-segment list overflow");

@@ -102,7 +102,9 @@ int dsss_ctx_kernel_times(dsss_ctx* ctx, char* buf, uint64_t len);
 int dsss_abi_version(void);
 
 /* Process-wide tuning knobs (no reference counterpart), read by every later
- * call; value -1 restores the default.  Results never depend on them.
+ * call; value -1 restores the default.  Results never depend on them.  The
+ * dp_ knobs concern the hash rounds of dsss_dp_prefixes; the full path takes
+ * the distinguishing prefixes from its global order's LCPs.
  *   dp_filter_min   hashed strings in a distinguishing-prefix round from which
  *                   duplicates are found through the fingerprint filter
  *                   (default 2^40, i.e. off: on B200 the filter's L2
@@ -149,10 +151,8 @@ int dsss_abi_version(void);
  *                   fewer passes cost more in the small-segment sorts, whose
  *                   buckets then cut across key bytes; values below 4096
  *                   count as 4096)
- *   dp_check        1: the arena-order rounds at depths 8, 24, 40 and 72,
- *                   which read the prefix hashes the string sort's first pass
- *                   stored, recompute each from the string and fail with
- *                   DSSS_EDEVICE on a mismatch (a self-check; default 0)
+ *   dp_check        0 (default) or 1: accepted, without effect (no round
+ *                   reads stored prefix hashes)
  *   sort_bits       1: MSD passes over plain keys split on the eight most
  *                   significant bits in which a segment's keys differ (over
  *                   small alphabets one pass then covers more than a key

@@ -2,17 +2,16 @@
 //
 // The full path (dsss_pd_sort) is laid out for one GPU holding every PE:
 //   1. one string sort of all n strings (K3, LCP as by-product);
-//   2. distinguishing prefixes from that order's LCPs (K1) — the result per
-//      string does not depend on the PE split;
-//   3. stable multisplit by PE of the global order gives each PE's local sorted
+//   2. stable multisplit by PE of the global order gives each PE's local sorted
 //      order (a subsequence of a sorted sequence is sorted), i.e. exactly what
-//      radixsort_CI3 produces per PE (prefix_doubling.hpp:228);
-//   4. partition (K5) on those local orders;
-//   5. every string's bucket follows from its PE and local index; a stable
-//      multisplit of the global order by bucket is each receiving PE's merged
-//      sequence — what AllToAllStringImplPrefixDoubling + choose_merge deliver
-//      (prefix_doubling.hpp:254-281) — with (local index, PE) as the
-//      permutation (:282-290) and merged LCPs taken from the global LCPs.
+//      radixsort_CI3 produces per PE (prefix_doubling.hpp:228), each string with
+//      its distinguishing prefix, which the order's LCPs decide (K1);
+//   3. splitters and bounds (K5) from positions and ranks in those orders;
+//   4. each receiving PE's merged sequence — what
+//      AllToAllStringImplPrefixDoubling + choose_merge deliver
+//      (prefix_doubling.hpp:254-281) — is the global order itself, its PEs and
+//      ranks the permutation (:282-290), unless equal strings fall on different
+//      sides of a splitter: then the stable multisplit of it by receiver.
 #include <algorithm>
 #include <cstring>
 #include <random>
@@ -24,6 +23,7 @@
 #include "merge.cuh"
 #include "partition.cuh"
 #include "pd.cuh"
+#include "project.cuh"
 #include "strsort.cuh"
 #include "util.cuh"
 
@@ -43,178 +43,6 @@ static ArenaDev view(const dsss_arena* a) { return ArenaDev{a->chars, a->offsets
 static uint32_t factor_of(const dsss_opts* o) { return (o && o->sampling_factor) ? o->sampling_factor : 2; }
 static uint32_t sampler_of(const dsss_opts* o) { return o ? o->sampler : DSSS_SAMPLER_NUM_STRINGS; }
 static uint32_t smallmax_of(const dsss_opts* o) { return o ? o->small_sort_max : 0; }
-
-// PE of every sorted position: the q with pb[q] <= ord[g] < pb[q + 1] in a
-// shared-memory copy of the PE bounds (npe + 1 <= 1025 entries), PE_IPT
-// positions per thread with their ids loaded before the lookups.  The first
-// guess is the PE that equal parts would give (id * p / n), moved by up to
-// two steps; a guess that is still off (PEs of very uneven sizes) falls back
-// to a binary search.
-constexpr int PE_NT = 256, PE_IPT = 8;
-__global__ void __launch_bounds__(PE_NT) k_pe_of(const uint32_t* ord, uint64_t n, const uint64_t* pb, uint32_t p,
-                                                 uint32_t* pe) {
-    extern __shared__ unsigned long long spb[];
-    for (uint32_t q = threadIdx.x; q <= p; q += PE_NT) spb[q] = pb[q];
-    const uint64_t g0 = (uint64_t)blockIdx.x * (PE_NT * PE_IPT) + threadIdx.x;
-    uint32_t s[PE_IPT];
-#pragma unroll
-    for (int j = 0; j < PE_IPT; ++j) {
-        const uint64_t g = g0 + (uint64_t)j * PE_NT;
-        s[j] = g < n ? ord[g] : 0u;
-    }
-    __syncthreads();
-    const float scale = (float)p / (float)(spb[p] ? spb[p] : 1ull);
-    uint32_t q[PE_IPT];
-#pragma unroll
-    for (int j = 0; j < PE_IPT; ++j) q[j] = min(p - 1, (uint32_t)((float)s[j] * scale));
-#pragma unroll
-    for (int step = 0; step < 2; ++step) {
-#pragma unroll
-        for (int j = 0; j < PE_IPT; ++j) {
-            if (spb[q[j]] > s[j]) --q[j];                        // q[j] > 0 here: spb[0] = 0
-            else if (spb[q[j] + 1] <= s[j]) ++q[j];              // q[j] + 1 < p here: spb[p] = n > s
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < PE_IPT; ++j) {
-        const uint64_t g = g0 + (uint64_t)j * PE_NT;
-        if (g >= n) continue;
-        uint32_t r = q[j];
-        if (spb[r] > s[j] || spb[r + 1] <= s[j]) {  // still off: the last r < p with pb[r] <= s
-            r = 0;
-            for (uint32_t st = 1u << (31 - __clz(p | 1u)); st; st >>= 1)
-                if (r + st < p && spb[r + st] <= s[j]) r += st;
-        }
-        pe[g] = r;
-    }
-}
-
-static int launch_pe_of(const uint32_t* ord, uint64_t n, const uint64_t* pb, uint32_t p, uint32_t* pe,
-                        cudaStream_t st) {
-    const uint64_t per = (uint64_t)PE_NT * PE_IPT;
-    DSSS_LAUNCH("k_pe_of", st,
-                k_pe_of<<<(unsigned)((n + per - 1) / per), PE_NT, (p + 1) * sizeof(unsigned long long), st>>>(
-                    ord, n, pb, p, pe));
-    return DSSS_OK;
-}
-
-// Receiving PE of every string: set s's PE q sends local positions
-// [bounds[(s*p+q)*(p+1) + r], … + r + 1) to the set's PE r; buckets are
-// numbered s*p + r.  src is q's global PE number, li the string's index in
-// q's local order; B is the bound table (u64 in global memory, or a u32 copy
-// in shared memory).
-template <typename B>
-__device__ __forceinline__ uint32_t bucket_of(const B* bounds, uint32_t p, uint32_t src, uint32_t li) {
-    const B* b = bounds + (uint64_t)src * (p + 1);
-    uint32_t lo = 0;  // the last r < p with b[r] <= li (b[0] = 0), in fixed steps
-    for (uint32_t step = 1u << (31 - __clz(p | 1u)); step; step >>= 1) {
-        const uint32_t m = lo + step;
-        if (m < p && b[m] <= li) lo = m;
-    }
-    return (src / p) * p + lo;
-}
-
-// k_bucket_of plus, for the common case, the merged sequences themselves: when
-// the buckets never decrease along the global order (no equal strings that two
-// PEs cut on different sides of a splitter), the stable partition by bucket
-// is the identity, so position g of the merged sequences is global position g:
-// its (local index, sender PE) and, unless it starts a receiving PE's run, the
-// global LCP.  *viol is set when some bucket decreases; the caller then runs
-// the multisplit, which rewrites every output (bucket, when given, receives
-// every position's bucket for it).  BD_IPT positions per thread, their inputs
-// loaded before the searches; with SMEM the bound table is searched in a u32
-// copy in shared memory; each position's predecessor bucket comes from the
-// tile's bucket row in shared memory.
-constexpr int BD_NT = 256, BD_IPT = 8, BD_TILE = BD_NT * BD_IPT;
-constexpr uint32_t BD_SMEM_BOUNDS = 8192;  // bound entries kept in shared memory (32 KiB)
-template <bool SMEM>
-__global__ void __launch_bounds__(BD_NT, 4) k_bucket_direct(const uint32_t* pe, const uint32_t* g2l,
-                                                         const uint64_t* bounds, uint32_t p, uint32_t npe, uint64_t n,
-                                                         int local_pe, const uint32_t* lcpg, uint32_t* bucket,
-                                                         uint32_t* pe_local, uint32_t* perm_index, uint32_t* perm_pe,
-                                                         uint32_t* merged, uint32_t* viol) {
-    extern __shared__ uint32_t sbd[];
-    uint32_t* sb = sbd;                  // the tile's buckets, after the one of the position before it
-    uint32_t* tab = sbd + BD_TILE + 1;   // SMEM: npe * (p + 1) bounds
-    const uint64_t t0 = (uint64_t)blockIdx.x * BD_TILE;
-    if (SMEM)
-        for (uint32_t k = threadIdx.x; k < npe * (p + 1); k += BD_NT) tab[k] = (uint32_t)bounds[k];
-    uint32_t src[BD_IPT], li[BD_IPT], lc[BD_IPT];
-#pragma unroll
-    for (int j = 0; j < BD_IPT; ++j) {
-        const uint64_t g = t0 + (uint64_t)j * BD_NT + threadIdx.x;
-        const bool v = g < n;
-        src[j] = v ? pe[g] : 0u;
-        li[j] = v ? g2l[g] : 0u;
-        lc[j] = v && merged ? lcpg[g] : 0u;
-    }
-    __syncthreads();
-    // the BD_IPT searches interleaved, in the fixed steps of bucket_of
-    uint32_t bk[BD_IPT];
-#pragma unroll
-    for (int j = 0; j < BD_IPT; ++j) bk[j] = 0;
-    for (uint32_t step = 1u << (31 - __clz(p | 1u)); step; step >>= 1) {
-#pragma unroll
-        for (int j = 0; j < BD_IPT; ++j) {
-            const uint32_t m = bk[j] + step;
-            if (m < p) {
-                const bool le = SMEM ? tab[src[j] * (p + 1) + m] <= li[j]
-                                     : bounds[(uint64_t)src[j] * (p + 1) + m] <= li[j];
-                if (le) bk[j] = m;
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < BD_IPT; ++j) {
-        bk[j] += (src[j] / p) * p;
-        sb[1 + j * BD_NT + threadIdx.x] = bk[j];
-    }
-    if (threadIdx.x == 0) {
-        uint32_t b = 0xFFFFFFFFu;
-        if (t0 && t0 <= n) {
-            const uint32_t s0 = pe[t0 - 1], l0 = g2l[t0 - 1];
-            b = SMEM ? bucket_of(tab, p, s0, l0) : bucket_of(bounds, p, s0, l0);
-        }
-        sb[0] = b;
-    }
-    __syncthreads();
-    bool bad = false;
-#pragma unroll
-    for (int j = 0; j < BD_IPT; ++j) {
-        const uint64_t g = t0 + (uint64_t)j * BD_NT + threadIdx.x;
-        if (g >= n) continue;
-        const uint32_t b = bk[j], bp = sb[j * BD_NT + threadIdx.x];
-        if (g && bp > b) bad = true;
-        const uint32_t ql = src[j] - (src[j] / p) * p;
-        if (bucket) bucket[g] = b;
-        if (pe_local) pe_local[g] = ql;
-        perm_index[g] = li[j];
-        perm_pe[g] = local_pe ? ql : src[j];
-        if (merged) merged[g] = (g == 0 || bp != b) ? 0u : lc[j];
-    }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicExch(viol, 1u);
-}
-
-static int launch_bucket_direct(const uint32_t* pe, const uint32_t* g2l, const uint64_t* bounds, uint32_t p,
-                                uint32_t npe, uint64_t n, int local_pe, const uint32_t* lcpg, uint32_t* bucket,
-                                uint32_t* pe_local, uint32_t* perm_index, uint32_t* perm_pe, uint32_t* merged,
-                                uint32_t* viol, cudaStream_t st) {
-    const unsigned grid = (unsigned)((n + BD_TILE - 1) / BD_TILE);
-    const uint64_t entries = (uint64_t)npe * (p + 1);
-    if (entries <= BD_SMEM_BOUNDS) {
-        const size_t sm = (BD_TILE + 1 + entries) * sizeof(uint32_t);
-        DSSS_LAUNCH("k_bucket_direct", st,
-                    k_bucket_direct<true><<<grid, BD_NT, sm, st>>>(pe, g2l, bounds, p, npe, n, local_pe, lcpg, bucket,
-                                                                   pe_local, perm_index, perm_pe, merged, viol));
-    } else {
-        const size_t sm = (BD_TILE + 1) * sizeof(uint32_t);
-        DSSS_LAUNCH("k_bucket_direct", st,
-                    k_bucket_direct<false><<<grid, BD_NT, sm, st>>>(pe, g2l, bounds, p, npe, n, local_pe, lcpg,
-                                                                    bucket, pe_local, perm_index, perm_pe, merged,
-                                                                    viol));
-    }
-    return DSSS_OK;
-}
 
 __global__ void k_merged_lcp(const uint32_t* out2g, const uint32_t* lcpg, const uint64_t* recv_begin, uint32_t p,
                              uint64_t n, uint32_t* merged) {
@@ -243,38 +71,54 @@ __global__ void k_zero_starts(uint32_t* a, const uint64_t* pb, uint32_t p) {
 
 struct PdLayout {
     ulonglong2* handles;
-    uint32_t *ord, *lcp, *dpg, *pe, *g2l, *tmp, *out2g, *pel, *nlong, *err, *viol;
-    uint64_t *pb, *bounds, *recv_begin;
+    LenStats* stats;
+    uint32_t *ord, *lcp, *bucket, *err, *nlong;
+    uint64_t* recv_begin;
     void* ms;
     SortLayout sort;
-    PartitionLayout part;
-    uint32_t* minlen;
+    ProjectLayout proj;
+    // after the sort, its buffers serve the multisplit of tied calls
+    uint32_t* tie[5];
 };
 
 // n strings in nsets sets of p PEs each.
-static void layout_pd(Carve& c, PdLayout& L, uint64_t n, uint32_t nsets, uint32_t p, uint32_t factor,
-                      uint32_t small_max) {
+static void layout_pd(Carve& c, PdLayout& L, uint64_t n, uint32_t nsets, uint32_t p, uint32_t small_max) {
     uint64_t N = n ? n : 1;
     const uint64_t npe = (uint64_t)nsets * p;
     L.handles = c.take<ulonglong2>(N);
+    L.stats = c.take<LenStats>(1);
     L.ord = c.take<uint32_t>(N);
     L.lcp = c.take<uint32_t>(N);
-    L.dpg = c.take<uint32_t>(N);
-    L.pe = c.take<uint32_t>(N);
-    L.g2l = c.take<uint32_t>(N);
-    L.tmp = c.take<uint32_t>(N);
-    L.out2g = c.take<uint32_t>(N);
-    L.pel = nsets > 1 ? c.take<uint32_t>(N) : nullptr;
-    L.nlong = c.take<uint32_t>(1);
+    L.bucket = c.take<uint32_t>(N);
     L.err = c.take<uint32_t>(1);
-    L.viol = c.take<uint32_t>(1);
-    L.pb = c.take<uint64_t>(npe + 1);
-    L.bounds = c.take<uint64_t>(npe * (p + 1));
+    L.nlong = c.take<uint32_t>(1);
     L.recv_begin = c.take<uint64_t>(npe + 1);
     L.ms = c.take<unsigned char>(multisplit_scratch_bytes(N, (uint32_t)npe));
+    layout_project(c, L.proj, N, nsets, p);
     layout_sort(c, L.sort, N, nsets, small_max);
-    layout_partition(c, L.part, N, p, factor, nsets);
-    L.minlen = c.take<uint32_t>(1);
+    L.tie[0] = L.sort.ord[0];
+    L.tie[1] = L.sort.ord[1];
+    L.tie[2] = (uint32_t*)L.sort.key[0];
+    L.tie[3] = c.sizing ? nullptr : (uint32_t*)L.sort.key[0] + N;
+    L.tie[4] = (uint32_t*)L.sort.key[1];
+}
+
+// Start of every receiver's strings, on the host and (for k_merged_lcp) on
+// the device.
+static int upload_recv_begin(const PdLayout& L, uint32_t npe, const uint64_t* recv_counts, void* pin,
+                             cudaStream_t st) {
+    uint64_t* h = (uint64_t*)pin;
+    h[0] = 0;
+    for (uint32_t r = 0; r < npe; ++r) h[r + 1] = h[r] + recv_counts[r];
+    DSSS_CUDA(cudaMemcpyAsync(L.recv_begin, h, (npe + 1) * 8, cudaMemcpyHostToDevice, st));
+    return DSSS_OK;
+}
+
+uint64_t pd_scratch_bytes(uint64_t n, uint32_t nsets, uint32_t p, const dsss_opts* opts) {
+    Carve sz(nullptr);
+    PdLayout L;
+    layout_pd(sz, L, n, nsets, p, smallmax_of(opts));
+    return sz.used;
 }
 
 // The fused path over nsets independent string sets of p PEs each (PE q of
@@ -282,13 +126,6 @@ static void layout_pd(Carve& c, PdLayout& L, uint64_t n, uint32_t nsets, uint32_
 // is the one a call on that set alone gives.  Per-string outputs keep the
 // arena's positions (set s's merged sequences fill the positions of its
 // strings), intervals and recv_counts are per set, one after the other.
-uint64_t pd_scratch_bytes(uint64_t n, uint32_t nsets, uint32_t p, const dsss_opts* opts) {
-    Carve sz(nullptr);
-    PdLayout L;
-    layout_pd(sz, L, n, nsets, p, factor_of(opts), smallmax_of(opts));
-    return sz.used;
-}
-
 int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, const uint64_t* pb,
                 const dsss_opts* opts, dsss_pd_result* out, cudaStream_t st) {
     DSSS_TRY(check_arena(in));
@@ -306,12 +143,15 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
     const bool want_local_lcp = opts && (opts->flags & DSSS_FLAG_LOCAL_LCP) && out->local_lcp;
     Carve sz(nullptr);
     PdLayout L;
-    layout_pd(sz, L, n, nsets, p, factor, smax);
+    layout_pd(sz, L, n, nsets, p, smax);
     DSSS_TRY(ensure_ws(ctx, sz.used));
-    DSSS_TRY(ensure_pin(ctx, 4096));
+    // the sort's counters, then the projection's staging area
+    const uint64_t pin_sort = 256;
+    DSSS_TRY(ensure_pin(ctx, std::max<uint64_t>(4096, pin_sort + project_pin_bytes(nsets, p))));
     Carve c(ctx->ws);
-    layout_pd(c, L, n, nsets, p, factor, smax);
-    uint32_t* pin = (uint32_t*)ctx->pin;  // re-read after any call that may grow it
+    layout_pd(c, L, n, nsets, p, smax);
+    uint32_t* pin = (uint32_t*)ctx->pin;
+    void* pinp = (char*)ctx->pin + pin_sort;
     ArenaDev a = view(in);
     if (n == 0) {
         for (uint32_t r = 0; r < npe; ++r) out->recv_counts[r] = 0;
@@ -321,87 +161,69 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
     }
     std::vector<uint64_t> set_begin(nsets + 1);
     for (uint32_t s = 0; s <= nsets; ++s) set_begin[s] = pb[(uint64_t)s * p];
-    make_handles(a, L.handles, st);
+    DSSS_TRY(make_handles(a, L.handles, st, L.stats));
     a.h = L.handles;
-    DSSS_CUDA(cudaMemsetAsync(L.err, 0, sizeof(uint32_t), st));
-    // 1. one sort per set, all sets in one segmented sort
+    // 1. one sort per set, all sets in one segmented sort; the global LCPs are
+    // the merged ones up to the receivers' starts
+    uint32_t* ord = p == 1 ? out->local_order : L.ord;
+    uint32_t* lcp = p > 1 && out->merged_lcp ? out->merged_lcp : p == 1 && want_local_lcp ? out->local_lcp : L.lcp;
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, L.ord, L.lcp, smax, pin, st));
+        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, ord, lcp, smax, pin, st));
     }
     if (p == 1) {  // prefix_doubling.hpp:236: one PE sorts locally and returns no permutation
-        DSSS_CUDA(cudaMemcpyAsync(out->local_order, L.ord, n * 4, cudaMemcpyDeviceToDevice, st));
-        if (want_local_lcp) DSSS_CUDA(cudaMemcpyAsync(out->local_lcp, L.lcp, n * 4, cudaMemcpyDeviceToDevice, st));
         for (uint32_t r = 0; r < npe; ++r) out->recv_counts[r] = 0;
         return DSSS_OK;
     }
-    // 2. distinguishing prefixes over each set's sorted order
+    // 2. the PEs' local orders with their distinguishing prefixes; position
+    // g's PE and its rank there are the (index, PE) permutation
+    uint32_t* pe = out->perm_pe;
+    uint32_t* bucket = nsets > 1 ? L.bucket : pe;
     {
-        StageTimer t("stage:dp", st);
-        DSSS_TRY(dp_from_lcps(a, n, L.ord, L.lcp, L.minlen, L.dpg, st));
+        StageTimer t("stage:local", st);
+        DSSS_TRY(project_setup(L.proj, nsets, p, pb, factor, pinp, st));
+        DSSS_TRY(project_local(L.proj, a, n, nsets, p, ord, lcp, L.stats, pe, bucket, out->local_order,
+                               out->perm_index, out->dp, st));
     }
-    // 3. local orders per PE
-    StageTimer t_local("stage:local", st);
-    DSSS_CUDA(cudaMemcpyAsync(L.pb, pb, (npe + 1) * 8, cudaMemcpyHostToDevice, st));
-    DSSS_TRY(launch_pe_of(L.ord, n, L.pb, npe, L.pe, st));
-    {
-        // local order and DP per PE: out[dest] = (string id, dp); g2l = rank inside the PE
-        const uint32_t* in[2] = {L.ord, L.dpg};
-        uint32_t* outs[2] = {out->local_order, out->dp};
-        DSSS_TRY(multisplit_payload(L.pe, n, npe, 2, in, outs, L.g2l, L.err, L.ms, st));
-    }
-    DSSS_CUDA(cudaGetLastError());
-    t_local.end();
-    // 4. partition
+    // 3. splitters and every PE's bounds; receiving PE (s, r) is bucket s*p + r
     {
         StageTimer t("stage:partition", st);
-        DSSS_TRY(partition_sets(L.part, ctx, a, nsets, p, pb, out->local_order, out->dp, sampler_of(opts), factor,
-                                out->intervals, st));
-    }
-    StageTimer t_merge("stage:merge", st);
-    // 5. buckets and the merged sequences; receiving PE (s, r) is bucket s*p + r
-    std::vector<uint64_t> bounds((uint64_t)npe * (p + 1)), recv(npe + 1, 0);
-    for (uint32_t g = 0; g < npe; ++g) {
-        const uint32_t s = g / p;
-        bounds[(uint64_t)g * (p + 1)] = 0;
-        for (uint32_t r = 0; r < p; ++r) {
-            uint64_t v = out->intervals[(uint64_t)g * p + r];
-            bounds[(uint64_t)g * (p + 1) + r + 1] = bounds[(uint64_t)g * (p + 1) + r] + v;
-            recv[(uint64_t)s * p + r + 1] += v;
-        }
-    }
-    for (uint32_t r = 0; r < npe; ++r) {
-        out->recv_counts[r] = recv[r + 1];
-        recv[r + 1] += recv[r];
-    }
-    DSSS_CUDA(cudaMemcpyAsync(L.bounds, bounds.data(), bounds.size() * 8, cudaMemcpyHostToDevice, st));
-    DSSS_CUDA(cudaMemcpyAsync(L.recv_begin, recv.data(), (npe + 1) * 8, cudaMemcpyHostToDevice, st));
-    DSSS_CUDA(cudaMemsetAsync(L.viol, 0, sizeof(uint32_t), st));
-    DSSS_TRY(launch_bucket_direct(L.pe, L.g2l, L.bounds, p, npe, n, nsets > 1, L.lcp, nullptr, L.pel,
-                                  out->perm_index, out->perm_pe, out->merged_lcp, L.viol, st));
-    pin = (uint32_t*)ctx->pin;  // the partition step may have grown the staging buffer
-    DSSS_CUDA(cudaMemcpyAsync(pin, L.viol, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    DSSS_CUDA(cudaStreamSynchronize(st));
-    if (pin[0]) {
-        // every position's bucket for the multisplit (the outputs are rewritten by it)
-        DSSS_TRY(launch_bucket_direct(L.pe, L.g2l, L.bounds, p, npe, n, nsets > 1, L.lcp, L.tmp, L.pel,
-                                      out->perm_index, out->perm_pe, nullptr, L.viol, st));
-        // merged sequences: (index in sender's local order, sender PE, global position)
-        const uint32_t* in[3] = {L.g2l, nsets > 1 ? L.pel : L.pe, nullptr};
-        uint32_t* outs[3] = {out->perm_index, out->perm_pe, L.out2g};
-        DSSS_TRY(multisplit_payload(L.tmp, n, npe, 3, in, outs, nullptr, L.err, L.ms, st));
-        if (out->merged_lcp)
-            DSSS_LAUNCH("k_merged_lcp", st,
-                        k_merged_lcp<<<grid_for(n, 256), 256, 0, st>>>(L.out2g, L.lcp, L.recv_begin, npe, n,
-                                                                      out->merged_lcp));
+        DSSS_TRY(project_partition(L.proj, a, n, nsets, p, factor,
+                                   sampler_of(opts) == DSSS_SAMPLER_INDEXED_NUM_STRINGS, nullptr, ord, lcp, bucket,
+                                   out->perm_index, out->merged_lcp, st));
+        DSSS_TRY(project_read_async(L.proj, nsets, p, pinp, st));
     }
     if (want_local_lcp) {
-        DSSS_TRY(adjacent_lcp(a, out->local_order, n, out->local_lcp, L.tmp, L.nlong, st));
-        DSSS_LAUNCH("k_zero_starts", st, k_zero_starts<<<grid_for(npe, 128), 128, 0, st>>>(out->local_lcp, L.pb, npe));
+        DSSS_TRY(adjacent_lcp(a, out->local_order, n, out->local_lcp, L.tie[0], L.nlong, st));
+        DSSS_LAUNCH("k_zero_starts", st,
+                    k_zero_starts<<<grid_for(npe, 128), 128, 0, st>>>(out->local_lcp, L.proj.pb, npe));
     }
     DSSS_CUDA(cudaGetLastError());
-    // The host vectors above were copied asynchronously; finish before they go.
-    pin = (uint32_t*)ctx->pin;  // the partition step may have grown the staging buffer
+    DSSS_CUDA(cudaStreamSynchronize(st));
+    bool ties = false;
+    DSSS_TRY(project_read(nsets, p, pinp, out->intervals, out->recv_counts, &ties));
+    if (!ties) return DSSS_OK;
+    // 4. equal strings on different sides of a splitter: the merged sequences
+    // are the stable multisplit of the global order by receiver
+    StageTimer t_merge("stage:merge", st);
+    DSSS_CUDA(cudaMemsetAsync(L.err, 0, sizeof(uint32_t), st));
+    DSSS_TRY(upload_recv_begin(L, npe, out->recv_counts, pinp, st));
+    DSSS_TRY(project_buckets(L.proj, n, p, bucket, out->perm_index, L.tie[2], st));
+    DSSS_CUDA(cudaMemcpyAsync(L.tie[0], out->perm_index, n * 4, cudaMemcpyDeviceToDevice, st));
+    DSSS_CUDA(cudaMemcpyAsync(L.tie[1], pe, n * 4, cudaMemcpyDeviceToDevice, st));
+    {
+        // (index in sender's local order, sender PE, global position)
+        const uint32_t* in3[3] = {L.tie[0], L.tie[1], nullptr};
+        uint32_t* outs[3] = {out->perm_index, out->perm_pe, L.tie[3]};
+        DSSS_TRY(multisplit_payload(L.tie[2], n, npe, 3, in3, outs, nullptr, L.err, L.ms, st));
+    }
+    if (out->merged_lcp) {
+        DSSS_CUDA(cudaMemcpyAsync(L.lcp, out->merged_lcp, n * 4, cudaMemcpyDeviceToDevice, st));
+        DSSS_LAUNCH("k_merged_lcp", st,
+                    k_merged_lcp<<<grid_for(n, 256), 256, 0, st>>>(L.tie[3], L.lcp, L.recv_begin, npe, n,
+                                                                  out->merged_lcp));
+    }
+    DSSS_CUDA(cudaGetLastError());
     DSSS_CUDA(cudaMemcpyAsync(pin, L.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));
     if (pin[0]) return fail(DSSS_EDEVICE, "pd sort: internal consistency guard tripped");
@@ -410,11 +232,10 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
 
 // ------------------------------------------------------- merge-sort path ----
 // DistributedMergeSort::sort on one GPU holding every PE: the global sort, the
-// local orders (multisplit by PE) and their LCP arrays, getAvgLcp, the
-// partition with samples cut to 200 (avg + 5) bytes, then the receiving PEs'
-// sequences as a projection of the global order (written directly, or by the
-// multisplit by bucket when ties cross a splitter) and their strings copied
-// out whole.
+// local orders and their LCP arrays, getAvgLcp, the partition with samples cut
+// to 200 (avg + 5) bytes, then the receiving PEs' sequences (the global order,
+// or its multisplit by receiver when ties cross a splitter) and their strings
+// copied out whole.
 
 __global__ void k_sum_u32_to_u64(const uint32_t* v, uint64_t n, unsigned long long* total) {
     unsigned long long s = 0;
@@ -425,20 +246,14 @@ __global__ void k_sum_u32_to_u64(const uint32_t* v, uint64_t n, unsigned long lo
     if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
 }
 
-__global__ void k_fill_u32(uint32_t* a, uint64_t n, uint32_t v) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) a[i] = v;
-}
-
 // Input index, source offset and length (+ 1 for the scan) of every output
-// string: the copy then reads its string's place sequentially instead of
-// gathering it again.
-__global__ void k_ms_source(const uint32_t* local_order, const uint64_t* pb, const uint32_t* perm_index,
-                            const uint32_t* perm_pe, ArenaDev a, uint64_t n, uint32_t* source, uint32_t* lengths,
-                            uint32_t* len1, uint64_t* src_off) {
+// string (the string at global position map[o], or o): the copy then reads its
+// string's place sequentially instead of gathering it again.
+__global__ void k_ms_source(const uint32_t* ord, const uint32_t* map, ArenaDev a, uint64_t n, uint32_t* source,
+                            uint32_t* lengths, uint32_t* len1, uint64_t* src_off) {
     const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= n) return;
-    const uint32_t id = perm_pe ? local_order[pb[perm_pe[o]] + perm_index[o]] : local_order[o];
+    const uint32_t id = ord[map ? map[o] : (uint32_t)o];
     uint64_t off;
     uint32_t len;
     str_of(a, id, off, len);
@@ -490,23 +305,29 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     const uint64_t n = in->n;
     const uint32_t factor = 2, smax = smallmax_of(opts);  // computePartition(..., 2): misc.hpp call in :238
     const uint64_t N = n ? n : 1;
-    Carve sz(nullptr);
     PdLayout L;
-    layout_pd(sz, L, n, 1, p, factor, smax);
-    uint32_t* src_tmp = sz.take<uint32_t>(N);
-    uint32_t* len1 = sz.take<uint32_t>(N);
-    uint64_t* srcoff = sz.take<uint64_t>(N);
-    unsigned long long* total = sz.take<unsigned long long>(2);
-    void* scan = sz.take<unsigned char>(scan_scratch_bytes(N));
+    uint32_t *src_tmp, *len1, *pe, *rank, *llcp;
+    uint64_t* srcoff;
+    unsigned long long* total;
+    void* scan;
+    auto plan = [&](Carve& c) {
+        layout_pd(c, L, n, 1, p, smax);
+        src_tmp = c.take<uint32_t>(N);
+        len1 = c.take<uint32_t>(N);
+        pe = c.take<uint32_t>(N);
+        rank = c.take<uint32_t>(N);
+        llcp = c.take<uint32_t>(N);
+        srcoff = c.take<uint64_t>(N);
+        total = c.take<unsigned long long>(2);
+        scan = c.take<unsigned char>(scan_scratch_bytes(N));
+    };
+    Carve sz(nullptr);
+    plan(sz);
     DSSS_TRY(ensure_ws(ctx, sz.used));
-    DSSS_TRY(ensure_pin(ctx, 4096));
+    const uint64_t pin_sort = 256;
+    DSSS_TRY(ensure_pin(ctx, std::max<uint64_t>(4096, pin_sort + project_pin_bytes(1, p))));
     Carve c(ctx->ws);
-    layout_pd(c, L, n, 1, p, factor, smax);
-    src_tmp = c.take<uint32_t>(N);
-    len1 = c.take<uint32_t>(N);
-    srcoff = c.take<uint64_t>(N);
-    total = c.take<unsigned long long>(2);
-    scan = c.take<unsigned char>(scan_scratch_bytes(N));
+    plan(c);
     uint32_t* source = out->source ? out->source : src_tmp;
     out->avg_lcp = 0;
     if (n == 0) {
@@ -515,108 +336,74 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
         return DSSS_OK;
     }
     ArenaDev a = view(in);
-    make_handles(a, L.handles, st);
+    DSSS_TRY(make_handles(a, L.handles, st, L.stats));
     a.h = L.handles;
     uint32_t* pin = (uint32_t*)ctx->pin;
+    void* pinp = (char*)ctx->pin + pin_sort;
+    LenStats* hstats = (LenStats*)((char*)ctx->pin + 128);
     DSSS_CUDA(cudaMemsetAsync(L.err, 0, sizeof(uint32_t), st));
     DSSS_CUDA(cudaMemsetAsync(total, 0, 2 * sizeof(unsigned long long), st));
+    DSSS_CUDA(cudaMemcpyAsync(hstats, L.stats, sizeof(LenStats), cudaMemcpyDeviceToHost, st));
     const uint64_t set_begin[2] = {0, n};
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, 1, set_begin, nullptr, L.ord, L.lcp, smax, pin, st));
+        DSSS_TRY(sort_strings(L.sort, a, n, 1, set_begin, nullptr, L.ord, out->lcp, smax, pin, st));
     }
+    const uint64_t bytes = hstats->sum + n;  // the sort has synchronised on st
     // local orders per PE and their LCP arrays (0 at each PE start)
     StageTimer t_local("stage:local", st);
-    DSSS_CUDA(cudaMemcpyAsync(L.pb, pb, (p + 1) * 8, cudaMemcpyHostToDevice, st));
-    DSSS_TRY(launch_pe_of(L.ord, n, L.pb, p, L.pe, st));
-    {
-        const uint32_t* ins[1] = {L.ord};
-        uint32_t* outs[1] = {out->local_order};
-        DSSS_TRY(multisplit_payload(L.pe, n, p, 1, ins, outs, L.g2l, L.err, L.ms, st));
-    }
-    // L.dpg holds the local LCPs, then the sample cut
-    DSSS_TRY(adjacent_lcp(a, out->local_order, n, L.dpg, L.tmp, L.nlong, st));
-    DSSS_LAUNCH("k_zero_starts", st, k_zero_starts<<<grid_for(p, 128), 128, 0, st>>>(L.dpg, L.pb, p));
-    DSSS_LAUNCH("k_sum_u32_to_u64", st, k_sum_u32_to_u64<<<148 * 4, 256, 0, st>>>(L.dpg, n, total));
-    pin = (uint32_t*)ctx->pin;
-    DSSS_CUDA(cudaMemcpyAsync(pin, total, 8, cudaMemcpyDeviceToHost, st));
-    DSSS_CUDA(cudaStreamSynchronize(st));
-    const uint64_t avg = *(const uint64_t*)pin / n;  // getAvgLcp (misc.hpp:68-87)
-    out->avg_lcp = avg;
+    DSSS_TRY(project_setup(L.proj, 1, p, pb, factor, pinp, st));
+    DSSS_TRY(project_local(L.proj, a, n, 1, p, L.ord, out->lcp, nullptr, pe, pe, out->local_order, rank, nullptr, st));
+    DSSS_TRY(adjacent_lcp(a, out->local_order, n, llcp, L.tie[0], L.nlong, st));
+    DSSS_LAUNCH("k_zero_starts", st, k_zero_starts<<<grid_for(p, 128), 128, 0, st>>>(llcp, L.proj.pb, p));
+    DSSS_LAUNCH("k_sum_u32_to_u64", st, k_sum_u32_to_u64<<<148 * 4, 256, 0, st>>>(llcp, n, total));
+    unsigned long long* hsum = (unsigned long long*)((char*)ctx->pin + 192);
+    DSSS_CUDA(cudaMemcpyAsync(hsum, total, 8, cudaMemcpyDeviceToHost, st));
     t_local.end();
+    const uint32_t* map = nullptr;
     if (p == 1) {  // lcp_aware_number_string_splitting.hpp:230-232: the local sort is the result
+        DSSS_CUDA(cudaStreamSynchronize(st));
         out->intervals[0] = n;
         out->recv_counts[0] = n;
-        StageTimer t("stage:merge", st);
-        DSSS_CUDA(cudaMemcpyAsync(out->lcp, L.dpg, n * 4, cudaMemcpyDeviceToDevice, st));
-        DSSS_LAUNCH("k_ms_source", st,
-                    k_ms_source<<<grid_for(n, 256), 256, 0, st>>>(out->local_order, L.pb, nullptr, nullptr, a, n,
-                                                                 source, out->lengths, len1, srcoff));
     } else {
         {
             StageTimer t("stage:partition", st);
-            const uint64_t cut = 2 * (100 * (avg + 5));  // misc.hpp:488 on 100 * globalLcpAvg (:238)
-            DSSS_LAUNCH("k_fill_u32", st,
-                        k_fill_u32<<<grid_for(n, 256), 256, 0, st>>>(L.dpg, n, cut > 0xFFFFFFFFull ? 0xFFFFFFFFu
-                                                                                                 : (uint32_t)cut));
-            DSSS_TRY(partition_sets(L.part, ctx, a, 1, p, pb, out->local_order, L.dpg, DSSS_SAMPLER_NUM_STRINGS,
-                                    factor, out->intervals, st));
+            DSSS_TRY(project_partition(L.proj, a, n, 1, p, factor, 0, total, L.ord, out->lcp, pe, rank, out->lcp, st));
+            DSSS_TRY(project_read_async(L.proj, 1, p, pinp, st));
+            DSSS_CUDA(cudaStreamSynchronize(st));
         }
         StageTimer t_merge("stage:merge", st);
-        std::vector<uint64_t> bounds((uint64_t)p * (p + 1)), recv(p + 1, 0);
-        for (uint32_t q = 0; q < p; ++q) {
-            bounds[(uint64_t)q * (p + 1)] = 0;
-            for (uint32_t r = 0; r < p; ++r) {
-                const uint64_t v = out->intervals[(uint64_t)q * p + r];
-                bounds[(uint64_t)q * (p + 1) + r + 1] = bounds[(uint64_t)q * (p + 1) + r] + v;
-                recv[r + 1] += v;
-            }
-        }
-        for (uint32_t r = 0; r < p; ++r) {
-            out->recv_counts[r] = recv[r + 1];
-            recv[r + 1] += recv[r];
-        }
-        DSSS_CUDA(cudaMemcpyAsync(L.bounds, bounds.data(), bounds.size() * 8, cudaMemcpyHostToDevice, st));
-        DSSS_CUDA(cudaMemcpyAsync(L.recv_begin, recv.data(), (p + 1) * 8, cudaMemcpyHostToDevice, st));
-        // (local index, sender PE) of every output position: perm_index in L.dpg, perm_pe in len1
-        DSSS_CUDA(cudaMemsetAsync(L.viol, 0, sizeof(uint32_t), st));
-        DSSS_TRY(launch_bucket_direct(L.pe, L.g2l, L.bounds, p, p, n, 0, L.lcp, nullptr, nullptr, L.dpg, len1,
-                                      out->lcp, L.viol, st));
-        pin = (uint32_t*)ctx->pin;
-        DSSS_CUDA(cudaMemcpyAsync(pin, L.viol, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));
-        if (pin[0]) {
-            DSSS_TRY(launch_bucket_direct(L.pe, L.g2l, L.bounds, p, p, n, 0, L.lcp, L.tmp, nullptr, L.dpg, len1,
-                                          nullptr, L.viol, st));
-            const uint32_t* ins[3] = {L.g2l, L.pe, nullptr};
-            uint32_t* outs[3] = {L.dpg, len1, L.out2g};
-            DSSS_TRY(multisplit_payload(L.tmp, n, p, 3, ins, outs, nullptr, L.err, L.ms, st));
+        bool ties = false;
+        DSSS_TRY(project_read(1, p, pinp, out->intervals, out->recv_counts, &ties));
+        if (ties) {
+            DSSS_TRY(upload_recv_begin(L, p, out->recv_counts, pinp, st));
+            DSSS_TRY(project_buckets(L.proj, n, p, pe, rank, L.tie[2], st));
+            const uint32_t* ins[1] = {nullptr};
+            uint32_t* outs[1] = {L.tie[3]};
+            DSSS_TRY(multisplit_payload(L.tie[2], n, p, 1, ins, outs, nullptr, L.err, L.ms, st));
+            DSSS_CUDA(cudaMemcpyAsync(L.lcp, out->lcp, n * 4, cudaMemcpyDeviceToDevice, st));
             DSSS_LAUNCH("k_merged_lcp", st,
-                        k_merged_lcp<<<grid_for(n, 256), 256, 0, st>>>(L.out2g, L.lcp, L.recv_begin, p, n, out->lcp));
+                        k_merged_lcp<<<grid_for(n, 256), 256, 0, st>>>(L.tie[3], L.lcp, L.recv_begin, p, n, out->lcp));
+            map = L.tie[3];
         }
-        DSSS_LAUNCH("k_ms_source", st,
-                    k_ms_source<<<grid_for(n, 256), 256, 0, st>>>(out->local_order, L.pb, L.dpg, len1, a, n, source,
-                                                                 out->lengths, src_tmp == source ? L.tmp : src_tmp,
-                                                                 srcoff));
-        len1 = src_tmp == source ? L.tmp : src_tmp;
     }
+    out->avg_lcp = *hsum / n;  // getAvgLcp (misc.hpp:68-87)
+    if (bytes > out->chars_capacity)
+        return fail(DSSS_EINVAL, "chars_capacity %llu is below the %llu output bytes",
+                    (unsigned long long)out->chars_capacity, (unsigned long long)bytes);
     // output layout and the strings themselves
     {
         StageTimer t("stage:copy", st);
+        DSSS_LAUNCH("k_ms_source", st,
+                    k_ms_source<<<grid_for(n, 256), 256, 0, st>>>(L.ord, map, a, n, source, out->lengths, len1,
+                                                                 srcoff));
         DSSS_TRY(exclusive_scan_u32_to_u64(len1, out->offsets, n, (uint64_t*)(total + 1), scan, st));
-        pin = (uint32_t*)ctx->pin;
-        DSSS_CUDA(cudaMemcpyAsync(pin, total + 1, 8, cudaMemcpyDeviceToHost, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));
-        const uint64_t bytes = *(const uint64_t*)pin;
-        if (bytes > out->chars_capacity)
-            return fail(DSSS_EINVAL, "chars_capacity %llu is below the %llu output bytes",
-                        (unsigned long long)out->chars_capacity, (unsigned long long)bytes);
         DSSS_TRY(launch_ms_copy(a.chars, srcoff, out->lengths, out->offsets, n, out->chars, st));
     }
-    pin = (uint32_t*)ctx->pin;
     DSSS_CUDA(cudaMemcpyAsync(pin, L.err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    DSSS_CUDA(cudaMemcpyAsync(pin + 1, L.proj.flags, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));
-    if (pin[0]) return fail(DSSS_EDEVICE, "ms sort: internal consistency guard tripped");
+    if (pin[0] || pin[1]) return fail(DSSS_EDEVICE, "ms sort: internal consistency guard tripped");
     return DSSS_OK;
 }
 
@@ -886,7 +673,8 @@ static int hq_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     auto plan = [&](Carve& c, ulonglong2*& handles, uint32_t*& ord, uint32_t*& lcp, uint16_t*& owner, uint32_t*& tmp,
                     uint32_t*& runx, uint32_t*& srcb, uint32_t*& tc, uint32_t*& off, uint32_t*& cnt, HqPe*& prm,
                     uint32_t*& cut, uint32_t*& dest, uint32_t*& err, uint64_t*& pbd, uint64_t*& total, void*& scan,
-                    uint64_t*& srcoff, SortLayout& sl) {
+                    uint64_t*& srcoff, LenStats*& stats, SortLayout& sl) {
+        stats = c.take<LenStats>(1);
         handles = c.take<ulonglong2>(N);
         ord = c.take<uint32_t>(N);
         lcp = c.take<uint32_t>(N);
@@ -913,18 +701,23 @@ static int hq_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     HqPe* prm;
     uint64_t *pbd, *total, *srcoff;
     void* scan;
+    LenStats* stats;
     SortLayout sl;
     Carve sz(nullptr);
-    plan(sz, handles, ord, lcp, owner, tmp, runx, srcb, tc, off, cnt, prm, cut, dest, err, pbd, total, scan, srcoff, sl);
+    plan(sz, handles, ord, lcp, owner, tmp, runx, srcb, tc, off, cnt, prm, cut, dest, err, pbd, total, scan, srcoff,
+         stats, sl);
     DSSS_TRY(ensure_ws(ctx, sz.used));
     const uint64_t pin_bytes = MAX_SPLIT_BUCKETS * (sizeof(uint32_t) + sizeof(HqPe)) + 64;
     DSSS_TRY(ensure_pin(ctx, pin_bytes < 4096 ? 4096 : pin_bytes));
     Carve c(ctx->ws);
-    plan(c, handles, ord, lcp, owner, tmp, runx, srcb, tc, off, cnt, prm, cut, dest, err, pbd, total, scan, srcoff, sl);
+    plan(c, handles, ord, lcp, owner, tmp, runx, srcb, tc, off, cnt, prm, cut, dest, err, pbd, total, scan, srcoff,
+         stats, sl);
     ArenaDev a = view(in);
-    make_handles(a, handles, st);
+    DSSS_TRY(make_handles(a, handles, st, stats));
     a.h = handles;
     DSSS_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
+    LenStats* hstats = (LenStats*)((char*)ctx->pin + 128);
+    DSSS_CUDA(cudaMemcpyAsync(hstats, stats, sizeof(LenStats), cudaMemcpyDeviceToHost, st));
     const uint64_t set_begin[2] = {0, n};
     {
         StageTimer t("stage:sort", st);
@@ -935,12 +728,10 @@ static int hq_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     {
         StageTimer t("stage:layout", st);
         DSSS_LAUNCH("k_ms_source", st,
-                    k_ms_source<<<grid_for(n, 256), 256, 0, st>>>(ord, nullptr, nullptr, nullptr, a, n, source,
-                                                                 out->lengths, tmp, srcoff));
+                    k_ms_source<<<grid_for(n, 256), 256, 0, st>>>(ord, nullptr, a, n, source, out->lengths, tmp,
+                                                                 srcoff));
         DSSS_TRY(exclusive_scan_u32_to_u64(tmp, out->offsets, n, total, scan, st));
-        DSSS_CUDA(cudaMemcpyAsync(ctx->pin, total, 8, cudaMemcpyDeviceToHost, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));
-        const uint64_t bytes = *(const uint64_t*)ctx->pin;
+        const uint64_t bytes = hstats->sum + n;  // the sort has synchronised on st
         if (bytes > out->chars_capacity)
             return fail(DSSS_EINVAL, "chars_capacity %llu is below the %llu output bytes",
                         (unsigned long long)out->chars_capacity, (unsigned long long)bytes);
@@ -1067,7 +858,7 @@ int dsss_local_sort_lcp(dsss_ctx* ctx, const dsss_arena* in, uint32_t p, const u
     ulonglong2* h = c.take<ulonglong2>(in->n ? in->n : 1);
     layout_sort(c, L, in->n, p, smax);
     ArenaDev a = view(in);
-    make_handles(a, h, st);
+    DSSS_TRY(make_handles(a, h, st));
     a.h = h;
     return sort_strings(L, a, in->n, p, part_begin, nullptr, order, lcp, smax, (uint32_t*)ctx->pin, st);
 }
@@ -1091,7 +882,7 @@ int dsss_dp_prefixes(dsss_ctx* ctx, const dsss_arena* in, uint32_t p, const uint
     ulonglong2* h = c.take<ulonglong2>(in->n ? in->n : 1);
     layout_dp(c, L, in->n);
     ArenaDev a = view(in);
-    make_handles(a, h, (cudaStream_t)stream);
+    DSSS_TRY(make_handles(a, h, (cudaStream_t)stream));
     a.h = h;
     // The PE split needs no extra handling: every PE's first LCP is 0, so no
     // string is an LCP duplicate of the previous PE's last one.
@@ -1258,7 +1049,7 @@ static int pd_sort_host(dsss_ctx* ctx, const dsss_arena* in, uint32_t nsets, uin
     // The io buffer sits in front of the pipeline's own scratch.
     Carve pdsz(nullptr);
     PdLayout PL;
-    layout_pd(pdsz, PL, n, nsets, p, factor_of(opts), smallmax_of(opts));
+    layout_pd(pdsz, PL, n, nsets, p, smallmax_of(opts));
     const uint64_t io_bytes = (sz.used + 255) & ~255ull;
     DSSS_TRY(ensure_ws(ctx, io_bytes + pdsz.used));
     Carve c(ctx->ws);

@@ -20,7 +20,7 @@
 // The hash table is sized by the number of strings hashed in the round.
 //
 // Where one GPU holds every PE, the global sorted order and its LCPs decide
-// the rounds without a hash (dp_from_lcps): the strings that share a string's
+// the rounds without a hash (k_local_scatter, project.cu): the strings that share a string's
 // d-byte prefix are its neighbours with LCPs of at least d, all of them still
 // candidates, since they share every shorter prefix too.  So a string stays in
 // the round at depth d exactly while m = max(LCP with its predecessor, LCP
@@ -117,38 +117,6 @@ __global__ void __launch_bounds__(256) k_min_nbr_lcp(const uint32_t* lcp, uint64
 #pragma unroll
     for (int o = 16; o; o >>= 1) m = min(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m != 0xFFFFFFFFu) atomicMin(out, m);
-}
-
-// The first depth above m of the schedule 8, 24, 40, 72, ..., 8 + 8 * 2^k.
-__device__ __forceinline__ uint64_t dp_depth_above(uint32_t m) {
-    if (m < 8) return 8;
-    const uint32_t k = 32 - __clz((m - 8) >> 3);  // the smallest k with 8 * 2^k > m - 8
-    return 8 + (8ull << max(k, 1u));
-}
-
-// One thread per sorted position.  Bound by HBM: 4 bytes of LCP read and 4
-// written per string; the length (a random read through the order) only where
-// the depth exceeds the shortest string.
-__global__ void __launch_bounds__(256) k_dp_from_lcps(ArenaDev a, const uint32_t* order, const uint32_t* lcp,
-                                                      uint64_t n, const uint32_t* minlen, uint32_t* dp) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint64_t d = dp_depth_above(max(i ? lcp[i] : 0u, i + 1 < n ? lcp[i + 1] : 0u));
-    if (d > *minlen) d = min(d, (uint64_t)a.len[order[i]]);
-    dp[i] = (uint32_t)d;
-}
-
-int dp_from_lcps(const ArenaDev& a, uint64_t n, const uint32_t* order, const uint32_t* lcp, uint32_t* minlen,
-                 uint32_t* dp, cudaStream_t st) {
-    if (n == 0) return DSSS_OK;
-    DSSS_CUDA(cudaMemsetAsync(minlen, 0xFF, sizeof(uint32_t), st));
-    DSSS_LAUNCH("k_min_len", st,
-                k_min_len<<<(unsigned)std::min<uint64_t>(grid_for(a.n, 256), 148 * 8), 256, 0, st>>>(a.len, a.h, a.n,
-                                                                                                   minlen));
-    DSSS_LAUNCH("k_dp_from_lcps", st,
-                k_dp_from_lcps<<<grid_for(n, 256), 256, 0, st>>>(a, order, lcp, n, minlen, dp));
-    DSSS_CUDA(cudaGetLastError());
-    return DSSS_OK;
 }
 
 // Adds the block's number of true flags to *ctr with one atomic per block

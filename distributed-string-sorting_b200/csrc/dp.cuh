@@ -64,11 +64,12 @@ int dp_rounds(const DpLayout& L, const ArenaDev& a, uint64_t n, const uint32_t* 
               uint32_t* dp, uint64_t* round_counts, uint32_t max_rounds, uint32_t* rounds, uint32_t* pin,
               cudaStream_t st);
 
-// Distinguishing prefixes of strings in their global sorted order (every PE's
-// strings in one order, lcp its LCP array with 0 at every set's first string):
-// dp[i] of the string at position i.  minlen: one word of scratch.
-int dp_from_lcps(const ArenaDev& a, uint64_t n, const uint32_t* order, const uint32_t* lcp, uint32_t* minlen,
-                 uint32_t* dp, cudaStream_t st);
+// The first depth above m of the schedule 8, 24, 40, 72, ..., 8 + 8 * 2^k.
+__device__ __forceinline__ uint64_t dp_depth_above(uint32_t m) {
+    if (m < 8) return 8;
+    const uint32_t k = 32 - __clz((m - 8) >> 3);  // the smallest k with 8 * 2^k > m - 8
+    return 8 + (8ull << max(k, 1u));
+}
 
 struct DpRoundLayout {
     DpLayout dp;

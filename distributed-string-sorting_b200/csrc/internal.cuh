@@ -177,8 +177,17 @@ __device__ __forceinline__ void str_of(const ArenaDev& a, uint32_t s, uint64_t& 
     }
 }
 
-// Builds the interleaved handle array for strings [0, n).
-void make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st);
+// The arena's shortest length (as the largest complement, so that zeroed
+// memory is the start of the reduction) and the sum of all lengths.
+struct LenStats {
+    uint32_t inv_min, pad;
+    unsigned long long sum;
+    __device__ __forceinline__ uint32_t min_len() const { return ~inv_min; }
+};
+
+// Builds the interleaved handle array for strings [0, n), and the length
+// statistics when asked for.
+int make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st, LenStats* stats = nullptr);
 
 int check_arena(const dsss_arena* a);
 

@@ -76,13 +76,56 @@ int adjacent_lcp(const ArenaDev& a, const uint32_t* order, uint64_t m, uint32_t*
     return DSSS_OK;
 }
 
-__global__ void k_make_handles(ArenaDev a, ulonglong2* h) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < a.n) h[i] = make_ulonglong2(a.off[i], a.len[i]);
+constexpr int MH_IPT = 4;
+__global__ void __launch_bounds__(256) k_make_handles(ArenaDev a, ulonglong2* h, LenStats* stats) {
+    const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint64_t off[MH_IPT];
+    uint32_t len[MH_IPT];
+#pragma unroll
+    for (int q = 0; q < MH_IPT; ++q) {
+        const uint64_t i = i0 + q * T;
+        off[q] = i < a.n ? a.off[i] : 0ull;
+        len[q] = i < a.n ? a.len[i] : 0u;
+    }
+    uint32_t inv = 0;
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int q = 0; q < MH_IPT; ++q) {
+        const uint64_t i = i0 + q * T;
+        if (i < a.n) {
+            h[i] = make_ulonglong2(off[q], len[q]);
+            inv = max(inv, ~len[q]);
+            sum += len[q];
+        }
+    }
+    if (!stats) return;
+    __shared__ uint32_t wi[8];
+    __shared__ unsigned long long wsum[8];
+    inv = __reduce_max_sync(0xffffffffu, inv);
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0) {
+        wi[threadIdx.x >> 5] = inv;
+        wsum[threadIdx.x >> 5] = sum;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            inv = max(inv, wi[w]);
+            sum += wsum[w];
+        }
+        atomicMax(&stats->inv_min, inv);
+        atomicAdd(&stats->sum, sum);
+    }
 }
 
-void make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st) {
-    if (a.n) DSSS_LAUNCH("k_make_handles", st, k_make_handles<<<grid_for(a.n, 256), 256, 0, st>>>(a, h));
+int make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st, LenStats* stats) {
+    if (stats) DSSS_CUDA(cudaMemsetAsync(stats, 0, sizeof(LenStats), st));
+    if (a.n)
+        DSSS_LAUNCH("k_make_handles", st,
+                    k_make_handles<<<grid_for((a.n + MH_IPT - 1) / MH_IPT, 256), 256, 0, st>>>(a, h, stats));
+    return DSSS_OK;
 }
 
 // ------------------------------------------------------------ multisplit ----

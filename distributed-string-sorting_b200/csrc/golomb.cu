@@ -14,12 +14,14 @@
 // Encoding is data-parallel: code lengths, a scan, then every code ORed into
 // its words.  A variable-length code is read sequentially; the decoder cuts
 // each block's bits into chunks of GB_CHUNK_BITS, reads every chunk from a
-// guessed code start and repeats, each chunk then starting where its
-// predecessor's last code ended, until no start changes.  The first chunk of
-// a block starts right, so the starts are exact once they agree; Golomb
-// codes fall back into step within a few codes, so nearly every guess holds
-// after the first repetition (and after as many repetitions as a block has
-// chunks in the worst case).
+// guessed code start and again from where its predecessor's last code ended,
+// until no start changes.  The first chunk of a block starts right, so the
+// starts are exact once they agree.  A reader that starts inside a code falls
+// into step with the codes after some of them (a few for short remainders,
+// some hundred for 40-bit ones), so the repetitions run inside a block of
+// threads, over 256 chunks in shared memory, and the blocks of threads then
+// agree among themselves in two rounds (in the worst case, as many as the
+// stream has such tiles).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -195,110 +197,347 @@ __global__ void k_gb_blocks(const unsigned long long* w, uint64_t nwords, uint32
     *nb = j;
 }
 
-struct GbChunk {
-    uint64_t cs, ce;     // the chunk's bits [cs, ce)
-    uint64_t bit1;       // end of its block's bits
-    uint64_t b, little;  // the block's parameters
-    uint32_t k, blk;
+// One block of the stream, as the chunk kernels use it.
+struct GbBlock {
+    uint64_t bit0, bit1;  // its code bits
+    uint64_t b, little;
+    uint64_t first;       // its uncoded first value
+    uint32_t chunk0;      // its first chunk (chunk0 of entry nb: all chunks)
+    uint32_t k;
 };
 
-// Bit t of the stream.
-__device__ __forceinline__ uint32_t gb_bit(const unsigned long long* w, uint64_t t) {
-    return (uint32_t)(w[t >> 6] >> (63 - (t & 63))) & 1u;
-}
+// A tile is GB_TILE consecutive chunks, one thread each; its words (and the
+// headers of the blocks that end inside it) are staged in shared memory as
+// 32-bit halves in stream order, one half of padding per 32 so that threads at
+// the same place of their chunks read different banks.
+constexpr uint32_t GB_TILE = 256;
+constexpr uint32_t GB_CUT = 1u << 31;  // in a chunk's count: its last code is cut off by the block's end
+constexpr uint32_t GB_STAGE = GB_TILE * (GB_CHUNK_BITS / 64) + 3 * GB_TILE + 2;
+__device__ __forceinline__ uint32_t gb_skew(uint32_t i) { return i + (i >> 5); }
+constexpr size_t GB_SMEM = (size_t)(2 * GB_STAGE + GB_STAGE / 16 + 2) * 4;
 
-// Reads the code at t (t < bit1).  Returns false at the stream's end (only
-// ones up to bit1: the padding); else sets the gap and moves t past the
-// code (t > bit1: the code is cut off).
-__device__ __forceinline__ bool gb_read(const unsigned long long* w, const GbChunk& C, uint64_t& t, uint64_t& gap) {
-    uint64_t q = 0;
-    for (;;) {  // ones up to the next zero, a word at a time
-        const uint32_t a = (uint32_t)(t & 63);
-        const uint64_t x = (uint64_t)w[t >> 6] << a;  // bits from t at the top
-        const uint32_t avail = 64 - a;
-        uint32_t ones = (uint32_t)__clzll(~x);  // leading ones (64 when all are)
-        if (ones > avail) ones = avail;
-        if (t + ones >= C.bit1) return false;  // no zero before the end
-        t += ones;
-        q += ones;
-        if (ones < avail) break;  // the zero is at t
-    }
-    ++t;  // the zero
-    uint64_t r = 0;
-    if (C.k) {
-        const uint32_t lo = C.k - 1;
-        for (uint32_t j = 0; j < lo; ++j) r = (r << 1) | (t < C.bit1 ? gb_bit(w, t++) : (++t, 0u));
-        if (r >= C.little) r = ((r << 1) | (t < C.bit1 ? gb_bit(w, t++) : (++t, 0u))) - C.little;
-    }
-    gap = q * C.b + r;
-    return true;
-}
-
-// One reading of every chunk from its start g[c]: cnt[c] codes start in
-// [g[c], ce), e[c] where the next code starts (bit1 at the stream's end).
-__global__ void k_gb_walk(const unsigned long long* w, const GbChunk* ch, uint64_t nch, const uint64_t* g, uint64_t* e,
-                          uint32_t* cnt, uint32_t* err) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nch) return;
-    const GbChunk C = ch[c];
-    uint64_t t = g[c];
-    uint32_t m = 0;
-    while (t < C.ce) {
-        uint64_t gap;
-        if (!gb_read(w, C, t, gap)) {
-            t = C.bit1;
-            break;
+struct GbReader {
+    const unsigned long long* w;   // the stream
+    const uint32_t* sw;            // words [w0, w1) of it, staged
+    uint64_t w0, w1, nwords, bit1;
+    uint64_t b, little;
+    uint32_t k;
+    __device__ __forceinline__ uint64_t word(uint64_t x) const {
+        if (x >= w0 && x < w1) {
+            const uint32_t i = 2 * (uint32_t)(x - w0);
+            return (uint64_t)sw[gb_skew(i)] << 32 | sw[gb_skew(i + 1)];
         }
-        ++m;
+        return x < nwords ? w[x] : 0ull;
     }
-    if (t > C.bit1) atomicOr(err, 4u);  // a code cut off by the block's end
-    e[c] = t;
-    cnt[c] = m;
+    // The 64 bits from bit t on, 0 past the block's end.
+    __device__ __forceinline__ uint64_t peek(uint64_t t) const {
+        if (t >= bit1) return 0;
+        const uint32_t a = (uint32_t)(t & 63);
+        const uint64_t x = t >> 6;
+        uint64_t v = word(x) << a;
+        if (a) v |= word(x + 1) >> (64 - a);
+        const uint64_t left = bit1 - t;
+        if (left < 64) v &= ~0ull << (64 - left);
+        return v;
+    }
+    // Reads the code at t (t < bit1).  Returns false at the stream's end (only
+    // ones up to bit1: the padding); else sets the gap and moves t past the
+    // code (t > bit1: the code is cut off).
+    __device__ __forceinline__ bool read(uint64_t& t, uint64_t& gap) const {
+        uint64_t q = 0;
+        for (;;) {
+            const uint32_t ones = (uint32_t)__clzll(~peek(t));
+            t += ones;
+            q += ones;
+            if (t >= bit1) return false;
+            if (ones < 64) break;
+        }
+        ++t;  // the zero
+        uint64_t r = 0;
+        if (k) {
+            const uint32_t lo = k - 1;
+            const uint64_t v = peek(t);
+            if (lo) r = v >> (64 - lo);
+            t += lo;
+            if (r >= little) {
+                r = ((r << 1) | ((v << lo) >> 63)) - little;
+                ++t;
+            }
+        }
+        gap = q * b + r;
+        return true;
+    }
+};
+
+// Chunk c: its block (the last j with chunk0 <= c) and its bits [cs, ce).
+__device__ __forceinline__ uint32_t gb_chunk(const GbBlock* blk, uint32_t nb, uint32_t c, uint64_t& cs, uint64_t& ce) {
+    uint32_t lo = 0, hi = nb;
+    while (hi - lo > 1) {
+        const uint32_t m = (lo + hi) >> 1;
+        if (blk[m].chunk0 <= c) lo = m;
+        else hi = m;
+    }
+    cs = blk[lo].bit0 + (uint64_t)(c - blk[lo].chunk0) * GB_CHUNK_BITS;
+    ce = min(cs + GB_CHUNK_BITS, blk[lo].bit1);
+    return lo;
 }
 
-// Each chunk starts where its predecessor in the block stopped.
-__global__ void k_gb_follow(const GbChunk* ch, uint64_t nch, const uint64_t* e, uint64_t* g, uint32_t* changed) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c == 0 || c >= nch || ch[c].blk != ch[c - 1].blk) return;
-    const uint64_t s = e[c - 1];
-    if (s != g[c]) {
-        g[c] = s;
-        *changed = 1;
+// Stages the tile's words (the block's threads together) and sets up each
+// thread's reader; cs, ce: the thread's chunk (cs = ce: none).  Returns its
+// block's number.
+__device__ __forceinline__ uint32_t gb_stage(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
+                                             uint32_t nb, uint32_t nch, uint32_t* sw, GbReader& R,
+                                             uint64_t& cs, uint64_t& ce) {
+    __shared__ unsigned long long s_range[2];
+    const uint32_t c0 = blockIdx.x * GB_TILE, c = c0 + threadIdx.x, cl = min(nch, c0 + GB_TILE) - 1;
+    uint32_t j = 0xFFFFFFFFu;
+    cs = ce = 0;
+    R.w = w;
+    R.sw = sw;
+    R.nwords = nwords;
+    R.bit1 = 0;
+    R.b = 1;
+    R.little = 0;
+    R.k = 0;
+    if (c < nch) {
+        j = gb_chunk(blk, nb, c, cs, ce);
+        R.bit1 = blk[j].bit1;
+        R.b = blk[j].b;
+        R.little = blk[j].little;
+        R.k = blk[j].k;
+        if (c == c0) s_range[0] = cs >> 6;
+        if (c == cl) s_range[1] = min((ce + 63) / 64 + 2, nwords);
+    }
+    __syncthreads();
+    R.w0 = s_range[0];
+    R.w1 = min((uint64_t)s_range[1], R.w0 + GB_STAGE);
+    for (uint32_t i = threadIdx.x; i < (uint32_t)(R.w1 - R.w0); i += GB_TILE) {
+        const uint64_t v = w[R.w0 + i];
+        sw[gb_skew(2 * i)] = (uint32_t)(v >> 32);
+        sw[gb_skew(2 * i + 1)] = (uint32_t)v;
+    }
+    __syncthreads();
+    return j;
+}
+
+// One reading of the tiles: every chunk is read from g[c] (round 0: its own
+// first bit) and then again from where its predecessor in the block stopped,
+// until no start of the tile changes.  A tile's first chunk starts where the
+// previous tile stopped in the previous round (end_in); a tile whose start
+// holds is left as it is.  cnt, sum: the codes that start in each chunk and
+// the sum of their gaps; end_out: where each tile stopped; *changed: some
+// tile now stops elsewhere.  A wrong start falls into step after some hundred
+// codes (20 chunks of 40-bit codes), far less than a tile, so two rounds
+// settle the stream.  (Rounds over the whole stream, each re-reading every
+// chunk, took 21 launches of 0.5 ms for 4e6 hashes, 20.5 of the 29 ms of a
+// there-and-back.)  Bound by the instructions per code and round: where b is a
+// power of two a code's length is its unary part plus a constant, so the
+// repetitions read one funnel-shifted word per code and no remainder (1.08 ->
+// 0.31 ms for the four launches); counts and gap sums are taken once, at the
+// end.
+__global__ void __launch_bounds__(GB_TILE) k_gb_walk(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
+                                                     uint32_t nb, uint32_t nch, int round, const uint64_t* end_in,
+                                                     uint64_t* end_out, uint64_t* g, uint32_t* cnt,
+                                                     unsigned long long* sum, uint32_t* changed) {
+    extern __shared__ __align__(16) uint32_t gb_sm[];
+    __shared__ unsigned long long e[GB_TILE];
+    const uint32_t c0 = blockIdx.x * GB_TILE, c = c0 + threadIdx.x;
+    if (round) {  // the tile's start: unchanged, or settled since the stream's (or the block's) first bit
+        uint64_t cs, ce;
+        const uint32_t j = gb_chunk(blk, nb, c0, cs, ce);
+        const bool keep = blockIdx.x == 0 || blk[j].chunk0 == c0 || g[c0] == end_in[blockIdx.x - 1];
+        if (keep) {  // the same for the whole block
+            if (threadIdx.x == 0) end_out[blockIdx.x] = end_in[blockIdx.x];
+            return;
+        }
+    }
+    GbReader R;
+    uint64_t cs, ce;
+    const uint32_t j = gb_stage(w, nwords, blk, nb, nch, gb_sm, R, cs, ce);
+    const bool valid = c < nch;
+    const bool chained = valid && threadIdx.x > 0 && blk[j].chunk0 != c;  // starts where the thread before stopped
+    uint64_t start = valid ? (round ? g[c] : cs) : 0;
+    if (round && threadIdx.x == 0) start = end_in[blockIdx.x - 1];
+    // the codes a repetition can step over by their unary part alone: b a
+    // power of two, the word read and the code's end inside the block
+    const uint64_t o = R.w0 * 64;
+    uint32_t lim = 0;
+    if (valid && R.little == 0) {
+        const uint64_t staged = (R.w1 - R.w0) * 64, left = R.bit1 - o;
+        const uint64_t room = min(staged, left);
+        if (room > 64ull + R.k + 33) lim = (uint32_t)(room - 64 - R.k - 33);
+    }
+    bool redo = valid;
+    uint64_t t = start;
+    for (;;) {
+        if (redo) {
+            t = start;
+            while (t < ce) {
+                const uint32_t u = (uint32_t)(t - o);  // t >= cs >= o: a chunk's codes start inside it
+                if (u < lim) {
+                    const uint32_t i = u >> 5;
+                    const uint32_t x = __funnelshift_l(gb_sm[gb_skew(i + 1)], gb_sm[gb_skew(i)], u & 31);
+                    const uint32_t ones = (uint32_t)__clz(~x);
+                    if (ones < 32) {
+                        t += ones + 1 + R.k;
+                        continue;
+                    }
+                }
+                uint64_t gap;
+                if (!R.read(t, gap)) {
+                    t = R.bit1;
+                    break;
+                }
+            }
+            e[threadIdx.x] = t;
+        }
+        __syncthreads();
+        redo = chained && e[threadIdx.x - 1] != start;
+        if (redo) start = e[threadIdx.x - 1];
+        if (!__syncthreads_or(redo)) break;
+    }
+    uint32_t m = 0;
+    unsigned long long s = 0;
+    if (valid) {
+        t = start;
+        while (t < ce) {
+            uint64_t gap;
+            if (!R.read(t, gap)) {
+                t = R.bit1;
+                break;
+            }
+            ++m;
+            s += gap;
+        }
+    }
+    if (!valid) return;
+    g[c] = start;
+    cnt[c] = m | (t > R.bit1 ? GB_CUT : 0u);
+    sum[c] = s;
+    if (threadIdx.x == GB_TILE - 1 || c + 1 == nch) {
+        if (round && t != end_in[blockIdx.x]) *changed = 1;
+        end_out[blockIdx.x] = t;
     }
 }
 
-// The values: chunk c's codes go to out[oc[c]..], each its block's first
-// value plus the gaps up to it (base[c] = that sum before the chunk).
-__global__ void k_gb_gaps(const unsigned long long* w, const GbChunk* ch, uint64_t nch, const uint64_t* g,
-                          const uint64_t* oc, unsigned long long* out, unsigned long long* csum) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nch) return;
-    const GbChunk C = ch[c];
-    uint64_t t = g[c], o = oc[c], s = 0;
-    while (t < C.ce) {
-        uint64_t gap;
-        if (!gb_read(w, C, t, gap)) break;
-        s += gap;
-        out[o++] = gap;
+// Exclusive scan of (m, s) over the block's threads, and the totals.
+__device__ __forceinline__ void gb_block_scan(uint32_t m, unsigned long long s, uint32_t& pm, unsigned long long& ps,
+                                              uint32_t& tm, unsigned long long& ts) {
+    __shared__ uint32_t wm[GB_TILE / 32];
+    __shared__ unsigned long long wsum[GB_TILE / 32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t x = m;
+    unsigned long long y = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t xx = __shfl_up_sync(0xffffffffu, x, o);
+        const unsigned long long yy = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) {
+            x += xx;
+            y += yy;
+        }
     }
-    csum[c] = s;
+    if (lane == 31) {
+        wm[w] = x;
+        wsum[w] = y;
+    }
+    __syncthreads();
+    pm = x - m;
+    ps = y - s;
+    tm = 0;
+    ts = 0;
+    for (int k = 0; k < (int)(GB_TILE / 32); ++k) {
+        if (k < w) {
+            pm += wm[k];
+            ps += wsum[k];
+        }
+        tm += wm[k];
+        ts += wsum[k];
+    }
+    __syncthreads();
 }
 
-// The blocks' uncoded first values: out[at[j]] = first[j].
-__global__ void k_gb_firsts(const uint64_t* at, const uint64_t* first, uint32_t nb, unsigned long long* out) {
+// Codes and gap sums before every chunk inside its tile, and the tiles' totals.
+__global__ void __launch_bounds__(GB_TILE) k_gb_prefix(uint32_t nch, const uint32_t* cnt, const unsigned long long* sum,
+                                                       uint32_t* pcnt, unsigned long long* psum, uint32_t* tcnt,
+                                                       unsigned long long* tsum, uint32_t* cut) {
+    const uint32_t c = blockIdx.x * GB_TILE + threadIdx.x;
+    const uint32_t v = c < nch ? cnt[c] : 0u;
+    if (v & GB_CUT) *cut = 1;
+    uint32_t pm, tm;
+    unsigned long long ps, ts;
+    gb_block_scan(v & ~GB_CUT, c < nch ? sum[c] : 0ull, pm, ps, tm, ts);
+    if (c < nch) {
+        pcnt[c] = pm;
+        psum[c] = ps;
+    }
+    if (threadIdx.x == 0) {
+        tcnt[blockIdx.x] = tm;
+        tsum[blockIdx.x] = ts;
+    }
+}
+
+// One block: codes and gap sums before every tile (entry `tiles`: all).
+__global__ void __launch_bounds__(GB_TILE) k_gb_tiles(uint32_t tiles, const uint32_t* tcnt,
+                                                      const unsigned long long* tsum, uint64_t* bcnt,
+                                                      unsigned long long* bsum) {
+    uint64_t cm = 0;
+    unsigned long long cs = 0;
+    for (uint32_t b = 0; b < tiles; b += GB_TILE) {
+        const uint32_t i = b + threadIdx.x;
+        uint32_t pm, tm;
+        unsigned long long ps, ts;
+        gb_block_scan(i < tiles ? tcnt[i] : 0u, i < tiles ? tsum[i] : 0ull, pm, ps, tm, ts);
+        if (i < tiles) {
+            bcnt[i] = cm + pm;
+            bsum[i] = cs + ps;
+        }
+        cm += tm;
+        cs += ts;
+    }
+    if (threadIdx.x == 0) {
+        bcnt[tiles] = cm;
+        bsum[tiles] = cs;
+    }
+}
+
+// Codes and gap sums before every block (entry nb: all).
+__global__ void k_gb_starts(const GbBlock* blk, uint32_t nb, uint32_t nch, uint32_t tiles, const uint64_t* bcnt,
+                            const unsigned long long* bsum, const uint32_t* pcnt, const unsigned long long* psum,
+                            uint64_t* ocnt, unsigned long long* osum) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < nb) out[at[j]] = first[j];
+    if (j > nb) return;
+    const uint32_t c = j < nb ? blk[j].chunk0 : nch;
+    ocnt[j] = c < nch ? bcnt[c / GB_TILE] + pcnt[c] : bcnt[tiles];
+    osum[j] = c < nch ? bsum[c / GB_TILE] + psum[c] : bsum[tiles];
 }
 
-__global__ void k_gb_sums(const GbChunk* ch, uint64_t nch, const uint64_t* oc, const uint32_t* cnt,
-                          const unsigned long long* base, unsigned long long* out) {
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The values: block j's uncoded first value goes to ocnt[j] + j, its chunks'
+// codes behind it, each the first value plus the gaps up to it.
+__global__ void k_gb_firsts(const GbBlock* blk, uint32_t nb, const uint64_t* ocnt, unsigned long long* out) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nb) out[ocnt[j] + j] = blk[j].first;
+}
+
+__global__ void __launch_bounds__(GB_TILE) k_gb_emit(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
+                                                     uint32_t nb, uint32_t nch, const uint64_t* g, const uint64_t* bcnt,
+                                                     const unsigned long long* bsum, const uint32_t* pcnt,
+                                                     const unsigned long long* psum, const unsigned long long* osum,
+                                                     unsigned long long* out) {
+    extern __shared__ __align__(16) uint32_t gb_sm[];
+    GbReader R;
+    uint64_t cs, ce;
+    const uint32_t j = gb_stage(w, nwords, blk, nb, nch, gb_sm, R, cs, ce);
+    const uint32_t c = blockIdx.x * GB_TILE + threadIdx.x;
     if (c >= nch) return;
-    uint64_t run = base[c];
-    const uint64_t o = oc[c];
-    for (uint32_t j = 0; j < cnt[c]; ++j) {
-        run += out[o + j];
-        out[o + j] = run;
+    uint64_t t = g[c];
+    uint64_t o = bcnt[blockIdx.x] + pcnt[c] + j + 1;
+    uint64_t run = blk[j].first + (bsum[blockIdx.x] + psum[c] - osum[j]);
+    while (t < ce) {
+        uint64_t gap;
+        if (!R.read(t, gap)) break;
+        run += gap;
+        out[o++] = run;
     }
 }
 
@@ -452,121 +691,98 @@ int dsss_golomb_decode(dsss_ctx* ctx, const uint64_t* words, uint64_t nwords, ui
         DSSS_CUDA(cudaStreamSynchronize(st));
         std::copy(pin64, pin64 + 4ull * nb, blk.begin());
     }
-    // 2. chunks of every block's bits
-    std::vector<GbChunk> ch;
-    std::vector<uint64_t> g0;
-    std::vector<uint64_t> first_chunk(nb + 1);
+    // 2. the blocks with their chunks
+    std::vector<GbBlock> hb(nb + 1);
+    uint64_t chunks = 0;
     for (uint32_t j = 0; j < nb; ++j) {
         const uint64_t pos = blk[4 * j], S = blk[4 * j + 1], b = blk[4 * j + 2];
         const uint32_t k = gb_ceil_log2(b);
-        const uint64_t little = (k >= 64 ? 0ull : (1ull << k)) - b;
         const uint64_t bit0 = (pos + 3) * 64, bit1 = (pos + 1 + S) * 64;
-        first_chunk[j] = ch.size();
-        for (uint64_t cs = bit0; cs < bit1; cs += GB_CHUNK_BITS) {
-            ch.push_back(GbChunk{cs, std::min(cs + GB_CHUNK_BITS, bit1), bit1, b, little, k, j});
-            g0.push_back(cs);
-        }
+        hb[j] = GbBlock{bit0, bit1, b, (k >= 64 ? 0ull : (1ull << k)) - b, blk[4 * j + 3], (uint32_t)chunks, k};
+        chunks += (bit1 - bit0 + GB_CHUNK_BITS - 1) / GB_CHUNK_BITS;
     }
-    first_chunk[nb] = ch.size();
-    const uint64_t nch = ch.size();
-    const uint64_t NC = nch ? nch : 1;
-    const uint64_t NB = nb ? nb : 1;
-    auto plan = [&](Carve& c, GbChunk*& dch, uint64_t*& g, uint64_t*& e, uint32_t*& cnt, uint64_t*& oc,
-                    unsigned long long*& csum, unsigned long long*& base, uint32_t*& flags, uint64_t*& fat) {
-        dch = c.take<GbChunk>(NC);
+    hb[nb] = GbBlock{};
+    hb[nb].chunk0 = (uint32_t)chunks;
+    if (chunks >= (1ull << 32) - GB_TILE) return fail(DSSS_ENOTSUP, "Golomb stream of 2^42 bits or more");
+    const uint32_t nch = (uint32_t)chunks, tiles = (nch + GB_TILE - 1) / GB_TILE;
+    const uint64_t NC = nch ? nch : 1, NT = (uint64_t)tiles + 1;
+    GbBlock* dblk;
+    uint64_t *g, *end[2], *bcnt, *ocnt;
+    uint32_t *cnt, *pcnt, *tcnt, *flags;
+    unsigned long long *sum, *psum, *tsum, *bsum, *osum;
+    auto plan = [&](Carve& c) {
+        dblk = c.take<GbBlock>(nb + 1);
         g = c.take<uint64_t>(NC);
-        e = c.take<uint64_t>(NC);
         cnt = c.take<uint32_t>(NC);
-        oc = c.take<uint64_t>(NC);
-        csum = c.take<unsigned long long>(NC);
-        base = c.take<unsigned long long>(NC);
-        flags = c.take<uint32_t>(2);
-        fat = c.take<uint64_t>(2 * NB);  // (output place, value) of every block's first value
+        sum = c.take<unsigned long long>(NC);
+        pcnt = c.take<uint32_t>(NC);
+        psum = c.take<unsigned long long>(NC);
+        end[0] = c.take<uint64_t>(NT);
+        end[1] = c.take<uint64_t>(NT);
+        tcnt = c.take<uint32_t>(NT);
+        tsum = c.take<unsigned long long>(NT);
+        bcnt = c.take<uint64_t>(NT);
+        bsum = c.take<unsigned long long>(NT);
+        ocnt = c.take<uint64_t>(nb + 1);
+        osum = c.take<unsigned long long>(nb + 1);
+        flags = c.take<uint32_t>(2);  // [0] a tile stopped elsewhere, [1] a code is cut off
     };
-    GbChunk* dch;
-    uint64_t *g, *e, *oc, *fat;
-    uint32_t *cnt, *flags;
-    unsigned long long *csum, *base;
     Carve s1(nullptr);
-    plan(s1, dch, g, e, cnt, oc, csum, base, flags, fat);
+    plan(s1);
     DSSS_TRY(ensure_ws(ctx, s1.used));
-    DSSS_TRY(ensure_pin(ctx, 16 * NC + 64));
     Carve c(ctx->ws);
-    plan(c, dch, g, e, cnt, oc, csum, base, flags, fat);
-    std::vector<uint32_t> hcnt(nch);
+    plan(c);
+    uint64_t* pin64 = (uint64_t*)ctx->pin;  // 32 max_blocks + 64 bytes, nb <= max_blocks
+    uint32_t* pin = (uint32_t*)(pin64 + nb + 1);
+    DSSS_CUDA(cudaMemcpyAsync(dblk, hb.data(), (nb + 1) * sizeof(GbBlock), cudaMemcpyHostToDevice, st));
+    DSSS_CUDA(cudaMemsetAsync(flags, 0, 8, st));
+    static std::atomic<uint64_t> walk_configured{0}, emit_configured{0};
+    DSSS_TRY(set_smem_once(walk_configured, k_gb_walk, (int)GB_SMEM));
+    DSSS_TRY(set_smem_once(emit_configured, k_gb_emit, (int)GB_SMEM));
     if (nch) {
-        DSSS_CUDA(cudaMemcpyAsync(dch, ch.data(), nch * sizeof(GbChunk), cudaMemcpyHostToDevice, st));
-        DSSS_CUDA(cudaMemcpyAsync(g, g0.data(), nch * 8, cudaMemcpyHostToDevice, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));  // the host vectors are reused below
-        uint32_t* pin = (uint32_t*)ctx->pin;
-        // 3. read every chunk until the starts agree (at most one round per
-        // chunk of the longest block, plus one)
-        uint64_t longest = 0;
-        for (uint32_t j = 0; j < nb; ++j) longest = std::max(longest, first_chunk[j + 1] - first_chunk[j]);
+        // 3. read the tiles until no tile stops elsewhere (each round settles
+        // at least one more tile of every block)
         bool settled = false;
-        for (uint64_t round = 0; round <= longest && !settled; ++round) {
-            DSSS_CUDA(cudaMemsetAsync(flags, 0, 8, st));
-            DSSS_LAUNCH("k_gb_walk", st, k_gb_walk<<<grid_for(nch, 128), 128, 0, st>>>(w, dch, nch, g, e, cnt,
-                                                                                       flags + 1));
-            DSSS_LAUNCH("k_gb_follow", st, k_gb_follow<<<grid_for(nch, 256), 256, 0, st>>>(dch, nch, e, g, flags));
-            DSSS_CUDA(cudaMemcpyAsync(pin, flags, 8, cudaMemcpyDeviceToHost, st));
+        for (uint32_t round = 0; round <= tiles + 1 && !settled; ++round) {
+            if (round > 1) DSSS_CUDA(cudaMemsetAsync(flags, 0, 4, st));
+            DSSS_LAUNCH("k_gb_walk", st,
+                        k_gb_walk<<<tiles, GB_TILE, GB_SMEM, st>>>(w, nwords, dblk, nb, nch, (int)round,
+                                                                  end[(round & 1) ^ 1], end[round & 1], g, cnt, sum,
+                                                                  flags));
+            if (round == 0) continue;
+            DSSS_CUDA(cudaGetLastError());
+            DSSS_CUDA(cudaMemcpyAsync(pin, flags, 4, cudaMemcpyDeviceToHost, st));
             DSSS_CUDA(cudaStreamSynchronize(st));
             settled = pin[0] == 0;
-            if (settled && (pin[1] & 4u)) return fail(DSSS_EINVAL, "a Golomb code is cut off by its block's end");
         }
         if (!settled) return fail(DSSS_EDEVICE, "Golomb chunk starts did not settle");
-        DSSS_CUDA(cudaMemcpyAsync(pin, cnt, nch * 4, cudaMemcpyDeviceToHost, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));
-        std::copy(pin, pin + nch, hcnt.begin());
     }
     // 4. output places: each block's first value, then its chunks' codes
-    std::vector<uint64_t> hoc(nch), first_at(nb);
-    uint64_t total = 0;
-    for (uint32_t j = 0; j < nb; ++j) {
-        first_at[j] = total++;
-        uint64_t m = 0;
-        for (uint64_t x = first_chunk[j]; x < first_chunk[j + 1]; ++x) {
-            hoc[x] = total;
-            total += hcnt[x];
-            m += hcnt[x];
-        }
-        if (j < max_blocks) block_counts[j] = m + 1;
-    }
+    if (nch)
+        DSSS_LAUNCH("k_gb_prefix", st,
+                    k_gb_prefix<<<tiles, GB_TILE, 0, st>>>(nch, cnt, sum, pcnt, psum, tcnt, tsum, flags + 1));
+    DSSS_LAUNCH("k_gb_tiles", st, k_gb_tiles<<<1, GB_TILE, 0, st>>>(tiles, tcnt, tsum, bcnt, bsum));
+    DSSS_LAUNCH("k_gb_starts", st,
+                k_gb_starts<<<grid_for(nb + 1, 128), 128, 0, st>>>(dblk, nb, nch, tiles, bcnt, bsum, pcnt, psum, ocnt,
+                                                                  osum));
+    DSSS_CUDA(cudaGetLastError());
+    DSSS_CUDA(cudaMemcpyAsync(pin64, ocnt, (nb + 1) * 8, cudaMemcpyDeviceToHost, st));
+    DSSS_CUDA(cudaMemcpyAsync(pin, flags, 8, cudaMemcpyDeviceToHost, st));
+    DSSS_CUDA(cudaStreamSynchronize(st));
+    if (pin[1]) return fail(DSSS_EINVAL, "a Golomb code is cut off by its block's end");
+    const uint64_t total = pin64[nb] + nb;
+    for (uint32_t j = 0; j < nb; ++j) block_counts[j] = pin64[j + 1] - pin64[j] + 1;
     *n_values = total;
     *nblocks = nb;
     if (!values) return DSSS_OK;  // size query
     if (total > cap_values) return fail(DSSS_EINVAL, "cap_values %llu below the %llu coded values",
                                         (unsigned long long)cap_values, (unsigned long long)total);
     unsigned long long* out = (unsigned long long*)values;
-    {  // the uncoded first values
-        std::vector<uint64_t> fa(2ull * nb);
-        for (uint32_t j = 0; j < nb; ++j) {
-            fa[j] = first_at[j];
-            fa[nb + j] = blk[4 * j + 3];
-        }
-        DSSS_CUDA(cudaMemcpyAsync(fat, fa.data(), 16ull * nb, cudaMemcpyHostToDevice, st));
-        DSSS_LAUNCH("k_gb_firsts", st, k_gb_firsts<<<grid_for(nb, 128), 128, 0, st>>>(fat, fat + nb, nb, out));
-        DSSS_CUDA(cudaStreamSynchronize(st));  // fa is released below
-    }
-    if (nch) {
-        DSSS_CUDA(cudaMemcpyAsync(oc, hoc.data(), nch * 8, cudaMemcpyHostToDevice, st));
-        DSSS_LAUNCH("k_gb_gaps", st, k_gb_gaps<<<grid_for(nch, 128), 128, 0, st>>>(w, dch, nch, g, oc, out, csum));
-        // each chunk's start: its block's first value plus the gaps before it
-        uint64_t* pin64 = (uint64_t*)ctx->pin;
-        std::vector<uint64_t> hs(nch), hb(nch);
-        DSSS_CUDA(cudaMemcpyAsync(pin64, csum, nch * 8, cudaMemcpyDeviceToHost, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));
-        std::copy(pin64, pin64 + nch, hs.begin());
-        for (uint32_t j = 0; j < nb; ++j) {
-            uint64_t run = blk[4 * j + 3];
-            for (uint64_t x = first_chunk[j]; x < first_chunk[j + 1]; ++x) {
-                hb[x] = run;
-                run += hs[x];
-            }
-        }
-        DSSS_CUDA(cudaMemcpyAsync(base, hb.data(), nch * 8, cudaMemcpyHostToDevice, st));
-        DSSS_LAUNCH("k_gb_sums", st, k_gb_sums<<<grid_for(nch, 128), 128, 0, st>>>(dch, nch, oc, cnt, base, out));
-    }
+    DSSS_LAUNCH("k_gb_firsts", st, k_gb_firsts<<<grid_for(nb, 128), 128, 0, st>>>(dblk, nb, ocnt, out));
+    if (nch)
+        DSSS_LAUNCH("k_gb_emit", st,
+                    k_gb_emit<<<tiles, GB_TILE, GB_SMEM, st>>>(w, nwords, dblk, nb, nch, g, bcnt, bsum, pcnt, psum,
+                                                              osum, out));
     DSSS_CUDA(cudaGetLastError());
     DSSS_CUDA(cudaStreamSynchronize(st));
     return DSSS_OK;

@@ -53,6 +53,8 @@ struct Seg {
     uint32_t nspl;
     unsigned long long spec_diff;
     uint32_t spl_slot, fix0;
+    // pivot pass: the pivot's string id (NO_PIVOT: the segment's first string)
+    uint32_t piv, pad;
     // OR and AND of the keys the previous pass's scatter wrote for this
     // segment (children with keys, when the child table is kept): the bits
     // that differ among its keys are kor ^ kand
@@ -76,6 +78,7 @@ constexpr int SPL_SAMPLE = 2048;
 constexpr uint32_t SPL_MAX = 255, SPL_STRIDE = 256, SPL_EQ_MAX = 127;
 constexpr uint32_t SPL_MIN_FLOOR = 4096;  // smallest sort_split_min other than 0 (off)
 constexpr uint32_t FIX_NONE = 0xFFFFFFFFu;
+constexpr uint32_t NO_PIVOT = 0xFFFFFFFFu;
 
 constexpr int NBINS = 4;
 __host__ __device__ constexpr int bin_cap(int b) { return b == 0 ? 32 : b == 1 ? 256 : b == 2 ? 1024 : 4096; }
@@ -154,6 +157,8 @@ __device__ __forceinline__ void push_small(const SortState& S, uint32_t start, u
     s.nspl = 0;
     s.spl_slot = 0;
     s.fix0 = 0;
+    s.piv = NO_PIVOT;
+    s.pad = 0;
     s.spec_diff = 0;
     s.kor = 0;
     s.kand = ~0ull;
@@ -181,6 +186,8 @@ __device__ __forceinline__ uint32_t push_large(const SortState& S, Seg* dst, uin
     s.nspl = 0;
     s.spl_slot = 0;
     s.fix0 = 0;
+    s.piv = NO_PIVOT;
+    s.pad = 0;
     s.spec_diff = 0;
     s.kor = 0;
     s.kand = ~0ull;
@@ -252,6 +259,59 @@ __device__ __forceinline__ void key_words(const uint8_t* chars, uint64_t off, ui
 constexpr int PF_W = 8;  // prefix words compared per batch (64 bytes)
 constexpr uint32_t SPEC_MAX = 56;  // speculated depths stay below d0 + 56 (key inside 64 bytes)
 
+// The pivot of a pivot pass: of PIVOT_SAMPLE evenly spaced members, the one
+// with the largest sum of LCPs (from the segment's depth, PIVOT_CAP bytes at
+// most) with the others.  In a chain of nested prefixes that is a string of the
+// longest shared part, so one pass peels nearly the whole chain; with the
+// segment's first string as pivot, every pass left the half of the chain that
+// shares more than it does.  Measured on 4e6 strings whose shared prefix has a
+// random length: 18 passes -> 4, 2.51 -> 1.69 ms per call.
+constexpr uint32_t PIVOT_SAMPLE = 64, PIVOT_WORDS = (PIVOT_CAP + 7) / 8;
+__device__ void choose_pivot(const SortState& S, Seg& sg, unsigned long long (*pw)[PIVOT_SAMPLE], uint32_t* psum,
+                             uint32_t* pid) {
+    const uint32_t* ord = S.ord[sg.flags & F_PARITY];
+    const uint32_t m = min(sg.size, PIVOT_SAMPLE), d0 = sg.depth;
+    for (uint32_t x = threadIdx.x; x < m * (PIVOT_WORDS / 4); x += blockDim.x) {
+        const uint32_t k = x % m, w0 = 4 * (x / m);
+        const uint32_t id = ord[sg.start + (uint32_t)((uint64_t)k * sg.size / m)];
+        uint64_t off, v[4];
+        uint32_t len;
+        str_of(S.a, id, off, len);
+        key_words<4>(S.a.chars, off, len, d0 + 8 * w0, 4, v);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) pw[w0 + q][k] = v[q];
+        if (w0 == 0) {
+            pid[k] = id;
+            psum[k] = 0;
+        }
+    }
+    __syncthreads();
+    for (uint32_t x = threadIdx.x; x < m * m; x += blockDim.x) {
+        const uint32_t i = x % m, j = x / m;
+        if (i >= j) continue;
+        uint32_t l = 8 * PIVOT_WORDS;
+        for (uint32_t w = 0; w < PIVOT_WORDS; ++w) {
+            const uint64_t a = pw[w][i], b = pw[w][j];
+            if (a != b) {
+                l = 8 * w + key_lcp(a, b);
+                break;
+            }
+            if (zero_byte(a) < 8) break;  // equal strings: the longest of LCPs
+        }
+        l = min(l, PIVOT_CAP);
+        atomicAdd(&psum[i], l);
+        atomicAdd(&psum[j], l);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        uint32_t best = 0;  // the sum (at most 63 * 127) above, the sample below
+        for (uint32_t k = threadIdx.x; k < m; k += 32) best = max(best, psum[k] << 8 | k);
+        best = __reduce_max_sync(0xffffffffu, best);
+        if (threadIdx.x == 0) sg.piv = pid[best & 0xFFu];
+    }
+    __syncthreads();  // the sample buffers are reused by the next segment
+}
+
 // Speculated common prefix of each segment without keys: the smallest LCP with
 // the segment's first string over up to 256 evenly spaced members, when it is
 // below d0 + SPEC_MAX.  k_prefix then reads each string once for both the
@@ -261,9 +321,15 @@ constexpr uint32_t SPEC_MAX = 56;  // speculated depths stay below d0 + 56 (key 
 // share SPEC_MAX bytes keep the plain prefix search (long common prefixes).
 __global__ void __launch_bounds__(256) k_spec(SortState S, Seg* segs, uint32_t nseg) {
     __shared__ uint32_t wmin[8];
+    __shared__ unsigned long long pw[PIVOT_WORDS][PIVOT_SAMPLE];
+    __shared__ uint32_t psum[PIVOT_SAMPLE], pid[PIVOT_SAMPLE];
     for (uint32_t si = blockIdx.x; si < nseg; si += gridDim.x) {
         Seg& sg = segs[si];
-        if (sg.flags & (F_KEYS | F_PIVOT)) continue;  // the same for the whole block
+        if (sg.flags & F_PIVOT) {  // the same for the whole block
+            choose_pivot(S, sg, pw, psum, pid);
+            continue;
+        }
+        if (sg.flags & F_KEYS) continue;
         const uint32_t* ord = S.ord[sg.flags & F_PARITY];
         const uint32_t d0 = sg.depth;
         uint32_t l = 0xFFFFFFFFu;
@@ -645,7 +711,7 @@ __global__ void __launch_bounds__(256) k_lcp_fix(SortState S) {
 
 // ----------------------------------------------------------------- pivot ----
 // Pivot pass of an F_PIVOT segment at depth d (all its strings share their
-// first d bytes) with s0 its first string.  For string x, l = LCP(x, s0)
+// first d bytes) with pivot s0, one of its strings.  For string x, l = LCP(x, s0)
 // counted from d and capped at PIVOT_CAP, and x's pseudo key holds
 //   byte 0: code = l            if x < s0 (x's byte at l is smaller: x ends
 //                               there or differs downwards),
@@ -712,7 +778,7 @@ __global__ void __launch_bounds__(LT_NT) k_pivot(SortState S, Seg* segs, uint32_
     const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
     uint64_t off0;
     uint32_t len0;
-    str_of(S.a, ord[sg.start], off0, len0);
+    str_of(S.a, sg.piv == NO_PIVOT ? ord[sg.start] : sg.piv, off0, len0);
     const uint64_t k0 = (uint64_t)PIVOT_CAP << 56;
     uint64_t df = 0;
     for (uint32_t i = tb + threadIdx.x; i < te; i += LT_NT) {
@@ -1043,8 +1109,7 @@ __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, uint32
             push_small(S, cs, total, depth, np | F_KEYS);
         }
     } else if (b == 0) {
-        // split by pivot code (only the pivot pass's own segment, whose first
-        // string is the pivot): large children keep the pseudo keys, small
+        // split by pivot code (only the pivot pass's own segment): large children keep the pseudo keys, small
         // ones restart from the depth their strings share
         if (total > S.small_max) {
             const uint32_t slot = push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO);
@@ -1054,7 +1119,7 @@ __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, uint32
             if (d == PIVOT_CAP) {
                 uint64_t o0;
                 uint32_t l0;
-                str_of(S.a, S.ord[par][sg.start], o0, l0);
+                str_of(S.a, sg.piv == NO_PIVOT ? S.ord[par][sg.start] : sg.piv, o0, l0);
                 cd = min(depth + PIVOT_CAP, l0);
             }
             push_small(S, cs, total, cd, np);

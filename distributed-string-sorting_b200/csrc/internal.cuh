@@ -146,7 +146,7 @@ enum TuneKnob : int {
                              // bits (several key bytes over small alphabets); 2: only where the first
                              // differing byte varies in at most four bits; 3: the same in the first pass
                              // only; 0: on one key byte (default)
-    TUNE_SORT_SEG_BITS,      // the same for the shared-memory passes of the segment sorter (default 0)
+    TUNE_SORT_SEG_BITS,      // accepted, without effect
     TUNE_COUNT
 };
 int64_t tune(TuneKnob k);

@@ -15,11 +15,11 @@
 // A child that keeps more than half of its parent (a chain of long shared
 // prefixes, e.g. suffixes inside repeats or strings that share a long common
 // head) would lose one byte per pass; it is flagged for a pivot pass instead:
-// every string's LCP with the segment's first string (up to 127 bytes) and
+// every string's LCP with one of the segment's strings (up to 127 bytes) and
 // the byte after it become a two-byte pseudo key whose order is the strings'
 // order, so one pass resolves up to 127 bytes of the chain.
-// Children of size <= small_max finish in one CTA (small_sort): bitonic sort
-// of (group, key, id) in shared memory, tie groups re-keyed 8 bytes deeper
+// Children of size <= small_max finish in one CTA (k_seg_sort): bucket passes
+// on the keys' differing bits in shared memory, ties re-keyed against a pivot
 // until every group is a single string or byte-identical strings.
 // LCPs are written where they become known: depth + first differing byte at
 // every bucket / group boundary, the length for byte-identical neighbours.
@@ -113,7 +113,6 @@ struct SortState {
     uint32_t small_max;
     uint32_t pivot;  // pivot passes enabled
     uint32_t bits;   // plain keys split on their top differing bits: 0 never, 1 always, 2 on narrow bytes
-    uint32_t seg_bits;  // the same inside the segment sorter
     uint32_t first;     // the first pass over the arena (host-driven passes)
     uint64_t cap_large, cap_small, cap_tiles, cap_chunks;
     // sampled splitters: segments of at least split_min strings (0: never);
@@ -1336,322 +1335,240 @@ __global__ void __launch_bounds__(LT_NT, 4) k_scatter(SortState S, const Seg* se
 
 // ------------------------------------------------------------ small sort ----
 // Segments of 2..small_max strings finish inside one CTA (the tail the MSD
-// passes hand over, like the reference's insertion-sort / multikey tail):
-//  - buckets of up to 32 strings, and of up to 64 from a wide split in the
-//    large variants: one warp, a bitonic network across the 32 lanes (two
-//    elements per lane above 32) on (group, key, id); groups of
-//    equal keys jump to the depth where a member leaves the group's head and
-//    are sorted again until each group is one string or byte-identical strings;
-//  - larger buckets: an MSD pass in shared memory on the first key byte that
-//    differs inside the bucket (warp-aggregated histogram, scan, stable
-//    scatter); children go on a shared-memory stack or to the warp list.
+// passes hand over, like the reference's insertion-sort / multikey tail), those
+// of up to 32 in one warp.  A group of strings is sorted by a 64-bit key:
+//   plain  : 8 bytes of each string from the group's depth;
+//   pseudo : each string's LCP l (from the depth) with one of the group, the
+//            pivot, as a 16-bit code that orders as the strings do, then the 6
+//            bytes behind it: a group whose 8-byte keys all agree goes on with
+//            these, since its strings often agree for long (suffixes of copied
+//            text, shared heads) and then leave the pivot at many depths;
+//   id     : the strings are equal; they keep ascending ids.
+// Equal keys that do not hold their strings' end form the next groups.
+//
+// A CTA takes groups of more than 32 strings through one bucket pass each: the
+// most significant bits in which the group's keys differ, as many as two
+// buckets per string need, pick a bucket; shared atomics count them and hand
+// out places (the order inside a bucket does not matter, every bucket is
+// sorted by (key, id) afterwards); buckets of 2..8 strings are sorted by one
+// thread each, up to 32 by a warp, larger ones return to the CTA's stack.
+// Over keys with enough differing bits nearly all buckets hold one string, so
+// a string costs about 60 thread instructions; the stable byte passes with
+// match instructions and bitonic networks that this replaces took 26 warp
+// instructions per string.  B200, 32e6 strings in segments of about 700:
+// 1.12 -> 0.49 ms; a 4e6-string request whose segments are chains of nested
+// prefixes: 0.61 -> 0.18 ms; 9e6 suffixes of copied text: 9.2 -> 6.5 ms.
 constexpr unsigned FULL = 0xffffffffu;
+enum GroupKind : uint32_t { G_PLAIN = 0, G_TIE = 1, G_ID = 2, G_PSEUDO = 3 };  // G_TIE: keys still to be made
+// Pivot code of a string with LCP l: l below the pivot, CODE_MID for strings
+// equal to it (or to CODE_CAP bytes of it), 0xBFFF - l above it.
+constexpr uint32_t CODE_MID = 0x4000u, CODE_TOP = 0xBFFFu, CODE_CAP = 0x3FFEu;
+constexpr uint32_t TINY_MAX = 8;  // largest bucket one thread sorts
 
-__device__ __forceinline__ bool lt3(uint32_t g1, uint64_t k1, uint32_t o1, uint32_t g2, uint64_t k2, uint32_t o2) {
-    return g1 < g2 || (g1 == g2 && (k1 < k2 || (k1 == k2 && o1 < o2)));
+// LCP part of a pivot code (the pivot's own is above all others).
+__device__ __forceinline__ uint32_t code_l(uint32_t c) { return c <= CODE_MID ? c : CODE_TOP - c; }
+
+// The key whose differing bits choose a group's buckets: above the pivot the
+// code counts down, so its LCP bits are flipped back.  In the key itself the
+// bits that then do not differ follow from the two highest ones.
+__device__ __forceinline__ uint64_t level_key(uint64_t k, bool pseudo) {
+    return pseudo && (k >> 63) ? k ^ 0x3FFFull << 48 : k;
 }
 
-// Lane i < size holds (key at `depth`, id).  On return lane i holds the i-th
-// smallest; lcp[lane] (lanes 1..size-1) gets the LCP with the predecessor.
-__device__ __forceinline__ void warp_sort(const ArenaDev& a, uint32_t size, uint32_t depth, uint64_t& key,
-                                          uint32_t& id, uint32_t* lcp) {
-    const int lane = threadIdx.x & 31;
-    const bool valid = (uint32_t)lane < size;
+// Bytes before the end that a key holds: plain, index of its first zero byte
+// (8: none); pseudo, index among its last six (6: none).
+__device__ __forceinline__ uint32_t key_end(uint64_t k, bool pseudo) {
+    return pseudo ? zero_byte(k | 0xFFFF000000000000ull) - 2 : zero_byte(k);
+}
+__device__ __forceinline__ bool key_ended(uint64_t k, bool pseudo) { return key_end(k, pseudo) < (pseudo ? 6u : 8u); }
+
+// LCP of two strings of a group of depth d whose keys differ.
+__device__ __forceinline__ uint32_t group_lcp(uint64_t x, uint64_t y, uint32_t d, bool pseudo) {
+    if (!pseudo) return d + key_lcp(x, y);
+    const uint32_t cx = (uint32_t)(x >> 48), cy = (uint32_t)(y >> 48);
+    if (cx != cy) return d + min(code_l(cx), code_l(cy));
+    return d + code_l(cx) + key_lcp(x, y) - 2;
+}
+
+// Depth up to which strings with the equal, not ended key k agree.
+__device__ __forceinline__ uint32_t tie_depth(uint64_t k, uint32_t d, bool pseudo) {
+    if (!pseudo) return d + 8;
+    const uint32_t c = (uint32_t)(k >> 48);
+    return c == CODE_MID ? d + CODE_CAP : d + code_l(c) + 6;
+}
+
+struct StrRef {
+    uint64_t off;
+    uint32_t len;
+};
+
+__device__ __forceinline__ StrRef ref_of(const ArenaDev& a, uint32_t id) {
+    StrRef r;
+    str_of(a, id, r.off, r.len);
+    return r;
+}
+
+// Each active lane's LCP with its own pivot h, both strings sharing their
+// first d bytes; at most d + CODE_CAP.  32 bytes per lane first; lanes still
+// equal then go one after another, the whole warp reading 256 bytes of a pair
+// at a time.  Every lane of the warp calls it.
+__device__ __forceinline__ uint32_t warp_lcp(const ArenaDev& a, StrRef x, StrRef h, uint32_t d, bool active) {
+    uint32_t l = d;
+    bool open = active;
+    if (active) {
+        uint64_t u[4], v[4];
+        key_words<4>(a.chars, x.off, x.len, d, 4, u);
+        key_words<4>(a.chars, h.off, h.len, d, 4, v);
+        l = d + 32;
+#pragma unroll
+        for (int w = 3; w >= 0; --w) {  // the first word that differs or ends wins
+            if (u[w] != v[w]) {
+                l = d + 8 * w + key_lcp(u[w], v[w]);
+                open = false;
+            } else if (zero_byte(u[w]) < 8) {
+                l = d + 8 * w + zero_byte(u[w]);
+                open = false;
+            }
+        }
+    }
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t todo = __ballot_sync(FULL, open); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const uint64_t ox = __shfl_sync(FULL, x.off, src), oh = __shfl_sync(FULL, h.off, src);
+        const uint32_t lx = __shfl_sync(FULL, x.len, src), lh = __shfl_sync(FULL, h.len, src);
+        const uint32_t d0 = __shfl_sync(FULL, d, src);
+        uint32_t at = d0 + 32;
+        for (;; at += 256) {
+            if (at >= d0 + CODE_CAP) {
+                at = d0 + CODE_CAP;
+                break;
+            }
+            const uint32_t p = at + 8 * lane;
+            const uint64_t u = key8(a.chars, ox, lx, p), v = key8(a.chars, oh, lh, p);
+            const uint32_t e = u != v ? key_lcp(u, v) : zero_byte(u);
+            const uint32_t hit = __ballot_sync(FULL, e < 8);
+            if (hit) {
+                const int f = __ffs(hit) - 1;
+                at = min(at + 8 * f + __shfl_sync(FULL, e, f), d0 + CODE_CAP);
+                break;
+            }
+        }
+        if (lane == (uint32_t)src) l = at;
+    }
+    return l;
+}
+
+// The pseudo key of string x against pivot h, l their LCP, d the group's
+// depth.
+__device__ __forceinline__ uint64_t pseudo_key(const ArenaDev& a, StrRef x, StrRef h, uint32_t l, uint32_t d) {
+    if (l >= d + CODE_CAP) return (uint64_t)CODE_MID << 48 | 0x010101010101ull;  // no end in sight
+    const uint64_t bx = key8(a.chars, x.off, x.len, l), bh = key8(a.chars, h.off, h.len, l);
+    const uint32_t xb = (uint32_t)(bx >> 56), hb = (uint32_t)(bh >> 56);
+    if (xb == hb) return (uint64_t)CODE_MID << 48;  // both end: equal strings
+    const uint32_t c = xb < hb ? l - d : CODE_TOP - (l - d);
+    return (uint64_t)c << 48 | bx >> 16;
+}
+
+// Compare-exchange network over the first P (a power of two) lanes.
+template <bool GRP>
+__device__ __forceinline__ void warp_network(uint32_t P, uint32_t& grp, uint64_t& key, uint32_t& id, uint32_t& dep) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (uint32_t k = 2; k <= 32; k <<= 1) {
+        if (k > P) break;
+#pragma unroll
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            const uint64_t pk = __shfl_xor_sync(FULL, key, j);
+            const uint32_t po = __shfl_xor_sync(FULL, id, j);
+            const bool want_min = ((lane & k) == 0) == ((lane & j) == 0);
+            if (GRP) {
+                const uint32_t pg = __shfl_xor_sync(FULL, grp, j), pd = __shfl_xor_sync(FULL, dep, j);
+                const bool less = pg < grp || (pg == grp && (pk < key || (pk == key && po < id)));
+                if (less == want_min) {
+                    grp = pg;
+                    key = pk;
+                    id = po;
+                    dep = pd;
+                }
+            } else {
+                const bool less = pk < key || (pk == key && po < id);
+                if (less == want_min) {
+                    key = pk;
+                    id = po;
+                }
+            }
+        }
+    }
+}
+
+// A group of size <= 32: lane i < size holds an id and, unless kind is G_TIE
+// or G_ID, its key.  On return lane i holds the i-th smallest string; lcp[i]
+// (1 <= i < size) gets the LCP with the predecessor (depth itself for G_ID).
+__device__ __forceinline__ void warp_group(const ArenaDev& a, uint32_t size, uint32_t depth, uint32_t kind,
+                                           uint64_t key, uint32_t& id, uint32_t* lcp) {
+    const uint32_t lane = threadIdx.x & 31;
+    const bool valid = lane < size;
+    const uint32_t P = size <= 2 ? 2u : 1u << (32 - __clz(size - 1));
     uint32_t grp = valid ? 0u : 0xFFFFFFFFu;
     uint32_t dep = depth;
+    bool pseudo = kind == G_PSEUDO;
     if (!valid) {
         key = ~0ull;
         id = 0xFFFFFFFFu;
+    } else if (kind == G_ID) {
+        key = 0;
     }
-    for (bool first = true;; first = false) {
-        if (first) {
-            // one group at one depth (invalid lanes carry the largest key
-            // and id, so they still sort last): (key, id) is the whole order
-#pragma unroll
-            for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const uint64_t pk = __shfl_xor_sync(FULL, key, j);
-                    const uint32_t po = __shfl_xor_sync(FULL, id, j);
-                    const bool want_min = ((lane & k) == 0) == ((lane & j) == 0);
-                    const bool less = pk < key || (pk == key && po < id);
-                    if (less == want_min) {
-                        key = pk;
-                        id = po;
-                    }
-                }
+    bool unres = valid && kind == G_TIE;
+    uint32_t rs = 0;
+    bool first = true;
+    for (;;) {
+        if (kind != G_TIE || !first) {
+            if (first) warp_network<false>(P, grp, key, id, dep);
+            else warp_network<true>(P, grp, key, id, dep);
+            const uint32_t qg = __shfl_up_sync(FULL, grp, 1);
+            const uint64_t qk = __shfl_up_sync(FULL, key, 1);
+            const bool head = lane == 0 || qg != grp || qk != key;
+            if (kind == G_ID) {
+                if (valid && lane > 0) lcp[lane] = depth;
+                return;
             }
-        } else {
-#pragma unroll
-            for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const uint32_t pg = __shfl_xor_sync(FULL, grp, j);
-                    const uint64_t pk = __shfl_xor_sync(FULL, key, j);
-                    const uint32_t po = __shfl_xor_sync(FULL, id, j);
-                    const uint32_t pd = __shfl_xor_sync(FULL, dep, j);
-                    const bool want_min = ((lane & k) == 0) == ((lane & j) == 0);
-                    const bool take = want_min ? lt3(pg, pk, po, grp, key, id) : lt3(grp, key, id, pg, pk, po);
-                    if (take) {
-                        grp = pg;
-                        key = pk;
-                        id = po;
-                        dep = pd;
-                    }
-                }
+            // dep of a resolved string is no longer used; neighbours in one
+            // group share it
+            if (valid && lane > 0 && qg == grp) {
+                if (qk != key) lcp[lane] = group_lcp(qk, key, dep, pseudo);
+                else if (key_ended(key, pseudo)) lcp[lane] = ref_of(a, id).len;  // equal strings
             }
+            const uint32_t heads = __ballot_sync(FULL, head);
+            rs = 31u - __clz(heads & ((2u << lane) - 1u));
+            const bool next_head = lane == 31 ? true : ((heads >> (lane + 1)) & 1u) != 0;
+            const bool multi = !head || (!next_head && lane + 1 < size);
+            unres = valid && multi && !key_ended(key, pseudo);
+            if (valid) grp = rs;
         }
-        const uint32_t qg = __shfl_up_sync(FULL, grp, 1);
-        const uint64_t qk = __shfl_up_sync(FULL, key, 1);
-        const bool head = lane == 0 || qg != grp || qk != key;
-        if (valid && lane > 0 && qg == grp) {
-            if (qk != key) {
-                lcp[lane] = dep + key_lcp(key, qk);
-            } else {
-                const uint32_t z = zero_byte(key);
-                if (z < 8) lcp[lane] = dep + z;  // byte-identical neighbours
-            }
-        }
-        const uint32_t heads = __ballot_sync(FULL, head);
-        const uint32_t rs = 31u - __clz(heads & ((2u << lane) - 1u));
-        const bool next_head = lane == 31 ? true : ((heads >> (lane + 1)) & 1u) != 0;
-        const bool multi = !head || (!next_head && (uint32_t)(lane + 1) < size);
-        const bool unres = valid && multi && zero_byte(key) == 8;
-        if (valid) grp = rs;
-        if (!__any_sync(FULL, unres)) break;
-        // Every unresolved run shares its 8-byte key: jump to the first depth
-        // where a member differs from the run head (or ends), the minimum over
-        // the run of each member's LCP with the head.
+        if (!__any_sync(FULL, unres)) return;
+        // every unresolved run goes on against its head
+        const uint32_t nd = first && kind == G_TIE ? depth : tie_depth(key, dep, pseudo);
         const uint32_t hid = __shfl_sync(FULL, id, rs);
-        uint32_t l = 0xFFFFFFFFu;
-        if (unres && (uint32_t)lane != rs) {
-            uint64_t off, offh;
-            uint32_t len, lenh;
-            str_of(a, id, off, len);
-            str_of(a, hid, offh, lenh);
-            for (uint32_t d = dep + 8;; d += 16) {
-                const uint64_t x0 = key8(a.chars, off, len, d), y0 = key8(a.chars, offh, lenh, d);
-                const uint64_t x1 = key8(a.chars, off, len, d + 8), y1 = key8(a.chars, offh, lenh, d + 8);
-                if (x0 != y0) { l = d + key_lcp(x0, y0); break; }
-                if (zero_byte(x0) < 8) { l = d + zero_byte(x0); break; }
-                if (x1 != y1) { l = d + 8 + key_lcp(x1, y1); break; }
-                if (zero_byte(x1) < 8) { l = d + 8 + zero_byte(x1); break; }
-            }
+        StrRef x{0, 0}, h{0, 0};
+        if (unres) {
+            x = ref_of(a, id);
+            h = ref_of(a, hid);
         }
-        const uint32_t run = __match_any_sync(FULL, unres ? rs : 32u + (uint32_t)lane);
-        const uint32_t nd = __reduce_min_sync(run, l);
+        const bool cmp = unres && lane != rs;
+        const uint32_t l = warp_lcp(a, x, h, nd, cmp);
+        // resolved strings keep a key that orders them among themselves
         if (unres) {
             dep = nd;
-            key = key8_of(a, id, dep);
+            key = cmp ? pseudo_key(a, x, h, l, nd) : (uint64_t)CODE_MID << 48;
+        } else if (valid) {
+            key = 0;  // alone in its group, or equal strings in id order
         }
-    }
-}
-
-// A bucket of at most T strings whose keys are in shared memory, sorted by
-// one thread: an odd-even transposition network on (key, id) in registers
-// (absent slots carry the largest pair, so they sort last), then the LCPs of
-// neighbours.  Returns false,
-// writing nothing, when two keys are equal and neither string ends inside
-// them (a warp sort then goes deeper).
-template <int T>
-__device__ __forceinline__ bool tiny_sort(const unsigned long long* sk, uint32_t* so, uint32_t* lcp, uint32_t ws,
-                                          uint32_t wn, uint32_t wd) {
-    uint64_t k[T];
-    uint32_t o[T];
-#pragma unroll
-    for (int i = 0; i < T; ++i) {
-        o[i] = 0xFFFFFFFFu;
-        k[i] = ~0ull;
-        if ((uint32_t)i < wn) {
-            o[i] = so[ws + i];
-            k[i] = sk[ws + i];
-        }
-    }
-#pragma unroll
-    for (int pass = 0; pass < T; ++pass) {
-#pragma unroll
-        for (int i = pass & 1; i + 1 < T; i += 2) {
-            if (k[i + 1] < k[i] || (k[i + 1] == k[i] && o[i + 1] < o[i])) {
-                const uint64_t tk = k[i];
-                k[i] = k[i + 1];
-                k[i + 1] = tk;
-                const uint32_t to = o[i];
-                o[i] = o[i + 1];
-                o[i + 1] = to;
-            }
-        }
-    }
-    bool ok = true;
-#pragma unroll
-    for (int i = 1; i < T; ++i)
-        if ((uint32_t)i < wn && k[i - 1] == k[i] && zero_byte(k[i]) == 8) ok = false;
-    if (!ok) return false;
-#pragma unroll
-    for (int i = 0; i < T; ++i) {
-        if ((uint32_t)i < wn) {
-            so[ws + i] = o[i];
-            if (i) lcp[ws + i] = k[i - 1] != k[i] ? wd + key_lcp(k[i - 1], k[i]) : wd + zero_byte(k[i]);
-        }
-    }
-    return true;
-}
-
-constexpr uint32_t WL_DONE = 1u << 31;  // warp-list entry finished by one thread
-constexpr uint32_t TINY_MAX = 8;       // largest bucket one thread sorts
-
-// Buckets of 33..64 strings: lane l holds positions l and l + 32 (elements 0
-// and 1).  The same bitonic order on (group, key, id) over 64 positions (the
-// stage j = 32 compares a lane's two elements), the same run handling as
-// warp_sort; the run minima go through `scratch` (>= size words of shared
-// memory owned by this warp).
-__device__ __forceinline__ void cx_key_id(uint64_t& key, uint32_t& id, int j, bool want_min) {
-    const uint64_t pk = __shfl_xor_sync(FULL, key, j);
-    const uint32_t po = __shfl_xor_sync(FULL, id, j);
-    const bool less = pk < key || (pk == key && po < id);
-    if (less == want_min) {
-        key = pk;
-        id = po;
-    }
-}
-
-__device__ __forceinline__ void cx_full(uint32_t& grp, uint64_t& key, uint32_t& id, uint32_t& dep, int j,
-                                        bool want_min) {
-    const uint32_t pg = __shfl_xor_sync(FULL, grp, j);
-    const uint64_t pk = __shfl_xor_sync(FULL, key, j);
-    const uint32_t po = __shfl_xor_sync(FULL, id, j);
-    const uint32_t pd = __shfl_xor_sync(FULL, dep, j);
-    const bool take = want_min ? lt3(pg, pk, po, grp, key, id) : lt3(grp, key, id, pg, pk, po);
-    if (take) {
-        grp = pg;
-        key = pk;
-        id = po;
-        dep = pd;
-    }
-}
-
-__device__ void warp_sort64(const ArenaDev& a, uint32_t size, uint32_t depth, uint64_t (&key)[2], uint32_t (&id)[2],
-                            uint32_t* lcp, uint32_t* scratch) {
-    const uint32_t lane = threadIdx.x & 31;
-    bool valid[2];
-    uint32_t grp[2], dep[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        valid[h] = lane + 32 * h < size;
-        grp[h] = valid[h] ? 0u : 0xFFFFFFFFu;
-        dep[h] = depth;
-        if (!valid[h]) {
-            key[h] = ~0ull;
-            id[h] = 0xFFFFFFFFu;
-        }
-    }
-    for (bool first = true;; first = false) {
-#pragma unroll
-        for (int k = 2; k <= 64; k <<= 1) {
-#pragma unroll
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                if (j == 32) {  // k == 64: ascending, element 0 takes the smaller
-                    // In the first network the group marks positions (valid
-                    // or padding) and the depth is uniform: only (key, id)
-                    // move, as in cx_key_id.
-                    const bool sw = first ? (key[1] < key[0] || (key[1] == key[0] && id[1] < id[0]))
-                                          : lt3(grp[1], key[1], id[1], grp[0], key[0], id[0]);
-                    if (sw) {
-                        uint64_t tk = key[0];
-                        key[0] = key[1];
-                        key[1] = tk;
-                        uint32_t t = id[0];
-                        id[0] = id[1];
-                        id[1] = t;
-                        if (!first) {
-                            t = grp[0];
-                            grp[0] = grp[1];
-                            grp[1] = t;
-                            t = dep[0];
-                            dep[0] = dep[1];
-                            dep[1] = t;
-                        }
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const uint32_t pos = lane + 32 * h;
-                    const bool want_min = ((pos & k) == 0) == ((pos & j) == 0);
-                    if (first) cx_key_id(key[h], id[h], j, want_min);
-                    else cx_full(grp[h], key[h], id[h], dep[h], j, want_min);
-                }
-            }
-        }
-        // predecessor of each position: lane - 1 of the same half, lane 31 of
-        // half 0 for position 32
-        const uint64_t k31 = __shfl_sync(FULL, key[0], 31);
-        const uint32_t g31 = __shfl_sync(FULL, grp[0], 31);
-        bool head[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint64_t qu = __shfl_up_sync(FULL, key[h], 1);
-            const uint32_t gu = __shfl_up_sync(FULL, grp[h], 1);
-            const uint64_t qk = lane == 0 ? k31 : qu;
-            const uint32_t qg = lane == 0 ? g31 : gu;
-            const bool has_pred = h == 1 || lane > 0;
-            head[h] = !has_pred || qg != grp[h] || qk != key[h];
-            if (valid[h] && has_pred && qg == grp[h]) {
-                const uint32_t pos = lane + 32 * h;
-                if (qk != key[h]) {
-                    lcp[pos] = dep[h] + key_lcp(key[h], qk);
-                } else {
-                    const uint32_t z = zero_byte(key[h]);
-                    if (z < 8) lcp[pos] = dep[h] + z;  // byte-identical neighbours
-                }
-            }
-        }
-        const uint64_t heads = (uint64_t)__ballot_sync(FULL, head[0]) | (uint64_t)__ballot_sync(FULL, head[1]) << 32;
-        bool unres[2];
-        uint32_t rs[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t pos = lane + 32 * h;
-            rs[h] = 63u - (uint32_t)__clzll(heads & ((2ull << pos) - 1ull));
-            const bool next_head = pos == 63 ? true : ((heads >> (pos + 1)) & 1ull) != 0;
-            const bool multi = !head[h] || (!next_head && pos + 1 < size);
-            unres[h] = valid[h] && multi && zero_byte(key[h]) == 8;
-            if (valid[h]) grp[h] = rs[h];
-        }
-        if (!__any_sync(FULL, unres[0] || unres[1])) break;
-        // Every unresolved run shares its 8-byte key: jump to the first depth
-        // where a member differs from the run head (or ends).
-        for (uint32_t x = lane; x < size; x += 32) scratch[x] = 0xFFFFFFFFu;
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t h0 = __shfl_sync(FULL, id[0], rs[h] & 31), h1 = __shfl_sync(FULL, id[1], rs[h] & 31);
-            const uint32_t hid = rs[h] < 32 ? h0 : h1;
-            if (unres[h] && lane + 32 * h != rs[h]) {
-                uint64_t off, offh;
-                uint32_t len, lenh;
-                str_of(a, id[h], off, len);
-                str_of(a, hid, offh, lenh);
-                uint32_t l;
-                for (uint32_t d = dep[h] + 8;; d += 16) {
-                    const uint64_t x0 = key8(a.chars, off, len, d), y0 = key8(a.chars, offh, lenh, d);
-                    const uint64_t x1 = key8(a.chars, off, len, d + 8), y1 = key8(a.chars, offh, lenh, d + 8);
-                    if (x0 != y0) { l = d + key_lcp(x0, y0); break; }
-                    if (zero_byte(x0) < 8) { l = d + zero_byte(x0); break; }
-                    if (x1 != y1) { l = d + 8 + key_lcp(x1, y1); break; }
-                    if (zero_byte(x1) < 8) { l = d + 8 + zero_byte(x1); break; }
-                }
-                atomicMin(&scratch[rs[h]], l);
-            }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (unres[h]) {
-                dep[h] = scratch[rs[h]];
-                key[h] = key8_of(a, id[h], dep[h]);
-            }
-        }
-        __syncwarp();
+        // the head shares its end with the strings that equal it, or the cap
+        const uint32_t capped = __ballot_sync(FULL, cmp && l >= nd + CODE_CAP);
+        const uint32_t run = __match_any_sync(FULL, unres ? rs : 32u + lane);
+        if (unres && lane == rs && (capped & run)) key |= 0x010101010101ull;
+        pseudo = true;
+        first = false;
     }
 }
 
@@ -1660,361 +1577,414 @@ __device__ void warp_sort64(const ArenaDev& a, uint32_t size, uint32_t depth, ui
 __global__ void __launch_bounds__(128) k_warp_segs(SortState S, const Seg* segs, uint32_t nseg, const uint32_t* dcount) {
     if (dcount) nseg = *dcount;
     for (uint32_t si = blockIdx.x * 4 + (threadIdx.x >> 5); si < nseg; si += gridDim.x * 4) {
-    const int lane = threadIdx.x & 31;
-    const Seg seg = segs[si];
-    const uint32_t* src = S.ord[seg.flags & F_PARITY];
-    uint32_t id = 0;
-    uint64_t key = 0;
-    if ((uint32_t)lane < seg.size) {
-        id = src[seg.start + lane];
-        key = (seg.flags & F_KEYS) ? S.key[seg.flags & F_PARITY][seg.start + lane]
-                                   : key8_of(S.a, id, seg.depth);
+        const uint32_t lane = threadIdx.x & 31;
+        const Seg seg = segs[si];
+        const uint32_t* src = S.ord[seg.flags & F_PARITY];
+        uint32_t id = 0;
+        uint64_t key = 0;
+        if (lane < seg.size) {
+            id = src[seg.start + lane];
+            key = (seg.flags & F_KEYS) ? S.key[seg.flags & F_PARITY][seg.start + lane] : key8_of(S.a, id, seg.depth);
+        }
+        warp_group(S.a, seg.size, seg.depth, G_PLAIN, key, id, S.lcp_out + seg.start);
+        if (lane < seg.size) S.ord_out[seg.start + lane] = id;
     }
-    warp_sort(S.a, seg.size, seg.depth, key, id, S.lcp_out + seg.start);
-    if ((uint32_t)lane < seg.size) S.ord_out[seg.start + lane] = id;
+}
+
+// The bits that pick a bucket: up to `want` of the most significant bits of
+// diff, in at most 8 runs of neighbouring bits.  A key's bucket is the OR over
+// the runs of ((key >> lo) >> sh) & mask; every bit above lo that is not
+// chosen is the same in all keys, so buckets order as keys do.
+// In a pseudo group whose code bits are all chosen, a bucket holds one code;
+// otherwise (LCPs over thousands of bytes) `mixed` is set.
+struct BucketBits {
+    uint32_t lo, nruns, wide, all;  // wide: the bits span more than 32; all: every differing bit is chosen
+    uint32_t mixed;
+    uint32_t sh[8], mask[8];
+};
+
+__device__ __forceinline__ uint32_t bucket_of_key(const BucketBits& B, uint64_t k) {
+    uint32_t b = 0;
+    for (uint32_t r = 0; r < B.nruns; ++r) b |= (uint32_t)(k >> (B.lo + B.sh[r])) & B.mask[r];
+    return b;
+}
+
+__device__ __forceinline__ void bucket_bits(BucketBits& B, uint64_t diff, uint32_t want) {
+    uint32_t at[8], len[8], n = 0, total = 0;
+    uint64_t x = diff;
+    const uint32_t hi = 63u - (uint32_t)__clzll(diff);
+    while (x && n < 8 && total < want) {
+        const uint32_t h = 63u - (uint32_t)__clzll(x);
+        const uint32_t run = (uint32_t)__clzll(~(x << (63u - h)));  // set bits from h down
+        const uint32_t take = min(run, want - total);
+        at[n] = h - take + 1;  // lowest bit taken
+        len[n] = take;
+        total += take;
+        x &= at[n] ? (1ull << at[n]) - 1 : 0ull;
+        ++n;
+    }
+    B.lo = at[n - 1];
+    B.nruns = n;
+    B.wide = hi - at[n - 1] >= 32;
+    B.all = x == 0;
+    B.mixed = (x >> 48) != 0;
+    uint32_t place = total;
+    for (uint32_t k = 0; k < n; ++k) {
+        place -= len[k];
+        B.sh[k] = at[k] - B.lo - place;
+        B.mask[k] = ((1u << len[k]) - 1u) << place;
+    }
+}
+
+// A group on the CTA's stack or the warps' list: positions [start, start +
+// size) of the segment, packed with the kind.
+__device__ __forceinline__ uint2 group_pack(uint32_t start, uint32_t size, uint32_t kind, uint32_t depth) {
+    return make_uint2(start | (size - 1) << 12 | kind << 24, depth);
+}
+__device__ __forceinline__ uint32_t group_start(uint2 g) { return g.x & 0xFFFu; }
+__device__ __forceinline__ uint32_t group_size(uint2 g) { return ((g.x >> 12) & 0xFFFu) + 1; }
+__device__ __forceinline__ uint32_t group_kind(uint2 g) { return g.x >> 24; }
+
+template <int CAP>
+struct SegSmem {
+    static constexpr int NB = CAP <= 256 ? 1024 : CAP <= 1024 ? 2048 : 4096;  // buckets
+    unsigned long long key[CAP];
+    uint32_t cnt[NB + 4];  // bucket counts, then starts (the last one the group's size)
+    uint32_t id[CAP];
+    uint2 wl[CAP / 2];         // groups for the warps
+    uint2 stk[CAP / 32 + 2];   // groups for the CTA
+};
+
+template <int CAP, int NT>
+__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_seg_sort(SortState S, const Seg* segs,
+                                                                                       uint32_t nseg,
+                                                                                       const uint32_t* dcount) {
+    constexpr int NW = NT / 32, IPT = CAP / NT, NB = SegSmem<CAP>::NB, PER = NB / NT;
+    extern __shared__ __align__(16) unsigned char smem[];
+    SegSmem<CAP>& M = *reinterpret_cast<SegSmem<CAP>*>(smem);
+    __shared__ unsigned long long s_or[NW], s_and[NW];
+    __shared__ uint32_t s_sum[NW], s_ns, s_nw, s_piv[8];
+    __shared__ uint2 s_cur;
+    __shared__ BucketBits s_bits;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (dcount) nseg = *dcount;
+    for (uint32_t bi = blockIdx.x; bi < nseg; bi += gridDim.x) {
+        const Seg seg = segs[bi];
+        const uint32_t start = seg.start, size = seg.size;
+        uint32_t* lcp = S.lcp_out + start;
+        {
+            const uint32_t* src = S.ord[seg.flags & F_PARITY] + start;
+            const unsigned long long* ksrc = S.key[seg.flags & F_PARITY] + start;
+            uint32_t o[IPT];
+            uint64_t k[IPT];
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                const uint32_t i = threadIdx.x + j * NT;
+                o[j] = i < size ? src[i] : 0u;
+                k[j] = i < size && (seg.flags & F_KEYS) ? ksrc[i] : 0ull;
+            }
+            if (!(seg.flags & F_KEYS)) {
+#pragma unroll
+                for (int j = 0; j < IPT; ++j)
+                    if (threadIdx.x + j * NT < size) k[j] = key8_of(S.a, o[j], seg.depth);
+            }
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                const uint32_t i = threadIdx.x + j * NT;
+                if (i < size) {
+                    M.id[i] = o[j];
+                    M.key[i] = k[j];
+                }
+            }
+        }
+        for (uint32_t x = threadIdx.x; x < NB; x += NT) M.cnt[x] = 0;
+        if (threadIdx.x == 0) {
+            const uint2 g = group_pack(0, size, G_PLAIN, seg.depth);
+            s_nw = size <= 32;
+            s_ns = size > 32;
+            if (size <= 32) M.wl[0] = g;
+            else M.stk[0] = g;
+        }
+        __syncthreads();
+        while (s_ns) {
+            if (threadIdx.x == 0) s_cur = M.stk[s_ns - 1];
+            __syncthreads();
+            const uint32_t bs = group_start(s_cur), bn = group_size(s_cur), dep = s_cur.y;
+            uint32_t kind = group_kind(s_cur);
+            if (threadIdx.x == 0) --s_ns;  // read again only after the next barrier
+            uint64_t k[IPT];
+            uint32_t o[IPT], br[IPT];
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                const uint32_t i = threadIdx.x + j * NT;
+                o[j] = i < bn ? M.id[bs + i] : 0u;
+                k[j] = i < bn ? (kind == G_ID ? (uint64_t)o[j] : M.key[bs + i]) : 0ull;
+            }
+            if (kind == G_TIE) {
+                // the pivot: of 8 evenly spaced strings the one with the
+                // largest sum of LCPs (256 bytes at most) with the others
+                for (uint32_t c = w; c < 8; c += NW) {
+                    const StrRef x = ref_of(S.a, M.id[bs + c * bn / 8]);
+                    const uint64_t kx = key8(S.a.chars, x.off, x.len, dep + 8 * lane);
+                    uint32_t sum = 0;
+#pragma unroll 4
+                    for (uint32_t q = 0; q < 8; ++q) {
+                        const StrRef y = ref_of(S.a, M.id[bs + q * bn / 8]);
+                        const uint64_t ky = key8(S.a.chars, y.off, y.len, dep + 8 * lane);
+                        const uint32_t e = kx != ky ? key_lcp(kx, ky) : 8u;
+                        const uint32_t hit = __ballot_sync(FULL, e < 8);
+                        const int f = hit ? __ffs(hit) - 1 : 0;
+                        const uint32_t ef = __shfl_sync(FULL, e, f);
+                        sum += hit ? 8 * f + ef : 256u;
+                    }
+                    if (lane == 0) s_piv[c] = sum << 3 | c;
+                }
+                __syncthreads();
+                uint32_t best = 0;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) best = max(best, s_piv[c]);
+                const uint32_t pid = M.id[bs + (best & 7u) * bn / 8];
+                const StrRef h = ref_of(S.a, pid);
+#pragma unroll 1
+                for (int j = 0; j < IPT; ++j) {
+                    const uint32_t i = threadIdx.x + j * NT;
+                    if (i - lane >= bn) break;  // the same for the whole warp
+                    const bool v = i < bn;
+                    StrRef x{0, 0};
+                    uint32_t oj = v ? M.id[bs + i] : 0u;
+                    if (v) x = ref_of(S.a, oj);
+                    const uint32_t l = warp_lcp(S.a, x, h, dep, v);
+                    if (v) M.key[bs + i] = pseudo_key(S.a, x, h, l, dep);
+                }
+                // a thread reads back only the keys it wrote
+#pragma unroll
+                for (int j = 0; j < IPT; ++j) {
+                    const uint32_t i = threadIdx.x + j * NT;
+                    if (i < bn) k[j] = M.key[bs + i];
+                }
+                kind = G_PSEUDO;
+            }
+            const bool pseudo = kind == G_PSEUDO;
+            // the bits in which the keys differ
+            uint64_t vo = 0, va = ~0ull;
+#pragma unroll
+            for (int j = 0; j < IPT; ++j)
+                if (threadIdx.x + j * NT < bn) {
+                    const uint64_t t = level_key(k[j], pseudo);
+                    vo |= t;
+                    va &= t;
+                }
+            const uint32_t olo = __reduce_or_sync(FULL, (uint32_t)vo), ohi = __reduce_or_sync(FULL, (uint32_t)(vo >> 32));
+            const uint32_t alo = __reduce_and_sync(FULL, (uint32_t)va);
+            const uint32_t ahi = __reduce_and_sync(FULL, (uint32_t)(va >> 32));
+            if (lane == 0) {
+                s_or[w] = (uint64_t)ohi << 32 | olo;
+                s_and[w] = (uint64_t)ahi << 32 | alo;
+            }
+            __syncthreads();
+            uint64_t diff;
+            {
+                uint64_t x = s_or[0], y = s_and[0];
+#pragma unroll
+                for (int v = 1; v < NW; ++v) {
+                    x |= s_or[v];
+                    y &= s_and[v];
+                }
+                diff = x ^ y;
+            }
+            if (diff == 0) {  // one key: equal strings, or the group goes deeper
+                if (threadIdx.x == 0) {
+                    const uint64_t k0 = k[0];
+                    M.stk[s_ns++] = key_ended(k0, pseudo) ? group_pack(bs, bn, G_ID, ref_of(S.a, o[0]).len)
+                                                          : group_pack(bs, bn, G_TIE, tie_depth(k0, dep, pseudo));
+                }
+                __syncthreads();
+                continue;
+            }
+            if (threadIdx.x == 0) {
+                constexpr uint32_t most = 31u - (uint32_t)__builtin_clz(NB);
+                bucket_bits(s_bits, diff, pseudo ? most : min(32u - (uint32_t)__clz(bn - 1) + 1u, most));
+            }
+            __syncthreads();
+            {
+                const uint32_t lo = s_bits.lo, nr = s_bits.nruns;
+                uint32_t x[IPT];
+#pragma unroll
+                for (int j = 0; j < IPT; ++j) {
+                    x[j] = (uint32_t)(k[j] >> lo);
+                    br[j] = 0;
+                }
+                for (uint32_t r = 0; r < nr; ++r) {
+                    const uint32_t sh = s_bits.sh[r], mask = s_bits.mask[r];
+                    if (s_bits.wide) {
+#pragma unroll
+                        for (int j = 0; j < IPT; ++j) br[j] |= (uint32_t)(k[j] >> (lo + sh)) & mask;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < IPT; ++j) br[j] |= (x[j] >> sh) & mask;
+                    }
+                }
+            }
+            // counts; br: the bucket and, above it, the place inside it
+#pragma unroll
+            for (int j = 0; j < IPT; ++j)
+                if (threadIdx.x + j * NT < bn) br[j] |= atomicAdd(&M.cnt[br[j]], 1u) << 16;
+            __syncthreads();
+            {
+                uint32_t v[PER], sum = 0;
+#pragma unroll
+                for (int q = 0; q < PER; q += 4) {
+                    const uint4 c = *reinterpret_cast<const uint4*>(&M.cnt[threadIdx.x * PER + q]);
+                    v[q] = c.x;
+                    v[q + 1] = c.y;
+                    v[q + 2] = c.z;
+                    v[q + 3] = c.w;
+                    sum += c.x + c.y + c.z + c.w;
+                }
+                uint32_t x = sum;
+#pragma unroll
+                for (int off = 1; off < 32; off <<= 1) {
+                    const uint32_t y = __shfl_up_sync(FULL, x, off);
+                    if (lane >= (uint32_t)off) x += y;
+                }
+                if (lane == 31) s_sum[w] = x;
+                __syncthreads();
+                uint32_t run = x - sum;
+#pragma unroll
+                for (int q = 0; q < NW; ++q)
+                    if ((uint32_t)q < w) run += s_sum[q];
+#pragma unroll
+                for (int q = 0; q < PER; q += 4) {
+                    uint4 c;
+                    c.x = run;
+                    c.y = c.x + v[q];
+                    c.z = c.y + v[q + 1];
+                    c.w = c.z + v[q + 2];
+                    run = c.w + v[q + 3];
+                    *reinterpret_cast<uint4*>(&M.cnt[threadIdx.x * PER + q]) = c;
+                }
+                if (threadIdx.x == NT - 1) M.cnt[NB] = run;
+            }
+            __syncthreads();
+            // places (a thread holds its strings, so the group is permuted in
+            // place); only the counts' sum bounds a place, never taken else
+            bool bad = false;
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                if (threadIdx.x + j * NT >= bn) continue;
+                const uint32_t at = M.cnt[br[j] & 0xFFFFu] + (br[j] >> 16);
+                if (at >= bn) {
+                    bad = true;
+                    continue;
+                }
+                M.key[bs + at] = k[j];
+                M.id[bs + at] = o[j];
+            }
+            if (bad) atomicExch(&S.counters[10], 1u);
+            __syncthreads();
+            // each bucket's first string: the LCP with the bucket before (any
+            // of its strings), and who sorts the bucket
+            const bool all = s_bits.all != 0, mixed = pseudo && s_bits.mixed;
+            uint32_t mine = 0;  // bit j: this thread sorts the bucket of string j
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                if (threadIdx.x + j * NT >= bn || (br[j] >> 16) != 0) continue;
+                const uint32_t b = br[j] & 0xFFFFu, s0 = M.cnt[b], c = M.cnt[b + 1] - s0;
+                if (s0) {
+                    uint64_t kp = M.key[bs + s0 - 1], kn = k[j];
+                    if (mixed) {  // the codes next to the boundary: the last of the bucket before, this one's first
+                        const uint32_t bp = bucket_of_key(s_bits, kp);
+                        for (uint32_t x = s0 - 1; x > 0 && bucket_of_key(s_bits, M.key[bs + x - 1]) == bp; --x)
+                            kp = max(kp, (uint64_t)M.key[bs + x - 1]);
+                        for (uint32_t x = 0; x < c; ++x) kn = min(kn, (uint64_t)M.key[bs + s0 + x]);
+                    }
+                    lcp[bs + s0] = kind == G_ID ? dep : group_lcp(kp, kn, dep, pseudo);
+                }
+                br[j] = s0 | c << 16;
+                if (c < 2) continue;
+                if (c <= TINY_MAX) {
+                    mine |= 1u << j;
+                    continue;
+                }
+                uint32_t gk = kind, gd = dep;
+                if (kind != G_ID && all) {  // one key in the bucket
+                    const bool ended = key_ended(k[j], pseudo);
+                    gk = ended ? G_ID : G_TIE;
+                    gd = ended ? ref_of(S.a, o[j]).len : tie_depth(k[j], dep, pseudo);
+                }
+                const uint2 g = group_pack(bs + s0, c, gk, gd);
+                if (c <= 32) M.wl[atomicAdd(&s_nw, 1u)] = g;
+                else M.stk[atomicAdd(&s_ns, 1u)] = g;
+            }
+            __syncthreads();
+            // buckets of 2..TINY_MAX strings: insertion sort on (key, id), then
+            // the neighbours' LCPs and the runs that go deeper
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                if (!((mine >> j) & 1u)) continue;
+                const uint32_t s0 = bs + (br[j] & 0xFFFFu), c = br[j] >> 16;
+                for (uint32_t x = 1; x < c; ++x) {
+                    const uint64_t kx = M.key[s0 + x];
+                    const uint32_t ox = M.id[s0 + x];
+                    uint32_t y = x;
+                    for (; y > 0; --y) {
+                        const uint64_t ky = M.key[s0 + y - 1];
+                        const uint32_t oy = M.id[s0 + y - 1];
+                        if (ky < kx || (ky == kx && oy < ox)) break;
+                        M.key[s0 + y] = ky;
+                        M.id[s0 + y] = oy;
+                    }
+                    M.key[s0 + y] = kx;
+                    M.id[s0 + y] = ox;
+                }
+                if (kind == G_ID) {
+                    for (uint32_t x = 1; x < c; ++x) lcp[s0 + x] = dep;
+                    continue;
+                }
+                uint64_t kp = M.key[s0];
+                uint32_t r0 = 0;  // start of the run of equal keys
+                for (uint32_t x = 1; x <= c; ++x) {
+                    const uint64_t kx = x < c ? M.key[s0 + x] : ~kp;
+                    if (kx == kp) continue;
+                    if (x - r0 > 1) {
+                        if (key_ended(kp, pseudo)) {
+                            const uint32_t len = ref_of(S.a, M.id[s0 + r0]).len;
+                            for (uint32_t y = r0 + 1; y < x; ++y) lcp[s0 + y] = len;
+                        } else {
+                            M.wl[atomicAdd(&s_nw, 1u)] = group_pack(s0 + r0, x - r0, G_TIE, tie_depth(kp, dep, pseudo));
+                        }
+                    }
+                    if (x < c) lcp[s0 + x] = group_lcp(kp, kx, dep, pseudo);
+                    kp = kx;
+                    r0 = x;
+                }
+            }
+            // the next pass counts from zero
+            for (uint32_t x = threadIdx.x; x < NB; x += NT) M.cnt[x] = 0;
+            __syncthreads();
+        }
+        const uint32_t nwl = s_nw;
+        for (uint32_t e = w; e < nwl; e += NW) {
+            const uint2 g = M.wl[e];
+            const uint32_t ws = group_start(g), wn = group_size(g);
+            uint64_t key = 0;
+            uint32_t id = 0;
+            if (lane < wn) {
+                id = M.id[ws + lane];
+                key = M.key[ws + lane];
+            }
+            warp_group(S.a, wn, g.y, group_kind(g), key, id, lcp + ws);
+            if (lane < wn) M.id[ws + lane] = id;
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < size; i += NT) S.ord_out[start + i] = M.id[i];
+        __syncthreads();  // shared memory is reused by the next segment
     }
 }
 
 template <int CAP>
 constexpr size_t seg_sort_smem() {
-    return (size_t)CAP * (8 + 8 + 4 + 4 + 4) + (size_t)(CAP / 2) * 3 * 4 * 2;
-}
-
-// Bucket flags inside k_seg_sort, packed above the 16-bit bucket size: the
-// keys must be gathered at the bucket depth first (SF_REKEY), a pivot pass is
-// due (SF_PIVOT), or the keys are pivot pseudo keys whose base depth is the
-// bucket depth (SF_PSEUDO).
-constexpr uint32_t SF_REKEY = 1u, SF_PIVOT = 2u, SF_PSEUDO = 4u;
-constexpr uint32_t WL_MAX = 64;  // largest bucket a warp sort takes (wide splits only)
-
-template <int CAP, int NT>
-__global__ void __launch_bounds__(NT) k_seg_sort(SortState S, const Seg* segs, uint32_t nseg, const uint32_t* dcount) {
-    constexpr int NW = NT / 32;
-    // the 64-wide warp sort only where segments are large enough to split
-    // wide (its registers would cost the small variant occupancy)
-    constexpr uint32_t WIDE_WL = CAP >= 1024 ? WL_MAX : 32;
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned long long* sk = (unsigned long long*)smem;
-    unsigned long long* tk = sk + CAP;
-    uint32_t* so = (uint32_t*)(tk + CAP);
-    uint32_t* to = so + CAP;
-    uint32_t* pk = to + CAP;  // digit << 24 | rank within the warp's chunk
-    uint32_t* stk = pk + CAP;  // (start, size | flags << 16, depth) of buckets > 32
-    uint32_t* wl = stk + 3 * (CAP / 2);  // (start, size | flags << 16, depth) of buckets <= WL_MAX
-    __shared__ uint32_t hist[256], bstart[256];
-    __shared__ uint32_t wcnt[NW][256];
-    __shared__ uint32_t s_top, s_nw, s_cur[3];
-    __shared__ unsigned long long s_diff;
-    __shared__ BitTables sbt;
-    if (dcount) nseg = *dcount;
-    for (uint32_t bi = blockIdx.x; bi < nseg; bi += gridDim.x) {
-    const Seg seg = segs[bi];
-    const uint32_t start = seg.start, size = seg.size;
-    const uint32_t* src = S.ord[seg.flags & F_PARITY];
-    uint32_t* lcp = S.lcp_out + start;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (seg.flags & F_KEYS) {
-        const unsigned long long* ksrc = S.key[seg.flags & F_PARITY];
-        for (uint32_t i = threadIdx.x; i < size; i += NT) {
-            so[i] = src[start + i];
-            sk[i] = ksrc[start + i];
-        }
-    } else {
-        for (uint32_t i = threadIdx.x; i < size; i += NT) {
-            const uint32_t o = src[start + i];
-            so[i] = o;
-            sk[i] = key8_of(S.a, o, seg.depth);
-        }
-    }
-    if (threadIdx.x == 0) {
-        s_top = 0;
-        s_nw = 0;
-        uint32_t* dst = size <= 32 ? wl : stk;
-        dst[0] = 0;
-        dst[1] = size;
-        dst[2] = seg.depth;
-        if (size <= 32) s_nw = 1;
-        else s_top = 1;
-        s_diff = 0;
-    }
-    __syncthreads();
-    for (;;) {
-        if (threadIdx.x == 0) {
-            if (s_top) {
-                --s_top;
-                s_cur[0] = stk[3 * s_top];
-                s_cur[1] = stk[3 * s_top + 1];
-                s_cur[2] = stk[3 * s_top + 2];
-            } else {
-                s_cur[1] = 0;
-            }
-        }
-        __syncthreads();
-        const uint32_t bs = s_cur[0], bn = s_cur[1] & 0xFFFFu, dep = s_cur[2];
-        uint32_t fl = s_cur[1] >> 16;
-        if (bn == 0) break;
-        if (fl & SF_REKEY) {
-            for (uint32_t i = threadIdx.x; i < bn; i += NT) sk[bs + i] = key8_of(S.a, so[bs + i], dep);
-            fl = 0;
-            __syncthreads();
-        } else if (fl & SF_PIVOT) {
-            uint64_t off0;
-            uint32_t len0;
-            str_of(S.a, so[bs], off0, len0);
-            for (uint32_t i = threadIdx.x; i < bn; i += NT) {
-                uint64_t off;
-                uint32_t len;
-                str_of(S.a, so[bs + i], off, len);
-                sk[bs + i] = pivot_key(S.a.chars, off, len, off0, len0, dep);
-            }
-            fl = SF_PSEUDO;
-            __syncthreads();
-        }
-        const bool pseudo = fl & SF_PSEUDO;
-        const uint64_t k0 = sk[bs];
-        uint64_t df = 0;
-        for (uint32_t i = threadIdx.x; i < bn; i += NT) df |= sk[bs + i] ^ k0;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) df |= __shfl_xor_sync(FULL, df, o);
-        if (lane == 0 && df) atomicOr(&s_diff, (unsigned long long)df);
-        __syncthreads();
-        df = s_diff;
-        if (df == 0) {
-            // one key for the whole bucket: byte-identical strings (their LCP
-            // is their length), or continue deeper
-            uint32_t fin = 0xFFFFFFFFu, cont = 0, cfl = SF_REKEY;
-            if (pseudo) {
-                const uint32_t code = (uint32_t)(k0 >> 56), byte = (uint32_t)(k0 >> 48) & 0xFFu;
-                if (code == PIVOT_CAP) {
-                    uint64_t o0;
-                    uint32_t l0;
-                    str_of(S.a, so[bs], o0, l0);
-                    if (l0 < dep + PIVOT_CAP) fin = l0;
-                    else cont = dep + PIVOT_CAP;
-                } else if (byte == 0) {
-                    fin = dep + pivot_l(code);
-                } else {
-                    cont = dep + pivot_l(code) + 1;
-                }
-                cfl = SF_PIVOT;
-            } else {
-                const uint32_t z = zero_byte(k0);
-                if (z < 8) fin = dep + z;
-                else cont = dep + 8;
-            }
-            if (fin != 0xFFFFFFFFu) {
-                for (uint32_t i = threadIdx.x + 1; i < bn; i += NT) lcp[bs + i] = fin;
-            } else if (threadIdx.x == 0) {
-                stk[3 * s_top] = bs;
-                stk[3 * s_top + 1] = bn | (cfl << 16);
-                stk[3 * s_top + 2] = cont;
-                ++s_top;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) s_diff = 0;
-            __syncthreads();
-            continue;
-        }
-        const uint32_t b = (uint32_t)(__clzll(df) >> 3);
-        const uint32_t shift = 56 - 8 * b;
-        // plain keys split on their top eight differing bits (seg_bits), pivot
-        // pseudo keys on a byte; digit 0 holds strings that end at byte b only
-        // when that byte has no constant nonzero part
-        const bool bits = S.seg_bits && !pseudo;
-        const BitDigit bd = bit_digit_spec(bits ? df : (0xFFull << shift));
-        if (!bd.whole) bit_tables_build(sbt, bd);  // ordered by the barrier below
-        const bool ended_ok = !bits || (((k0 >> shift) & 0xFFu) & ~((df >> shift) & 0xFFu)) == 0;
-        for (uint32_t x = threadIdx.x; x < NW * 256; x += NT) (&wcnt[0][0])[x] = 0;
-        __syncthreads();
-        // stable ranks: warp w owns the contiguous chunk [w*cs, min((w+1)*cs, bn))
-        const uint32_t cs = ((bn + NW - 1) / NW + 31) & ~31u;
-        const uint32_t ce = min((uint32_t)(w + 1) * cs, bn);
-        for (uint32_t base = (uint32_t)w * cs; base < ce; base += 32) {
-            const uint32_t i = base + lane;
-            const bool v = i < ce;
-            const uint32_t d = v ? bit_digit(sk[bs + i], bd, sbt) : 0x100u + lane;
-            const uint32_t peers = __match_any_sync(FULL, d);
-            const uint32_t r = __popc(peers & ((1u << lane) - 1u));
-            const uint32_t prev = v ? wcnt[w][d] : 0u;
-            __syncwarp();
-            if (v && lane == __ffs(peers) - 1) wcnt[w][d] = prev + __popc(peers);
-            __syncwarp();
-            if (v) pk[bs + i] = (d << 24) | (prev + r);
-        }
-        __syncthreads();
-        for (uint32_t d = threadIdx.x; d < 256; d += NT) {
-            uint32_t run = 0;
-#pragma unroll
-            for (int ww = 0; ww < NW; ++ww) {
-                const uint32_t v = wcnt[ww][d];
-                wcnt[ww][d] = run;
-                run += v;
-            }
-            hist[d] = run;
-        }
-        __syncthreads();
-        if (w == 0) {  // exclusive scan of the 256 digit totals, 8 per lane
-            uint32_t v[8], sum = 0;
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                v[t] = hist[lane * 8 + t];
-                sum += v[t];
-            }
-            uint32_t x = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, x, o);
-                if (lane >= o) x += y;
-            }
-            uint32_t ex = x - sum;
-#pragma unroll
-            for (int t = 0; t < 8; ++t) {
-                bstart[lane * 8 + t] = ex;
-                ex += v[t];
-            }
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < bn; i += NT) {
-            const uint32_t x = pk[bs + i];
-            const uint32_t d = x >> 24;
-            const uint32_t dest = bstart[d] + wcnt[i / cs][d] + (x & 0xFFFFFFu);
-            if (dest >= bn) {  // never taken when the counts agree
-                atomicExch(&S.counters[10], 1u);
-                continue;
-            }
-            tk[bs + dest] = sk[bs + i];
-            to[bs + dest] = so[bs + i];
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < bn; i += NT) {
-            sk[bs + i] = tk[bs + i];
-            so[bs + i] = to[bs + i];
-        }
-        __syncthreads();
-        // split by pivot code, by the byte after a pivot code's shared
-        // prefix, or by a plain key byte
-        const bool code_split = pseudo && b == 0;
-        const uint32_t lin = pseudo ? dep + pivot_l((uint32_t)(k0 >> 56)) : dep + b;
-        for (uint32_t d = threadIdx.x; d < 256; d += NT) {
-            const uint32_t cnt = hist[d];
-            if (!cnt) continue;
-            const uint32_t c0 = bs + bstart[d];
-            if (c0 != bs) {  // boundary to the previous non-empty bucket
-                uint32_t l = lin;
-                if (code_split || !bd.whole) {
-                    uint32_t pd = d - 1;
-                    while (pd > 0 && bstart[pd] == bstart[d]) --pd;
-                    // pivot codes: d + min(l, l'); bit digits: the byte of the
-                    // highest bit in which the two buckets' digits differ
-                    l = code_split ? dep + min(pivot_l(d), pivot_l(pd))
-                                   : dep + bit_digit_byte(bd, 31u - (uint32_t)__clz(d ^ pd));
-                }
-                lcp[c0] = l;
-            }
-            if (d == 0 && !code_split && ended_ok) {  // strings that end here: byte-identical
-                for (uint32_t k = 1; k < cnt; ++k) lcp[c0 + k] = lin;
-                continue;
-            }
-            if (cnt < 2) continue;
-            uint32_t cd, cf;
-            if (!pseudo) {
-                if (S.pivot && cnt > 32 && 2 * cnt > bn) {
-                    cd = dep + b + 1;  // keeps most of the bucket: pivot pass next
-                    cf = SF_PIVOT;
-                } else {
-                    cd = dep;
-                    cf = 0;
-                }
-            } else if (code_split) {
-                if (cnt > 32) {
-                    cd = dep;
-                    cf = SF_PSEUDO;
-                } else {
-                    cd = dep + pivot_l(d);
-                    if (d == PIVOT_CAP) {
-                        uint64_t o0;
-                        uint32_t l0;
-                        str_of(S.a, so[c0], o0, l0);
-                        cd = min(dep + PIVOT_CAP, l0);
-                    }
-                    cf = SF_REKEY;
-                }
-            } else {
-                cd = lin + 1;
-                cf = (S.pivot && cnt > 32 && 2 * cnt > bn) ? SF_PIVOT : SF_REKEY;
-            }
-            // Warp list: up to 32 strings, or up to WL_MAX with plain keys
-            // (valid or re-gathered) from a wide split (at most 1/8 of the
-            // bucket: the keys' remaining bytes are likely to tell the strings
-            // apart in one network).  Narrow splits and chains stay with the
-            // block: a deep 64-string bucket on one warp would work through
-            // all of its runs alone, where a block pass hands them to 8 warps,
-            // and a chain of long shared prefixes gets the pivot pass.
-            uint32_t* dst;
-            uint32_t slot;
-            if (cnt <= 32 || (cnt <= WIDE_WL && 8 * cnt <= bn && !(cf & (SF_PIVOT | SF_PSEUDO)))) {
-                slot = atomicAdd(&s_nw, 1u);
-                dst = wl + 3 * slot;
-            } else {
-                slot = atomicAdd(&s_top, 1u);
-                dst = stk + 3 * slot;
-            }
-            dst[0] = c0;
-            dst[1] = cnt | (cf << 16);
-            dst[2] = cd;
-        }
-        if (threadIdx.x == 0) s_diff = 0;
-        __syncthreads();
-    }
-    const uint32_t nwl = s_nw;
-    // buckets of up to TINY_MAX strings: one thread each
-    for (uint32_t e = threadIdx.x; e < nwl; e += NT) {
-        const uint32_t ws = wl[3 * e], wn = wl[3 * e + 1] & 0xFFFFu, wd = wl[3 * e + 2];
-        // keys that must be gathered first stay with a warp (32 gathers at once)
-        if (wn > TINY_MAX || ((wl[3 * e + 1] >> 16) & SF_REKEY)) continue;
-        const bool done = wn <= 4 ? tiny_sort<4>(sk, so, lcp, ws, wn, wd) : tiny_sort<8>(sk, so, lcp, ws, wn, wd);
-        if (done) wl[3 * e + 1] |= WL_DONE;
-    }
-    __syncthreads();
-    for (uint32_t e = w; e < nwl; e += NW) {
-        if (wl[3 * e + 1] & WL_DONE) continue;
-        const uint32_t ws = wl[3 * e], wn = wl[3 * e + 1] & 0xFFFFu, wd = wl[3 * e + 2];
-        const bool rekey = (wl[3 * e + 1] >> 16) & SF_REKEY;
-        if (WIDE_WL == 32 || wn <= 32) {
-            uint64_t key = 0;
-            uint32_t id = 0;
-            if ((uint32_t)lane < wn) {
-                id = so[ws + lane];
-                key = rekey ? key8_of(S.a, id, wd) : sk[ws + lane];
-            }
-            warp_sort(S.a, wn, wd, key, id, lcp + ws);
-            if ((uint32_t)lane < wn) so[ws + lane] = id;
-        } else {
-            // pk of this bucket's positions is free once the block passes end
-            uint64_t key[2];
-            uint32_t id[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t pos = (uint32_t)lane + 32 * h;
-                id[h] = 0;
-                key[h] = 0;
-                if (pos < wn) {
-                    id[h] = so[ws + pos];
-                    key[h] = rekey ? key8_of(S.a, id[h], wd) : sk[ws + pos];
-                }
-            }
-            if constexpr (WIDE_WL > 32) warp_sort64(S.a, wn, wd, key, id, lcp + ws, pk + ws);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t pos = (uint32_t)lane + 32 * h;
-                if (pos < wn) so[ws + pos] = id[h];
-            }
-        }
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < size; i += NT) S.ord_out[start + i] = so[i];
-    __syncthreads();  // shared memory is reused by the next segment
-    }
+    return sizeof(SegSmem<CAP>);
 }
 
 template <int CAP, int NT>
@@ -2185,7 +2155,7 @@ static int sort_strings_graph(const SortLayout& L, SortState S, uint64_t n, uint
         k_warp_segs<<<148 * 8, 128, 0, st>>>(S, S.small[0], 0, S.counters + 1);
         k_seg_sort<256, 128><<<148 * 8, 128, seg_sort_smem<256>(), st>>>(S, S.small[1], 0, S.counters + 2);
         k_seg_sort<1024, 256><<<148 * 4, 256, seg_sort_smem<1024>(), st>>>(S, S.small[2], 0, S.counters + 3);
-        k_seg_sort<4096, 256><<<148, 256, seg_sort_smem<4096>(), st>>>(S, S.small[3], 0, S.counters + 4);
+        k_seg_sort<4096, 512><<<148 * 2, 512, seg_sort_smem<4096>(), st>>>(S, S.small[3], 0, S.counters + 4);
         if (S.split_min) k_lcp_fix<<<148 * 4, 256, 0, st>>>(S);
         cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
     }
@@ -2274,7 +2244,6 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     S.small_max = clamp_small_max(small_max);
     S.pivot = tune(TUNE_SORT_PIVOT) ? 1u : 0u;
     S.bits = (uint32_t)tune(TUNE_SORT_BITS);
-    S.seg_bits = tune(TUNE_SORT_SEG_BITS) ? 1u : 0u;
     S.first = 0;
     S.cap_large = L.cap_large;
     S.cap_small = L.cap_small;
@@ -2296,7 +2265,7 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
         static std::atomic<uint64_t> c256{0}, c1024{0}, c4096{0};
         DSSS_TRY(set_smem_once(c256, k_seg_sort<256, 128>, (int)seg_sort_smem<256>()));
         DSSS_TRY(set_smem_once(c1024, k_seg_sort<1024, 256>, (int)seg_sort_smem<1024>()));
-        DSSS_TRY(set_smem_once(c4096, k_seg_sort<4096, 256>, (int)seg_sort_smem<4096>()));
+        DSSS_TRY(set_smem_once(c4096, k_seg_sort<4096, 512>, (int)seg_sort_smem<4096>()));
         S.large[0] = large_list(L, 0);
         S.large[1] = large_list(L, 1);
         S.child = nullptr;  // every pass of the graph reads the keys itself
@@ -2366,7 +2335,7 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     }
     DSSS_TRY((launch_seg_sort<256, 128>(S, S.small[1], pin[2], "k_seg_sort256", st)));
     DSSS_TRY((launch_seg_sort<1024, 256>(S, S.small[2], pin[3], "k_seg_sort1024", st)));
-    DSSS_TRY((launch_seg_sort<4096, 256>(S, S.small[3], pin[4], "k_seg_sort4096", st)));
+    DSSS_TRY((launch_seg_sort<4096, 512>(S, S.small[3], pin[4], "k_seg_sort4096", st)));
     if (pin[5]) DSSS_LAUNCH("k_lcp_fix", st, k_lcp_fix<<<grid_for(std::min<uint64_t>(pin[5], L.cap_fix), 256), 256, 0, st>>>(S));
     DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));

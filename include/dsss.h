@@ -112,7 +112,8 @@ int dsss_abi_version(void);
  *   dp_filter_bits  filter bits per hashed string (default 16)
  *   sort_small_max  small-segment cutoff of the string sort when dsss_opts
  *                   gives 0 (2..4096, default 4096)
- *   sort_pivot      pivot passes of the string sort on/off (default 1)
+ *   sort_pivot      pivot passes of the string sort's MSD passes on/off
+ *                   (default 1)
  *   dp_table        hash-table slots per hashed string in a distinguishing-
  *                   prefix round, rounded up to a power of two (2..8, default 2)
  *   sort_graph_max_n  largest n whose string sort runs as one CUDA graph with
@@ -159,9 +160,8 @@ int dsss_abi_version(void);
  *                   byte); 2: only where the first differing key byte varies
  *                   in at most four bits; 3: the same in the first pass only;
  *                   0: on the first differing key byte (default)
- *   sort_seg_bits   the same for the shared-memory passes of the segment
- *                   sorter (segments up to the small-segment cutoff; 0:
- *                   one key byte, the default) */
+ *   sort_seg_bits   0 (default) or 1: accepted, without effect (segments up to
+ *                   the small-segment cutoff always split on differing bits) */
 int dsss_tune_set(const char* name, int64_t value);
 int dsss_tune_get(const char* name, int64_t* value);
 

@@ -37,16 +37,15 @@ constexpr unsigned PJ_FULL = 0xffffffffu;
 
 // ------------------------------------------------------------- local orders --
 // PE of every position and the PE counts of each tile.  The PE bounds are
-// searched in shared memory: the first guess is the PE that equal parts would
-// give, moved by up to two steps; PEs of very uneven sizes fall back to a
-// binary search.  Bound by the 4-byte id read and the 4-byte PE written per
+// looked up in shared memory: the PE that equal parts would give, or one of
+// its neighbours; PEs of very uneven sizes fall back to a binary search.  Bound by the 4-byte id read and the 4-byte PE written per
 // position (one pass where finding the PEs and counting them were two).
 __global__ void __launch_bounds__(PJ_NT) k_pe_hist(const uint32_t* ord, uint64_t n, const uint64_t* pb, uint32_t npe,
                                                    uint32_t p, uint64_t tiles, uint32_t* pe, uint32_t* bucket,
                                                    uint32_t* hist) {
-    extern __shared__ unsigned long long spb[];
-    uint32_t* h = reinterpret_cast<uint32_t*>(spb + npe + 1);  // a row of npe counts per warp
-    for (uint32_t q = threadIdx.x; q <= npe; q += PJ_NT) spb[q] = pb[q];
+    extern __shared__ uint32_t spb[];
+    uint32_t* h = spb + npe + 1;  // a row of npe counts per warp
+    for (uint32_t q = threadIdx.x; q <= npe; q += PJ_NT) spb[q] = (uint32_t)pb[q];  // n < 2^32
     for (uint32_t q = threadIdx.x; q < npe * PJ_NW; q += PJ_NT) h[q] = 0;
     const uint64_t g0 = (uint64_t)blockIdx.x * PJ_TILE + threadIdx.x;
     uint32_t s[PJ_IPT];
@@ -56,28 +55,25 @@ __global__ void __launch_bounds__(PJ_NT) k_pe_hist(const uint32_t* ord, uint64_t
         s[j] = g < n ? ord[g] : 0u;
     }
     __syncthreads();
-    const float scale = (float)npe / (float)(spb[npe] ? spb[npe] : 1ull);
+    const float scale = (float)npe / (float)max(spb[npe], 1u);
     uint32_t q[PJ_IPT];
 #pragma unroll
     for (int j = 0; j < PJ_IPT; ++j) q[j] = min(npe - 1, (uint32_t)((float)s[j] * scale));
-#pragma unroll
-    for (int step = 0; step < 2; ++step) {
-#pragma unroll
-        for (int j = 0; j < PJ_IPT; ++j) {
-            if (spb[q[j]] > s[j]) --q[j];            // q[j] > 0 here: spb[0] = 0
-            else if (spb[q[j] + 1] <= s[j]) ++q[j];  // q[j] + 1 < npe here: spb[npe] = n > s
-        }
-    }
     uint32_t* hw = h + (threadIdx.x >> 5) * npe;
 #pragma unroll
     for (int j = 0; j < PJ_IPT; ++j) {
         const uint64_t g = g0 + (uint64_t)j * PJ_NT;
         if (g >= n) continue;
         uint32_t r = q[j];
-        if (spb[r] > s[j] || spb[r + 1] <= s[j]) {  // still off: the last r < npe with pb[r] <= s
-            r = 0;
-            for (uint32_t st = 1u << (31 - __clz(npe | 1u)); st; st >>= 1)
-                if (r + st < npe && spb[r + st] <= s[j]) r += st;
+        if (spb[r] > s[j] || spb[r + 1] <= s[j]) {
+            // off by one (r stays in range: spb[0] = 0, spb[npe] = n > s), or
+            // further: the last r < npe with pb[r] <= s
+            r = spb[r] > s[j] ? r - 1 : r + 1;
+            if (spb[r] > s[j] || spb[r + 1] <= s[j]) {
+                r = 0;
+                for (uint32_t st = 1u << (31 - __clz(npe | 1u)); st; st >>= 1)
+                    if (r + st < npe && spb[r + st] <= s[j]) r += st;
+            }
         }
         pe[g] = p < npe ? r % p : r;
         if (bucket != pe) bucket[g] = r;
@@ -549,7 +545,7 @@ int project_local(const ProjectLayout& L, const ArenaDev& a, uint64_t n, uint32_
     const uint32_t npe = nsets * p;
     const uint64_t cells = L.tiles * npe;
     if (cells >= (1ull << 32)) return fail(DSSS_ENOTSUP, "local orders: too many tiles x PEs");
-    const size_t hsm = (npe + 1) * sizeof(unsigned long long) + (size_t)npe * PJ_NW * sizeof(uint32_t);
+    const size_t hsm = (npe + 1 + (size_t)npe * PJ_NW) * sizeof(uint32_t);
     DSSS_LAUNCH("k_pe_hist", st,
                 k_pe_hist<<<(unsigned)L.tiles, PJ_NT, hsm, st>>>(ord, n, L.pb, npe, p, L.tiles, pe, bucket, L.hist));
     DSSS_TRY(exclusive_scan_u32(L.hist, L.off, cells, nullptr, L.scan, st));

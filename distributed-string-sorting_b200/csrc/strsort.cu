@@ -1652,6 +1652,7 @@ struct SegSmem {
     uint32_t cnt[NB + 4];  // bucket counts, then starts (the last one the group's size)
     uint32_t id[CAP];
     uint2 wl[CAP / 2];         // groups for the warps
+    uint32_t tl[CAP / 2];      // the pass's buckets of 2..TINY_MAX strings
     uint2 stk[CAP / 32 + 2];   // groups for the CTA
 };
 
@@ -1663,7 +1664,7 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
     extern __shared__ __align__(16) unsigned char smem[];
     SegSmem<CAP>& M = *reinterpret_cast<SegSmem<CAP>*>(smem);
     __shared__ unsigned long long s_or[NW], s_and[NW];
-    __shared__ uint32_t s_sum[NW], s_ns, s_nw, s_piv[8];
+    __shared__ uint32_t s_sum[NW], s_ns, s_nw, s_nt, s_piv[8];
     __shared__ uint2 s_cur;
     __shared__ BucketBits s_bits;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1702,6 +1703,7 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
             const uint2 g = group_pack(0, size, G_PLAIN, seg.depth);
             s_nw = size <= 32;
             s_ns = size > 32;
+            s_nt = 0;
             if (size <= 32) M.wl[0] = g;
             else M.stk[0] = g;
         }
@@ -1885,7 +1887,6 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
             // each bucket's first string: the LCP with the bucket before (any
             // of its strings), and who sorts the bucket
             const bool all = s_bits.all != 0, mixed = pseudo && s_bits.mixed;
-            uint32_t mine = 0;  // bit j: this thread sorts the bucket of string j
 #pragma unroll
             for (int j = 0; j < IPT; ++j) {
                 if (threadIdx.x + j * NT >= bn || (br[j] >> 16) != 0) continue;
@@ -1900,10 +1901,9 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
                     }
                     lcp[bs + s0] = kind == G_ID ? dep : group_lcp(kp, kn, dep, pseudo);
                 }
-                br[j] = s0 | c << 16;
                 if (c < 2) continue;
                 if (c <= TINY_MAX) {
-                    mine |= 1u << j;
+                    M.tl[atomicAdd(&s_nt, 1u)] = s0 | c << 16;
                     continue;
                 }
                 uint32_t gk = kind, gd = dep;
@@ -1919,10 +1919,9 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
             __syncthreads();
             // buckets of 2..TINY_MAX strings: insertion sort on (key, id), then
             // the neighbours' LCPs and the runs that go deeper
-#pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                if (!((mine >> j) & 1u)) continue;
-                const uint32_t s0 = bs + (br[j] & 0xFFFFu), c = br[j] >> 16;
+            const uint32_t nt = s_nt;
+            for (uint32_t e = threadIdx.x; e < nt; e += NT) {
+                const uint32_t s0 = bs + (M.tl[e] & 0xFFFFu), c = M.tl[e] >> 16;
                 for (uint32_t x = 1; x < c; ++x) {
                     const uint64_t kx = M.key[s0 + x];
                     const uint32_t ox = M.id[s0 + x];
@@ -1962,6 +1961,7 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
             // the next pass counts from zero
             for (uint32_t x = threadIdx.x; x < NB; x += NT) M.cnt[x] = 0;
             __syncthreads();
+            if (threadIdx.x == 0) s_nt = 0;  // pushed to again only after the next pass's barriers
         }
         const uint32_t nwl = s_nw;
         for (uint32_t e = w; e < nwl; e += NW) {

@@ -1610,29 +1610,31 @@ __device__ __forceinline__ uint32_t bucket_of_key(const BucketBits& B, uint64_t 
 }
 
 __device__ __forceinline__ void bucket_bits(BucketBits& B, uint64_t diff, uint32_t want) {
-    uint32_t at[8], len[8], n = 0, total = 0;
+    uint32_t n = 0, left = want, lo = 0;
     uint64_t x = diff;
     const uint32_t hi = 63u - (uint32_t)__clzll(diff);
-    while (x && n < 8 && total < want) {
+    // a run's lowest bit and length, for the second loop
+    do {
         const uint32_t h = 63u - (uint32_t)__clzll(x);
-        const uint32_t run = (uint32_t)__clzll(~(x << (63u - h)));  // set bits from h down
-        const uint32_t take = min(run, want - total);
-        at[n] = h - take + 1;  // lowest bit taken
-        len[n] = take;
-        total += take;
-        x &= at[n] ? (1ull << at[n]) - 1 : 0ull;
+        const uint32_t take = min((uint32_t)__clzll(~(x << (63u - h))), left);  // set bits from h down
+        lo = h - take + 1;
+        B.sh[n] = lo;
+        B.mask[n] = (1u << take) - 1u;
+        left -= take;
+        x &= (1ull << lo) - 1;
         ++n;
-    }
-    B.lo = at[n - 1];
+    } while (x && n < 8 && left);
+    B.lo = lo;
     B.nruns = n;
-    B.wide = hi - at[n - 1] >= 32;
+    B.wide = hi - lo >= 32;
     B.all = x == 0;
     B.mixed = (x >> 48) != 0;
-    uint32_t place = total;
-    for (uint32_t k = 0; k < n; ++k) {
-        place -= len[k];
-        B.sh[k] = at[k] - B.lo - place;
-        B.mask[k] = ((1u << len[k]) - 1u) << place;
+    uint32_t place = 0;
+    for (uint32_t k = n; k-- > 0;) {
+        const uint32_t m = B.mask[k];
+        B.sh[k] = B.sh[k] - lo - place;
+        B.mask[k] = m << place;
+        place += (uint32_t)__popc(m);
     }
 }
 

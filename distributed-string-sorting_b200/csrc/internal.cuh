@@ -131,7 +131,7 @@ enum TuneKnob : int {
     TUNE_SORT_SMALL_MAX,     // small-segment cutoff when the options give 0
     TUNE_SORT_PIVOT,         // pivot passes on (1) or off (0)
     TUNE_DP_TABLE,           // DP hash-table slots per hashed string (rounded up to a power of two)
-    TUNE_SORT_GRAPH,         // largest n sorted by the device-driven graph (0: never)
+    TUNE_SORT_GRAPH,         // accepted, without effect
     TUNE_MERGE_SORT,         // receive containers merged by sorting their union (1), by merge rounds (0) or
                              // by co-ranked tiles of all runs at once (2)
     TUNE_MERGE_LANES,        // threads per chunk of strings in the prefix decompression (0: from the length)
@@ -140,12 +140,8 @@ enum TuneKnob : int {
     TUNE_DP_DIGEST,          // hash rounds in which at least 1/k of the positions hash run in arena order
                              // (k_dp_arena_hash); 0 turns the arena-order form off
     TUNE_DP_CHECK,           // accepted, without effect
-    TUNE_SORT_SPLIT_MIN,     // smallest large segment that may split by sampled splitters instead of a key
-                             // byte (0: never, the default; values below 4096 count as 4096)
-    TUNE_SORT_BITS,          // 1: passes over plain keys split on the keys' eight most significant differing
-                             // bits (several key bytes over small alphabets); 2: only where the first
-                             // differing byte varies in at most four bits; 3: the same in the first pass
-                             // only; 0: on one key byte (default)
+    TUNE_SORT_SPLIT_MIN,     // accepted, without effect
+    TUNE_SORT_BITS,          // accepted, without effect
     TUNE_SORT_SEG_BITS,      // accepted, without effect
     TUNE_COUNT
 };

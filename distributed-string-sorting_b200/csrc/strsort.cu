@@ -9,9 +9,12 @@
 //              first one), so a segment's key starts at its first differing byte;
 //   keys/diff: gather the 8-byte key at that depth, OR of (key ^ key0) tells
 //              which key byte is the first to differ;
-//   hist     : warp-aggregated 256-bin histogram of that byte per 4096-element tile;
-//   scan     : per segment, bucket starts and per-tile offsets (chunked);
-//   scatter  : stable scatter of ids (and keys of children that stay large).
+//   hist     : per segment, counts of a digit of up to 8 bits: the most
+//              significant bits in which its keys may differ;
+//   scan     : per segment, bucket starts, bucket-start LCPs, the children;
+//   scatter  : ids and keys to their buckets, places reserved per tile by one
+//              atomic per digit (the order inside a bucket does not matter:
+//              equal strings are ordered by id at the end).
 // A child that keeps more than half of its parent (a chain of long shared
 // prefixes, e.g. suffixes inside repeats or strings that share a long common
 // head) would lose one byte per pass; it is flagged for a pivot pass instead:
@@ -31,65 +34,55 @@
 
 namespace dsss {
 
-constexpr int LT_NT = 256, LT_IPT = 8, LT_TILE = LT_NT * LT_IPT;
-constexpr int CHUNK_TILES = 32;
+constexpr int LT_NT = 256, LT_IPT = 16, LT_TILE = LT_NT * LT_IPT;
 constexpr uint32_t PREFIX_CAP = 256;
 // F_KEYS: the key array holds the segment's keys at Seg.depth; F_PIVOT: the
-// next pass is a pivot pass; F_PSEUDO: the keys are pivot pseudo keys.
-constexpr uint32_t F_PARITY = 1u, F_KEYS = 2u, F_PIVOT = 4u, F_PSEUDO = 8u;
+// next pass is a pivot pass; F_PSEUDO: the keys are pivot pseudo keys; F_ID:
+// the strings are equal (Seg.depth their length) and are sorted by id.
+constexpr uint32_t F_PARITY = 1u, F_KEYS = 2u, F_PIVOT = 4u, F_PSEUDO = 8u, F_ID = 16u;
 constexpr uint32_t PIVOT_CAP = 127;  // pseudo key byte 0 holds codes 0 .. 2 * PIVOT_CAP
+constexpr uint32_t NO_PIVOT = 0xFFFFFFFFu;
+
+// The bits that pick a key's bucket: up to `want` of the most significant
+// bits of diff, in at most 8 runs of neighbouring bits.  A key's bucket is the
+// OR over the runs of ((key >> lo) >> sh) & mask; every bit above lo that is
+// not chosen is the same in all keys, so buckets order as keys do.  In a
+// pseudo group of the segment sorter whose code bits are all chosen, a bucket
+// holds one code; otherwise (LCPs over thousands of bytes) `mixed` is set.
+struct BucketBits {
+    uint32_t lo, nruns, wide, all;  // wide: the bits span more than 32; all: every differing bit is chosen
+    uint32_t mixed;
+    uint32_t sh[8], mask[8];
+};
 
 struct Seg {
     uint32_t start, size, depth, flags;
     uint32_t newdepth;
-    uint32_t first_digit;
-    unsigned long long diff;
     // speculated common-prefix depth + 1 (0: none) and the OR of key ^ key0
     // over the keys k_prefix wrote at that depth (segments without keys)
     uint32_t spec;
-    // this pass's digit: the key byte at the first difference (nspl = 0), or
-    // the bucket among nspl sampled splitters (table spl_slot; bucket-start
-    // LCPs into the fix list from fix0)
-    uint32_t nspl;
     unsigned long long spec_diff;
-    uint32_t spl_slot, fix0;
-    // pivot pass: the pivot's string id (NO_PIVOT: the segment's first string)
-    uint32_t piv, pad;
-    // OR and AND of the keys the previous pass's scatter wrote for this
-    // segment (children with keys, when the child table is kept): the bits
-    // that differ among its keys are kor ^ kand
-    unsigned long long kor, kand;
+    // bits in which the keys may differ: exact for keys made in this pass, the
+    // parent's bits below its digit for keys carried over
+    unsigned long long diff;
+    uint32_t piv;    // pivot pass: the pivot's string id (NO_PIVOT: the first string)
+    uint32_t ended;  // bucket 0 holds the strings that end at the first differing byte
+    BucketBits bits;  // this pass's digit
 };
 
-// Sampled splitters.  Where the key byte at a large segment's first
-// difference takes few values (letters, DNA), a byte digit splits the segment
-// only a few ways per pass.  Instead, the distinct keys among every 8th of an
-// evenly spaced, sorted sample of SPL_SAMPLE keys become m <= 255 splitters.
-// With more than SPL_EQ_MAX of them a key's bucket is the number of
-// splitters below it (about 1/256 of the segment each; two splitters are
-// keys of the segment in different buckets, so it splits).  With fewer (few
-// distinct keys: frequent ones), bucket 2j holds the keys between splitters
-// j-1 and j and bucket 2j+1 the keys equal to splitter j, so every sampled
-// key lands in an equality bucket and the others elsewhere.  Equal keys
-// always share a bucket, and two neighbours across a bucket boundary have
-// different keys, so their LCP is the depth plus the LCP of the two keys; it
-// is written once the final order is known (k_lcp_fix).
-constexpr int SPL_SAMPLE = 2048;
-constexpr uint32_t SPL_MAX = 255, SPL_STRIDE = 256, SPL_EQ_MAX = 127;
-constexpr uint32_t SPL_MIN_FLOOR = 4096;  // smallest sort_split_min other than 0 (off)
-constexpr uint32_t FIX_NONE = 0xFFFFFFFFu;
-constexpr uint32_t NO_PIVOT = 0xFFFFFFFFu;
+struct SmallSeg {
+    uint32_t start, size, depth, flags;
+};
 
 constexpr int NBINS = 4;
 __host__ __device__ constexpr int bin_cap(int b) { return b == 0 ? 32 : b == 1 ? 256 : b == 2 ? 1024 : 4096; }
-__device__ __forceinline__ int bin_of(uint32_t size) {
+__host__ __device__ __forceinline__ int bin_of(uint32_t size) {
     return size <= 32 ? 0 : size <= 256 ? 1 : size <= 1024 ? 2 : 3;
 }
 
-// Counters block (device): [0] n_large_next, [1..4] n_small per bin, [5]
-// fix-list slots reserved, [6] splitter tables of the pass, [8] total tiles,
-// [9] total chunks, [10] error flag (a guard tripped), [11] large segments of
-// the next pass without keys or with a pivot pass.
+// Counters block (device): [0] n_large_next, [1..4] n_small per bin, [8] total
+// tiles, [10] error flag (a guard tripped), [11] large segments of the next
+// pass without keys or with a pivot pass.
 struct SortState {
     ArenaDev a;
     uint32_t* ord[2];
@@ -97,101 +90,68 @@ struct SortState {
     uint32_t* ord_out;
     uint32_t* lcp_out;
     Seg* large[2];
-    Seg* small[NBINS];
+    SmallSeg* small[NBINS];
     uint32_t* tile0;
-    uint32_t* chunk0;
-    uint32_t* tmp_counts;
-    uint32_t* tile_hist;
-    uint32_t* chunk_pre;
-    uint32_t* bucket;  // 257 per large segment
+    uint32_t* hist;    // 256 per large segment, zero between passes
+    uint32_t* bucket;  // 257 per large segment: where the buckets start
+    uint32_t* cursor;  // 256 per large segment: where their next tile goes
     uint32_t* counters;
-    // child table (optional, 256 per large segment): the next list's slot of
-    // digit d's child when it is large and keeps the keys (~0u otherwise); the
-    // scatter then folds the keys it writes into that child's kor / kand
-    uint32_t* child;
-    Seg* nxt;  // the next pass's list (the scatter's children)
     uint32_t small_max;
     uint32_t pivot;  // pivot passes enabled
-    uint32_t bits;   // plain keys split on their top differing bits: 0 never, 1 always, 2 on narrow bytes
-    uint32_t first;     // the first pass over the arena (host-driven passes)
-    uint64_t cap_large, cap_small, cap_tiles, cap_chunks;
-    // sampled splitters: segments of at least split_min strings (0: never);
-    // cap_spl tables of SPL_STRIDE keys per pass; the fix list holds
-    // (position, depth) pairs of bucket starts whose LCP k_lcp_fix writes
-    uint32_t split_min;
+    uint32_t iota;   // first pass over the whole arena: position i holds id i
+    uint64_t n;
+    uint64_t cap_large, cap_small[NBINS], cap_tiles;
     const uint32_t* seg_depth;  // optional: each segment's shared prefix length
-    unsigned long long* spl;
-    uint32_t* fix;
-    uint64_t cap_spl, cap_fix;
 };
 
+__device__ __forceinline__ uint32_t ord_of(const SortState& S, uint32_t par, uint32_t i) {
+    return S.iota ? i : S.ord[par][i];
+}
+
+// The last s with first[s] <= t, by all lanes of a warp together (32 probes
+// per step: three dependent reads for 32768 segments).
 __device__ __forceinline__ uint32_t find_seg(const uint32_t* first, uint32_t nseg, uint32_t t) {
-    // last s with first[s] <= t
     uint32_t lo = 0, hi = nseg;
     while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (first[mid] <= t) lo = mid;
-        else hi = mid;
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t x = lo + (threadIdx.x & 31) * step;
+        const uint32_t below = __popc(__ballot_sync(0xffffffffu, x < hi && first[x] <= t));
+        lo += (below - 1) * step;
+        hi = min(hi, lo + step);
     }
     return lo;
 }
 
 __device__ __forceinline__ void push_small(const SortState& S, uint32_t start, uint32_t size, uint32_t depth,
                                            uint32_t flags) {
-    int b = bin_of(size);
-    uint32_t slot = atomicAdd(&S.counters[1 + b], 1u);
-    if (slot >= S.cap_small) {
+    const int b = bin_of(size);
+    const uint32_t slot = atomicAdd(&S.counters[1 + b], 1u);
+    if (slot >= S.cap_small[b]) {
         atomicExch(&S.counters[10], 1u);
         return;
     }
-    Seg s;
-    s.start = start;
-    s.size = size;
-    s.depth = depth;
-    s.flags = flags;
-    s.newdepth = 0xFFFFFFFFu;
-    s.first_digit = 0;
-    s.diff = 0;
-    s.spec = 0;
-    s.nspl = 0;
-    s.spl_slot = 0;
-    s.fix0 = 0;
-    s.piv = NO_PIVOT;
-    s.pad = 0;
-    s.spec_diff = 0;
-    s.kor = 0;
-    s.kand = ~0ull;
-    S.small[b][slot] = s;
+    S.small[b][slot] = SmallSeg{start, size, depth, flags};
 }
 
-// Returns the segment's slot in dst (~0u when the list is full).
-__device__ __forceinline__ uint32_t push_large(const SortState& S, Seg* dst, uint32_t start, uint32_t size,
-                                               uint32_t depth, uint32_t flags) {
-    uint32_t slot = atomicAdd(&S.counters[0], 1u);
+__device__ __forceinline__ void push_large(const SortState& S, Seg* dst, uint32_t start, uint32_t size, uint32_t depth,
+                                           uint32_t flags, uint64_t diff = 0) {
+    const uint32_t slot = atomicAdd(&S.counters[0], 1u);
     if (slot >= S.cap_large) {
         atomicExch(&S.counters[10], 1u);
-        return 0xFFFFFFFFu;
+        return;
     }
-    if (!(flags & F_KEYS) || (flags & F_PIVOT)) atomicAdd(&S.counters[11], 1u);
-    Seg s;
+    if (!(flags & F_KEYS)) atomicAdd(&S.counters[11], 1u);
+    Seg& s = dst[slot];
     s.start = start;
     s.size = size;
     s.depth = depth;
     s.flags = flags;
     s.newdepth = 0xFFFFFFFFu;
-    s.first_digit = 0;
-    s.diff = 0;
     s.spec = 0;
-    s.nspl = 0;
-    s.spl_slot = 0;
-    s.fix0 = 0;
-    s.piv = NO_PIVOT;
-    s.pad = 0;
     s.spec_diff = 0;
-    s.kor = 0;
-    s.kand = ~0ull;
-    dst[slot] = s;
-    return slot;
+    s.diff = diff;
+    s.piv = NO_PIVOT;
+    s.ended = 0;
 }
 
 // ------------------------------------------------------------------ init ----
@@ -200,29 +160,21 @@ __global__ void k_init_ids(uint32_t* ord, const uint32_t* in, uint64_t n) {
     if (i < n) ord[i] = in ? in[i] : (uint32_t)i;
 }
 
+// pb: p + 1 segment bounds (NULL: one segment of n strings).
 __global__ void k_init_segs(SortState S, const uint64_t* pb, uint32_t p) {
-    uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= p) return;
-    uint32_t start = (uint32_t)pb[q], size = (uint32_t)(pb[q + 1] - pb[q]);
+    const uint32_t start = pb ? (uint32_t)pb[q] : 0u, size = pb ? (uint32_t)(pb[q + 1] - pb[q]) : (uint32_t)S.n;
     if (size == 0) return;
     S.lcp_out[start] = 0;
     if (size == 1) {
-        S.ord_out[start] = S.ord[0][start];
+        S.ord_out[start] = ord_of(S, 0, start);
         return;
     }
     // a segment whose strings are known to share their first bytes starts there
     const uint32_t d = S.seg_depth ? S.seg_depth[q] : 0u;
     if (size > S.small_max) push_large(S, S.large[0], start, size, d, 0);
     else push_small(S, start, size, d, 0);
-}
-
-// --------------------------------------------------------- tile indexing ----
-__global__ void k_tile_counts(const Seg* segs, uint32_t nseg, uint32_t* tiles, uint32_t* chunks) {
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nseg) return;
-    uint32_t t = (segs[s].size + LT_TILE - 1) / LT_TILE;
-    tiles[s] = t;
-    chunks[s] = (t + CHUNK_TILES - 1) / CHUNK_TILES;
 }
 
 // ---------------------------------------------------------------- prefix ----
@@ -328,17 +280,17 @@ __global__ void __launch_bounds__(256) k_spec(SortState S, Seg* segs, uint32_t n
             choose_pivot(S, sg, pw, psum, pid);
             continue;
         }
-        if (sg.flags & F_KEYS) continue;
-        const uint32_t* ord = S.ord[sg.flags & F_PARITY];
+        if (sg.flags & (F_KEYS | F_ID)) continue;
+        const uint32_t par = sg.flags & F_PARITY;
         const uint32_t d0 = sg.depth;
         uint32_t l = 0xFFFFFFFFu;
         const uint32_t m = sg.size < 256u ? sg.size : 256u;
         if (threadIdx.x < m) {
             uint64_t off0, off;
             uint32_t len0, len;
-            str_of(S.a, ord[sg.start], off0, len0);
+            str_of(S.a, ord_of(S, par, sg.start), off0, len0);
             const uint32_t i = sg.start + (uint32_t)((uint64_t)threadIdx.x * sg.size / m);
-            str_of(S.a, ord[i], off, len);
+            str_of(S.a, ord_of(S, par, i), off, len);
             uint64_t x[7], y[7];
             key_words<7>(S.a.chars, off, len, d0, 7, x);
             key_words<7>(S.a.chars, off0, len0, d0, 7, y);
@@ -364,21 +316,16 @@ __global__ void __launch_bounds__(256) k_spec(SortState S, Seg* segs, uint32_t n
 }
 
 __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
     Seg& sg = segs[si];
-    if (sg.flags & (F_KEYS | F_PIVOT)) return;
+    if (sg.flags & (F_KEYS | F_PIVOT | F_ID)) return;
     const uint32_t par = sg.flags & F_PARITY;
-    const uint32_t* ord = S.ord[par];
     const uint32_t tb = sg.start + (t - S.tile0[si]) * LT_TILE;
     const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
     const uint32_t d0 = sg.depth, cap = d0 + PREFIX_CAP;
-    const uint32_t s0 = ord[sg.start];
+    const uint32_t s0 = ord_of(S, par, sg.start);
     uint64_t off0;
     uint32_t len0;
     str_of(S.a, s0, off0, len0);
@@ -404,8 +351,7 @@ __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uin
         for (uint32_t i = tb + threadIdx.x; i < te; i += LT_NT) {
             uint64_t off;
             uint32_t len;
-            const uint32_t s = ord[i];
-            str_of(S.a, s, off, len);
+            str_of(S.a, ord_of(S, par, i), off, len);
             uint64_t x[PF_W];
             key_words<PF_W>(S.a.chars, off, len, d0, want, x);
             uint32_t l = D;
@@ -442,8 +388,7 @@ __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uin
     for (uint32_t i = tb + threadIdx.x; i < te; i += LT_NT) {
         uint64_t off;
         uint32_t len;
-        const uint32_t s = ord[i];
-        str_of(S.a, s, off, len);
+        str_of(S.a, ord_of(S, par, i), off, len);
         // no need to compare past this thread's minimum so far
         const uint32_t lim = min(cap, mn);
         uint32_t l = 0;
@@ -514,198 +459,65 @@ __global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uin
 // ------------------------------------------------------------- keys/diff ----
 constexpr int KD_ILP = 8;
 __global__ void __launch_bounds__(LT_NT) k_keys_diff(SortState S, Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
     Seg& sg = segs[si];
-    if (sg.flags & F_PIVOT) return;  // keys and diff come from k_pivot
-    if (!(sg.flags & F_KEYS) && sg.spec && sg.newdepth == sg.spec - 1) {
+    if (sg.flags & (F_KEYS | F_PIVOT)) return;  // keys carried over, or made by k_pivot
+    const bool by_id = sg.flags & F_ID;
+    if (!by_id && sg.spec && sg.newdepth == sg.spec - 1) {
         // the speculated depth was the common prefix: k_prefix wrote the keys
         if (t == S.tile0[si] && threadIdx.x == 0) sg.diff = sg.spec_diff;
         return;
     }
-    const uint32_t par = sg.flags & F_PARITY;
-    const bool valid = sg.flags & F_KEYS;
-    const uint32_t depth = valid ? sg.depth : sg.newdepth;
-    const uint32_t* ord = S.ord[par];
+    const uint32_t par = sg.flags & F_PARITY, depth = sg.newdepth;
     unsigned long long* key = S.key[par];
     const uint32_t tb = sg.start + (t - S.tile0[si]) * LT_TILE;
     const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
-    uint64_t k0;
-    if (valid) {
-        k0 = key[sg.start];
-    } else {
-        uint32_t s0 = ord[sg.start];
-        k0 = key8_of(S.a, s0, depth);
-    }
+    const uint32_t s0 = ord_of(S, par, sg.start);
+    const uint64_t k0 = by_id ? (uint64_t)s0 : key8_of(S.a, s0, depth);
     uint64_t df = 0;
-    if (valid) {
-        // the tile's keys all in flight before any is used
-        uint64_t k[LT_IPT];
+    // KD_ILP independent gathers in flight per thread
+    for (uint32_t i0 = tb + threadIdx.x; i0 < te; i0 += KD_ILP * LT_NT) {
+        uint32_t s[KD_ILP];
+        uint64_t off[KD_ILP];
+        uint32_t len[KD_ILP];
 #pragma unroll
-        for (int j = 0; j < LT_IPT; ++j) {
-            const uint32_t i = tb + j * LT_NT + threadIdx.x;
-            k[j] = i < te ? key[i] : k0;
+        for (int q = 0; q < KD_ILP; ++q) {
+            const uint32_t i = i0 + q * LT_NT;
+            s[q] = i < te ? ord_of(S, par, i) : 0u;
         }
-#pragma unroll
-        for (int j = 0; j < LT_IPT; ++j) df |= k[j] ^ k0;
-    } else {
-        // KD_ILP independent gathers in flight per thread
-        for (uint32_t i0 = tb + threadIdx.x; i0 < te; i0 += KD_ILP * LT_NT) {
-            uint32_t s[KD_ILP];
-            uint64_t off[KD_ILP];
-            uint32_t len[KD_ILP];
-#pragma unroll
-            for (int q = 0; q < KD_ILP; ++q) {
-                const uint32_t i = i0 + q * LT_NT;
-                s[q] = i < te ? ord[i] : 0u;
-            }
-#pragma unroll
-            for (int q = 0; q < KD_ILP; ++q) {
-                const uint32_t i = i0 + q * LT_NT;
-                off[q] = 0;
-                len[q] = 0;
-                if (i < te) str_of(S.a, s[q], off[q], len[q]);
-            }
+        if (by_id) {
 #pragma unroll
             for (int q = 0; q < KD_ILP; ++q) {
                 const uint32_t i = i0 + q * LT_NT;
                 if (i < te) {
-                    const uint64_t k = key8(S.a.chars, off[q], len[q], depth);
-                    key[i] = k;
-                    df |= k ^ k0;
+                    key[i] = s[q];
+                    df |= s[q] ^ k0;
                 }
+            }
+            continue;
+        }
+#pragma unroll
+        for (int q = 0; q < KD_ILP; ++q) {
+            const uint32_t i = i0 + q * LT_NT;
+            off[q] = 0;
+            len[q] = 0;
+            if (i < te) str_of(S.a, s[q], off[q], len[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < KD_ILP; ++q) {
+            const uint32_t i = i0 + q * LT_NT;
+            if (i < te) {
+                const uint64_t k = key8(S.a.chars, off[q], len[q], depth);
+                key[i] = k;
+                df |= k ^ k0;
             }
         }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) df |= __shfl_xor_sync(0xffffffffu, df, o);
     if ((threadIdx.x & 31) == 0 && df) atomicOr(&sg.diff, (unsigned long long)df);
-}
-
-// ------------------------------------------------------ sampled splitters ----
-// Per large segment with keys (not a pivot pass) of at least split_min
-// strings: the sample's byte-digit histogram at the first difference decides
-// whether splitters pay (its largest bucket holds more than 1/64 of the
-// sample, four times what a splitter bucket holds); if so, the sorted
-// sample's every 8th key, distinct, become the splitters.  One block of
-// SPL_SAMPLE / 2 threads per segment.
-__global__ void __launch_bounds__(SPL_SAMPLE / 2) k_split_sample(SortState S, Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
-    __shared__ unsigned long long sk[SPL_SAMPLE];
-    __shared__ uint32_t bcnt[256];
-    __shared__ uint32_t s_fix0, s_nres;
-    for (uint32_t si = blockIdx.x; si < nseg; si += gridDim.x) {
-        Seg& sg = segs[si];
-        const bool use = S.split_min && sg.size >= S.split_min && sg.diff != 0 && !(sg.flags & (F_PIVOT | F_PSEUDO));
-        if (!use) {  // the same for the whole block
-            if (threadIdx.x == 0) sg.nspl = 0;
-            continue;
-        }
-        const unsigned long long* key = S.key[sg.flags & F_PARITY];
-        const uint32_t shift = 56 - 8 * (uint32_t)(__clzll(sg.diff) >> 3);
-        if (threadIdx.x < 256) bcnt[threadIdx.x] = 0;
-        __syncthreads();
-        for (uint32_t j = threadIdx.x; j < (uint32_t)SPL_SAMPLE; j += blockDim.x) {
-            const unsigned long long k = key[sg.start + (uint32_t)((uint64_t)j * sg.size / SPL_SAMPLE)];
-            sk[j] = k;
-            atomicAdd(&bcnt[(uint32_t)(k >> shift) & 0xFFu], 1u);
-        }
-        __syncthreads();
-        // bitonic sort of the sample, ascending: thread t compares index i
-        // (bit j clear) with i | j
-        for (uint32_t k = 2; k <= (uint32_t)SPL_SAMPLE; k <<= 1) {
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                const uint32_t i = ((threadIdx.x & ~(j - 1)) << 1) | (threadIdx.x & (j - 1));
-                const unsigned long long a = sk[i], b = sk[i | j];
-                if ((a > b) == ((i & k) == 0)) {
-                    sk[i] = b;
-                    sk[i | j] = a;
-                }
-                __syncthreads();
-            }
-        }
-        if (threadIdx.x == 0) {
-            uint32_t mx = 0;
-            for (int d = 0; d < 256; ++d) mx = max(mx, bcnt[d]);
-            uint32_t m = 0, slot = 0, fix0 = 0, nres = 0;
-            if (64 * mx > (uint32_t)SPL_SAMPLE) {
-                slot = atomicAdd(&S.counters[6], 1u);
-                if (slot < S.cap_spl) {
-                    unsigned long long* spl = S.spl + (uint64_t)slot * SPL_STRIDE;
-                    for (uint32_t q = 0; q < SPL_MAX; ++q) {
-                        const unsigned long long c = sk[(q + 1) * (SPL_SAMPLE / SPL_STRIDE) - 1];
-                        if (m == 0 || c != spl[m - 1]) spl[m++] = c;
-                    }
-                    for (uint32_t q = m; q < SPL_STRIDE; ++q) spl[q] = ~0ull;
-                    // bucket-start slots in the fix list, one per bucket
-                    nres = m > SPL_EQ_MAX ? m + 1 : 2 * m + 1;
-                    fix0 = atomicAdd(&S.counters[5], nres);
-                    if ((uint64_t)fix0 + nres > S.cap_fix) m = 0;
-                }
-            }
-            s_fix0 = fix0;
-            s_nres = nres;
-            sg.nspl = m;
-            sg.spl_slot = slot;
-            sg.fix0 = fix0;
-        }
-        __syncthreads();
-        // every reserved fix slot starts empty (also a reservation past the
-        // list's end, as far as the list goes)
-        if (s_nres) {
-            const uint64_t e = min((uint64_t)s_fix0 + s_nres, S.cap_fix);
-            for (uint64_t f = (uint64_t)s_fix0 + threadIdx.x; f < e; f += blockDim.x) S.fix[2 * f] = FIX_NONE;
-        }
-        __syncthreads();  // the sample buffer is reused by the next segment
-    }
-}
-
-// Bucket of key k among m sorted splitters (the table padded to SPL_STRIDE
-// with ~0): j = the number of splitters below k (at most m, eight fixed
-// steps); with more than SPL_EQ_MAX splitters j, else 2j, or 2j + 1 when k
-// equals splitter j.
-__device__ __forceinline__ uint32_t spl_bucket(const unsigned long long* spl, uint32_t m, unsigned long long k) {
-    uint32_t j = 0;
-#pragma unroll
-    for (uint32_t step = SPL_STRIDE / 2; step; step >>= 1)
-        if (spl[j + step - 1] < k) j += step;
-    if (m > SPL_EQ_MAX) return j;
-    return 2 * j + (j < m && spl[j] == k ? 1u : 0u);
-}
-
-// LCPs at the bucket starts of splitter passes, once the order is final: the
-// two neighbours have different keys at depth d.
-__global__ void __launch_bounds__(256) k_lcp_fix(SortState S) {
-    const uint64_t m = min((uint64_t)S.counters[5], S.cap_fix);
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t f = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; f < m; f += stride) {
-        const uint32_t pos = S.fix[2 * f];
-        if (pos == FIX_NONE) continue;
-        uint32_t l = S.fix[2 * f + 1];
-        const uint32_t x = S.ord_out[pos - 1], y = S.ord_out[pos];
-        for (;;) {
-            const uint64_t kx = key8_of(S.a, x, l), ky = key8_of(S.a, y, l);
-            if (kx != ky) {
-                l += key_lcp(kx, ky);
-                break;
-            }
-            const uint32_t z = zero_byte(kx);
-            if (z < 8) {
-                l += z;
-                break;
-            }
-            l += 8;
-        }
-        S.lcp_out[pos] = l;
-    }
 }
 
 // ----------------------------------------------------------------- pivot ----
@@ -761,10 +573,6 @@ __device__ __forceinline__ uint64_t pivot_key(const uint8_t* chars, uint64_t off
 }
 
 __global__ void __launch_bounds__(LT_NT) k_pivot(SortState S, Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
@@ -794,218 +602,159 @@ __global__ void __launch_bounds__(LT_NT) k_pivot(SortState S, Seg* segs, uint32_
 }
 
 // ------------------------------------------------------------------ hist ----
-__device__ __forceinline__ uint32_t digit_of(uint64_t k, uint32_t shift) { return (uint32_t)(k >> shift) & 0xFFu; }
-
-// The digit of a pass over plain keys: the (up to) eight most significant
-// bits in which the segment's keys differ, packed in key order.  Every bit
-// above the lowest of them that is not one of them is the same in all keys,
-// so the digit orders the keys as their first bytes do.  Where the key byte
-// at the first difference varies in all eight bits this is that byte; over a
-// small alphabet (letters vary in 5 or 6 bits of a byte, DNA in 4) a digit
-// covers more than one key byte, and a pass splits up to 256 ways instead of
-// as many ways as the byte has values.  sh[j]: the right shift that brings
-// digit bit j (most significant first) to bit 0.
-struct BitDigit {
-    uint32_t nb;     // bits in the digit (1..8)
-    uint32_t sh[8];
-    bool whole;      // one whole key byte: (k >> sh[7]) & 0xFF
-};
-
-// Whether a pass over plain keys splits on bits: knob sort_bits 1 always, 2
-// where the first differing key byte varies in at most four bits (DNA, or a
-// leading digit with few values), 3 the same in the first pass only, 0
-// never; and only for segments of more than four times the small-segment
-// cutoff (a 256-way split of a segment just above the cutoff leaves children
-// of a few strings each, whose segment records cost more than sorting them).
-__device__ __forceinline__ bool use_bits(uint32_t mode, uint64_t diff, uint32_t shift, uint32_t size,
-                                         uint32_t small_max, uint32_t first) {
-    if ((uint64_t)size <= 4ull * small_max) return false;
-    const bool narrow = __popc((uint32_t)(diff >> shift) & 0xFFu) <= 4;
-    return mode == 1 || (mode == 2 && narrow) || (mode == 3 && first && narrow);
+__device__ __forceinline__ uint32_t bucket_of_key(const BucketBits& B, uint64_t k) {
+    uint32_t b = 0;
+    for (uint32_t r = 0; r < B.nruns; ++r) b |= (uint32_t)(k >> (B.lo + B.sh[r])) & B.mask[r];
+    return b;
 }
 
-__device__ __forceinline__ BitDigit bit_digit_spec(uint64_t diff) {
-    BitDigit d;
-    d.nb = 0;
+__device__ __forceinline__ void bucket_bits(BucketBits& B, uint64_t diff, uint32_t want) {
+    uint32_t n = 0, left = want, lo = 0;
     uint64_t x = diff;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        d.sh[j] = 0;
-        if (x) {
-            const uint32_t at = 63u - (uint32_t)__clzll(x);
-            d.sh[j] = at;
-            x &= ~(1ull << at);
-            ++d.nb;
-        }
-    }
-    d.whole = d.nb == 8 && (d.sh[0] & 7u) == 7u && d.sh[7] + 7u == d.sh[0];
-    return d;
-}
-
-// Digit lookup in shared memory: for each key byte that holds digit bits,
-// tab[q][v] is the digit bits of byte value v, packed and moved to their place
-// in the digit; a key's digit is the OR over those bytes (usually two).
-struct BitTables {
-    uint8_t tab[8][256];
-    uint32_t n;      // key bytes holding digit bits
-    uint32_t sh[8];  // right shift of each such byte
-};
-
-// Builds the tables of digit d; every thread of the block calls it, and a
-// barrier follows before the first lookup.
-__device__ __forceinline__ void bit_tables_build(BitTables& T, const BitDigit& d) {
-    uint64_t chosen = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if ((uint32_t)j < d.nb) chosen |= 1ull << d.sh[j];
-    for (uint32_t v = threadIdx.x; v < 256; v += blockDim.x) {
-        uint32_t q = 0, below = (uint32_t)__popcll(chosen);
-        for (int J = 0; J < 8; ++J) {
-            const uint32_t sh = 56u - 8u * (uint32_t)J;
-            const uint32_t sel = (uint32_t)(chosen >> sh) & 0xFFu;
-            if (!sel) continue;
-            below -= (uint32_t)__popc(sel);  // digit bits in later key bytes
-            uint32_t x = 0;                  // the bits of v that sel selects, packed
-            for (int bit = 7; bit >= 0; --bit)
-                if ((sel >> bit) & 1u) x = (x << 1) | ((v >> bit) & 1u);
-            T.tab[q][v] = (uint8_t)(x << below);
-            if (v == 0) T.sh[q] = sh;
-            ++q;
-        }
-        if (v == 0) T.n = q;
+    const uint32_t hi = 63u - (uint32_t)__clzll(diff);
+    // a run's lowest bit and length, for the second loop
+    do {
+        const uint32_t h = 63u - (uint32_t)__clzll(x);
+        const uint32_t take = min((uint32_t)__clzll(~(x << (63u - h))), left);  // set bits from h down
+        lo = h - take + 1;
+        B.sh[n] = lo;
+        B.mask[n] = (1u << take) - 1u;
+        left -= take;
+        x &= (1ull << lo) - 1;
+        ++n;
+    } while (x && n < 8 && left);
+    B.lo = lo;
+    B.nruns = n;
+    B.wide = hi - lo >= 32;
+    B.all = x == 0;
+    B.mixed = (x >> 48) != 0;
+    uint32_t place = 0;
+    for (uint32_t k = n; k-- > 0;) {
+        const uint32_t m = B.mask[k];
+        B.sh[k] = B.sh[k] - lo - place;
+        B.mask[k] = m << place;
+        place += (uint32_t)__popc(m);
     }
 }
 
-__device__ __forceinline__ uint32_t bit_digit(uint64_t k, const BitDigit& d, const BitTables& T) {
-    if (d.whole) return (uint32_t)(k >> d.sh[7]) & 0xFFu;
-    uint32_t v = 0;
-    for (uint32_t q = 0; q < T.n; ++q) v |= T.tab[q][(uint32_t)(k >> T.sh[q]) & 0xFFu];
-    return v;
+// This pass's digit of a segment: pivot pseudo keys split on a whole byte (the
+// code, then the byte behind the LCP), other keys on their most significant
+// differing bits, as many (up to 8) as leave about DIGIT_TARGET strings per
+// bucket.  A digit of 8 bits over letters (5 differing bits per byte) or DNA (4)
+// covers more than a byte, so 32e6 random six-letter keys take two passes where
+// byte digits took four; narrower digits for segments just above the cutoff
+// keep their children from being a few strings each.
+constexpr uint32_t DIGIT_TARGET = 640;
+__device__ __forceinline__ void segment_digit(BucketBits& B, uint64_t diff, uint32_t flags, uint32_t size) {
+    if (flags & (F_PIVOT | F_PSEUDO)) {
+        B.lo = 56 - 8 * (uint32_t)(__clzll(diff) >> 3);
+        B.nruns = 1;
+        B.wide = 0;
+        B.all = 0;
+        B.mixed = 0;
+        B.sh[0] = 0;
+        B.mask[0] = 0xFFu;
+        return;
+    }
+    const uint32_t parts = size / DIGIT_TARGET;
+    bucket_bits(B, diff, min(8u, max(3u, 33u - (uint32_t)__clz(parts | 1u))));
 }
 
-// Key byte (from the key's first byte) that holds digit bit h (0: least
-// significant): two keys whose digits first differ in bit h share exactly
-// that many bytes past the segment depth.
-__device__ __forceinline__ uint32_t bit_digit_byte(const BitDigit& d, uint32_t h) {
-    uint32_t byte = 0;
+// The bits of a key that a digit holds.
+__device__ __forceinline__ uint64_t digit_mask(const BucketBits& B) {
+    uint64_t m = 0;
+    for (uint32_t r = 0; r < B.nruns; ++r) m |= (uint64_t)B.mask[r] << (B.lo + B.sh[r]);
+    return m;
+}
+
+// Bucket numbers of N keys (the runs outermost: one shared read per run).
+template <int N>
+__device__ __forceinline__ void digits_of(const BucketBits& B, const uint64_t (&k)[N], uint32_t (&d)[N]) {
+    const uint32_t lo = B.lo, nr = B.nruns;
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if ((uint32_t)j + 1 + h == d.nb) byte = (63u - d.sh[j]) >> 3;
-    return byte;
+    for (int j = 0; j < N; ++j) d[j] = 0;
+    if (B.wide) {
+        for (uint32_t r = 0; r < nr; ++r) {
+            const uint32_t sh = lo + B.sh[r], mask = B.mask[r];
+#pragma unroll
+            for (int j = 0; j < N; ++j) d[j] |= (uint32_t)(k[j] >> sh) & mask;
+        }
+        return;
+    }
+    uint32_t x[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] = (uint32_t)(k[j] >> lo);
+    for (uint32_t r = 0; r < nr; ++r) {
+        const uint32_t sh = B.sh[r], mask = B.mask[r];
+#pragma unroll
+        for (int j = 0; j < N; ++j) d[j] |= (x[j] >> sh) & mask;
+    }
 }
 
-// BITS: the bit-digit form (its tables and registers only where the knob asks
-// for it; the byte form keeps the occupancy of a 32-register kernel).
-template <bool BITS>
+// Counts per segment and digit: a tile's counts in shared memory (one row per
+// warp), then one global atomic per digit.  Bound by the 8-byte key read.
 __global__ void __launch_bounds__(LT_NT) k_hist(SortState S, const Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
-    // one 256-bin histogram per warp (shared-memory atomics contend only
-    // inside a warp), summed per digit at the end
     __shared__ uint32_t hist[LT_NT / 32][256];
-    __shared__ unsigned long long s_spl[SPL_STRIDE];
+    __shared__ BucketBits B;
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
-    const Seg sg = segs[si];
-    if (sg.diff == 0) return;
-    const uint32_t shift = 56 - 8 * (uint32_t)(__clzll(sg.diff) >> 3);
-    const uint32_t m = sg.nspl;
-    // plain keys split on their top differing bits, pivot pseudo keys on a byte
-    const bool bits = BITS && !m && !(sg.flags & (F_PIVOT | F_PSEUDO)) && use_bits(S.bits, sg.diff, shift, sg.size, S.small_max, S.first);
-    const BitDigit bd = bit_digit_spec(bits ? (uint64_t)sg.diff : (0xFFull << shift));
-    __shared__ BitTables bt;
-    if (BITS && !bd.whole) bit_tables_build(bt, bd);
-    const unsigned long long* key = S.key[sg.flags & F_PARITY];
-#pragma unroll
-    for (int w = 0; w < LT_NT / 32; ++w) hist[w][threadIdx.x] = 0;
-    if (m)
-        for (uint32_t q = threadIdx.x; q < SPL_STRIDE; q += LT_NT) s_spl[q] = S.spl[(uint64_t)sg.spl_slot * SPL_STRIDE + q];
-    __syncthreads();
-    const uint32_t tb = sg.start + (t - S.tile0[si]) * LT_TILE;
-    const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
-    uint32_t* wh = hist[threadIdx.x >> 5];
-    // the tile's keys loaded before any is counted (one DRAM wait, not LT_IPT)
+    const Seg& sg = segs[si];
+    const uint64_t diff = sg.diff;
+    if (diff == 0) return;
+    const uint32_t start = sg.start, size = sg.size, flags = sg.flags;
+    const uint32_t tb = start + (t - S.tile0[si]) * LT_TILE;
+    const uint32_t te = min(start + size, tb + LT_TILE);
+    const unsigned long long* key = S.key[flags & F_PARITY];
+    // the tile's keys loaded before the digit is known (one DRAM wait)
     uint64_t k[LT_IPT];
 #pragma unroll
     for (int j = 0; j < LT_IPT; ++j) {
         const uint32_t i = tb + j * LT_NT + threadIdx.x;
         k[j] = i < te ? key[i] : 0;
     }
+    if (threadIdx.x == 0) segment_digit(B, diff, flags, size);
 #pragma unroll
-    for (int j = 0; j < LT_IPT; ++j) {
-        const uint32_t i = tb + j * LT_NT + threadIdx.x;
-        if (i < te)
-            atomicAdd(&wh[m ? spl_bucket(s_spl, m, k[j]) : BITS ? bit_digit(k[j], bd, bt) : digit_of(k[j], shift)], 1u);
-    }
+    for (int w = 0; w < LT_NT / 32; ++w) hist[w][threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t d[LT_IPT];
+    digits_of(B, k, d);
+    uint32_t* wh = hist[threadIdx.x >> 5];
+#pragma unroll
+    for (int j = 0; j < LT_IPT; ++j)
+        if (tb + j * LT_NT + threadIdx.x < te) atomicAdd(&wh[d[j]], 1u);
     __syncthreads();
     uint32_t c = 0;
 #pragma unroll
     for (int w = 0; w < LT_NT / 32; ++w) c += hist[w][threadIdx.x];
-    S.tile_hist[(uint64_t)t * 256 + threadIdx.x] = c;
-}
-
-// ------------------------------------------------------------ chunk sums ----
-__global__ void k_chunk_sum(SortState S, const Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
-    const uint32_t c = blockIdx.x;
-    if (c >= S.counters[9]) return;
-    const uint32_t si = find_seg(S.chunk0, nseg, c);
-    const Seg sg = segs[si];
-    if (sg.diff == 0) return;
-    const uint32_t ntiles = (sg.size + LT_TILE - 1) / LT_TILE;
-    const uint32_t t0 = S.tile0[si] + (c - S.chunk0[si]) * CHUNK_TILES;
-    const uint32_t t1 = min(S.tile0[si] + ntiles, t0 + CHUNK_TILES);
-    // each tile's count becomes its exclusive prefix inside the chunk (one
-    // read for the scatter instead of the chunk's earlier tiles); every load
-    // of the chunk in flight before the first store
-    uint32_t v[CHUNK_TILES];
-#pragma unroll
-    for (int q = 0; q < CHUNK_TILES; ++q)
-        v[q] = t0 + q < t1 ? S.tile_hist[(uint64_t)(t0 + q) * 256 + threadIdx.x] : 0u;
-    uint32_t s = 0;
-#pragma unroll
-    for (int q = 0; q < CHUNK_TILES; ++q) {
-        if (t0 + q < t1) S.tile_hist[(uint64_t)(t0 + q) * 256 + threadIdx.x] = s;
-        s += v[q];
-    }
-    S.chunk_pre[(uint64_t)c * 256 + threadIdx.x] = s;
+    if (c) atomicAdd(&S.hist[(uint64_t)si * 256 + threadIdx.x], c);
 }
 
 // ----------------------------------------------------------- segment scan ----
-__global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, uint32_t nseg, Seg* next) {
-    __shared__ uint32_t sh[32];
-    __shared__ uint32_t s_first;
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        const uint32_t c = S.counters[12];
-        segs = S.large[c];
-        next = S.large[c ^ 1u];
-        nseg = S.counters[13];
-    }
+// One block per segment: bucket starts, the LCPs at bucket starts, and the
+// segment's children.
+__global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, Seg* next) {
+    __shared__ uint32_t wsum[8], wany[8];
+    __shared__ BucketBits B;
     const uint32_t si = blockIdx.x;
-    if (si >= nseg) return;
     Seg& sg = segs[si];
-    const uint32_t par = sg.flags & F_PARITY;
-    const bool pseudo = (sg.flags & (F_PIVOT | F_PSEUDO)) != 0;
-    const uint32_t depth = (sg.flags & (F_KEYS | F_PIVOT)) ? sg.depth : sg.newdepth;
+    const uint32_t start = sg.start, size = sg.size, flags = sg.flags, par = flags & F_PARITY, np = par ^ 1u;
+    const uint64_t diff = sg.diff;
+    const bool pseudo = (flags & (F_PIVOT | F_PSEUDO)) != 0, by_id = (flags & F_ID) != 0;
+    const uint32_t depth = (flags & (F_KEYS | F_PIVOT | F_ID)) ? sg.depth : sg.newdepth;
+    const uint64_t k0 = S.key[par][start];
     const uint32_t d = threadIdx.x;
-    if (sg.diff == 0) {
+    if (diff == 0) {
         // Every key equal: byte-identical strings if the key holds their end,
         // else continue deeper without keys.
-        const uint64_t k0 = S.key[par][sg.start];
-        const uint32_t* ord = S.ord[par];
+        if (d != 0) return;
         uint32_t fin = 0xFFFFFFFFu, cont = 0, cflags = par;
         if (pseudo) {
             const uint32_t code = (uint32_t)(k0 >> 56), byte = (uint32_t)(k0 >> 48) & 0xFFu;
             if (code == PIVOT_CAP) {
                 uint64_t o0;
                 uint32_t l0;
-                str_of(S.a, ord[sg.start], o0, l0);
+                str_of(S.a, ord_of(S, par, start), o0, l0);
                 if (l0 < depth + PIVOT_CAP) fin = l0;  // all equal the pivot
                 else cont = depth + PIVOT_CAP;
             } else if (byte == 0) {
@@ -1019,319 +768,210 @@ __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, uint32
             if (z < 8) fin = depth + z;
             else cont = depth + 8;
         }
-        if (fin != 0xFFFFFFFFu) {
-            for (uint32_t i = threadIdx.x; i < sg.size; i += blockDim.x) {
-                S.ord_out[sg.start + i] = ord[sg.start + i];
-                if (i) S.lcp_out[sg.start + i] = fin;
-            }
-        } else if (threadIdx.x == 0) {
-            push_large(S, next, sg.start, sg.size, cont, cflags);
-        }
+        if (fin != 0xFFFFFFFFu) push_large(S, next, start, size, fin, par | F_ID);
+        else push_large(S, next, start, size, cont, cflags);
         return;
     }
-    const uint32_t b = (uint32_t)(__clzll(sg.diff) >> 3);
-    const uint32_t c0 = S.chunk0[si];
-    const uint32_t ntiles = (sg.size + LT_TILE - 1) / LT_TILE;
-    const uint32_t nch = (ntiles + CHUNK_TILES - 1) / CHUNK_TILES;
-    // the digit's column of chunk sums, eight loads in flight (a segment of
-    // n strings has n / 64 Ki chunks, walked by one block)
-    uint32_t run = 0;
-    for (uint32_t c = 0; c < nch; c += 8) {
-        uint32_t v[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = c + q < nch ? S.chunk_pre[(uint64_t)(c0 + c + q) * 256 + d] : 0u;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            if (c + q < nch) S.chunk_pre[(uint64_t)(c0 + c + q) * 256 + d] = run;
-            run += v[q];
-        }
-    }
-    const uint32_t total = run;
-    // block exclusive scan over the 256 digits
+    const uint32_t total = S.hist[(uint64_t)si * 256 + d];
+    S.hist[(uint64_t)si * 256 + d] = 0;
+    if (d == 0) segment_digit(B, diff, flags, size);
+    // block exclusive scan over the 256 digits, and the digits that occur
     const int lane = d & 31, w = d >> 5;
     uint32_t x = total;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    if (lane == 31) sh[w] = x;
-    if (d == 0) s_first = 256;
+    const uint32_t any = __ballot_sync(0xffffffffu, total != 0);
+    if (lane == 31) wsum[w] = x;
+    if (lane == 0) wany[w] = any;
     __syncthreads();
-    uint32_t wb = 0;
-    for (int k = 0; k < w; ++k) wb += sh[k];
-    const uint32_t excl = wb + x - total;
-    if (total) atomicMin(&s_first, d);
-    uint32_t* bk = S.bucket + (uint64_t)si * 257;
-    bk[d] = sg.start + excl;
-    if (d == 255) bk[256] = sg.start + sg.size;
-    __syncthreads();
+    uint32_t excl = x - total;
+    for (int k = 0; k < w; ++k) excl += wsum[k];
+    const uint32_t cs = start + excl;
+    S.bucket[(uint64_t)si * 257 + d] = cs;
+    if (d == 255) S.bucket[(uint64_t)si * 257 + 256] = start + size;
+    S.cursor[(uint64_t)si * 256 + d] = cs;
+    // byte b is the first that may differ; bucket 0 holds the strings that end
+    // there if that byte's differing bits are all in the digit and it has no
+    // constant nonzero part
+    const uint32_t b = (uint32_t)(__clzll(diff) >> 3), shift = 56 - 8 * b;
+    const uint64_t mask = digit_mask(B), rest = diff & ~mask;
+    const bool plain = !pseudo && !by_id, code_split = pseudo && b == 0;
+    const bool ended = plain ? (((k0 >> shift) & ~(diff >> shift)) & 0xFFu) == 0 && ((rest >> shift) & 0xFFu) == 0
+                             : pseudo && !code_split;
+    const uint32_t lcp_here = pseudo ? depth + pivot_l((uint32_t)(k0 >> 56)) : depth + b;
     if (d == 0) {
-        sg.first_digit = s_first;
-        sg.depth = depth;
+        sg.bits = B;
+        sg.ended = ended;
     }
-    uint32_t* child = S.child ? S.child + (uint64_t)si * 256 + d : nullptr;
-    if (child) *child = 0xFFFFFFFFu;  // set below for a large child that keeps the keys
+    if (total == 0) return;
+    if (cs != start) {
+        // LCP with the bucket before (the last smaller digit that occurs)
+        uint32_t m = any & ((1u << lane) - 1u);
+        int pw = w;
+        while (m == 0) m = wany[--pw];
+        const uint32_t pd = (uint32_t)pw * 32 + 31u - (uint32_t)__clz(m);
+        uint32_t l = lcp_here;
+        if (by_id) {
+            l = depth;
+        } else if (code_split) {
+            l = depth + min(pivot_l(d), pivot_l(pd));
+        } else if (plain) {
+            // the byte of the highest bit in which the two digits differ
+            const uint32_t h = 31u - (uint32_t)__clz(d ^ pd);
+            for (uint32_t r = 0; r < B.nruns; ++r)
+                if ((B.mask[r] >> h) & 1u) l = depth + ((63u - (B.lo + B.sh[r] + h)) >> 3);
+        }
+        S.lcp_out[cs] = l;
+    }
     if (total < 2) return;
-    const uint32_t cs = sg.start + excl;
-    const uint32_t np = par ^ 1u;
-    if (sg.nspl) {
-        // splitter buckets: children keep the keys at this depth (an
-        // equality bucket's keys are all equal: its next pass goes deeper)
-        if (total > S.small_max) {
-            const uint32_t slot = push_large(S, next, cs, total, depth, np | F_KEYS);
-            if (child) *child = slot;
-        } else {
-            push_small(S, cs, total, depth, np | F_KEYS);
-        }
-    } else if (!pseudo) {
-        // digit 0 holds the strings that end at byte b, unless byte b has a
-        // constant nonzero part (then no string ends there and digit 0 is an
-        // ordinary bucket)
-        bool ended_ok = true;
-        if (S.bits) {
-            const uint32_t shift = 56 - 8 * b;
-            const uint64_t k0 = S.key[par][sg.start];
-            ended_ok = (((k0 >> shift) & 0xFFu) & ~((sg.diff >> shift) & 0xFFu)) == 0;
-        }
-        if (d == 0 && ended_ok) return;  // strings that end here: written by the scatter
-        // children keep the parent's keys: their first b+1 key bytes are now
-        // common; one that keeps most of the parent gets a pivot pass
-        if (total > S.small_max) {
-            if (S.pivot && 2 * (uint64_t)total > sg.size) {
-                push_large(S, next, cs, total, depth + b + 1, np | F_PIVOT);
-            } else {
-                const uint32_t slot = push_large(S, next, cs, total, depth, np | F_KEYS);
-                if (child) *child = slot;
-            }
-        } else {
-            push_small(S, cs, total, depth, np | F_KEYS);
-        }
-    } else if (b == 0) {
-        // split by pivot code (only the pivot pass's own segment): large children keep the pseudo keys, small
-        // ones restart from the depth their strings share
-        if (total > S.small_max) {
-            const uint32_t slot = push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO);
-            if (child) *child = slot;
+    const bool big = total > S.small_max;
+    const bool chain = S.pivot && 2 * (uint64_t)total > size;
+    if (by_id) {
+        if (big) push_large(S, next, cs, total, depth, np | F_KEYS | F_ID, rest);
+        else push_small(S, cs, total, depth, np | F_ID);
+    } else if (ended && d == 0) {
+        // equal strings (they may end before byte b when no key differs at
+        // all): the scatter makes their ids the keys
+        const uint32_t fin = plain ? depth + min(b, zero_byte(k0)) : lcp_here;
+        if (big) push_large(S, next, cs, total, fin, np | F_KEYS | F_ID,
+                            (2ull << (63 - __clzll(max(S.n, S.a.n)))) - 1);
+        else push_small(S, cs, total, fin, np | F_ID);
+    } else if (plain) {
+        // children keep the parent's keys, whose bits down to the digit's
+        // lowest are now common; one that keeps most of the parent gets a
+        // pivot pass
+        if (!big) push_small(S, cs, total, depth, np | F_KEYS);
+        else if (chain) push_large(S, next, cs, total, depth + ((64u - B.lo) >> 3), np | F_PIVOT);
+        else push_large(S, next, cs, total, depth, np | F_KEYS, rest);
+    } else if (code_split) {
+        // split by pivot code (only the pivot pass's own segment): large
+        // children keep the pseudo keys, small ones restart from the depth
+        // their strings share
+        if (big) {
+            // (the code of the pivot itself has no byte behind it)
+            push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO, d == PIVOT_CAP ? 0 : rest & ~(0xFFull << 56));
         } else {
             uint32_t cd = depth + pivot_l(d);
             if (d == PIVOT_CAP) {
                 uint64_t o0;
                 uint32_t l0;
-                str_of(S.a, sg.piv == NO_PIVOT ? S.ord[par][sg.start] : sg.piv, o0, l0);
+                str_of(S.a, sg.piv == NO_PIVOT ? ord_of(S, par, start) : sg.piv, o0, l0);
                 cd = min(depth + PIVOT_CAP, l0);
             }
             push_small(S, cs, total, cd, np);
         }
     } else {
-        // split by the byte after the shared d + l bytes; byte 0: strings that
-        // end there, written by the scatter
-        if (d == 0) return;
-        const uint32_t cd = depth + pivot_l((uint32_t)(S.key[par][sg.start] >> 56)) + 1;
-        if (total > S.small_max) push_large(S, next, cs, total, cd, np | (S.pivot && 2 * (uint64_t)total > sg.size ? F_PIVOT : 0u));
+        // split by the byte after the shared d + l bytes
+        const uint32_t cd = lcp_here + 1;
+        if (big) push_large(S, next, cs, total, cd, np | (chain ? F_PIVOT : 0u));
         else push_small(S, cs, total, cd, np);
     }
 }
 
 // --------------------------------------------------------------- scatter ----
-// Ranks are stable within the tile (warp-aggregated per digit); the tile is
-// first reordered by digit in shared memory so that the global writes of each
-// digit's run are contiguous.
-constexpr size_t SCATTER_SMEM = (size_t)LT_TILE * (8 + 4 + 1);
+// The tile is reordered by digit in shared memory, places from shared
+// atomics, so that the global writes of each digit's run are contiguous; one
+// global atomic per digit reserves the run's place in its bucket.  Bound by
+// the 24 bytes moved per key and the shared-memory round trip; with stable
+// ranks from match instructions, per-tile counts and their scans, and keys
+// folded for the children, a pass over 32e6 keys took 0.31 ms; now 0.15 to
+// 0.19 ms.
+constexpr int SC_NT = 512, SC_IPT = LT_TILE / SC_NT;
+constexpr size_t SCATTER_SMEM = (size_t)LT_TILE * (8 + 4 + 2);
 
-__global__ void __launch_bounds__(LT_NT, 4) k_scatter(SortState S, const Seg* segs, uint32_t nseg) {
-    if (!segs) {  // graph mode: this pass's list and count live on the device
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
+__global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* segs, uint32_t nseg) {
     extern __shared__ __align__(16) unsigned char sm_scatter[];
     unsigned long long* skey = (unsigned long long*)sm_scatter;
     uint32_t* sord = (uint32_t*)(skey + LT_TILE);
-    uint8_t* sdig = (uint8_t*)(sord + LT_TILE);
-    __shared__ uint32_t base[256];
-    __shared__ uint32_t bstart[257];
-    __shared__ uint32_t tloff[256];
-    __shared__ uint32_t wcnt[LT_NT / 32][256];
-    __shared__ uint32_t wsum[LT_NT / 32];
-    __shared__ uint32_t schild[256];
-    __shared__ uint32_t actm[LT_NT / 32];  // per warp: the digits (d & 7 == warp) whose keys it folds
-    __shared__ unsigned long long s_spl[SPL_STRIDE];
+    uint16_t* sdig = (uint16_t*)(sord + LT_TILE);
+    __shared__ uint32_t cnt[256], tloff[256], wsum[8];
+    __shared__ uint2 dst[256];  // place of the digit's run minus its place in the tile; whether its bucket is one string
+    __shared__ BucketBits B;
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
-    const Seg sg = segs[si];
-    if (sg.diff == 0) return;
-    const uint32_t par = sg.flags & F_PARITY;
-    const uint32_t b = (uint32_t)(__clzll(sg.diff) >> 3);
-    const uint32_t shift = 56 - 8 * b;
-    const uint32_t depth = sg.depth;
-    const uint32_t m = sg.nspl;  // splitter buckets (0: the byte digit)
-    const bool pseudo = (sg.flags & (F_PIVOT | F_PSEUDO)) != 0;
-    // plain keys split on their top differing bits, pivot pseudo keys on a byte
-    const bool bits = S.bits && !m && !pseudo && use_bits(S.bits, sg.diff, shift, sg.size, S.small_max, S.first);
-    const BitDigit bd = bit_digit_spec(bits ? (uint64_t)sg.diff : (0xFFull << shift));
-    __shared__ BitTables bt;
-    if (!bd.whole) bit_tables_build(bt, bd);  // the barrier after the block's set-up follows
-    // digit 0 holds the strings that end at byte b unless byte b has a
-    // constant nonzero part
-    bool ended_ok = true;
-    if (bits) {
-        const uint64_t k0 = S.key[par][sg.start];
-        ended_ok = (((k0 >> shift) & 0xFFu) & ~((sg.diff >> shift) & 0xFFu)) == 0;
-    }
-    // LCP inside the group of strings that end here and at bucket starts
-    // (pivot code splits: d + min(l, l') from the two codes)
-    const bool code_split = pseudo && b == 0;
-    const uint32_t lcp_here = pseudo ? depth + pivot_l((uint32_t)(S.key[par][sg.start] >> 56)) : depth + b;
-    const uint32_t tloc = t - S.tile0[si];
-    const uint32_t c = S.chunk0[si] + tloc / CHUNK_TILES;
-    {
-        const uint32_t d = threadIdx.x;
-        const uint32_t* bk = S.bucket + (uint64_t)si * 257;
-        // k_chunk_sum left the tile's prefix inside its chunk in tile_hist
-        base[d] = bk[d] + S.chunk_pre[(uint64_t)c * 256 + d] + S.tile_hist[(uint64_t)t * 256 + d];
-        bstart[d] = bk[d];
-        if (d == 0) bstart[256] = bk[256];
-        if (S.child) schild[d] = S.child[(uint64_t)si * 256 + d];
-        if (d < LT_NT / 32) actm[d] = 0;
-#pragma unroll
-        for (int w = 0; w < LT_NT / 32; ++w) wcnt[w][d] = 0;
-        if (m)
-            for (uint32_t q = d; q < SPL_STRIDE; q += LT_NT) s_spl[q] = S.spl[(uint64_t)sg.spl_slot * SPL_STRIDE + q];
-    }
-    __syncthreads();
-    const uint32_t* ord = S.ord[par];
-    const unsigned long long* key = S.key[par];
-    uint32_t* ord_dst = S.ord[par ^ 1u];
-    unsigned long long* key_dst = S.key[par ^ 1u];
-    const uint32_t tb = sg.start + tloc * LT_TILE;
-    const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
+    const Seg& sg = segs[si];
+    const uint32_t start = sg.start, end = start + sg.size, flags = sg.flags, par = flags & F_PARITY;
+    const uint32_t tb = start + (t - S.tile0[si]) * LT_TILE;
+    const uint32_t te = min(end, tb + LT_TILE);
     const uint32_t tn = te - tb;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t wb = tb + (uint32_t)w * 32 * LT_IPT;
-    uint64_t k[LT_IPT];
-    uint32_t o[LT_IPT];
-    uint32_t rk[LT_IPT];
+    if (sg.diff == 0) {  // the segment stays where it is (its ids must exist)
+        if (S.iota)
+            for (uint32_t i = tb + threadIdx.x; i < te; i += SC_NT) S.ord[par][i] = i;
+        return;
+    }
+    const unsigned long long* key = S.key[par];
+    uint64_t k[SC_IPT];
+    uint32_t o[SC_IPT];
 #pragma unroll
-    for (int j = 0; j < LT_IPT; ++j) {
-        const uint32_t i = wb + j * 32 + lane;
+    for (int j = 0; j < SC_IPT; ++j) {
+        const uint32_t i = tb + j * SC_NT + threadIdx.x;
         k[j] = i < te ? key[i] : 0;
-        o[j] = i < te ? ord[i] : 0;
+        o[j] = i < te ? ord_of(S, par, i) : 0;
     }
-#pragma unroll
-    for (int j = 0; j < LT_IPT; ++j) {
-        const uint32_t i = wb + j * 32 + lane;
-        const uint32_t dg = i < te ? (m ? spl_bucket(s_spl, m, k[j]) : bit_digit(k[j], bd, bt)) : 0x100u + lane;
-        const uint32_t peers = __match_any_sync(0xffffffffu, dg);
-        const uint32_t r = __popc(peers & ((1u << lane) - 1));
-        const uint32_t prev = dg < 256 ? wcnt[w][dg] : 0;
-        __syncwarp();
-        if (dg < 256 && lane == __ffs(peers) - 1) wcnt[w][dg] = prev + __popc(peers);
-        __syncwarp();
-        rk[j] = (dg & 0xFFu) << 24 | (prev + r);  // the digit kept for the placement below
-    }
+    if (threadIdx.x < sizeof(BucketBits) / 4) ((uint32_t*)&B)[threadIdx.x] = ((const uint32_t*)&sg.bits)[threadIdx.x];
+    const bool ended = sg.ended;
+    if (threadIdx.x < 256) cnt[threadIdx.x] = 0;
     __syncthreads();
-    {
-        // exclusive over warps per digit, then over digits within the tile
-        const uint32_t d = threadIdx.x;
-        uint32_t run = 0;
+    uint32_t d[SC_IPT];
+    digits_of(B, k, d);
 #pragma unroll
-        for (int ww = 0; ww < LT_NT / 32; ++ww) {
-            const uint32_t v = wcnt[ww][d];
-            wcnt[ww][d] = run;
-            run += v;
-        }
-        uint32_t x = run;
+    for (int j = 0; j < SC_IPT; ++j)
+        if (tb + j * SC_NT + threadIdx.x < te) d[j] |= atomicAdd(&cnt[d[j]], 1u) << 8;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t c = 0, x = 0;
+    if (threadIdx.x < 256) {
+        c = cnt[threadIdx.x];
+        x = c;
 #pragma unroll
         for (int off = 1; off < 32; off <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
             if (lane >= off) x += y;
         }
         if (lane == 31) wsum[w] = x;
-        __syncthreads();
-        uint32_t wpre = 0;
-        for (int ww = 0; ww < w; ++ww) wpre += wsum[ww];
-        tloff[d] = wpre + x - run;
-        if (S.child && run && schild[d] < S.cap_large) atomicOr(&actm[d & 7], 1u << (d >> 3));
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+        uint32_t at = x - c;
+        for (int ww = 0; ww < w; ++ww) at += wsum[ww];
+        tloff[threadIdx.x] = at;
+        const uint32_t* bk = S.bucket + (uint64_t)si * 257 + threadIdx.x;
+        const uint32_t base = c ? atomicAdd(&S.cursor[(uint64_t)si * 256 + threadIdx.x], c) : 0u;
+        dst[threadIdx.x] = make_uint2(base - at, bk[1] - bk[0] == 1);
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < LT_IPT; ++j) {
-        const uint32_t i = wb + j * 32 + lane;
-        if (i >= te) continue;
-        const uint32_t dg = rk[j] >> 24;
-        const uint32_t lp = tloff[dg] + wcnt[w][dg] + (rk[j] & 0xFFFFFFu);
-        if (lp >= tn) {  // never taken when the counts agree
-            atomicExch(&S.counters[10], 1u);
-            continue;
-        }
-        skey[lp] = k[j];
+    for (int j = 0; j < SC_IPT; ++j) {
+        if (tb + j * SC_NT + threadIdx.x >= te) continue;
+        const uint32_t dg = d[j] & 0xFFu, lp = tloff[dg] + (d[j] >> 8);
+        skey[lp] = ended && dg == 0 ? (uint64_t)o[j] : k[j];  // equal strings go on by id
         sord[lp] = o[j];
-        sdig[lp] = (uint8_t)dg;
+        sdig[lp] = (uint16_t)dg;
     }
     __syncthreads();
-    if (S.child) {
-        // the OR and AND of the keys each large child that keeps them gets
-        // from this tile (one warp per digit, over the digit's run in shared
-        // memory): its next pass needs no key read to find the byte where its
-        // keys differ
-        for (uint32_t m = actm[w]; m; m &= m - 1) {
-            const uint32_t dg = ((uint32_t)(__ffs(m) - 1) << 3) | (uint32_t)w;
-            const uint32_t r0 = tloff[dg], r1 = dg < 255 ? tloff[dg + 1] : tn;
-            unsigned long long vo = 0, va = ~0ull;
-            for (uint32_t x = r0 + lane; x < r1; x += 32) {
-                const unsigned long long v = skey[x];
-                vo |= v;
-                va &= v;
-            }
-            const uint32_t olo = __reduce_or_sync(0xffffffffu, (uint32_t)vo);
-            const uint32_t ohi = __reduce_or_sync(0xffffffffu, (uint32_t)(vo >> 32));
-            const uint32_t alo = __reduce_and_sync(0xffffffffu, (uint32_t)va);
-            const uint32_t ahi = __reduce_and_sync(0xffffffffu, (uint32_t)(va >> 32));
-            if (lane == 0) {
-                const uint32_t slot = schild[dg];
-                atomicOr(&S.nxt[slot].kor, ((unsigned long long)ohi << 32) | olo);
-                atomicAnd(&S.nxt[slot].kand, ((unsigned long long)ahi << 32) | alo);
-            }
-        }
-    }
-    for (uint32_t x = threadIdx.x; x < tn; x += LT_NT) {
-        const uint32_t dg = sdig[x];
-        const uint32_t dest = base[dg] + (x - tloff[dg]);
-        const uint32_t bs = bstart[dg], cnt = bstart[dg + 1] - bs;
-        if (dest < bs || dest >= bs + cnt) {  // never taken when the counts agree
+    uint32_t* ord_dst = S.ord[par ^ 1u];
+    unsigned long long* key_dst = S.key[par ^ 1u];
+    for (uint32_t i = threadIdx.x; i < tn; i += SC_NT) {
+        const uint2 to = dst[sdig[i]];
+        const uint32_t at = to.x + i;
+        if (at < start || at >= end) {  // never taken when the counts agree
             atomicExch(&S.counters[10], 1u);
             continue;
         }
-        const uint32_t oo = sord[x];
-        const bool ended = !m && dg == 0 && !code_split && ended_ok;
-        if (ended || cnt == 1) {
-            S.ord_out[dest] = oo;
-            if (ended && dest != bs) S.lcp_out[dest] = lcp_here;
+        const uint32_t oo = sord[i];
+        if (to.y) {
+            S.ord_out[at] = oo;
         } else {
-            ord_dst[dest] = oo;
-            key_dst[dest] = skey[x];
-        }
-        if (m) {
-            // a splitter bucket's start: its LCP once the order is final
-            if (dest == bs && dg != sg.first_digit) {
-                S.fix[2 * ((uint64_t)sg.fix0 + dg)] = dest;
-                S.fix[2 * ((uint64_t)sg.fix0 + dg) + 1] = depth;
-            }
-        } else if (dest == bs && dg != sg.first_digit) {
-            uint32_t l = lcp_here;
-            if (code_split || !bd.whole) {
-                uint32_t pd = dg - 1;  // previous non-empty bucket (exists: dg is not the first)
-                while (pd > 0 && bstart[pd] == bs) --pd;
-                // pivot codes: d + min(l, l'); bit digits: the byte of the
-                // highest bit in which the two buckets' digits differ
-                l = code_split ? depth + min(pivot_l(dg), pivot_l(pd))
-                               : depth + bit_digit_byte(bd, 31u - (uint32_t)__clz(dg ^ pd));
-            }
-            S.lcp_out[dest] = l;
+            ord_dst[at] = oo;
+            key_dst[at] = skey[i];
         }
     }
 }
+
 
 // ------------------------------------------------------------ small sort ----
 // Segments of 2..small_max strings finish inside one CTA (the tail the MSD
@@ -1573,68 +1213,20 @@ __device__ __forceinline__ void warp_group(const ArenaDev& a, uint32_t size, uin
 }
 
 // Segments of 2..32 strings: one warp each, four per CTA.
-// dcount (graph mode): the segment count on the device; blocks stride over it.
-__global__ void __launch_bounds__(128) k_warp_segs(SortState S, const Seg* segs, uint32_t nseg, const uint32_t* dcount) {
-    if (dcount) nseg = *dcount;
+__global__ void __launch_bounds__(128) k_warp_segs(SortState S, const SmallSeg* segs, uint32_t nseg) {
     for (uint32_t si = blockIdx.x * 4 + (threadIdx.x >> 5); si < nseg; si += gridDim.x * 4) {
         const uint32_t lane = threadIdx.x & 31;
-        const Seg seg = segs[si];
+        const SmallSeg seg = segs[si];
         const uint32_t* src = S.ord[seg.flags & F_PARITY];
         uint32_t id = 0;
         uint64_t key = 0;
         if (lane < seg.size) {
             id = src[seg.start + lane];
-            key = (seg.flags & F_KEYS) ? S.key[seg.flags & F_PARITY][seg.start + lane] : key8_of(S.a, id, seg.depth);
+            if (seg.flags & F_ID) key = 0;
+            else key = (seg.flags & F_KEYS) ? S.key[seg.flags & F_PARITY][seg.start + lane] : key8_of(S.a, id, seg.depth);
         }
-        warp_group(S.a, seg.size, seg.depth, G_PLAIN, key, id, S.lcp_out + seg.start);
+        warp_group(S.a, seg.size, seg.depth, (seg.flags & F_ID) ? G_ID : G_PLAIN, key, id, S.lcp_out + seg.start);
         if (lane < seg.size) S.ord_out[seg.start + lane] = id;
-    }
-}
-
-// The bits that pick a bucket: up to `want` of the most significant bits of
-// diff, in at most 8 runs of neighbouring bits.  A key's bucket is the OR over
-// the runs of ((key >> lo) >> sh) & mask; every bit above lo that is not
-// chosen is the same in all keys, so buckets order as keys do.
-// In a pseudo group whose code bits are all chosen, a bucket holds one code;
-// otherwise (LCPs over thousands of bytes) `mixed` is set.
-struct BucketBits {
-    uint32_t lo, nruns, wide, all;  // wide: the bits span more than 32; all: every differing bit is chosen
-    uint32_t mixed;
-    uint32_t sh[8], mask[8];
-};
-
-__device__ __forceinline__ uint32_t bucket_of_key(const BucketBits& B, uint64_t k) {
-    uint32_t b = 0;
-    for (uint32_t r = 0; r < B.nruns; ++r) b |= (uint32_t)(k >> (B.lo + B.sh[r])) & B.mask[r];
-    return b;
-}
-
-__device__ __forceinline__ void bucket_bits(BucketBits& B, uint64_t diff, uint32_t want) {
-    uint32_t n = 0, left = want, lo = 0;
-    uint64_t x = diff;
-    const uint32_t hi = 63u - (uint32_t)__clzll(diff);
-    // a run's lowest bit and length, for the second loop
-    do {
-        const uint32_t h = 63u - (uint32_t)__clzll(x);
-        const uint32_t take = min((uint32_t)__clzll(~(x << (63u - h))), left);  // set bits from h down
-        lo = h - take + 1;
-        B.sh[n] = lo;
-        B.mask[n] = (1u << take) - 1u;
-        left -= take;
-        x &= (1ull << lo) - 1;
-        ++n;
-    } while (x && n < 8 && left);
-    B.lo = lo;
-    B.nruns = n;
-    B.wide = hi - lo >= 32;
-    B.all = x == 0;
-    B.mixed = (x >> 48) != 0;
-    uint32_t place = 0;
-    for (uint32_t k = n; k-- > 0;) {
-        const uint32_t m = B.mask[k];
-        B.sh[k] = B.sh[k] - lo - place;
-        B.mask[k] = m << place;
-        place += (uint32_t)__popc(m);
     }
 }
 
@@ -1659,9 +1251,9 @@ struct SegSmem {
 };
 
 template <int CAP, int NT>
-__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_seg_sort(SortState S, const Seg* segs,
-                                                                                       uint32_t nseg,
-                                                                                       const uint32_t* dcount) {
+__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_seg_sort(SortState S,
+                                                                                       const SmallSeg* segs,
+                                                                                       uint32_t nseg) {
     constexpr int NW = NT / 32, IPT = CAP / NT, NB = SegSmem<CAP>::NB, PER = NB / NT;
     extern __shared__ __align__(16) unsigned char smem[];
     SegSmem<CAP>& M = *reinterpret_cast<SegSmem<CAP>*>(smem);
@@ -1670,9 +1262,8 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
     __shared__ uint2 s_cur;
     __shared__ BucketBits s_bits;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (dcount) nseg = *dcount;
     for (uint32_t bi = blockIdx.x; bi < nseg; bi += gridDim.x) {
-        const Seg seg = segs[bi];
+        const SmallSeg seg = segs[bi];
         const uint32_t start = seg.start, size = seg.size;
         uint32_t* lcp = S.lcp_out + start;
         {
@@ -1686,7 +1277,7 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
                 o[j] = i < size ? src[i] : 0u;
                 k[j] = i < size && (seg.flags & F_KEYS) ? ksrc[i] : 0ull;
             }
-            if (!(seg.flags & F_KEYS)) {
+            if (!(seg.flags & (F_KEYS | F_ID))) {
 #pragma unroll
                 for (int j = 0; j < IPT; ++j)
                     if (threadIdx.x + j * NT < size) k[j] = key8_of(S.a, o[j], seg.depth);
@@ -1702,7 +1293,7 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
         }
         for (uint32_t x = threadIdx.x; x < NB; x += NT) M.cnt[x] = 0;
         if (threadIdx.x == 0) {
-            const uint2 g = group_pack(0, size, G_PLAIN, seg.depth);
+            const uint2 g = group_pack(0, size, (seg.flags & F_ID) ? G_ID : G_PLAIN, seg.depth);
             s_nw = size <= 32;
             s_ns = size > 32;
             s_nt = 0;
@@ -1990,194 +1581,53 @@ constexpr size_t seg_sort_smem() {
 }
 
 template <int CAP, int NT>
-static int launch_seg_sort(const SortState& S, const Seg* segs, uint32_t n, const char* name, cudaStream_t st) {
+static int launch_seg_sort(const SortState& S, const SmallSeg* segs, uint32_t n, const char* name, cudaStream_t st) {
     if (!n) return DSSS_OK;
     constexpr size_t shm = seg_sort_smem<CAP>();
     static std::atomic<uint64_t> configured{0};
     DSSS_TRY(set_smem_once(configured, k_seg_sort<CAP, NT>, (int)shm));
-    DSSS_LAUNCH(name, st, k_seg_sort<CAP, NT><<<n, NT, shm, st>>>(S, segs, n, nullptr));
+    DSSS_LAUNCH(name, st, k_seg_sort<CAP, NT><<<n, NT, shm, st>>>(S, segs, n));
     DSSS_CUDA(cudaGetLastError());
     return DSSS_OK;
 }
 
 
-// ------------------------------------------------------- graph mode ----
-// For n up to sort_graph_max_n (off by default) the MSD passes run as one CUDA graph: the pass
-// is the body of a conditional WHILE node, the number of large segments and
-// the parity of their list live on the device (counters[13], [12]), grids are
-// the layout's capacities (blocks past the real tiles exit), and a one-thread
-// kernel at the end of each pass sets the loop condition — no host round trip
-// per pass.  The small-segment sorters then stride over the device counts.
-
-// One block: per large segment its first tile and chunk (exclusive prefix
-// over the list), totals into counters[8], [9]; resets the next-list count.
-__global__ void __launch_bounds__(1024) k_seg_offsets(SortState S, Seg* segs, uint32_t nseg) {
-    __shared__ uint32_t st_[1024], sc_[1024];
-    if (!segs) {
-        segs = S.large[S.counters[12]];
-        nseg = S.counters[13];
-    }
+// ------------------------------------------------------------------ host ----
+// One block: per large segment its first tile (exclusive prefix over the
+// list), the total into counters[8]; resets the next list's counts.
+__global__ void __launch_bounds__(1024) k_seg_offsets(SortState S, const Seg* segs, uint32_t nseg) {
+    __shared__ uint32_t wsum[32];
     const uint32_t per = (nseg + 1023) / 1024;
     const uint32_t b = min(nseg, threadIdx.x * per), e = min(nseg, b + per);
-    uint32_t tt = 0, tc = 0;
-    for (uint32_t i = b; i < e; ++i) {
-        const uint32_t t = (segs[i].size + LT_TILE - 1) / LT_TILE;
-        tt += t;
-        tc += (t + CHUNK_TILES - 1) / CHUNK_TILES;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t tt = 0;
+    for (uint32_t i = b; i < e; ++i) tt += (segs[i].size + LT_TILE - 1) / LT_TILE;
+    uint32_t x = tt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
     }
-    st_[threadIdx.x] = tt;
-    sc_[threadIdx.x] = tc;
+    if (lane == 31) wsum[w] = x;
     __syncthreads();
-    for (int off = 1; off < 1024; off <<= 1) {
-        const uint32_t vt = threadIdx.x >= (unsigned)off ? st_[threadIdx.x - off] : 0;
-        const uint32_t vc = threadIdx.x >= (unsigned)off ? sc_[threadIdx.x - off] : 0;
-        __syncthreads();
-        st_[threadIdx.x] += vt;
-        sc_[threadIdx.x] += vc;
-        __syncthreads();
+    uint32_t rt = x - tt, total = 0;
+    for (int k = 0; k < 32; ++k) {
+        if (k < w) rt += wsum[k];
+        total += wsum[k];
     }
-    uint32_t rt = st_[threadIdx.x] - tt, rc = sc_[threadIdx.x] - tc;
     for (uint32_t i = b; i < e; ++i) {
-        const uint32_t t = (segs[i].size + LT_TILE - 1) / LT_TILE;
-        // keys folded by the previous scatter: the bits where they differ
-        if (S.child && (segs[i].flags & (F_KEYS | F_PIVOT)) == F_KEYS) segs[i].diff = segs[i].kor ^ segs[i].kand;
         S.tile0[i] = rt;
-        S.chunk0[i] = rc;
-        rt += t;
-        rc += (t + CHUNK_TILES - 1) / CHUNK_TILES;
+        rt += (segs[i].size + LT_TILE - 1) / LT_TILE;
     }
-    if (threadIdx.x == 1023) {
-        S.counters[8] = st_[1023];
-        S.counters[9] = sc_[1023];
-        if (st_[1023] > S.cap_tiles || sc_[1023] > S.cap_chunks) {
-            S.counters[8] = 0;  // nothing runs; the guard stops the loop
-            S.counters[9] = 0;
-            S.counters[10] = 1;
-        }
+    if (threadIdx.x == 0) {
+        const bool over = total > S.cap_tiles;
+        S.counters[8] = over ? 0u : total;  // nothing runs past the plan; the guard stops the loop
+        if (over) S.counters[10] = 1;
         S.counters[0] = 0;   // large segments of the next pass
         S.counters[11] = 0;  // of them, without keys or with a pivot pass
-        S.counters[6] = 0;   // splitter tables of this pass
     }
 }
 
-__global__ void k_loop_init(SortState S, cudaGraphConditionalHandle h) {
-    S.counters[12] = 0;
-    S.counters[13] = S.counters[0];
-    S.counters[14] = 0;
-    cudaGraphSetConditional(h, S.counters[13] > 0 ? 1u : 0u);
-}
-
-// Ends a pass: the next list becomes current; loop while it is not empty,
-// no guard tripped and the pass count stays sane.
-__global__ void k_pass_end(SortState S, cudaGraphConditionalHandle h) {
-    uint32_t next = S.counters[0];
-    if (next > S.cap_large) {
-        S.counters[10] = 1;
-        next = 0;
-    }
-    S.counters[12] ^= 1u;
-    S.counters[13] = next;
-    const uint32_t passes = ++S.counters[14];
-    if (passes > (1u << 20)) S.counters[10] = 1;
-    cudaGraphSetConditional(h, (next > 0 && S.counters[10] == 0) ? 1u : 0u);
-}
-
-// Two streams per host thread and device to capture on (the caller's stream
-// may be the legacy default stream, which cannot be captured); the graph is
-// then launched on the caller's stream.
-static int capture_streams(cudaStream_t* cap, cudaStream_t* body) {
-    constexpr int MAXDEV = 64;
-    thread_local cudaStream_t tl[MAXDEV][2] = {};
-    int dev = 0;
-    DSSS_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= MAXDEV) return fail(DSSS_ENOTSUP, "device %d out of range", dev);
-    for (int k = 0; k < 2; ++k)
-        if (!tl[dev][k]) DSSS_CUDA(cudaStreamCreateWithFlags(&tl[dev][k], cudaStreamNonBlocking));
-    *cap = tl[dev][0];
-    *body = tl[dev][1];
-    return DSSS_OK;
-}
-
-static int sort_strings_graph(const SortLayout& L, SortState S, uint64_t n, uint32_t p, const uint32_t* ids_in,
-                              uint32_t* pin, cudaStream_t run_st) {
-    cudaStream_t st = nullptr, bst = nullptr;
-    DSSS_TRY(capture_streams(&st, &bst));
-    struct Res {
-        cudaGraph_t g = nullptr;
-        cudaGraphExec_t x = nullptr;
-        ~Res() {
-            if (x) cudaGraphExecDestroy(x);
-            if (g) cudaGraphDestroy(g);
-        }
-    } res;
-    const unsigned tiles = (unsigned)L.cap_tiles, chunks = (unsigned)L.cap_chunks, large = (unsigned)L.cap_large;
-    DSSS_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(L.counters, 0, 16 * sizeof(uint32_t), st);
-    k_init_ids<<<grid_for(n, 256), 256, 0, st>>>(S.ord[0], ids_in, n);
-    k_init_segs<<<grid_for(p, 128), 128, 0, st>>>(S, L.pb, p);
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t g = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    cudaError_t e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &ndeps);
-    cudaGraphConditionalHandle h{};
-    if (e == cudaSuccess) e = cudaGraphConditionalHandleCreate(&h, g, 0, 0);
-    if (e == cudaSuccess) k_loop_init<<<1, 1, 0, st>>>(S, h);
-    if (e == cudaSuccess) e = cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &ndeps);
-    cudaGraphNodeParams np{};
-    np.type = cudaGraphNodeTypeConditional;
-    np.conditional.handle = h;
-    np.conditional.type = cudaGraphCondTypeWhile;
-    np.conditional.size = 1;
-    cudaGraphNode_t cond = nullptr;
-    if (e == cudaSuccess) e = cudaGraphAddNode(&cond, g, deps, ndeps, &np);
-    if (e == cudaSuccess) e = cudaStreamUpdateCaptureDependencies(st, &cond, 1, cudaStreamSetCaptureDependencies);
-    if (e == cudaSuccess) {
-        // the loop body: one MSD pass, captured on a second stream into the body graph
-        cudaGraph_t body = np.conditional.phGraph_out[0];
-        e = cudaStreamBeginCaptureToGraph(bst, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            k_seg_offsets<<<1, 1024, 0, bst>>>(S, nullptr, 0);
-            k_prefix<<<tiles, LT_NT, 0, bst>>>(S, nullptr, 0);
-            k_pivot<<<tiles, LT_NT, 0, bst>>>(S, nullptr, 0);
-            k_keys_diff<<<tiles, LT_NT, 0, bst>>>(S, nullptr, 0);
-            if (S.split_min) k_split_sample<<<148, SPL_SAMPLE / 2, 0, bst>>>(S, nullptr, 0);
-            if (S.bits) k_hist<true><<<tiles, LT_NT, 0, bst>>>(S, nullptr, 0);
-            else k_hist<false><<<tiles, LT_NT, 0, bst>>>(S, nullptr, 0);
-            k_chunk_sum<<<chunks, 256, 0, bst>>>(S, nullptr, 0);
-            k_seg_scan<<<large, 256, 0, bst>>>(S, nullptr, 0, nullptr);
-            k_scatter<<<tiles, LT_NT, SCATTER_SMEM, bst>>>(S, nullptr, 0);
-            k_pass_end<<<1, 1, 0, bst>>>(S, h);
-            cudaGraph_t got = nullptr;
-            e = cudaStreamEndCapture(bst, &got);
-        }
-    }
-    if (e == cudaSuccess) {
-        // small segments, striding over the device counts
-        k_warp_segs<<<148 * 8, 128, 0, st>>>(S, S.small[0], 0, S.counters + 1);
-        k_seg_sort<256, 128><<<148 * 8, 128, seg_sort_smem<256>(), st>>>(S, S.small[1], 0, S.counters + 2);
-        k_seg_sort<1024, 256><<<148 * 4, 256, seg_sort_smem<1024>(), st>>>(S, S.small[2], 0, S.counters + 3);
-        k_seg_sort<4096, 512><<<148 * 2, 512, seg_sort_smem<4096>(), st>>>(S, S.small[3], 0, S.counters + 4);
-        if (S.split_min) k_lcp_fix<<<148 * 4, 256, 0, st>>>(S);
-        cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
-    }
-    cudaGraph_t whole = nullptr;
-    const cudaError_t e2 = cudaStreamEndCapture(st, &whole);
-    res.g = whole;
-    if (e != cudaSuccess || e2 != cudaSuccess)
-        return fail(DSSS_EDEVICE, "string sort graph: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
-    DSSS_CUDA(cudaGraphInstantiate(&res.x, whole, 0));
-    {
-        StageTimer t("graph:sort", run_st);
-        DSSS_CUDA(cudaGraphLaunch(res.x, run_st));
-    }
-    DSSS_CUDA(cudaStreamSynchronize(run_st));
-    if (pin[10]) return fail(DSSS_EDEVICE, "string sort: internal consistency guard tripped");
-    return DSSS_OK;
-}
-
-// ------------------------------------------------------------------ host ----
-static Seg* large_list(const SortLayout& L, int k) { return (Seg*)L.large[k]; }
 static uint32_t clamp_small_max(uint32_t m) {
     if (m == 0) m = (uint32_t)tune(TUNE_SORT_SMALL_MAX);
     return (m == 0 || m > (uint32_t)bin_cap(NBINS - 1)) ? (uint32_t)bin_cap(NBINS - 1) : (m < 2 ? 2 : m);
@@ -2191,33 +1641,20 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
     L.key[0] = c.take<unsigned long long>(N);
     L.key[1] = c.take<unsigned long long>(N);
     L.cap_large = N / (small_max + 1) + p + 1;
-    L.cap_small = N / 2 + p + 1;
     L.cap_tiles = N / LT_TILE + L.cap_large + 1;
-    L.cap_chunks = L.cap_tiles / CHUNK_TILES + L.cap_large + 1;
     L.large[0] = c.take<unsigned char>(L.cap_large * sizeof(Seg));
     L.large[1] = c.take<unsigned char>(L.cap_large * sizeof(Seg));
-    for (int b = 0; b < NBINS; ++b) L.small[b] = c.take<unsigned char>(L.cap_small * sizeof(Seg));
+    for (int b = 0; b < NBINS; ++b) {
+        // segments of a bin are disjoint and larger than the bin below
+        L.cap_small[b] = N / (b ? bin_cap(b - 1) + 1 : 2) + p + 1;
+        L.small[b] = c.take<unsigned char>(L.cap_small[b] * sizeof(SmallSeg));
+    }
     L.tile0 = c.take<uint32_t>(L.cap_large);
-    L.chunk0 = c.take<uint32_t>(L.cap_large);
-    L.tmp_counts = c.take<uint32_t>(2 * L.cap_large);
-    L.tile_hist = c.take<uint32_t>(L.cap_tiles * 256);
-    L.chunk_pre = c.take<uint32_t>(L.cap_chunks * 256);
+    L.hist = c.take<uint32_t>(L.cap_large * 256);
     L.bucket = c.take<uint32_t>(L.cap_large * 257);
-    // the child table: 256 slots per large segment, about 4 bytes per string
-    // once large segments hold more than 256 strings (smaller cut-offs keep
-    // the per-pass key reads instead)
-    L.child = small_max >= 256 ? c.take<uint32_t>(L.cap_large * 256) : nullptr;
+    L.cursor = c.take<uint32_t>(L.cap_large * 256);
     L.counters = c.take<uint32_t>(16);
     L.pb = c.take<uint64_t>(p + 1);
-    L.scan = c.take<unsigned char>(scan_scratch_bytes(L.cap_large));
-    // splitter tables: segments of at least SPL_MIN_FLOOR strings per pass;
-    // fix list: (position, depth) pairs (when it runs short, passes keep the
-    // byte digit)
-    L.cap_spl = N / SPL_MIN_FLOOR + p + 1;
-    L.spl = c.take<unsigned long long>(L.cap_spl * SPL_STRIDE);
-    L.cap_fix = N / 16 + 65536;
-    L.fix = c.take<uint32_t>(2 * L.cap_fix);
-    L.pin = nullptr;
 }
 
 int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
@@ -2233,112 +1670,82 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     S.ord_out = ord_out;
     S.lcp_out = lcp_out;
     Seg* large[2] = {(Seg*)L.large[0], (Seg*)L.large[1]};
-    for (int b = 0; b < NBINS; ++b) S.small[b] = (Seg*)L.small[b];
-    S.tile0 = L.tile0;
-    S.chunk0 = L.chunk0;
-    S.tmp_counts = L.tmp_counts;
-    S.tile_hist = L.tile_hist;
-    S.chunk_pre = L.chunk_pre;
-    S.bucket = L.bucket;
-    S.counters = L.counters;
-    S.child = L.child;
-    S.nxt = nullptr;
-    S.small_max = clamp_small_max(small_max);
-    S.pivot = tune(TUNE_SORT_PIVOT) ? 1u : 0u;
-    S.bits = (uint32_t)tune(TUNE_SORT_BITS);
-    S.first = 0;
-    S.cap_large = L.cap_large;
-    S.cap_small = L.cap_small;
-    S.cap_tiles = L.cap_tiles;
-    S.cap_chunks = L.cap_chunks;
-    {
-        const int64_t v = tune(TUNE_SORT_SPLIT_MIN);
-        S.split_min = v <= 0 ? 0u : (uint32_t)std::min<int64_t>(std::max<int64_t>(v, SPL_MIN_FLOOR), 0xFFFFFFFFll);
-    }
-    S.seg_depth = seg_depth;
-    S.spl = L.spl;
-    S.fix = L.fix;
-    S.cap_spl = L.cap_spl;
-    S.cap_fix = L.cap_fix;
-    static std::atomic<uint64_t> scatter_configured{0};
-    DSSS_TRY(set_smem_once(scatter_configured, k_scatter, (int)SCATTER_SMEM));
-    DSSS_CUDA(cudaMemcpyAsync(L.pb, pb_host, (p + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
-    if (n <= (uint64_t)tune(TUNE_SORT_GRAPH)) {
-        static std::atomic<uint64_t> c256{0}, c1024{0}, c4096{0};
-        DSSS_TRY(set_smem_once(c256, k_seg_sort<256, 128>, (int)seg_sort_smem<256>()));
-        DSSS_TRY(set_smem_once(c1024, k_seg_sort<1024, 256>, (int)seg_sort_smem<1024>()));
-        DSSS_TRY(set_smem_once(c4096, k_seg_sort<4096, 512>, (int)seg_sort_smem<4096>()));
-        S.large[0] = large_list(L, 0);
-        S.large[1] = large_list(L, 1);
-        S.child = nullptr;  // every pass of the graph reads the keys itself
-        return sort_strings_graph(L, S, n, p, ids_in, pin, st);
-    }
-    DSSS_CUDA(cudaMemsetAsync(L.counters, 0, 16 * sizeof(uint32_t), st));
-    DSSS_LAUNCH("k_init_ids", st, k_init_ids<<<grid_for(n, 256), 256, 0, st>>>(S.ord[0], ids_in, n));
     S.large[0] = large[0];
     S.large[1] = large[1];
-    DSSS_LAUNCH("k_init_segs", st, k_init_segs<<<grid_for(p, 128), 128, 0, st>>>(S, L.pb, p));
+    for (int b = 0; b < NBINS; ++b) {
+        S.small[b] = (SmallSeg*)L.small[b];
+        S.cap_small[b] = L.cap_small[b];
+    }
+    S.tile0 = L.tile0;
+    S.hist = L.hist;
+    S.bucket = L.bucket;
+    S.cursor = L.cursor;
+    S.counters = L.counters;
+    S.small_max = clamp_small_max(small_max);
+    S.pivot = tune(TUNE_SORT_PIVOT) ? 1u : 0u;
+    S.n = n;
+    S.cap_large = L.cap_large;
+    S.cap_tiles = L.cap_tiles;
+    S.seg_depth = seg_depth;
+    // the first lists' sizes follow from the bounds: nothing to read back
+    uint32_t nlarge = 0, nsmall[NBINS] = {};
+    for (uint32_t q = 0; q < p; ++q) {
+        const uint64_t size = pb_host[q + 1] - pb_host[q];
+        if (size > S.small_max) ++nlarge;
+        else if (size > 1) ++nsmall[bin_of((uint32_t)size)];
+    }
+    const bool all_large = !nsmall[0] && !nsmall[1] && !nsmall[2] && !nsmall[3];
+    S.iota = !ids_in && all_large;
+    static std::atomic<uint64_t> scatter_configured{0};
+    DSSS_TRY(set_smem_once(scatter_configured, k_scatter, (int)SCATTER_SMEM));
+    DSSS_CUDA(cudaMemsetAsync(L.counters, 0, 16 * sizeof(uint32_t), st));
+    if (nlarge) DSSS_CUDA(cudaMemsetAsync(L.hist, 0, L.cap_large * 256 * sizeof(uint32_t), st));
+    if (!S.iota) DSSS_LAUNCH("k_init_ids", st, k_init_ids<<<grid_for(n, 256), 256, 0, st>>>(S.ord[0], ids_in, n));
+    const bool one = p == 1 && pb_host[0] == 0 && pb_host[1] == n;
+    if (!one) DSSS_CUDA(cudaMemcpyAsync(L.pb, pb_host, (p + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+    DSSS_LAUNCH("k_init_segs", st, k_init_segs<<<grid_for(p, 128), 128, 0, st>>>(S, one ? nullptr : L.pb, p));
     DSSS_CUDA(cudaGetLastError());
-    DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    DSSS_CUDA(cudaStreamSynchronize(st));
-    uint32_t nlarge = pin[0];
     int cur = 0;
     uint32_t guard = 0;
-    S.first = 1;
-    // whether the list holds a segment without keys folded by the previous
-    // scatter (no keys, a pivot pass, or the first pass): only then the
-    // prefix, pivot and key passes run
+    // whether the list holds a segment without keys (the first pass, a pivot
+    // pass, equal strings): only then the passes that make keys run
     bool keyless = true;
     while (nlarge) {
         if (++guard > (1u << 24)) return fail(DSSS_EDEVICE, "string sort made no progress");
         Seg* segs = large[cur];
         Seg* next = large[cur ^ 1];
-        // tile / chunk indexing
-        // tile / chunk indexing (and the next list's count reset): one block
+        // an upper bound for the grids (kernels exit past the real count)
+        const unsigned tiles = (unsigned)std::min<uint64_t>(L.cap_tiles, n / LT_TILE + nlarge + 1);
         DSSS_LAUNCH("k_seg_offsets", st, k_seg_offsets<<<1, 1024, 0, st>>>(S, segs, nlarge));
-        // upper bounds for the grids (kernels exit past the real counts)
-        uint64_t max_tiles = std::min<uint64_t>(L.cap_tiles, n / LT_TILE + nlarge + 1);
-        uint64_t max_chunks = std::min<uint64_t>(L.cap_chunks, max_tiles / CHUNK_TILES + nlarge + 1);
-        S.large[0] = segs;
-        S.nxt = next;
         if (keyless) {
             DSSS_LAUNCH("k_spec", st, k_spec<<<std::min<uint32_t>(nlarge, 148 * 16), 256, 0, st>>>(S, segs, nlarge));
-            DSSS_LAUNCH("k_prefix", st, k_prefix<<<(unsigned)max_tiles, LT_NT, 0, st>>>(S, segs, nlarge));
-            DSSS_LAUNCH("k_pivot", st, k_pivot<<<(unsigned)max_tiles, LT_NT, 0, st>>>(S, segs, nlarge));
-            DSSS_LAUNCH("k_keys_diff", st, k_keys_diff<<<(unsigned)max_tiles, LT_NT, 0, st>>>(S, segs, nlarge));
+            DSSS_LAUNCH("k_prefix", st, k_prefix<<<tiles, LT_NT, 0, st>>>(S, segs, nlarge));
+            if (guard > 1) DSSS_LAUNCH("k_pivot", st, k_pivot<<<tiles, LT_NT, 0, st>>>(S, segs, nlarge));
+            DSSS_LAUNCH("k_keys_diff", st, k_keys_diff<<<tiles, LT_NT, 0, st>>>(S, segs, nlarge));
         }
-        if (S.split_min)
-            DSSS_LAUNCH("k_split_sample", st,
-                        k_split_sample<<<std::min<uint32_t>(nlarge, 148 * 2), SPL_SAMPLE / 2, 0, st>>>(S, segs, nlarge));
-        // the bit-digit histogram only in passes that can split on bits (its
-        // tables and registers cost the byte form's occupancy)
-        if (S.bits && (S.bits != 3 || S.first))
-            DSSS_LAUNCH("k_hist", st, k_hist<true><<<(unsigned)max_tiles, LT_NT, 0, st>>>(S, segs, nlarge));
-        else
-            DSSS_LAUNCH("k_hist", st, k_hist<false><<<(unsigned)max_tiles, LT_NT, 0, st>>>(S, segs, nlarge));
-        DSSS_LAUNCH("k_chunk_sum", st, k_chunk_sum<<<(unsigned)max_chunks, 256, 0, st>>>(S, segs, nlarge));
-        DSSS_LAUNCH("k_seg_scan", st, k_seg_scan<<<nlarge, 256, 0, st>>>(S, segs, nlarge, next));
-        DSSS_LAUNCH("k_scatter", st, k_scatter<<<(unsigned)max_tiles, LT_NT, SCATTER_SMEM, st>>>(S, segs, nlarge));
+        DSSS_LAUNCH("k_hist", st, k_hist<<<tiles, LT_NT, 0, st>>>(S, segs, nlarge));
+        DSSS_LAUNCH("k_seg_scan", st, k_seg_scan<<<nlarge, 256, 0, st>>>(S, segs, next));
+        DSSS_LAUNCH("k_scatter", st, k_scatter<<<tiles, SC_NT, SCATTER_SMEM, st>>>(S, segs, nlarge));
         DSSS_CUDA(cudaGetLastError());
         DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         DSSS_CUDA(cudaStreamSynchronize(st));
         nlarge = pin[0];
-        keyless = !S.child || pin[11] != 0;
+        keyless = pin[11] != 0;
         if (pin[10]) return fail(DSSS_EDEVICE, "string sort: internal consistency guard tripped");
         if (nlarge > L.cap_large) return fail(DSSS_EDEVICE, "string sort: large-segment list overflow");
         cur ^= 1;
-        S.first = 0;
+        S.iota = 0;
+        for (int b = 0; b < NBINS; ++b) nsmall[b] = pin[1 + b];
     }
     for (int b = 0; b < NBINS; ++b)
-        if (pin[1 + b] > L.cap_small) return fail(DSSS_EDEVICE, "string sort: small-segment list overflow");
-    if (pin[1]) {
-        DSSS_LAUNCH("k_warp_segs", st, k_warp_segs<<<(pin[1] + 3) / 4, 128, 0, st>>>(S, S.small[0], pin[1], nullptr));
+        if (nsmall[b] > L.cap_small[b]) return fail(DSSS_EDEVICE, "string sort: small-segment list overflow");
+    if (nsmall[0]) {
+        DSSS_LAUNCH("k_warp_segs", st, k_warp_segs<<<(nsmall[0] + 3) / 4, 128, 0, st>>>(S, S.small[0], nsmall[0]));
         DSSS_CUDA(cudaGetLastError());
     }
-    DSSS_TRY((launch_seg_sort<256, 128>(S, S.small[1], pin[2], "k_seg_sort256", st)));
-    DSSS_TRY((launch_seg_sort<1024, 256>(S, S.small[2], pin[3], "k_seg_sort1024", st)));
-    DSSS_TRY((launch_seg_sort<4096, 512>(S, S.small[3], pin[4], "k_seg_sort4096", st)));
-    if (pin[5]) DSSS_LAUNCH("k_lcp_fix", st, k_lcp_fix<<<grid_for(std::min<uint64_t>(pin[5], L.cap_fix), 256), 256, 0, st>>>(S));
+    DSSS_TRY((launch_seg_sort<256, 128>(S, S.small[1], nsmall[1], "k_seg_sort256", st)));
+    DSSS_TRY((launch_seg_sort<1024, 256>(S, S.small[2], nsmall[2], "k_seg_sort1024", st)));
+    DSSS_TRY((launch_seg_sort<4096, 512>(S, S.small[3], nsmall[3], "k_seg_sort4096", st)));
     DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));
     if (pin[10]) return fail(DSSS_EDEVICE, "string sort: internal consistency guard tripped");

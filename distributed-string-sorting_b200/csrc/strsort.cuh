@@ -10,19 +10,12 @@ struct SortLayout {
     unsigned char* large[2];
     unsigned char* small[4];
     uint32_t* tile0;
-    uint32_t* chunk0;
-    uint32_t* tmp_counts;
-    uint32_t* tile_hist;
-    uint32_t* chunk_pre;
+    uint32_t* hist;
     uint32_t* bucket;
-    uint32_t* child;  // 256 per large segment (NULL: the passes read the keys themselves)
+    uint32_t* cursor;
     uint32_t* counters;
     uint64_t* pb;
-    unsigned char* scan;
-    unsigned long long* spl;  // sampled splitter tables
-    uint32_t* fix;            // bucket starts whose LCP is written at the end
-    uint32_t* pin;
-    uint64_t cap_large, cap_small, cap_tiles, cap_chunks, cap_spl, cap_fix;
+    uint64_t cap_large, cap_small[4], cap_tiles;
 };
 
 constexpr uint32_t SORT_SMALL_MAX_DEFAULT = 4096;

@@ -116,11 +116,7 @@ int dsss_abi_version(void);
  *                   (default 1)
  *   dp_table        hash-table slots per hashed string in a distinguishing-
  *                   prefix round, rounded up to a power of two (2..8, default 2)
- *   sort_graph_max_n  largest n whose string sort runs as one CUDA graph with
- *                   a device-side pass loop (default 0 = never: measured on
- *                   B200 no faster than the host-driven loop, whose per-pass
- *                   read-back costs less than the graph's capacity-sized grids
- *                   and per-call instantiation)
+ *   sort_graph_max_n  0 (default) to 2^32: accepted, without effect
  *   merge_by_sort   dsss_lcp_merge: decompressed runs merged by one segmented
  *                   string sort (1, default), by pairwise merge-path rounds
  *                   (0), or all p runs at once by co-ranked tiles (2: every
@@ -145,21 +141,12 @@ int dsss_abi_version(void);
  *                   and the outcome read back as one bit per sorted position
  *                   (k = 1..64, default 4); 0 hashes every round by gathering
  *                   the prefixes in sorted order
- *   sort_split_min  smallest segment of the string sort's MSD passes that
- *                   may split by up to 255 splitters sampled from its keys
- *                   instead of by one key byte, where that byte takes few
- *                   values (letters, DNA; default 0 = never: on B200 the
- *                   fewer passes cost more in the small-segment sorts, whose
- *                   buckets then cut across key bytes; values below 4096
- *                   count as 4096)
+ *   sort_split_min  0 (default) to 2^32: accepted, without effect
  *   dp_check        0 (default) or 1: accepted, without effect (no round
  *                   reads stored prefix hashes)
- *   sort_bits       1: MSD passes over plain keys split on the eight most
- *                   significant bits in which a segment's keys differ (over
- *                   small alphabets one pass then covers more than a key
- *                   byte); 2: only where the first differing key byte varies
- *                   in at most four bits; 3: the same in the first pass only;
- *                   0: on the first differing key byte (default)
+ *   sort_bits       0 (default) to 3: accepted, without effect (the passes
+ *                   choose their digit from the keys' differing bits and the
+ *                   segment's size)
  *   sort_seg_bits   0 (default) or 1: accepted, without effect (segments up to
  *                   the small-segment cutoff always split on differing bits) */
 int dsss_tune_set(const char* name, int64_t value);

@@ -67,6 +67,8 @@ struct Seg {
     unsigned long long diff;
     uint32_t piv;    // pivot pass: the pivot's string id (NO_PIVOT: the first string)
     uint32_t ended;  // bucket 0 holds the strings that end at the first differing byte
+    unsigned long long exact;  // the bits in which the keys do differ (k_hist)
+    uint32_t stay, pad;        // the pass does not move the segment
     BucketBits bits;  // this pass's digit
 };
 
@@ -92,9 +94,10 @@ struct SortState {
     Seg* large[2];
     SmallSeg* small[NBINS];
     uint32_t* tile0;
-    uint32_t* hist;    // 256 per large segment, zero between passes
-    uint32_t* bucket;  // 257 per large segment: where the buckets start
-    uint32_t* cursor;  // 256 per large segment: where their next tile goes
+    uint32_t* hist;    // D per large segment, zero between passes
+    uint32_t* bucket;  // D + 1 per large segment: where the buckets start
+    uint32_t* cursor;  // D per large segment: where their next tile goes
+    uint32_t dbits;    // digits of up to dbits bits, D = 1 << dbits
     uint32_t* counters;
     uint32_t small_max;
     uint32_t pivot;  // pivot passes enabled
@@ -152,6 +155,9 @@ __device__ __forceinline__ void push_large(const SortState& S, Seg* dst, uint32_
     s.diff = diff;
     s.piv = NO_PIVOT;
     s.ended = 0;
+    s.exact = 0;
+    s.stay = 0;
+    s.pad = 0;
 }
 
 // ------------------------------------------------------------------ init ----
@@ -537,39 +543,34 @@ __global__ void __launch_bounds__(LT_NT) k_keys_diff(SortState S, Seg* segs, uin
 // strings with different codes is d + min(l, l').
 __device__ __forceinline__ uint32_t pivot_l(uint32_t code) { return code <= PIVOT_CAP ? code : 2 * PIVOT_CAP - code; }
 
-// Pseudo key of string (off, len) against the pivot (off0, len0), both
-// sharing their first d0 bytes.
-__device__ __forceinline__ uint64_t pivot_key(const uint8_t* chars, uint64_t off, uint32_t len, uint64_t off0,
-                                              uint32_t len0, uint32_t d0) {
-    uint32_t code = PIVOT_CAP, byte = 0;
-    bool done = false;
-    for (uint32_t c = 0; c < PIVOT_CAP && !done; c += 16) {
-        // 16 bytes per step: two independent 8-byte compares
-        uint64_t x[2], y[2];
+// Pseudo key of string (off, len) against the pivot, whose big-endian words
+// from depth d0 (zero past its end) are y[0..PIVOT_WORDS): 32 bytes of the
+// string per step, all their loads in flight together.
+__device__ __forceinline__ uint64_t pivot_key(const uint8_t* chars, uint64_t off, uint32_t len,
+                                              const unsigned long long* y, uint32_t d0) {
+    for (uint32_t c = 0; c < PIVOT_WORDS; c += 4) {
+        uint64_t x[4];
+        key_words<4>(chars, off, len, d0 + 8 * c, 4, x);
+        uint32_t l = 0xFFFFFFFFu;
+        uint64_t xw = 0, yw = 0;
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            x[q] = key8(chars, off, len, d0 + c + 8 * q);
-            y[q] = key8(chars, off0, len0, d0 + c + 8 * q);
-        }
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            if (done) continue;
-            if (x[q] != y[q]) {
-                const uint32_t j = key_lcp(x[q], y[q]);
-                const uint32_t l = c + 8 * q + j;
-                if (l < PIVOT_CAP) {
-                    const uint32_t bx = (uint32_t)(x[q] >> (56 - 8 * j)) & 0xFFu;
-                    const uint32_t by = (uint32_t)(y[q] >> (56 - 8 * j)) & 0xFFu;
-                    code = bx < by ? l : 2 * PIVOT_CAP - l;
-                    byte = bx;
-                }
-                done = true;
-            } else if (zero_byte(x[q]) < 8) {
-                done = true;  // equal to the pivot
+        for (int q = 3; q >= 0; --q) {  // the first word that differs or ends wins
+            const uint64_t v = y[c + q];
+            if (x[q] != v || zero_byte(v) < 8) {
+                l = 8 * (c + q);
+                xw = x[q];
+                yw = v;
             }
         }
+        if (l == 0xFFFFFFFFu) continue;
+        if (xw == yw) break;  // equal to the pivot
+        const uint32_t j = key_lcp(xw, yw);
+        l += j;
+        if (l >= PIVOT_CAP) break;
+        const uint32_t bx = (uint32_t)(xw >> (56 - 8 * j)) & 0xFFu, by = (uint32_t)(yw >> (56 - 8 * j)) & 0xFFu;
+        return (uint64_t)(bx < by ? l : 2 * PIVOT_CAP - l) << 56 | (uint64_t)bx << 48;
     }
-    return (uint64_t)code << 56 | (uint64_t)byte << 48;
+    return (uint64_t)PIVOT_CAP << 56;
 }
 
 __global__ void __launch_bounds__(LT_NT) k_pivot(SortState S, Seg* segs, uint32_t nseg) {
@@ -583,16 +584,21 @@ __global__ void __launch_bounds__(LT_NT) k_pivot(SortState S, Seg* segs, uint32_
     unsigned long long* key = S.key[par];
     const uint32_t tb = sg.start + (t - S.tile0[si]) * LT_TILE;
     const uint32_t te = min(sg.start + sg.size, tb + LT_TILE);
-    uint64_t off0;
-    uint32_t len0;
-    str_of(S.a, sg.piv == NO_PIVOT ? ord[sg.start] : sg.piv, off0, len0);
+    __shared__ unsigned long long y[PIVOT_WORDS];
+    if (threadIdx.x < PIVOT_WORDS) {
+        uint64_t off0;
+        uint32_t len0;
+        str_of(S.a, sg.piv == NO_PIVOT ? ord[sg.start] : sg.piv, off0, len0);
+        y[threadIdx.x] = key8(S.a.chars, off0, len0, sg.depth + 8 * threadIdx.x);
+    }
+    __syncthreads();
     const uint64_t k0 = (uint64_t)PIVOT_CAP << 56;
     uint64_t df = 0;
     for (uint32_t i = tb + threadIdx.x; i < te; i += LT_NT) {
         uint64_t off;
         uint32_t len;
         str_of(S.a, ord[i], off, len);
-        const uint64_t k = pivot_key(S.a.chars, off, len, off0, len0, sg.depth);
+        const uint64_t k = pivot_key(S.a.chars, off, len, y, sg.depth);
         key[i] = k;
         df |= k ^ k0;
     }
@@ -639,13 +645,17 @@ __device__ __forceinline__ void bucket_bits(BucketBits& B, uint64_t diff, uint32
 
 // This pass's digit of a segment: pivot pseudo keys split on a whole byte (the
 // code, then the byte behind the LCP), other keys on their most significant
-// differing bits, as many (up to 8) as leave about DIGIT_TARGET strings per
-// bucket.  A digit of 8 bits over letters (5 differing bits per byte) or DNA (4)
-// covers more than a byte, so 32e6 random six-letter keys take two passes where
-// byte digits took four; narrower digits for segments just above the cutoff
-// keep their children from being a few strings each.
-constexpr uint32_t DIGIT_TARGET = 640;
-__device__ __forceinline__ void segment_digit(BucketBits& B, uint64_t diff, uint32_t flags, uint32_t size) {
+// differing bits: as many as leave about DIGIT_TARGET strings per bucket, in
+// equal parts where one pass of DIGIT_BITS_MAX is too few.  A digit over letters
+// (5 differing bits per byte) or DNA (4) covers more than a byte: 1e8 random
+// six-letter keys take two passes, four by bytes and three by 8 bits (whose
+// last one leaves segments of 100 to 200 strings: counts, scatters and segment
+// sorter 4.7 ms, with passes of 9 and 10 bits 3.4 ms); narrower digits for
+// segments just above the cutoff keep their children from being a few strings
+// each.
+constexpr uint32_t DIGIT_TARGET = 1200, DIGIT_BITS_MAX = 10, DIGIT_MAX = 1u << DIGIT_BITS_MAX;
+__device__ __forceinline__ void segment_digit(BucketBits& B, uint64_t diff, uint32_t flags, uint32_t size,
+                                              uint32_t dbits) {
     if (flags & (F_PIVOT | F_PSEUDO)) {
         B.lo = 56 - 8 * (uint32_t)(__clzll(diff) >> 3);
         B.nruns = 1;
@@ -656,8 +666,9 @@ __device__ __forceinline__ void segment_digit(BucketBits& B, uint64_t diff, uint
         B.mask[0] = 0xFFu;
         return;
     }
-    const uint32_t parts = size / DIGIT_TARGET;
-    bucket_bits(B, diff, min(8u, max(3u, 33u - (uint32_t)__clz(parts | 1u))));
+    const uint32_t need = max(3u, 33u - (uint32_t)__clz((size / DIGIT_TARGET) | 1u));
+    const uint32_t passes = (need + dbits - 1) / dbits;
+    bucket_bits(B, diff, (need + passes - 1) / passes);
 }
 
 // The bits of a key that a digit holds.
@@ -691,15 +702,18 @@ __device__ __forceinline__ void digits_of(const BucketBits& B, const uint64_t (&
     }
 }
 
-// Counts per segment and digit: a tile's counts in shared memory (one row per
-// warp), then one global atomic per digit.  Bound by the 8-byte key read.
-__global__ void __launch_bounds__(LT_NT) k_hist(SortState S, const Seg* segs, uint32_t nseg) {
-    __shared__ uint32_t hist[LT_NT / 32][256];
+// Counts per segment and digit, and the bits in which the keys do differ: a tile's counts in shared memory (a row for
+// every two warps), then one global atomic per digit.  Bound by the 8-byte key
+// read.
+constexpr int HIST_ROWS = LT_NT / 64;
+__global__ void __launch_bounds__(LT_NT) k_hist(SortState S, Seg* segs, uint32_t nseg) {
+    __shared__ uint32_t hist[HIST_ROWS][DIGIT_MAX];
+    __shared__ unsigned long long s_diff[LT_NT / 32];
     __shared__ BucketBits B;
-    const uint32_t t = blockIdx.x;
+    const uint32_t t = blockIdx.x, D = 1u << S.dbits;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
-    const Seg& sg = segs[si];
+    Seg& sg = segs[si];
     const uint64_t diff = sg.diff;
     if (diff == 0) return;
     const uint32_t start = sg.start, size = sg.size, flags = sg.flags;
@@ -713,41 +727,64 @@ __global__ void __launch_bounds__(LT_NT) k_hist(SortState S, const Seg* segs, ui
         const uint32_t i = tb + j * LT_NT + threadIdx.x;
         k[j] = i < te ? key[i] : 0;
     }
-    if (threadIdx.x == 0) segment_digit(B, diff, flags, size);
+    const uint64_t k0 = key[start];
+    if (threadIdx.x == 0) segment_digit(B, diff, flags, size, S.dbits);
 #pragma unroll
-    for (int w = 0; w < LT_NT / 32; ++w) hist[w][threadIdx.x] = 0;
+    for (int w = 0; w < HIST_ROWS; ++w)
+        for (uint32_t x = threadIdx.x; x < D; x += LT_NT) hist[w][x] = 0;
     __syncthreads();
     uint32_t d[LT_IPT];
     digits_of(B, k, d);
-    uint32_t* wh = hist[threadIdx.x >> 5];
+    uint32_t* wh = hist[threadIdx.x >> 6];
 #pragma unroll
     for (int j = 0; j < LT_IPT; ++j)
         if (tb + j * LT_NT + threadIdx.x < te) atomicAdd(&wh[d[j]], 1u);
-    __syncthreads();
-    uint32_t c = 0;
+    uint64_t df = 0;
 #pragma unroll
-    for (int w = 0; w < LT_NT / 32; ++w) c += hist[w][threadIdx.x];
-    if (c) atomicAdd(&S.hist[(uint64_t)si * 256 + threadIdx.x], c);
+    for (int j = 0; j < LT_IPT; ++j)
+        if (tb + j * LT_NT + threadIdx.x < te) df |= k[j] ^ k0;
+    const uint32_t dlo = __reduce_or_sync(0xffffffffu, (uint32_t)df);
+    const uint32_t dhi = __reduce_or_sync(0xffffffffu, (uint32_t)(df >> 32));
+    if ((threadIdx.x & 31) == 0) s_diff[threadIdx.x >> 5] = (unsigned long long)dhi << 32 | dlo;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long x = 0;
+#pragma unroll
+        for (int w = 0; w < LT_NT / 32; ++w) x |= s_diff[w];
+        if (x) atomicOr(&sg.exact, x);
+    }
+    for (uint32_t x = threadIdx.x; x < D; x += LT_NT) {
+        uint32_t c = 0;
+#pragma unroll
+        for (int w = 0; w < HIST_ROWS; ++w) c += hist[w][x];
+        if (c) atomicAdd(&S.hist[((uint64_t)si << S.dbits) + x], c);
+    }
 }
 
 // ----------------------------------------------------------- segment scan ----
 // One block per segment: bucket starts, the LCPs at bucket starts, and the
-// segment's children.
+// segment's children; DPT consecutive digits per thread.
+template <int DPT>
 __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, Seg* next) {
-    __shared__ uint32_t wsum[8], wany[8];
+    constexpr uint32_t D = 256 * DPT;
+    __shared__ uint32_t wsum[8], any[D / 32];  // any: the digits that occur
+    __shared__ uint32_t s_small[NBINS], s_base[NBINS];
     __shared__ BucketBits B;
     const uint32_t si = blockIdx.x;
     Seg& sg = segs[si];
     const uint32_t start = sg.start, size = sg.size, flags = sg.flags, par = flags & F_PARITY, np = par ^ 1u;
-    const uint64_t diff = sg.diff;
+    const uint64_t diff = sg.exact;
     const bool pseudo = (flags & (F_PIVOT | F_PSEUDO)) != 0, by_id = (flags & F_ID) != 0;
     const uint32_t depth = (flags & (F_KEYS | F_PIVOT | F_ID)) ? sg.depth : sg.newdepth;
     const uint64_t k0 = S.key[par][start];
-    const uint32_t d = threadIdx.x;
     if (diff == 0) {
         // Every key equal: byte-identical strings if the key holds their end,
         // else continue deeper without keys.
-        if (d != 0) return;
+        // (counted in one bucket when the parent left bits open)
+        uint32_t* hist = S.hist + (uint64_t)si * D + threadIdx.x * DPT;
+        for (int q = 0; q < DPT; ++q) hist[q] = 0;
+        if (threadIdx.x != 0) return;
+        sg.stay = 1;
         uint32_t fin = 0xFFFFFFFFu, cont = 0, cflags = par;
         if (pseudo) {
             const uint32_t code = (uint32_t)(k0 >> 56), byte = (uint32_t)(k0 >> 48) & 0xFFu;
@@ -772,102 +809,148 @@ __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, Seg* n
         else push_large(S, next, start, size, cont, cflags);
         return;
     }
-    const uint32_t total = S.hist[(uint64_t)si * 256 + d];
-    S.hist[(uint64_t)si * 256 + d] = 0;
-    if (d == 0) segment_digit(B, diff, flags, size);
-    // block exclusive scan over the 256 digits, and the digits that occur
-    const int lane = d & 31, w = d >> 5;
-    uint32_t x = total;
+    uint32_t tot[DPT], sum = 0, occ = 0;
+    uint32_t* hist = S.hist + (uint64_t)si * D + threadIdx.x * DPT;
+#pragma unroll
+    for (int q = 0; q < DPT; ++q) {
+        tot[q] = hist[q];
+        hist[q] = 0;
+        sum += tot[q];
+        occ |= (tot[q] != 0 ? 1u : 0u) << q;
+    }
+    if (threadIdx.x < D / 32) any[threadIdx.x] = 0;
+    if (threadIdx.x < NBINS) s_small[threadIdx.x] = 0;
+    if (threadIdx.x == 0) segment_digit(B, sg.diff, flags, size, S.dbits);
+    // block exclusive scan over the digits
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t x = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    const uint32_t any = __ballot_sync(0xffffffffu, total != 0);
     if (lane == 31) wsum[w] = x;
-    if (lane == 0) wany[w] = any;
     __syncthreads();
-    uint32_t excl = x - total;
-    for (int k = 0; k < w; ++k) excl += wsum[k];
-    const uint32_t cs = start + excl;
-    S.bucket[(uint64_t)si * 257 + d] = cs;
-    if (d == 255) S.bucket[(uint64_t)si * 257 + 256] = start + size;
-    S.cursor[(uint64_t)si * 256 + d] = cs;
+    if (occ) atomicOr(&any[threadIdx.x * DPT / 32], occ << (threadIdx.x * DPT % 32));
+    uint32_t cs = start + x - sum;
+    for (int k = 0; k < w; ++k) cs += wsum[k];
+    __syncthreads();
     // byte b is the first that may differ; bucket 0 holds the strings that end
     // there if that byte's differing bits are all in the digit and it has no
     // constant nonzero part
     const uint32_t b = (uint32_t)(__clzll(diff) >> 3), shift = 56 - 8 * b;
     const uint64_t mask = digit_mask(B), rest = diff & ~mask;
     const bool plain = !pseudo && !by_id, code_split = pseudo && b == 0;
+    if ((diff & mask) == 0) {  // one bucket: the same keys again, on the bits that do differ
+        if (threadIdx.x == 0) {
+            sg.stay = 1;
+            push_large(S, next, start, size, depth, par | F_KEYS | (flags & F_ID) | (pseudo ? F_PSEUDO : 0u), diff);
+        }
+        return;
+    }
     const bool ended = plain ? (((k0 >> shift) & ~(diff >> shift)) & 0xFFu) == 0 && ((rest >> shift) & 0xFFu) == 0
                              : pseudo && !code_split;
     const uint32_t lcp_here = pseudo ? depth + pivot_l((uint32_t)(k0 >> 56)) : depth + b;
-    if (d == 0) {
+    if (threadIdx.x == 0) {
         sg.bits = B;
         sg.ended = ended;
+        S.bucket[(uint64_t)si * (D + 1) + D] = start + size;
     }
-    if (total == 0) return;
-    if (cs != start) {
-        // LCP with the bucket before (the last smaller digit that occurs)
-        uint32_t m = any & ((1u << lane) - 1u);
-        int pw = w;
-        while (m == 0) m = wany[--pw];
-        const uint32_t pd = (uint32_t)pw * 32 + 31u - (uint32_t)__clz(m);
-        uint32_t l = lcp_here;
-        if (by_id) {
-            l = depth;
-        } else if (code_split) {
-            l = depth + min(pivot_l(d), pivot_l(pd));
-        } else if (plain) {
-            // the byte of the highest bit in which the two digits differ
-            const uint32_t h = 31u - (uint32_t)__clz(d ^ pd);
-            for (uint32_t r = 0; r < B.nruns; ++r)
-                if ((B.mask[r] >> h) & 1u) l = depth + ((63u - (B.lo + B.sh[r] + h)) >> 3);
-        }
-        S.lcp_out[cs] = l;
-    }
-    if (total < 2) return;
-    const bool big = total > S.small_max;
-    const bool chain = S.pivot && 2 * (uint64_t)total > size;
-    if (by_id) {
-        if (big) push_large(S, next, cs, total, depth, np | F_KEYS | F_ID, rest);
-        else push_small(S, cs, total, depth, np | F_ID);
-    } else if (ended && d == 0) {
-        // equal strings (they may end before byte b when no key differs at
-        // all): the scatter makes their ids the keys
-        const uint32_t fin = plain ? depth + min(b, zero_byte(k0)) : lcp_here;
-        if (big) push_large(S, next, cs, total, fin, np | F_KEYS | F_ID,
-                            (2ull << (63 - __clzll(max(S.n, S.a.n)))) - 1);
-        else push_small(S, cs, total, fin, np | F_ID);
-    } else if (plain) {
-        // children keep the parent's keys, whose bits down to the digit's
-        // lowest are now common; one that keeps most of the parent gets a
-        // pivot pass
-        if (!big) push_small(S, cs, total, depth, np | F_KEYS);
-        else if (chain) push_large(S, next, cs, total, depth + ((64u - B.lo) >> 3), np | F_PIVOT);
-        else push_large(S, next, cs, total, depth, np | F_KEYS, rest);
-    } else if (code_split) {
-        // split by pivot code (only the pivot pass's own segment): large
-        // children keep the pseudo keys, small ones restart from the depth
-        // their strings share
-        if (big) {
-            // (the code of the pivot itself has no byte behind it)
-            push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO, d == PIVOT_CAP ? 0 : rest & ~(0xFFull << 56));
-        } else {
-            uint32_t cd = depth + pivot_l(d);
-            if (d == PIVOT_CAP) {
-                uint64_t o0;
-                uint32_t l0;
-                str_of(S.a, sg.piv == NO_PIVOT ? ord_of(S, par, start) : sg.piv, o0, l0);
-                cd = min(depth + PIVOT_CAP, l0);
+    // small children get their places by one global atomic per bin and block
+    uint32_t sdepth[DPT], sflags[DPT], sslot[DPT];
+#pragma unroll
+    for (int q = 0; q < DPT; ++q) sslot[q] = 0xFFFFFFFFu;
+    auto small = [&](int q, uint32_t dp, uint32_t fl) {
+        sdepth[q] = dp;
+        sflags[q] = fl;
+        sslot[q] = atomicAdd(&s_small[bin_of(tot[q])], 1u);
+    };
+    const uint32_t cs0 = cs;
+#pragma unroll
+    for (int q = 0; q < DPT; ++q) {
+        const uint32_t d = threadIdx.x * DPT + q, total = tot[q];
+        if (q) cs += tot[q - 1];
+        S.bucket[(uint64_t)si * (D + 1) + d] = cs;
+        S.cursor[(uint64_t)si * D + d] = cs;
+        if (total == 0) continue;
+        if (cs != start) {
+            // LCP with the bucket before (the last smaller digit that occurs)
+            int pw = (int)(d >> 5);
+            uint32_t m = any[pw] & ((1u << (d & 31)) - 1u);
+            while (m == 0) m = any[--pw];
+            const uint32_t pd = (uint32_t)pw * 32 + 31u - (uint32_t)__clz(m);
+            uint32_t l = lcp_here;
+            if (by_id) {
+                l = depth;
+            } else if (code_split) {
+                l = depth + min(pivot_l(d), pivot_l(pd));
+            } else if (plain) {
+                // the byte of the highest bit in which the two digits differ
+                const uint32_t h = 31u - (uint32_t)__clz(d ^ pd);
+                for (uint32_t r = 0; r < B.nruns; ++r)
+                    if ((B.mask[r] >> h) & 1u) l = depth + ((63u - (B.lo + B.sh[r] + h)) >> 3);
             }
-            push_small(S, cs, total, cd, np);
+            S.lcp_out[cs] = l;
         }
-    } else {
-        // split by the byte after the shared d + l bytes
-        const uint32_t cd = lcp_here + 1;
-        if (big) push_large(S, next, cs, total, cd, np | (chain ? F_PIVOT : 0u));
-        else push_small(S, cs, total, cd, np);
+        if (total < 2) continue;
+        const bool big = total > S.small_max;
+        // a chain: most strings stay together, and not because most of the
+        // digit's bits, left open by the parent, do not differ here
+        const bool chain = S.pivot && 2 * (uint64_t)total > size &&
+                           (pseudo || rest == 0 || 2 * __popcll(diff & mask) >= __popcll(mask));
+        if (by_id) {
+            if (big) push_large(S, next, cs, total, depth, np | F_KEYS | F_ID, rest);
+            else small(q, depth, np | F_ID);
+        } else if (ended && d == 0) {
+            // equal strings: the scatter makes their ids the keys
+            const uint32_t fin = lcp_here;
+            if (big) push_large(S, next, cs, total, fin, np | F_KEYS | F_ID,
+                                (2ull << (63 - __clzll(max(S.n, S.a.n)))) - 1);
+            else small(q, fin, np | F_ID);
+        } else if (plain) {
+            // children keep the parent's keys, whose bits down to the digit's
+            // lowest are now common; one that keeps most of the parent gets a
+            // pivot pass
+            if (!big) small(q, depth, np | F_KEYS);
+            else if (chain) push_large(S, next, cs, total, depth + ((64u - B.lo) >> 3), np | F_PIVOT);
+            else push_large(S, next, cs, total, depth, np | F_KEYS, rest);
+        } else if (code_split) {
+            // split by pivot code (only the pivot pass's own segment): large
+            // children keep the pseudo keys, small ones restart from the depth
+            // their strings share
+            if (big) {
+                // (the code of the pivot itself has no byte behind it)
+                push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO, d == PIVOT_CAP ? 0 : rest & ~(0xFFull << 56));
+            } else {
+                uint32_t cd = depth + pivot_l(d);
+                if (d == PIVOT_CAP) {
+                    uint64_t o0;
+                    uint32_t l0;
+                    str_of(S.a, sg.piv == NO_PIVOT ? ord_of(S, par, start) : sg.piv, o0, l0);
+                    cd = min(depth + PIVOT_CAP, l0);
+                }
+                small(q, cd, np);
+            }
+        } else {
+            // split by the byte after the shared d + l bytes
+            const uint32_t cd = lcp_here + 1;
+            if (big) push_large(S, next, cs, total, cd, np | (chain ? F_PIVOT : 0u));
+            else small(q, cd, np);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < NBINS) s_base[threadIdx.x] = s_small[threadIdx.x] ? atomicAdd(&S.counters[1 + threadIdx.x], s_small[threadIdx.x]) : 0u;
+    __syncthreads();
+    cs = cs0;
+#pragma unroll
+    for (int q = 0; q < DPT; ++q) {
+        if (sslot[q] != 0xFFFFFFFFu) {
+            const int bin = bin_of(tot[q]);
+            const uint32_t at = s_base[bin] + sslot[q];
+            if (at < S.cap_small[bin]) S.small[bin][at] = SmallSeg{cs, tot[q], sdepth[q], sflags[q]};
+            else atomicExch(&S.counters[10], 1u);
+        }
+        cs += tot[q];
     }
 }
 
@@ -887,18 +970,19 @@ __global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* se
     unsigned long long* skey = (unsigned long long*)sm_scatter;
     uint32_t* sord = (uint32_t*)(skey + LT_TILE);
     uint16_t* sdig = (uint16_t*)(sord + LT_TILE);
-    __shared__ uint32_t cnt[256], tloff[256], wsum[8];
-    __shared__ uint2 dst[256];  // place of the digit's run minus its place in the tile; whether its bucket is one string
+    __shared__ uint32_t cnt[DIGIT_MAX], tloff[DIGIT_MAX], wsum[SC_NT / 32];
+    __shared__ uint2 dst[DIGIT_MAX];  // place of the digit's run minus its place in the tile; whether its bucket is one string
     __shared__ BucketBits B;
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
+    const uint32_t D = 1u << S.dbits;
     const uint32_t si = find_seg(S.tile0, nseg, t);
     const Seg& sg = segs[si];
     const uint32_t start = sg.start, end = start + sg.size, flags = sg.flags, par = flags & F_PARITY;
     const uint32_t tb = start + (t - S.tile0[si]) * LT_TILE;
     const uint32_t te = min(end, tb + LT_TILE);
     const uint32_t tn = te - tb;
-    if (sg.diff == 0) {  // the segment stays where it is (its ids must exist)
+    if (sg.stay) {  // the segment stays where it is (its ids must exist)
         if (S.iota)
             for (uint32_t i = tb + threadIdx.x; i < te; i += SC_NT) S.ord[par][i] = i;
         return;
@@ -914,40 +998,48 @@ __global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* se
     }
     if (threadIdx.x < sizeof(BucketBits) / 4) ((uint32_t*)&B)[threadIdx.x] = ((const uint32_t*)&sg.bits)[threadIdx.x];
     const bool ended = sg.ended;
-    if (threadIdx.x < 256) cnt[threadIdx.x] = 0;
+#pragma unroll
+    for (uint32_t x = 0; x < DIGIT_MAX / SC_NT; ++x) cnt[x * SC_NT + threadIdx.x] = 0;
     __syncthreads();
     uint32_t d[SC_IPT];
     digits_of(B, k, d);
 #pragma unroll
     for (int j = 0; j < SC_IPT; ++j)
-        if (tb + j * SC_NT + threadIdx.x < te) d[j] |= atomicAdd(&cnt[d[j]], 1u) << 8;
+        if (tb + j * SC_NT + threadIdx.x < te) d[j] |= atomicAdd(&cnt[d[j]], 1u) << DIGIT_BITS_MAX;
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    uint32_t c = 0, x = 0;
-    if (threadIdx.x < 256) {
-        c = cnt[threadIdx.x];
-        x = c;
+    constexpr int PER = DIGIT_MAX / SC_NT;
+    uint32_t c[PER], x = 0;
 #pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (lane == 31) wsum[w] = x;
+    for (int q = 0; q < PER; ++q) x += c[q] = cnt[threadIdx.x * PER + q];
+    const uint32_t mine = x;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+        if (lane >= off) x += y;
     }
+    if (lane == 31) wsum[w] = x;
     __syncthreads();
-    if (threadIdx.x < 256) {
-        uint32_t at = x - c;
-        for (int ww = 0; ww < w; ++ww) at += wsum[ww];
-        tloff[threadIdx.x] = at;
-        const uint32_t* bk = S.bucket + (uint64_t)si * 257 + threadIdx.x;
-        const uint32_t base = c ? atomicAdd(&S.cursor[(uint64_t)si * 256 + threadIdx.x], c) : 0u;
-        dst[threadIdx.x] = make_uint2(base - at, bk[1] - bk[0] == 1);
+    uint32_t at = x - mine;
+#pragma unroll
+    for (int ww = 0; ww < SC_NT / 32; ++ww)
+        if (ww < w) at += wsum[ww];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+        const uint32_t dg = threadIdx.x * PER + q;
+        tloff[dg] = at;
+        if (c[q]) {  // then dg < D
+            const uint32_t* bk = S.bucket + (uint64_t)si * (D + 1) + dg;
+            const uint32_t base = atomicAdd(&S.cursor[(uint64_t)si * D + dg], c[q]);
+            dst[dg] = make_uint2(base - at, bk[1] - bk[0] == 1);
+        }
+        at += c[q];
     }
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < SC_IPT; ++j) {
         if (tb + j * SC_NT + threadIdx.x >= te) continue;
-        const uint32_t dg = d[j] & 0xFFu, lp = tloff[dg] + (d[j] >> 8);
+        const uint32_t dg = d[j] & (DIGIT_MAX - 1), lp = tloff[dg] + (d[j] >> DIGIT_BITS_MAX);
         skey[lp] = ended && dg == 0 ? (uint64_t)o[j] : k[j];  // equal strings go on by id
         sord[lp] = o[j];
         sdig[lp] = (uint16_t)dg;
@@ -1650,9 +1742,13 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
         L.small[b] = c.take<unsigned char>(L.cap_small[b] * sizeof(SmallSeg));
     }
     L.tile0 = c.take<uint32_t>(L.cap_large);
-    L.hist = c.take<uint32_t>(L.cap_large * 256);
-    L.bucket = c.take<uint32_t>(L.cap_large * 257);
-    L.cursor = c.take<uint32_t>(L.cap_large * 256);
+    // a segment of a few hundred strings needs no wide digit (and such cutoffs
+    // allow many segments)
+    L.dbits = small_max >= 256 ? DIGIT_BITS_MAX : 8;
+    const uint64_t D = 1ull << L.dbits;
+    L.hist = c.take<uint32_t>(L.cap_large * D);
+    L.bucket = c.take<uint32_t>(L.cap_large * (D + 1));
+    L.cursor = c.take<uint32_t>(L.cap_large * D);
     L.counters = c.take<uint32_t>(16);
     L.pb = c.take<uint64_t>(p + 1);
 }
@@ -1680,6 +1776,7 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     S.hist = L.hist;
     S.bucket = L.bucket;
     S.cursor = L.cursor;
+    S.dbits = L.dbits;
     S.counters = L.counters;
     S.small_max = clamp_small_max(small_max);
     S.pivot = tune(TUNE_SORT_PIVOT) ? 1u : 0u;
@@ -1699,7 +1796,7 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
     static std::atomic<uint64_t> scatter_configured{0};
     DSSS_TRY(set_smem_once(scatter_configured, k_scatter, (int)SCATTER_SMEM));
     DSSS_CUDA(cudaMemsetAsync(L.counters, 0, 16 * sizeof(uint32_t), st));
-    if (nlarge) DSSS_CUDA(cudaMemsetAsync(L.hist, 0, L.cap_large * 256 * sizeof(uint32_t), st));
+    if (nlarge) DSSS_CUDA(cudaMemsetAsync(L.hist, 0, (L.cap_large << L.dbits) * sizeof(uint32_t), st));
     if (!S.iota) DSSS_LAUNCH("k_init_ids", st, k_init_ids<<<grid_for(n, 256), 256, 0, st>>>(S.ord[0], ids_in, n));
     const bool one = p == 1 && pb_host[0] == 0 && pb_host[1] == n;
     if (!one) DSSS_CUDA(cudaMemcpyAsync(L.pb, pb_host, (p + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
@@ -1724,7 +1821,8 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
             DSSS_LAUNCH("k_keys_diff", st, k_keys_diff<<<tiles, LT_NT, 0, st>>>(S, segs, nlarge));
         }
         DSSS_LAUNCH("k_hist", st, k_hist<<<tiles, LT_NT, 0, st>>>(S, segs, nlarge));
-        DSSS_LAUNCH("k_seg_scan", st, k_seg_scan<<<nlarge, 256, 0, st>>>(S, segs, next));
+        if (S.dbits == 8) DSSS_LAUNCH("k_seg_scan", st, k_seg_scan<1><<<nlarge, 256, 0, st>>>(S, segs, next));
+        else DSSS_LAUNCH("k_seg_scan", st, k_seg_scan<4><<<nlarge, 256, 0, st>>>(S, segs, next));
         DSSS_LAUNCH("k_scatter", st, k_scatter<<<tiles, SC_NT, SCATTER_SMEM, st>>>(S, segs, nlarge));
         DSSS_CUDA(cudaGetLastError());
         DSSS_CUDA(cudaMemcpyAsync(pin, L.counters, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));

@@ -15,6 +15,7 @@ struct SortLayout {
     uint32_t* cursor;
     uint32_t* counters;
     uint64_t* pb;
+    uint32_t dbits;
     uint64_t cap_large, cap_small[4], cap_tiles;
 };
 

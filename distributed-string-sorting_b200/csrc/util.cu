@@ -181,8 +181,8 @@ __global__ void __launch_bounds__(MS_NT) k_ms_scatter(const uint32_t* bucket, ui
 #pragma unroll
     for (int j = 0; j < MS_IPT; ++j) {
         uint64_t i = wb + j * 32 + lane;
-        uint32_t d = i < n ? bucket[i] : 0xFFFFFFFFu - lane;
-        uint32_t peers = __match_any_sync(0xffffffffu, d);
+        uint32_t d = i < n ? bucket[i] : 0;
+        uint32_t peers = same_lanes(d, i < n, P);
         uint32_t r = __popc(peers & ((1u << lane) - 1));
         uint32_t prev = i < n ? wcnt[w * P + d] : 0;
         __syncwarp();
@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(MS_NT, 5) k_ms_scatter_pay(const uint32_t* buc
 #pragma unroll
     for (int j = 0; j < MS_IPT; ++j) {
         const uint64_t i = wb + j * 32 + lane;
-        const uint32_t d = i < n ? bucket[i] : 0xFFFFFFFFu - lane;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
+        const uint32_t d = i < n ? bucket[i] : 0;
+        const uint32_t peers = same_lanes(d, i < n, P);
         const uint32_t r = __popc(peers & ((1u << lane) - 1));
         const uint32_t prev = i < n ? wcnt[w * P + d] : 0;
         __syncwarp();

@@ -161,15 +161,15 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
     }
     std::vector<uint64_t> set_begin(nsets + 1);
     for (uint32_t s = 0; s <= nsets; ++s) set_begin[s] = pb[(uint64_t)s * p];
-    DSSS_TRY(make_handles(a, L.handles, st, L.stats));
-    a.h = L.handles;
+    if (p > 1) DSSS_TRY(length_stats(a, L.stats, st));
     // 1. one sort per set, all sets in one segmented sort; the global LCPs are
     // the merged ones up to the receivers' starts
     uint32_t* ord = p == 1 ? out->local_order : L.ord;
     uint32_t* lcp = p > 1 && out->merged_lcp ? out->merged_lcp : p == 1 && want_local_lcp ? out->local_lcp : L.lcp;
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, ord, lcp, smax, pin, st));
+        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, ord, lcp, smax, pin, st,
+                              L.handles));
     }
     if (p == 1) {  // prefix_doubling.hpp:236: one PE sorts locally and returns no permutation
         for (uint32_t r = 0; r < npe; ++r) out->recv_counts[r] = 0;
@@ -336,8 +336,7 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
         return DSSS_OK;
     }
     ArenaDev a = view(in);
-    DSSS_TRY(make_handles(a, L.handles, st, L.stats));
-    a.h = L.handles;
+    DSSS_TRY(length_stats(a, L.stats, st));
     uint32_t* pin = (uint32_t*)ctx->pin;
     void* pinp = (char*)ctx->pin + pin_sort;
     LenStats* hstats = (LenStats*)((char*)ctx->pin + 128);
@@ -347,7 +346,11 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     const uint64_t set_begin[2] = {0, n};
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, 1, set_begin, nullptr, L.ord, out->lcp, smax, pin, st));
+        DSSS_TRY(sort_strings(L.sort, a, n, 1, set_begin, nullptr, L.ord, out->lcp, smax, pin, st, L.handles));
+    }
+    if (!a.h) {  // every string is gathered below
+        DSSS_TRY(make_handles(a, L.handles, st));
+        a.h = L.handles;
     }
     const uint64_t bytes = hstats->sum + n;  // the sort has synchronised on st
     // local orders per PE and their LCP arrays (0 at each PE start)
@@ -713,15 +716,18 @@ static int hq_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     plan(c, handles, ord, lcp, owner, tmp, runx, srcb, tc, off, cnt, prm, cut, dest, err, pbd, total, scan, srcoff,
          stats, sl);
     ArenaDev a = view(in);
-    DSSS_TRY(make_handles(a, handles, st, stats));
-    a.h = handles;
+    DSSS_TRY(length_stats(a, stats, st));
     DSSS_CUDA(cudaMemsetAsync(err, 0, sizeof(uint32_t), st));
     LenStats* hstats = (LenStats*)((char*)ctx->pin + 128);
     DSSS_CUDA(cudaMemcpyAsync(hstats, stats, sizeof(LenStats), cudaMemcpyDeviceToHost, st));
     const uint64_t set_begin[2] = {0, n};
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(sl, a, n, 1, set_begin, nullptr, ord, lcp, smax, (uint32_t*)ctx->pin, st));
+        DSSS_TRY(sort_strings(sl, a, n, 1, set_begin, nullptr, ord, lcp, smax, (uint32_t*)ctx->pin, st, handles));
+    }
+    if (!a.h) {  // every string is gathered below
+        DSSS_TRY(make_handles(a, handles, st));
+        a.h = handles;
     }
     // the output layout: the PEs' sorted data in rank order is the global order
     uint32_t* source = out->source ? out->source : srcb;
@@ -858,9 +864,7 @@ int dsss_local_sort_lcp(dsss_ctx* ctx, const dsss_arena* in, uint32_t p, const u
     ulonglong2* h = c.take<ulonglong2>(in->n ? in->n : 1);
     layout_sort(c, L, in->n, p, smax);
     ArenaDev a = view(in);
-    DSSS_TRY(make_handles(a, h, st));
-    a.h = h;
-    return sort_strings(L, a, in->n, p, part_begin, nullptr, order, lcp, smax, (uint32_t*)ctx->pin, st);
+    return sort_strings(L, a, in->n, p, part_begin, nullptr, order, lcp, smax, (uint32_t*)ctx->pin, st, h);
 }
 
 int dsss_dp_prefixes(dsss_ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_t* part_begin,

@@ -181,9 +181,9 @@ struct LenStats {
     __device__ __forceinline__ uint32_t min_len() const { return ~inv_min; }
 };
 
-// Builds the interleaved handle array for strings [0, n), and the length
-// statistics when asked for.
-int make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st, LenStats* stats = nullptr);
+// Builds the interleaved handle array for strings [0, n).
+int make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st);
+int length_stats(const ArenaDev& a, LenStats* stats, cudaStream_t st);
 
 int check_arena(const dsss_arena* a);
 

@@ -799,7 +799,7 @@ int lcp_merge(Ctx* ctx, const uint8_t* chars, uint64_t bytes, const uint32_t* ch
         DSSS_CUDA(cudaStreamSynchronize(st));
         // every tile sorted on its own, from its strings' shared prefix
         DSSS_TRY(sort_strings(K.SL, fa, n, (uint32_t)P.nt, ts.data(), K.gathered, order, mlcp, 0, (uint32_t*)ctx->pin,
-                              st, K.tdepth));
+                              st, nullptr, K.tdepth));
         DSSS_LAUNCH("k_kw_lcp_fix", st,
                     k_kw_lcp_fix<<<grid_for(P.nt, 256), 256, 0, st>>>(f, K.tstart, K.tb, nrecv, order, mlcp));
         DSSS_LAUNCH("k_merge_tags", st,

@@ -1753,9 +1753,9 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
     L.pb = c.take<uint64_t>(p + 1);
 }
 
-int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
+int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
                  const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t small_max,
-                 uint32_t* pin, cudaStream_t st, const uint32_t* seg_depth) {
+                 uint32_t* pin, cudaStream_t st, ulonglong2* handles, const uint32_t* seg_depth) {
     if (n == 0) return DSSS_OK;
     SortState S;
     S.a = a;
@@ -1833,6 +1833,11 @@ int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p,
         if (nlarge > L.cap_large) return fail(DSSS_EDEVICE, "string sort: large-segment list overflow");
         cur ^= 1;
         S.iota = 0;
+        if (nlarge && keyless && handles && !a.h) {
+            // keys are gathered from here on: one 16-byte read per string
+            DSSS_TRY(make_handles(a, handles, st));
+            a.h = S.a.h = handles;
+        }
         for (int b = 0; b < NBINS; ++b) nsmall[b] = pin[1 + b];
     }
     for (int b = 0; b < NBINS; ++b)

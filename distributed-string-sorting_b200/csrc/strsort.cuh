@@ -30,8 +30,11 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
 // host buffer of >= 16 u32 for count read-backs (the call synchronises on st).
 // seg_depth (optional, device, p entries): the strings of segment q share
 // their first seg_depth[q] bytes (the sort starts there).
-int sort_strings(const SortLayout& L, const ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
+// handles (optional, a.n entries, with a.h NULL): built, and put into a.h, once
+// the sort goes back to the strings in an order other than the arena's; a sort
+// whose first keys tell all strings apart never needs them.
+int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
                  const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t small_max,
-                 uint32_t* pin, cudaStream_t st, const uint32_t* seg_depth = nullptr);
+                 uint32_t* pin, cudaStream_t st, ulonglong2* handles = nullptr, const uint32_t* seg_depth = nullptr);
 
 }  // namespace dsss

@@ -76,30 +76,31 @@ int adjacent_lcp(const ArenaDev& a, const uint32_t* order, uint64_t m, uint32_t*
     return DSSS_OK;
 }
 
-constexpr int MH_IPT = 4;
-__global__ void __launch_bounds__(256) k_make_handles(ArenaDev a, ulonglong2* h, LenStats* stats) {
-    const uint64_t T = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t off[MH_IPT];
-    uint32_t len[MH_IPT];
+__global__ void __launch_bounds__(256) k_make_handles(ArenaDev a, ulonglong2* h) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < a.n) h[i] = make_ulonglong2(a.off[i], a.len[i]);
+}
+
+int make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st) {
+    if (a.n) DSSS_LAUNCH("k_make_handles", st, k_make_handles<<<grid_for(a.n, 256), 256, 0, st>>>(a, h));
+    return DSSS_OK;
+}
+
+constexpr int LS_IPT = 8;
+__global__ void __launch_bounds__(256) k_len_stats(const uint32_t* len, uint64_t n, LenStats* stats) {
+    const uint64_t i0 = (uint64_t)blockIdx.x * (256 * LS_IPT) + threadIdx.x;
+    uint32_t v[LS_IPT];
 #pragma unroll
-    for (int q = 0; q < MH_IPT; ++q) {
-        const uint64_t i = i0 + q * T;
-        off[q] = i < a.n ? a.off[i] : 0ull;
-        len[q] = i < a.n ? a.len[i] : 0u;
-    }
+    for (int q = 0; q < LS_IPT; ++q) v[q] = i0 + q * 256 < n ? len[i0 + q * 256] : 0xFFFFFFFFu;
     uint32_t inv = 0;
     unsigned long long sum = 0;
 #pragma unroll
-    for (int q = 0; q < MH_IPT; ++q) {
-        const uint64_t i = i0 + q * T;
-        if (i < a.n) {
-            h[i] = make_ulonglong2(off[q], len[q]);
-            inv = max(inv, ~len[q]);
-            sum += len[q];
+    for (int q = 0; q < LS_IPT; ++q) {
+        if (i0 + q * 256 < n) {
+            inv = max(inv, ~v[q]);
+            sum += v[q];
         }
     }
-    if (!stats) return;
     __shared__ uint32_t wi[8];
     __shared__ unsigned long long wsum[8];
     inv = __reduce_max_sync(0xffffffffu, inv);
@@ -120,11 +121,11 @@ __global__ void __launch_bounds__(256) k_make_handles(ArenaDev a, ulonglong2* h,
     }
 }
 
-int make_handles(const ArenaDev& a, ulonglong2* h, cudaStream_t st, LenStats* stats) {
-    if (stats) DSSS_CUDA(cudaMemsetAsync(stats, 0, sizeof(LenStats), st));
+int length_stats(const ArenaDev& a, LenStats* stats, cudaStream_t st) {
+    DSSS_CUDA(cudaMemsetAsync(stats, 0, sizeof(LenStats), st));
     if (a.n)
-        DSSS_LAUNCH("k_make_handles", st,
-                    k_make_handles<<<grid_for((a.n + MH_IPT - 1) / MH_IPT, 256), 256, 0, st>>>(a, h, stats));
+        DSSS_LAUNCH("k_len_stats", st,
+                    k_len_stats<<<grid_for(a.n, 256 * LS_IPT), 256, 0, st>>>(a.len, a.n, stats));
     return DSSS_OK;
 }
 

@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(256) k_spec(SortState S, Seg* segs, uint32_t n
     }
 }
 
-__global__ void __launch_bounds__(LT_NT, 4) k_prefix(SortState S, Seg* segs, uint32_t nseg) {
+__global__ void __launch_bounds__(LT_NT, 6) k_prefix(SortState S, Seg* segs, uint32_t nseg) {
     const uint32_t t = blockIdx.x;
     if (t >= S.counters[8]) return;
     const uint32_t si = find_seg(S.tile0, nseg, t);
@@ -706,7 +706,7 @@ __device__ __forceinline__ void digits_of(const BucketBits& B, const uint64_t (&
 // every two warps), then one global atomic per digit.  Bound by the 8-byte key
 // read.
 constexpr int HIST_ROWS = LT_NT / 64;
-__global__ void __launch_bounds__(LT_NT) k_hist(SortState S, Seg* segs, uint32_t nseg) {
+__global__ void __launch_bounds__(LT_NT, 4) k_hist(SortState S, Seg* segs, uint32_t nseg) {
     __shared__ uint32_t hist[HIST_ROWS][DIGIT_MAX];
     __shared__ unsigned long long s_diff[LT_NT / 32];
     __shared__ BucketBits B;
@@ -1358,11 +1358,12 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
         const SmallSeg seg = segs[bi];
         const uint32_t start = seg.start, size = seg.size;
         uint32_t* lcp = S.lcp_out + start;
+        // the current group's strings; the whole segment first
+        uint32_t o[IPT];
+        uint64_t k[IPT];
         {
             const uint32_t* src = S.ord[seg.flags & F_PARITY] + start;
             const unsigned long long* ksrc = S.key[seg.flags & F_PARITY] + start;
-            uint32_t o[IPT];
-            uint64_t k[IPT];
 #pragma unroll
             for (int j = 0; j < IPT; ++j) {
                 const uint32_t i = threadIdx.x + j * NT;
@@ -1383,7 +1384,9 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
                 }
             }
         }
-        for (uint32_t x = threadIdx.x; x < NB; x += NT) M.cnt[x] = 0;
+#pragma unroll
+        for (int q = 0; q < PER; q += 4)
+            *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
         if (threadIdx.x == 0) {
             const uint2 g = group_pack(0, size, (seg.flags & F_ID) ? G_ID : G_PLAIN, seg.depth);
             s_nw = size <= 32;
@@ -1399,13 +1402,18 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
             const uint32_t bs = group_start(s_cur), bn = group_size(s_cur), dep = s_cur.y;
             uint32_t kind = group_kind(s_cur);
             if (threadIdx.x == 0) --s_ns;  // read again only after the next barrier
-            uint64_t k[IPT];
-            uint32_t o[IPT], br[IPT];
+            uint32_t br[IPT];
+            if (bn != size) {  // (the whole segment is still in registers)
 #pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                const uint32_t i = threadIdx.x + j * NT;
-                o[j] = i < bn ? M.id[bs + i] : 0u;
-                k[j] = i < bn ? (kind == G_ID ? (uint64_t)o[j] : M.key[bs + i]) : 0ull;
+                for (int j = 0; j < IPT; ++j) {
+                    const uint32_t i = threadIdx.x + j * NT;
+                    o[j] = i < bn ? M.id[bs + i] : 0u;
+                    k[j] = i < bn ? M.key[bs + i] : 0ull;
+                }
+            }
+            if (kind == G_ID) {
+#pragma unroll
+                for (int j = 0; j < IPT; ++j) k[j] = o[j];
             }
             if (kind == G_TIE) {
                 // the pivot: of 8 evenly spaced strings the one with the
@@ -1469,17 +1477,20 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
                 s_and[w] = (uint64_t)ahi << 32 | alo;
             }
             __syncthreads();
-            uint64_t diff;
-            {
-                uint64_t x = s_or[0], y = s_and[0];
-#pragma unroll
-                for (int v = 1; v < NW; ++v) {
-                    x |= s_or[v];
-                    y &= s_and[v];
+            if (w == 0) {
+                uint64_t x = lane < NW ? s_or[lane] : 0ull, y = lane < NW ? s_and[lane] : ~0ull;
+                const uint32_t dl = __reduce_or_sync(FULL, (uint32_t)x) ^ __reduce_and_sync(FULL, (uint32_t)y);
+                const uint32_t dh = __reduce_or_sync(FULL, (uint32_t)(x >> 32)) ^ __reduce_and_sync(FULL, (uint32_t)(y >> 32));
+                if (lane == 0) {
+                    constexpr uint32_t most = 31u - (uint32_t)__builtin_clz(NB);
+                    const uint64_t diff = (uint64_t)dh << 32 | dl;
+                    s_bits.nruns = 0;
+                    if (diff)
+                        bucket_bits(s_bits, diff, pseudo ? most : min(32u - (uint32_t)__clz(bn - 1) + 1u, most));
                 }
-                diff = x ^ y;
             }
-            if (diff == 0) {  // one key: equal strings, or the group goes deeper
+            __syncthreads();
+            if (s_bits.nruns == 0) {  // one key: equal strings, or the group goes deeper
                 if (threadIdx.x == 0) {
                     const uint64_t k0 = k[0];
                     M.stk[s_ns++] = key_ended(k0, pseudo) ? group_pack(bs, bn, G_ID, ref_of(S.a, o[0]).len)
@@ -1488,11 +1499,6 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
                 __syncthreads();
                 continue;
             }
-            if (threadIdx.x == 0) {
-                constexpr uint32_t most = 31u - (uint32_t)__builtin_clz(NB);
-                bucket_bits(s_bits, diff, pseudo ? most : min(32u - (uint32_t)__clz(bn - 1) + 1u, most));
-            }
-            __syncthreads();
             {
                 const uint32_t lo = s_bits.lo, nr = s_bits.nruns;
                 uint32_t x[IPT];
@@ -1644,7 +1650,9 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_s
                 }
             }
             // the next pass counts from zero
-            for (uint32_t x = threadIdx.x; x < NB; x += NT) M.cnt[x] = 0;
+#pragma unroll
+            for (int q = 0; q < PER; q += 4)
+                *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
             if (threadIdx.x == 0) s_nt = 0;  // pushed to again only after the next pass's barriers
         }

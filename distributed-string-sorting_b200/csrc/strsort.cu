@@ -1083,19 +1083,31 @@ __global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* se
 // buckets per string need, pick a bucket; shared atomics count them and hand
 // out places (the order inside a bucket does not matter, every bucket is
 // sorted by (key, id) afterwards); buckets of 2..8 strings are sorted by one
-// thread each, up to 32 by a warp, larger ones return to the CTA's stack.
+// thread each, up to 64 by a warp, larger ones return to the CTA's stack.
+// The first pass, which is all that most segments need, stands by itself: the
+// rest is one call behind it, whose registers would else cut into the first
+// pass's (1e8 strings in segments of about 700: 1.32 ms inlined, 1.18 ms as a
+// call, 1.03 ms with the five blocks per SM that then fit; six: 1.04).
+//
+// What bounds the groups that go deeper is latency, not instructions: a group
+// of the CTA takes a dozen barriers, of the warps a chain of loads per round.
+// So warps claim groups from a list, several small ones at a time in their 64
+// elements, and all lanes of a comparison step on together (text with repeats,
+// 9e6 strings: 32 elements and one group per warp, comparisons beyond 32 bytes
+// one lane after another: 5.4 ms; this: 3.8; groups up to 128 by a warp: 4.1).
 // Over keys with enough differing bits nearly all buckets hold one string, so
 // a string costs about 60 thread instructions; the stable byte passes with
 // match instructions and bitonic networks that this replaces took 26 warp
 // instructions per string.  B200, 32e6 strings in segments of about 700:
-// 1.12 -> 0.49 ms; a 4e6-string request whose segments are chains of nested
-// prefixes: 0.61 -> 0.18 ms; 9e6 suffixes of copied text: 9.2 -> 6.5 ms.
+// 1.12 -> 0.34 ms; a 4e6-string request whose segments are chains of nested
+// prefixes: 0.61 -> 0.17 ms; 9e6 suffixes of copied text: 9.2 -> 3.8 ms.
 constexpr unsigned FULL = 0xffffffffu;
 enum GroupKind : uint32_t { G_PLAIN = 0, G_TIE = 1, G_ID = 2, G_PSEUDO = 3 };  // G_TIE: keys still to be made
 // Pivot code of a string with LCP l: l below the pivot, CODE_MID for strings
 // equal to it (or to CODE_CAP bytes of it), 0xBFFF - l above it.
 constexpr uint32_t CODE_MID = 0x4000u, CODE_TOP = 0xBFFFu, CODE_CAP = 0x3FFEu;
 constexpr uint32_t TINY_MAX = 8;  // largest bucket one thread sorts
+constexpr uint32_t MID_MAX = 64;  // largest group that one warp sorts
 
 // LCP part of a pivot code (the pivot's own is above all others).
 __device__ __forceinline__ uint32_t code_l(uint32_t c) { return c <= CODE_MID ? c : CODE_TOP - c; }
@@ -1141,47 +1153,57 @@ __device__ __forceinline__ StrRef ref_of(const ArenaDev& a, uint32_t id) {
 }
 
 // Each active lane's LCP with its own pivot h, both strings sharing their
-// first d bytes; at most d + CODE_CAP.  32 bytes per lane first; lanes still
-// equal then go one after another, the whole warp reading 256 bytes of a pair
-// at a time.  Every lane of the warp calls it.
-__device__ __forceinline__ uint32_t warp_lcp(const ArenaDev& a, StrRef x, StrRef h, uint32_t d, bool active) {
+// first d bytes; at most d + CODE_CAP.  Lanes take 32 bytes of their own pair
+// at a time; once at most four are still equal these go one after another, the
+// whole warp reading 256 bytes of a pair at a time.  Every lane of the warp
+// calls it.
+__device__ __forceinline__ uint32_t warp_lcp(const uint8_t* chars, StrRef x, StrRef h, uint32_t d, bool active) {
     uint32_t l = d;
     bool open = active;
-    if (active) {
-        uint64_t u[4], v[4];
-        key_words<4>(a.chars, x.off, x.len, d, 4, u);
-        key_words<4>(a.chars, h.off, h.len, d, 4, v);
-        l = d + 32;
+    uint32_t todo;
+    do {
+        if (open) {
+            const uint32_t at = l;
+            uint64_t u[4], v[4];
+            key_words<4>(chars, x.off, x.len, at, 4, u);
+            key_words<4>(chars, h.off, h.len, at, 4, v);
+            l = at + 32;
 #pragma unroll
-        for (int w = 3; w >= 0; --w) {  // the first word that differs or ends wins
-            if (u[w] != v[w]) {
-                l = d + 8 * w + key_lcp(u[w], v[w]);
-                open = false;
-            } else if (zero_byte(u[w]) < 8) {
-                l = d + 8 * w + zero_byte(u[w]);
+            for (int w = 3; w >= 0; --w) {  // the first word that differs or ends wins
+                if (u[w] != v[w]) {
+                    l = at + 8 * w + key_lcp(u[w], v[w]);
+                    open = false;
+                } else if (zero_byte(u[w]) < 8) {
+                    l = at + 8 * w + zero_byte(u[w]);
+                    open = false;
+                }
+            }
+            if (l >= d + CODE_CAP) {
+                l = d + CODE_CAP;
                 open = false;
             }
         }
-    }
+        todo = __ballot_sync(FULL, open);
+    } while (__popc(todo) > 4);
     const uint32_t lane = threadIdx.x & 31;
-    for (uint32_t todo = __ballot_sync(FULL, open); todo; todo &= todo - 1) {
+    for (; todo; todo &= todo - 1) {
         const int src = __ffs(todo) - 1;
         const uint64_t ox = __shfl_sync(FULL, x.off, src), oh = __shfl_sync(FULL, h.off, src);
         const uint32_t lx = __shfl_sync(FULL, x.len, src), lh = __shfl_sync(FULL, h.len, src);
-        const uint32_t d0 = __shfl_sync(FULL, d, src);
-        uint32_t at = d0 + 32;
+        const uint32_t cap = __shfl_sync(FULL, d, src) + CODE_CAP;
+        uint32_t at = __shfl_sync(FULL, l, src);
         for (;; at += 256) {
-            if (at >= d0 + CODE_CAP) {
-                at = d0 + CODE_CAP;
+            if (at >= cap) {
+                at = cap;
                 break;
             }
             const uint32_t p = at + 8 * lane;
-            const uint64_t u = key8(a.chars, ox, lx, p), v = key8(a.chars, oh, lh, p);
+            const uint64_t u = key8(chars, ox, lx, p), v = key8(chars, oh, lh, p);
             const uint32_t e = u != v ? key_lcp(u, v) : zero_byte(u);
             const uint32_t hit = __ballot_sync(FULL, e < 8);
             if (hit) {
                 const int f = __ffs(hit) - 1;
-                at = min(at + 8 * f + __shfl_sync(FULL, e, f), d0 + CODE_CAP);
+                at = min(at + 8 * f + __shfl_sync(FULL, e, f), cap);
                 break;
             }
         }
@@ -1201,111 +1223,208 @@ __device__ __forceinline__ uint64_t pseudo_key(const ArenaDev& a, StrRef x, StrR
     return (uint64_t)c << 48 | bx >> 16;
 }
 
-// Compare-exchange network over the first P (a power of two) lanes.
-template <bool GRP>
-__device__ __forceinline__ void warp_network(uint32_t P, uint32_t& grp, uint64_t& key, uint32_t& id, uint32_t& dep) {
+// Pseudo key of string id against pivot hid of a group of depth d, and
+// whether the comparison ended at the cap; every lane of the warp calls it.
+struct PivotKey {
+    uint64_t key;
+    bool capped;
+};
+__device__ __forceinline__ PivotKey pivot_key(const ArenaDev& a, uint32_t id, uint32_t hid, uint32_t d, bool active) {
+    StrRef x{0, 0}, h{0, 0};
+    if (active) {
+        x = ref_of(a, id);
+        h = ref_of(a, hid);
+    }
+    const uint32_t l = warp_lcp(a.chars, x, h, d, active);
+    PivotKey r{0, false};
+    if (active) {
+        r.key = pseudo_key(a, x, h, l, d);
+        r.capped = l >= d + CODE_CAP;
+    }
+    return r;
+}
+
+// Compare-exchange network on (grp, key, id) over the first P (a power of two)
+// elements of a warp's 32 * I; element 32 * q + lane is item q of the lane.
+template <int I>
+__device__ __forceinline__ void warp_network(uint32_t P, uint32_t (&grp)[I], uint64_t (&key)[I], uint32_t (&id)[I]) {
     const uint32_t lane = threadIdx.x & 31;
-#pragma unroll
-    for (uint32_t k = 2; k <= 32; k <<= 1) {
-        if (k > P) break;
-#pragma unroll
+#pragma unroll 1
+    for (uint32_t k = 2; k <= P; k <<= 1) {
+#pragma unroll 1
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            const uint64_t pk = __shfl_xor_sync(FULL, key, j);
-            const uint32_t po = __shfl_xor_sync(FULL, id, j);
-            const bool want_min = ((lane & k) == 0) == ((lane & j) == 0);
-            if (GRP) {
-                const uint32_t pg = __shfl_xor_sync(FULL, grp, j), pd = __shfl_xor_sync(FULL, dep, j);
-                const bool less = pg < grp || (pg == grp && (pk < key || (pk == key && po < id)));
-                if (less == want_min) {
-                    grp = pg;
-                    key = pk;
-                    id = po;
-                    dep = pd;
+            if (I > 1 && j >= 32) {
+#pragma unroll
+                for (int q = 0; q < I; ++q) {
+#pragma unroll
+                    for (int r = q + 1; r < I; ++r) {
+                        if ((uint32_t)(q ^ r) * 32 != j) continue;
+                        const bool less = grp[r] < grp[q] || (grp[r] == grp[q] && (key[r] < key[q] || (key[r] == key[q] && id[r] < id[q])));
+                        if (less == ((q * 32 & k) == 0)) {
+                            const uint32_t tg = grp[q], to = id[q];
+                            const uint64_t tk = key[q];
+                            grp[q] = grp[r];
+                            key[q] = key[r];
+                            id[q] = id[r];
+                            grp[r] = tg;
+                            key[r] = tk;
+                            id[r] = to;
+                        }
+                    }
                 }
-            } else {
-                const bool less = pk < key || (pk == key && po < id);
+                continue;
+            }
+#pragma unroll
+            for (int q = 0; q < I; ++q) {
+                if (I > 1 && (uint32_t)q * 32 >= P) break;
+                const uint64_t pk = __shfl_xor_sync(FULL, key[q], j);
+                const uint32_t po = __shfl_xor_sync(FULL, id[q], j), pg = __shfl_xor_sync(FULL, grp[q], j);
+                const bool want_min = (((q * 32 + lane) & k) == 0) == ((lane & j) == 0);
+                const bool less = pg < grp[q] || (pg == grp[q] && (pk < key[q] || (pk == key[q] && po < id[q])));
                 if (less == want_min) {
-                    key = pk;
-                    id = po;
+                    grp[q] = pg;
+                    key[q] = pk;
+                    id[q] = po;
                 }
             }
         }
     }
 }
 
-// A group of size <= 32: lane i < size holds an id and, unless kind is G_TIE
-// or G_ID, its key.  On return lane i holds the i-th smallest string; lcp[i]
-// (1 <= i < size) gets the LCP with the predecessor (depth itself for G_ID).
-__device__ __forceinline__ void warp_group(const ArenaDev& a, uint32_t size, uint32_t depth, uint32_t kind,
-                                           uint64_t key, uint32_t& id, uint32_t* lcp) {
+// Groups of one warp, back to back in its n <= 32 * I elements.  An element
+// holds the element at which its group starts (grp), the group's depth and
+// kind, its own place pos (with its LCP at lcp[pos]), a string of the group
+// and, unless kind is G_TIE or G_ID, the string's key.  On return the ids of
+// each group are in order and every element but a group's first has its LCP
+// with its predecessor (the depth itself for G_ID).
+//
+// All groups go through each round together: sort by (group, key, id), then
+// every run of equal keys that has not ended becomes a group of its own and
+// compares with its first string.
+template <int I>
+__device__ __forceinline__ void warp_groups(const ArenaDev& a, uint32_t n, uint32_t (&grp)[I], uint32_t (&dep)[I],
+                                            uint32_t (&kind)[I], const uint32_t (&pos)[I], uint64_t (&key)[I],
+                                            uint32_t (&id)[I], uint32_t* lcp) {
     const uint32_t lane = threadIdx.x & 31;
-    const bool valid = lane < size;
-    const uint32_t P = size <= 2 ? 2u : 1u << (32 - __clz(size - 1));
-    uint32_t grp = valid ? 0u : 0xFFFFFFFFu;
-    uint32_t dep = depth;
-    bool pseudo = kind == G_PSEUDO;
-    if (!valid) {
-        key = ~0ull;
-        id = 0xFFFFFFFFu;
-    } else if (kind == G_ID) {
-        key = 0;
+    const uint32_t P = n <= 2 ? 2u : 1u << (32 - __clz(n - 1));
+    uint32_t rs[I];  // start of the element's run
+    bool unres[I];   // the run goes on
+    bool sort = false;
+#pragma unroll
+    for (int q = 0; q < I; ++q) {
+        const bool valid = q * 32 + lane < n;
+        if (!valid) {
+            grp[q] = 0xFFFFFFFFu;
+            id[q] = 0xFFFFFFFFu;
+            kind[q] = G_TIE;
+        }
+        if (kind[q] == G_TIE || kind[q] == G_ID) key[q] = 0;
+        rs[q] = grp[q];
+        unres[q] = valid && kind[q] == G_TIE;
+        sort = sort || kind[q] != G_TIE;
     }
-    bool unres = valid && kind == G_TIE;
-    uint32_t rs = 0;
-    bool first = true;
+    sort = __any_sync(FULL, sort);
     for (;;) {
-        if (kind != G_TIE || !first) {
-            if (first) warp_network<false>(P, grp, key, id, dep);
-            else warp_network<true>(P, grp, key, id, dep);
-            const uint32_t qg = __shfl_up_sync(FULL, grp, 1);
-            const uint64_t qk = __shfl_up_sync(FULL, key, 1);
-            const bool head = lane == 0 || qg != grp || qk != key;
-            if (kind == G_ID) {
-                if (valid && lane > 0) lcp[lane] = depth;
-                return;
+        if (sort) {
+            warp_network<I>(P, grp, key, id);
+            uint32_t heads[I];
+            bool head[I];
+#pragma unroll
+            for (int q = 0; q < I; ++q) {
+                const uint32_t e = q * 32 + lane;
+                uint64_t qk = __shfl_up_sync(FULL, key[q], 1);
+                if (I > 1 && q > 0) {
+                    const uint64_t last = __shfl_sync(FULL, key[q > 0 ? q - 1 : 0], 31);
+                    if (lane == 0) qk = last;
+                }
+                const bool valid = e < n, inner = valid && e != grp[q];
+                const bool pseudo = kind[q] == G_PSEUDO;
+                head[q] = !inner || qk != key[q];
+                if (inner && kind[q] != G_TIE) {
+                    if (kind[q] == G_ID) lcp[pos[q]] = dep[q];
+                    else if (qk != key[q]) lcp[pos[q]] = group_lcp(qk, key[q], dep[q], pseudo);
+                    else if (key_ended(key[q], pseudo)) lcp[pos[q]] = ref_of(a, id[q]).len;  // equal strings
+                }
+                heads[q] = __ballot_sync(FULL, head[q]);
             }
-            // dep of a resolved string is no longer used; neighbours in one
-            // group share it
-            if (valid && lane > 0 && qg == grp) {
-                if (qk != key) lcp[lane] = group_lcp(qk, key, dep, pseudo);
-                else if (key_ended(key, pseudo)) lcp[lane] = ref_of(a, id).len;  // equal strings
+#pragma unroll
+            for (int q = 0; q < I; ++q) {
+                const uint32_t e = q * 32 + lane;
+                const bool valid = e < n;
+#pragma unroll
+                for (int r = 0; r <= q; ++r) {
+                    const uint32_t m = r < q ? heads[r] : heads[q] & ((2u << lane) - 1u);
+                    if (m) rs[q] = r * 32 + 31u - __clz(m);
+                }
+                const bool next_head = lane < 31 ? (heads[q] >> (lane + 1) & 1u) != 0
+                                                 : (q + 1 < I ? (heads[q + 1 < I ? q + 1 : 0] & 1u) != 0 : true);
+                unres[q] = valid && kind[q] != G_ID && !(head[q] && next_head) &&
+                           (kind[q] == G_TIE || !key_ended(key[q], kind[q] == G_PSEUDO));
+                if (valid) grp[q] = unres[q] ? rs[q] : e;  // a resolved string stays at its place
             }
-            const uint32_t heads = __ballot_sync(FULL, head);
-            rs = 31u - __clz(heads & ((2u << lane) - 1u));
-            const bool next_head = lane == 31 ? true : ((heads >> (lane + 1)) & 1u) != 0;
-            const bool multi = !head || (!next_head && lane + 1 < size);
-            unres = valid && multi && !key_ended(key, pseudo);
-            if (valid) grp = rs;
         }
-        if (!__any_sync(FULL, unres)) return;
-        // every unresolved run goes on against its head
-        const uint32_t nd = first && kind == G_TIE ? depth : tie_depth(key, dep, pseudo);
-        const uint32_t hid = __shfl_sync(FULL, id, rs);
-        StrRef x{0, 0}, h{0, 0};
-        if (unres) {
-            x = ref_of(a, id);
-            h = ref_of(a, hid);
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < I; ++q) any = any || unres[q];
+        if (!__any_sync(FULL, any)) return;
+        // every unresolved run goes on against its first string
+        uint32_t hid[I];
+#pragma unroll
+        for (int q = 0; q < I; ++q) {
+            hid[q] = 0;
+#pragma unroll
+            for (int r = 0; r <= q; ++r) {
+                const uint32_t t = __shfl_sync(FULL, id[r], rs[q] & 31u);
+                if (rs[q] >> 5 == (uint32_t)r) hid[q] = t;
+            }
         }
-        const bool cmp = unres && lane != rs;
-        const uint32_t l = warp_lcp(a, x, h, nd, cmp);
-        // resolved strings keep a key that orders them among themselves
-        if (unres) {
-            dep = nd;
-            key = cmp ? pseudo_key(a, x, h, l, nd) : (uint64_t)CODE_MID << 48;
-        } else if (valid) {
-            key = 0;  // alone in its group, or equal strings in id order
+        bool capped[I];
+#pragma unroll
+        for (int q = 0; q < I; ++q) capped[q] = false;
+#pragma unroll 1
+        for (int q = 0; q < I; ++q) {  // one copy of the comparison's code: warps are at different places in it
+            uint32_t qi = id[0], qh = hid[0], qd = dep[0], qt = kind[0], qr = rs[0];
+            uint64_t qk = key[0];
+            bool qu = unres[0];
+#pragma unroll
+            for (int r = 1; r < I; ++r)
+                if (r == q) {
+                    qi = id[r];
+                    qh = hid[r];
+                    qd = dep[r];
+                    qt = kind[r];
+                    qr = rs[r];
+                    qk = key[r];
+                    qu = unres[r];
+                }
+            if (I > 1 && !__any_sync(FULL, qu)) continue;
+            if (qt != G_TIE) qd = tie_depth(qk, qd, qt == G_PSEUDO);
+            const bool cmp = qu && q * 32 + lane != qr;
+            const PivotKey t = pivot_key(a, qi, qh, qd, cmp);
+#pragma unroll
+            for (int r = 0; r < I; ++r)
+                if (r == q && qu) {
+                    dep[r] = qd;
+                    kind[r] = G_PSEUDO;
+                    key[r] = cmp ? t.key : (uint64_t)CODE_MID << 48;
+                    capped[r] = cmp && t.capped;
+                }
         }
-        // the head shares its end with the strings that equal it, or the cap
-        const uint32_t capped = __ballot_sync(FULL, cmp && l >= nd + CODE_CAP);
-        const uint32_t run = __match_any_sync(FULL, unres ? rs : 32u + lane);
-        if (unres && lane == rs && (capped & run)) key |= 0x010101010101ull;
-        pseudo = true;
-        first = false;
+        // a run's first string keeps to those that agree with it up to the cap
+#pragma unroll
+        for (int q = 0; q < I; ++q)
+            for (uint32_t m = __ballot_sync(FULL, capped[q]); m; m &= m - 1) {
+                const uint32_t f = __shfl_sync(FULL, rs[q], __ffs(m) - 1);
+#pragma unroll
+                for (int r = 0; r <= q; ++r)
+                    if (f == r * 32 + lane) key[r] |= 0x010101010101ull;
+            }
+        sort = true;
     }
 }
 
 // Segments of 2..32 strings: one warp each, four per CTA.
-__global__ void __launch_bounds__(128) k_warp_segs(SortState S, const SmallSeg* segs, uint32_t nseg) {
+__global__ void __launch_bounds__(128) k_warp_segs(const __grid_constant__ SortState S, const SmallSeg* segs, uint32_t nseg) {
     for (uint32_t si = blockIdx.x * 4 + (threadIdx.x >> 5); si < nseg; si += gridDim.x * 4) {
         const uint32_t lane = threadIdx.x & 31;
         const SmallSeg seg = segs[si];
@@ -1317,8 +1436,12 @@ __global__ void __launch_bounds__(128) k_warp_segs(SortState S, const SmallSeg* 
             if (seg.flags & F_ID) key = 0;
             else key = (seg.flags & F_KEYS) ? S.key[seg.flags & F_PARITY][seg.start + lane] : key8_of(S.a, id, seg.depth);
         }
-        warp_group(S.a, seg.size, seg.depth, (seg.flags & F_ID) ? G_ID : G_PLAIN, key, id, S.lcp_out + seg.start);
-        if (lane < seg.size) S.ord_out[seg.start + lane] = id;
+        uint32_t grp1[1] = {0}, dep1[1] = {seg.depth}, kind1[1] = {(seg.flags & F_ID) ? (uint32_t)G_ID : (uint32_t)G_PLAIN};
+        const uint32_t pos1[1] = {lane};
+        uint64_t key1[1] = {key};
+        uint32_t id1[1] = {id};
+        warp_groups<1>(S.a, seg.size, grp1, dep1, kind1, pos1, key1, id1, S.lcp_out + seg.start);
+        if (lane < seg.size) S.ord_out[seg.start + lane] = id1[0];
     }
 }
 
@@ -1331,359 +1454,412 @@ __device__ __forceinline__ uint32_t group_start(uint2 g) { return g.x & 0xFFFu; 
 __device__ __forceinline__ uint32_t group_size(uint2 g) { return ((g.x >> 12) & 0xFFFu) + 1; }
 __device__ __forceinline__ uint32_t group_kind(uint2 g) { return g.x >> 24; }
 
-template <int CAP>
+template <int CAP, int NT>
 struct SegSmem {
+    static constexpr int NW = NT / 32;
     static constexpr int NB = CAP <= 256 ? 1024 : CAP <= 1024 ? 2048 : 4096;  // buckets
     unsigned long long key[CAP];
     uint32_t cnt[NB + 4];  // bucket counts, then starts (the last one the group's size)
     uint32_t id[CAP];
     uint2 wl[CAP / 2];         // groups for the warps
     uint32_t tl[CAP / 2];      // the pass's buckets of 2..TINY_MAX strings
-    uint2 stk[CAP / 32 + 2];   // groups for the CTA
+    uint2 stk[CAP / MID_MAX + 2];  // groups for the CTA
+    // per pass: OR and AND of the warps' keys, the warps' counts, the LCP sums of the pivot's candidates
+    unsigned long long orv[NW], andv[NW];
+    uint32_t sum[NW], piv[8];
+    BucketBits bits;
+    uint32_t ns, nw, nt, claim;  // lengths of stk, wl and tl; groups of wl taken
 };
 
+// The keys of a group that goes deeper: pivot, then every string's pseudo key.
 template <int CAP, int NT>
-__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 4 : 8) k_seg_sort(SortState S,
+__device__ __forceinline__ void cta_pivot_keys(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bs, uint32_t bn, uint32_t dep) {
+    constexpr int NW = NT / 32, IPT = CAP / NT;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+                    // the pivot: of 8 evenly spaced strings the one with the
+                    // largest sum of LCPs (256 bytes at most) with the others
+                    for (uint32_t c = w; c < 8; c += NW) {
+                        const StrRef x = ref_of(S.a, M.id[bs + c * bn / 8]);
+                        const uint64_t kx = key8(S.a.chars, x.off, x.len, dep + 8 * lane);
+                        uint32_t sum = 0;
+    #pragma unroll 4
+                        for (uint32_t q = 0; q < 8; ++q) {
+                            const StrRef y = ref_of(S.a, M.id[bs + q * bn / 8]);
+                            const uint64_t ky = key8(S.a.chars, y.off, y.len, dep + 8 * lane);
+                            const uint32_t e = kx != ky ? key_lcp(kx, ky) : 8u;
+                            const uint32_t hit = __ballot_sync(FULL, e < 8);
+                            const int f = hit ? __ffs(hit) - 1 : 0;
+                            const uint32_t ef = __shfl_sync(FULL, e, f);
+                            sum += hit ? 8 * f + ef : 256u;
+                        }
+                        if (lane == 0) M.piv[c] = sum << 3 | c;
+                    }
+                    __syncthreads();
+                    uint32_t best = 0;
+    #pragma unroll
+                    for (int c = 0; c < 8; ++c) best = max(best, M.piv[c]);
+                    const uint32_t pid = M.id[bs + (best & 7u) * bn / 8];
+                    const StrRef h = ref_of(S.a, pid);
+    #pragma unroll 1
+                    for (int j = 0; j < IPT; ++j) {
+                        const uint32_t i = threadIdx.x + j * NT;
+                        if (i - lane >= bn) break;  // the same for the whole warp
+                        const bool v = i < bn;
+                        StrRef x{0, 0};
+                        uint32_t oj = v ? M.id[bs + i] : 0u;
+                        if (v) x = ref_of(S.a, oj);
+                        const uint32_t l = warp_lcp(S.a.chars, x, h, dep, v);
+                        if (v) M.key[bs + i] = pseudo_key(S.a, x, h, l, dep);
+                    }
+}
+
+// The groups on the warps' list, claimed up to 8 at a time; as many of these
+// together as fit into a warp's 64 elements.
+template <int CAP, int NT>
+__device__ __forceinline__ void warps_sort_groups(const SortState& S, SegSmem<CAP, NT>& M, uint32_t* lcp) {
+    const uint32_t ng = M.nw, lane = threadIdx.x & 31, per = min(8u, 1 + ng / (NT / 16));
+    for (;;) {
+        uint32_t e0 = 0;
+        if (lane == 0) e0 = atomicAdd(&M.claim, per);
+        e0 = __shfl_sync(FULL, e0, 0);
+        if (e0 >= ng) break;
+        uint2 g = make_uint2(0, 0);
+        uint32_t left = min(per, ng - e0), sz = 0;  // lane t < left: the t-th group still to be sorted
+        if (lane < left) {
+            g = M.wl[e0 + lane];
+            sz = group_size(g);
+        }
+        while (left) {
+            uint32_t end = sz;  // inclusive sums of the sizes
+#pragma unroll
+            for (int off = 1; off < 8; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, end, off);
+                if (lane >= (uint32_t)off) end += y;
+            }
+            const uint32_t take = __popc(__ballot_sync(FULL, lane < left && end <= 64));
+            const uint32_t n = __shfl_sync(FULL, end, take - 1);
+            uint32_t grp[2], dep[2], kind[2], pos[2], id[2];
+            uint64_t key[2];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const uint32_t e = q * 32 + lane;
+                uint32_t t = 0;  // the element's group
+                for (uint32_t r = 0; r + 1 < take; ++r) t += e >= __shfl_sync(FULL, end, r);
+                const uint32_t gx = __shfl_sync(FULL, g.x, t);
+                grp[q] = __shfl_sync(FULL, end - sz, t);
+                dep[q] = __shfl_sync(FULL, g.y, t);
+                kind[q] = gx >> 24;
+                pos[q] = (gx & 0xFFFu) + e - grp[q];
+                id[q] = e < n ? M.id[pos[q]] : 0u;
+                key[q] = e < n ? M.key[pos[q]] : 0ull;
+            }
+            warp_groups<2>(S.a, n, grp, dep, kind, pos, key, id, lcp);
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                if (q * 32 + lane < n) M.id[pos[q]] = id[q];
+            left -= take;
+            g.x = __shfl_down_sync(FULL, g.x, take);
+            g.y = __shfl_down_sync(FULL, g.y, take);
+            sz = __shfl_down_sync(FULL, sz, take);
+            if (lane >= left) sz = 0;
+        }
+    }
+}
+
+// One bucket pass over the CTA's group at [bs, bs + bn): thread t holds its
+// strings t, t + NT, ... (o) and their keys (k).  Every count in cnt is zero
+// before and after.  FIRST: the whole segment, not yet in shared memory, with
+// plain keys or ids.
+template <int CAP, int NT, bool FIRST>
+__device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bs, uint32_t bn, uint32_t dep,
+                                         uint32_t kind, const uint32_t (&o)[CAP / NT], const uint64_t (&k)[CAP / NT],
+                                         uint32_t* lcp) {
+    constexpr int NW = NT / 32, IPT = CAP / NT, NB = SegSmem<CAP, NT>::NB, PER = NB / NT;
+    const ArenaDev& a = S.a;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t br[IPT];
+    const bool pseudo = !FIRST && kind == G_PSEUDO;
+    // the bits in which the keys differ
+    uint64_t vo = 0, va = ~0ull;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j)
+        if (threadIdx.x + j * NT < bn) {
+            const uint64_t t = level_key(k[j], pseudo);
+            vo |= t;
+            va &= t;
+        }
+    const uint32_t olo = __reduce_or_sync(FULL, (uint32_t)vo), ohi = __reduce_or_sync(FULL, (uint32_t)(vo >> 32));
+    const uint32_t alo = __reduce_and_sync(FULL, (uint32_t)va);
+    const uint32_t ahi = __reduce_and_sync(FULL, (uint32_t)(va >> 32));
+    if (lane == 0) {
+        M.orv[w] = (uint64_t)ohi << 32 | olo;
+        M.andv[w] = (uint64_t)ahi << 32 | alo;
+    }
+    __syncthreads();
+    if (w == 0) {
+        uint64_t x = lane < NW ? M.orv[lane] : 0ull, y = lane < NW ? M.andv[lane] : ~0ull;
+        const uint32_t dl = __reduce_or_sync(FULL, (uint32_t)x) ^ __reduce_and_sync(FULL, (uint32_t)y);
+        const uint32_t dh = __reduce_or_sync(FULL, (uint32_t)(x >> 32)) ^ __reduce_and_sync(FULL, (uint32_t)(y >> 32));
+        if (lane == 0) {
+            constexpr uint32_t most = 31u - (uint32_t)__builtin_clz(NB);
+            const uint64_t diff = (uint64_t)dh << 32 | dl;
+            M.bits.nruns = 0;
+            if (diff)
+                bucket_bits(M.bits, diff, pseudo ? most : min(32u - (uint32_t)__clz(bn - 1) + 1u, most));
+        }
+    }
+    __syncthreads();
+    if (M.bits.nruns == 0) {  // one key: equal strings, or the group goes deeper
+        if (FIRST) {
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) {
+                const uint32_t i = threadIdx.x + j * NT;
+                if (i < bn) M.id[i] = o[j];
+            }
+        }
+        if (threadIdx.x == 0) {
+            const uint64_t k0 = k[0];
+            const uint2 g = key_ended(k0, pseudo) ? group_pack(bs, bn, G_ID, ref_of(a, o[0]).len)
+                                                  : group_pack(bs, bn, G_TIE, tie_depth(k0, dep, pseudo));
+            if (bn <= MID_MAX) M.wl[M.nw++] = g;
+            else M.stk[M.ns++] = g;
+        }
+        __syncthreads();
+        return;
+    }
+    {
+        const uint32_t lo = M.bits.lo, nr = M.bits.nruns;
+        uint32_t x[IPT];
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            x[j] = (uint32_t)(k[j] >> lo);
+            br[j] = 0;
+        }
+        for (uint32_t r = 0; r < nr; ++r) {
+            const uint32_t sh = M.bits.sh[r], mask = M.bits.mask[r];
+            if (M.bits.wide) {
+#pragma unroll
+                for (int j = 0; j < IPT; ++j) br[j] |= (uint32_t)(k[j] >> (lo + sh)) & mask;
+            } else {
+#pragma unroll
+                for (int j = 0; j < IPT; ++j) br[j] |= (x[j] >> sh) & mask;
+            }
+        }
+    }
+    // counts; br: the bucket and, above it, the place inside it
+#pragma unroll
+    for (int j = 0; j < IPT; ++j)
+        if (threadIdx.x + j * NT < bn) br[j] |= atomicAdd(&M.cnt[br[j]], 1u) << 16;
+    __syncthreads();
+    {
+        uint32_t v[PER], sum = 0;
+#pragma unroll
+        for (int q = 0; q < PER; q += 4) {
+            const uint4 c = *reinterpret_cast<const uint4*>(&M.cnt[threadIdx.x * PER + q]);
+            v[q] = c.x;
+            v[q + 1] = c.y;
+            v[q + 2] = c.z;
+            v[q + 3] = c.w;
+            sum += c.x + c.y + c.z + c.w;
+        }
+        uint32_t x = sum;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, x, off);
+            if (lane >= (uint32_t)off) x += y;
+        }
+        if (lane == 31) M.sum[w] = x;
+        __syncthreads();
+        uint32_t run = x - sum;
+#pragma unroll
+        for (int q = 0; q < NW; ++q)
+            if ((uint32_t)q < w) run += M.sum[q];
+#pragma unroll
+        for (int q = 0; q < PER; q += 4) {
+            uint4 c;
+            c.x = run;
+            c.y = c.x + v[q];
+            c.z = c.y + v[q + 1];
+            c.w = c.z + v[q + 2];
+            run = c.w + v[q + 3];
+            *reinterpret_cast<uint4*>(&M.cnt[threadIdx.x * PER + q]) = c;
+        }
+        if (threadIdx.x == NT - 1) M.cnt[NB] = run;
+    }
+    __syncthreads();
+    // places (a thread holds its strings, so the group is permuted in
+    // place); only the counts' sum bounds a place, never taken else
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+        if (threadIdx.x + j * NT >= bn) continue;
+        const uint32_t at = M.cnt[br[j] & 0xFFFFu] + (br[j] >> 16);
+        if (at >= bn) {
+            bad = true;
+            continue;
+        }
+        M.key[bs + at] = k[j];
+        M.id[bs + at] = o[j];
+    }
+    if (bad) atomicExch(&S.counters[10], 1u);
+    __syncthreads();
+    // each bucket's first string: the LCP with the bucket before (any
+    // of its strings), and who sorts the bucket
+    const bool all = M.bits.all != 0, mixed = pseudo && M.bits.mixed;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+        if (threadIdx.x + j * NT >= bn || (br[j] >> 16) != 0) continue;
+        const uint32_t b = br[j] & 0xFFFFu, s0 = M.cnt[b], c = M.cnt[b + 1] - s0;
+        if (s0) {
+            uint64_t kp = M.key[bs + s0 - 1], kn = k[j];
+            if (mixed) {  // the codes next to the boundary: the last of the bucket before, this one's first
+                const uint32_t bp = bucket_of_key(M.bits, kp);
+                for (uint32_t x = s0 - 1; x > 0 && bucket_of_key(M.bits, M.key[bs + x - 1]) == bp; --x)
+                    kp = max(kp, (uint64_t)M.key[bs + x - 1]);
+                for (uint32_t x = 0; x < c; ++x) kn = min(kn, (uint64_t)M.key[bs + s0 + x]);
+            }
+            lcp[bs + s0] = kind == G_ID ? dep : group_lcp(kp, kn, dep, pseudo);
+        }
+        if (c < 2) continue;
+        if (c <= TINY_MAX) {
+            M.tl[atomicAdd(&M.nt, 1u)] = s0 | c << 16;
+            continue;
+        }
+        uint32_t gk = kind, gd = dep;
+        if (kind != G_ID && all) {  // one key in the bucket
+            const bool ended = key_ended(k[j], pseudo);
+            gk = ended ? G_ID : G_TIE;
+            gd = ended ? ref_of(a, o[j]).len : tie_depth(k[j], dep, pseudo);
+        }
+        const uint2 g = group_pack(bs + s0, c, gk, gd);
+        if (c <= MID_MAX) M.wl[atomicAdd(&M.nw, 1u)] = g;
+        else M.stk[atomicAdd(&M.ns, 1u)] = g;
+    }
+    __syncthreads();
+    // buckets of 2..TINY_MAX strings: insertion sort on (key, id), then
+    // the neighbours' LCPs and the runs that go deeper
+    const uint32_t nt = M.nt;
+    for (uint32_t e = threadIdx.x; e < nt; e += NT) {
+        const uint32_t s0 = bs + (M.tl[e] & 0xFFFFu), c = M.tl[e] >> 16;
+        for (uint32_t x = 1; x < c; ++x) {
+            const uint64_t kx = M.key[s0 + x];
+            const uint32_t ox = M.id[s0 + x];
+            uint32_t y = x;
+            for (; y > 0; --y) {
+                const uint64_t ky = M.key[s0 + y - 1];
+                const uint32_t oy = M.id[s0 + y - 1];
+                if (ky < kx || (ky == kx && oy < ox)) break;
+                M.key[s0 + y] = ky;
+                M.id[s0 + y] = oy;
+            }
+            M.key[s0 + y] = kx;
+            M.id[s0 + y] = ox;
+        }
+        if (kind == G_ID) {
+            for (uint32_t x = 1; x < c; ++x) lcp[s0 + x] = dep;
+            continue;
+        }
+        uint64_t kp = M.key[s0];
+        uint32_t r0 = 0;  // start of the run of equal keys
+        for (uint32_t x = 1; x <= c; ++x) {
+            const uint64_t kx = x < c ? M.key[s0 + x] : ~kp;
+            if (kx == kp) continue;
+            if (x - r0 > 1) {
+                if (key_ended(kp, pseudo)) {
+                    const uint32_t len = ref_of(a, M.id[s0 + r0]).len;
+                    for (uint32_t y = r0 + 1; y < x; ++y) lcp[s0 + y] = len;
+                } else {
+                    M.wl[atomicAdd(&M.nw, 1u)] = group_pack(s0 + r0, x - r0, G_TIE, tie_depth(kp, dep, pseudo));
+                }
+            }
+            if (x < c) lcp[s0 + x] = group_lcp(kp, kx, dep, pseudo);
+            kp = kx;
+            r0 = x;
+        }
+    }
+    // the next pass counts from zero
+#pragma unroll
+    for (int q = 0; q < PER; q += 4)
+        *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    if (threadIdx.x == 0) M.nt = 0;  // pushed to again only after the next pass's barriers
+}
+
+// Everything after a segment's first pass: the CTA's stack of groups, then the
+// warps' list.
+template <int CAP, int NT>
+__device__ __noinline__ void sort_rest(const SortState& S, uint32_t* lcp) {
+    constexpr int IPT = CAP / NT;
+    extern __shared__ __align__(16) unsigned char smem[];
+    SegSmem<CAP, NT>& M = *reinterpret_cast<SegSmem<CAP, NT>*>(smem);
+    while (M.ns) {
+        const uint2 g = M.stk[M.ns - 1];
+        const uint32_t bs = group_start(g), bn = group_size(g), dep = g.y;
+        uint32_t kind = group_kind(g);
+        __syncthreads();
+        if (threadIdx.x == 0) --M.ns;  // read again only after the pass's barriers
+        if (kind == G_TIE) {
+            cta_pivot_keys<CAP, NT>(S, M, bs, bn, dep);
+            kind = G_PSEUDO;  // a thread reads back only the keys it wrote
+        }
+        uint32_t o[IPT];
+        uint64_t k[IPT];
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) {
+            const uint32_t i = threadIdx.x + j * NT;
+            o[j] = i < bn ? M.id[bs + i] : 0u;
+            k[j] = i < bn ? (kind == G_ID ? o[j] : M.key[bs + i]) : 0ull;
+        }
+        cta_pass<CAP, NT, false>(S, M, bs, bn, dep, kind, o, k, lcp);
+    }
+    if (M.nw) warps_sort_groups<CAP, NT>(S, M, lcp);
+}
+
+template <int CAP, int NT>
+__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 5 : 8) k_seg_sort(const __grid_constant__ SortState S,
                                                                                        const SmallSeg* segs,
                                                                                        uint32_t nseg) {
-    constexpr int NW = NT / 32, IPT = CAP / NT, NB = SegSmem<CAP>::NB, PER = NB / NT;
+    constexpr int IPT = CAP / NT, PER = SegSmem<CAP, NT>::NB / NT;
     extern __shared__ __align__(16) unsigned char smem[];
-    SegSmem<CAP>& M = *reinterpret_cast<SegSmem<CAP>*>(smem);
-    __shared__ unsigned long long s_or[NW], s_and[NW];
-    __shared__ uint32_t s_sum[NW], s_ns, s_nw, s_nt, s_piv[8];
-    __shared__ uint2 s_cur;
-    __shared__ BucketBits s_bits;
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    SegSmem<CAP, NT>& M = *reinterpret_cast<SegSmem<CAP, NT>*>(smem);
     for (uint32_t bi = blockIdx.x; bi < nseg; bi += gridDim.x) {
         const SmallSeg seg = segs[bi];
         const uint32_t start = seg.start, size = seg.size;
         uint32_t* lcp = S.lcp_out + start;
-        // the current group's strings; the whole segment first
         uint32_t o[IPT];
         uint64_t k[IPT];
-        {
-            const uint32_t* src = S.ord[seg.flags & F_PARITY] + start;
-            const unsigned long long* ksrc = S.key[seg.flags & F_PARITY] + start;
+        const uint32_t* src = S.ord[seg.flags & F_PARITY] + start;
+        const unsigned long long* ksrc = S.key[seg.flags & F_PARITY] + start;
 #pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                const uint32_t i = threadIdx.x + j * NT;
-                o[j] = i < size ? src[i] : 0u;
-                k[j] = i < size && (seg.flags & F_KEYS) ? ksrc[i] : 0ull;
-            }
-            if (!(seg.flags & (F_KEYS | F_ID))) {
+        for (int j = 0; j < IPT; ++j) {
+            const uint32_t i = threadIdx.x + j * NT;
+            o[j] = i < size ? src[i] : 0u;
+            k[j] = i < size && (seg.flags & F_KEYS) ? ksrc[i] : 0ull;
+        }
+        if (seg.flags & F_ID) {
 #pragma unroll
-                for (int j = 0; j < IPT; ++j)
-                    if (threadIdx.x + j * NT < size) k[j] = key8_of(S.a, o[j], seg.depth);
-            }
+            for (int j = 0; j < IPT; ++j) k[j] = o[j];
+        } else if (!(seg.flags & F_KEYS)) {
 #pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                const uint32_t i = threadIdx.x + j * NT;
-                if (i < size) {
-                    M.id[i] = o[j];
-                    M.key[i] = k[j];
-                }
-            }
+            for (int j = 0; j < IPT; ++j)
+                if (threadIdx.x + j * NT < size) k[j] = key8_of(S.a, o[j], seg.depth);
         }
 #pragma unroll
         for (int q = 0; q < PER; q += 4)
             *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
-        if (threadIdx.x == 0) {
-            const uint2 g = group_pack(0, size, (seg.flags & F_ID) ? G_ID : G_PLAIN, seg.depth);
-            s_nw = size <= 32;
-            s_ns = size > 32;
-            s_nt = 0;
-            if (size <= 32) M.wl[0] = g;
-            else M.stk[0] = g;
-        }
-        __syncthreads();
-        while (s_ns) {
-            if (threadIdx.x == 0) s_cur = M.stk[s_ns - 1];
-            __syncthreads();
-            const uint32_t bs = group_start(s_cur), bn = group_size(s_cur), dep = s_cur.y;
-            uint32_t kind = group_kind(s_cur);
-            if (threadIdx.x == 0) --s_ns;  // read again only after the next barrier
-            uint32_t br[IPT];
-            if (bn != size) {  // (the whole segment is still in registers)
-#pragma unroll
-                for (int j = 0; j < IPT; ++j) {
-                    const uint32_t i = threadIdx.x + j * NT;
-                    o[j] = i < bn ? M.id[bs + i] : 0u;
-                    k[j] = i < bn ? M.key[bs + i] : 0ull;
-                }
-            }
-            if (kind == G_ID) {
-#pragma unroll
-                for (int j = 0; j < IPT; ++j) k[j] = o[j];
-            }
-            if (kind == G_TIE) {
-                // the pivot: of 8 evenly spaced strings the one with the
-                // largest sum of LCPs (256 bytes at most) with the others
-                for (uint32_t c = w; c < 8; c += NW) {
-                    const StrRef x = ref_of(S.a, M.id[bs + c * bn / 8]);
-                    const uint64_t kx = key8(S.a.chars, x.off, x.len, dep + 8 * lane);
-                    uint32_t sum = 0;
-#pragma unroll 4
-                    for (uint32_t q = 0; q < 8; ++q) {
-                        const StrRef y = ref_of(S.a, M.id[bs + q * bn / 8]);
-                        const uint64_t ky = key8(S.a.chars, y.off, y.len, dep + 8 * lane);
-                        const uint32_t e = kx != ky ? key_lcp(kx, ky) : 8u;
-                        const uint32_t hit = __ballot_sync(FULL, e < 8);
-                        const int f = hit ? __ffs(hit) - 1 : 0;
-                        const uint32_t ef = __shfl_sync(FULL, e, f);
-                        sum += hit ? 8 * f + ef : 256u;
-                    }
-                    if (lane == 0) s_piv[c] = sum << 3 | c;
-                }
-                __syncthreads();
-                uint32_t best = 0;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) best = max(best, s_piv[c]);
-                const uint32_t pid = M.id[bs + (best & 7u) * bn / 8];
-                const StrRef h = ref_of(S.a, pid);
-#pragma unroll 1
-                for (int j = 0; j < IPT; ++j) {
-                    const uint32_t i = threadIdx.x + j * NT;
-                    if (i - lane >= bn) break;  // the same for the whole warp
-                    const bool v = i < bn;
-                    StrRef x{0, 0};
-                    uint32_t oj = v ? M.id[bs + i] : 0u;
-                    if (v) x = ref_of(S.a, oj);
-                    const uint32_t l = warp_lcp(S.a, x, h, dep, v);
-                    if (v) M.key[bs + i] = pseudo_key(S.a, x, h, l, dep);
-                }
-                // a thread reads back only the keys it wrote
-#pragma unroll
-                for (int j = 0; j < IPT; ++j) {
-                    const uint32_t i = threadIdx.x + j * NT;
-                    if (i < bn) k[j] = M.key[bs + i];
-                }
-                kind = G_PSEUDO;
-            }
-            const bool pseudo = kind == G_PSEUDO;
-            // the bits in which the keys differ
-            uint64_t vo = 0, va = ~0ull;
-#pragma unroll
-            for (int j = 0; j < IPT; ++j)
-                if (threadIdx.x + j * NT < bn) {
-                    const uint64_t t = level_key(k[j], pseudo);
-                    vo |= t;
-                    va &= t;
-                }
-            const uint32_t olo = __reduce_or_sync(FULL, (uint32_t)vo), ohi = __reduce_or_sync(FULL, (uint32_t)(vo >> 32));
-            const uint32_t alo = __reduce_and_sync(FULL, (uint32_t)va);
-            const uint32_t ahi = __reduce_and_sync(FULL, (uint32_t)(va >> 32));
-            if (lane == 0) {
-                s_or[w] = (uint64_t)ohi << 32 | olo;
-                s_and[w] = (uint64_t)ahi << 32 | alo;
-            }
-            __syncthreads();
-            if (w == 0) {
-                uint64_t x = lane < NW ? s_or[lane] : 0ull, y = lane < NW ? s_and[lane] : ~0ull;
-                const uint32_t dl = __reduce_or_sync(FULL, (uint32_t)x) ^ __reduce_and_sync(FULL, (uint32_t)y);
-                const uint32_t dh = __reduce_or_sync(FULL, (uint32_t)(x >> 32)) ^ __reduce_and_sync(FULL, (uint32_t)(y >> 32));
-                if (lane == 0) {
-                    constexpr uint32_t most = 31u - (uint32_t)__builtin_clz(NB);
-                    const uint64_t diff = (uint64_t)dh << 32 | dl;
-                    s_bits.nruns = 0;
-                    if (diff)
-                        bucket_bits(s_bits, diff, pseudo ? most : min(32u - (uint32_t)__clz(bn - 1) + 1u, most));
-                }
-            }
-            __syncthreads();
-            if (s_bits.nruns == 0) {  // one key: equal strings, or the group goes deeper
-                if (threadIdx.x == 0) {
-                    const uint64_t k0 = k[0];
-                    M.stk[s_ns++] = key_ended(k0, pseudo) ? group_pack(bs, bn, G_ID, ref_of(S.a, o[0]).len)
-                                                          : group_pack(bs, bn, G_TIE, tie_depth(k0, dep, pseudo));
-                }
-                __syncthreads();
-                continue;
-            }
-            {
-                const uint32_t lo = s_bits.lo, nr = s_bits.nruns;
-                uint32_t x[IPT];
-#pragma unroll
-                for (int j = 0; j < IPT; ++j) {
-                    x[j] = (uint32_t)(k[j] >> lo);
-                    br[j] = 0;
-                }
-                for (uint32_t r = 0; r < nr; ++r) {
-                    const uint32_t sh = s_bits.sh[r], mask = s_bits.mask[r];
-                    if (s_bits.wide) {
-#pragma unroll
-                        for (int j = 0; j < IPT; ++j) br[j] |= (uint32_t)(k[j] >> (lo + sh)) & mask;
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < IPT; ++j) br[j] |= (x[j] >> sh) & mask;
-                    }
-                }
-            }
-            // counts; br: the bucket and, above it, the place inside it
-#pragma unroll
-            for (int j = 0; j < IPT; ++j)
-                if (threadIdx.x + j * NT < bn) br[j] |= atomicAdd(&M.cnt[br[j]], 1u) << 16;
-            __syncthreads();
-            {
-                uint32_t v[PER], sum = 0;
-#pragma unroll
-                for (int q = 0; q < PER; q += 4) {
-                    const uint4 c = *reinterpret_cast<const uint4*>(&M.cnt[threadIdx.x * PER + q]);
-                    v[q] = c.x;
-                    v[q + 1] = c.y;
-                    v[q + 2] = c.z;
-                    v[q + 3] = c.w;
-                    sum += c.x + c.y + c.z + c.w;
-                }
-                uint32_t x = sum;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const uint32_t y = __shfl_up_sync(FULL, x, off);
-                    if (lane >= (uint32_t)off) x += y;
-                }
-                if (lane == 31) s_sum[w] = x;
-                __syncthreads();
-                uint32_t run = x - sum;
-#pragma unroll
-                for (int q = 0; q < NW; ++q)
-                    if ((uint32_t)q < w) run += s_sum[q];
-#pragma unroll
-                for (int q = 0; q < PER; q += 4) {
-                    uint4 c;
-                    c.x = run;
-                    c.y = c.x + v[q];
-                    c.z = c.y + v[q + 1];
-                    c.w = c.z + v[q + 2];
-                    run = c.w + v[q + 3];
-                    *reinterpret_cast<uint4*>(&M.cnt[threadIdx.x * PER + q]) = c;
-                }
-                if (threadIdx.x == NT - 1) M.cnt[NB] = run;
-            }
-            __syncthreads();
-            // places (a thread holds its strings, so the group is permuted in
-            // place); only the counts' sum bounds a place, never taken else
-            bool bad = false;
-#pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                if (threadIdx.x + j * NT >= bn) continue;
-                const uint32_t at = M.cnt[br[j] & 0xFFFFu] + (br[j] >> 16);
-                if (at >= bn) {
-                    bad = true;
-                    continue;
-                }
-                M.key[bs + at] = k[j];
-                M.id[bs + at] = o[j];
-            }
-            if (bad) atomicExch(&S.counters[10], 1u);
-            __syncthreads();
-            // each bucket's first string: the LCP with the bucket before (any
-            // of its strings), and who sorts the bucket
-            const bool all = s_bits.all != 0, mixed = pseudo && s_bits.mixed;
-#pragma unroll
-            for (int j = 0; j < IPT; ++j) {
-                if (threadIdx.x + j * NT >= bn || (br[j] >> 16) != 0) continue;
-                const uint32_t b = br[j] & 0xFFFFu, s0 = M.cnt[b], c = M.cnt[b + 1] - s0;
-                if (s0) {
-                    uint64_t kp = M.key[bs + s0 - 1], kn = k[j];
-                    if (mixed) {  // the codes next to the boundary: the last of the bucket before, this one's first
-                        const uint32_t bp = bucket_of_key(s_bits, kp);
-                        for (uint32_t x = s0 - 1; x > 0 && bucket_of_key(s_bits, M.key[bs + x - 1]) == bp; --x)
-                            kp = max(kp, (uint64_t)M.key[bs + x - 1]);
-                        for (uint32_t x = 0; x < c; ++x) kn = min(kn, (uint64_t)M.key[bs + s0 + x]);
-                    }
-                    lcp[bs + s0] = kind == G_ID ? dep : group_lcp(kp, kn, dep, pseudo);
-                }
-                if (c < 2) continue;
-                if (c <= TINY_MAX) {
-                    M.tl[atomicAdd(&s_nt, 1u)] = s0 | c << 16;
-                    continue;
-                }
-                uint32_t gk = kind, gd = dep;
-                if (kind != G_ID && all) {  // one key in the bucket
-                    const bool ended = key_ended(k[j], pseudo);
-                    gk = ended ? G_ID : G_TIE;
-                    gd = ended ? ref_of(S.a, o[j]).len : tie_depth(k[j], dep, pseudo);
-                }
-                const uint2 g = group_pack(bs + s0, c, gk, gd);
-                if (c <= 32) M.wl[atomicAdd(&s_nw, 1u)] = g;
-                else M.stk[atomicAdd(&s_ns, 1u)] = g;
-            }
-            __syncthreads();
-            // buckets of 2..TINY_MAX strings: insertion sort on (key, id), then
-            // the neighbours' LCPs and the runs that go deeper
-            const uint32_t nt = s_nt;
-            for (uint32_t e = threadIdx.x; e < nt; e += NT) {
-                const uint32_t s0 = bs + (M.tl[e] & 0xFFFFu), c = M.tl[e] >> 16;
-                for (uint32_t x = 1; x < c; ++x) {
-                    const uint64_t kx = M.key[s0 + x];
-                    const uint32_t ox = M.id[s0 + x];
-                    uint32_t y = x;
-                    for (; y > 0; --y) {
-                        const uint64_t ky = M.key[s0 + y - 1];
-                        const uint32_t oy = M.id[s0 + y - 1];
-                        if (ky < kx || (ky == kx && oy < ox)) break;
-                        M.key[s0 + y] = ky;
-                        M.id[s0 + y] = oy;
-                    }
-                    M.key[s0 + y] = kx;
-                    M.id[s0 + y] = ox;
-                }
-                if (kind == G_ID) {
-                    for (uint32_t x = 1; x < c; ++x) lcp[s0 + x] = dep;
-                    continue;
-                }
-                uint64_t kp = M.key[s0];
-                uint32_t r0 = 0;  // start of the run of equal keys
-                for (uint32_t x = 1; x <= c; ++x) {
-                    const uint64_t kx = x < c ? M.key[s0 + x] : ~kp;
-                    if (kx == kp) continue;
-                    if (x - r0 > 1) {
-                        if (key_ended(kp, pseudo)) {
-                            const uint32_t len = ref_of(S.a, M.id[s0 + r0]).len;
-                            for (uint32_t y = r0 + 1; y < x; ++y) lcp[s0 + y] = len;
-                        } else {
-                            M.wl[atomicAdd(&s_nw, 1u)] = group_pack(s0 + r0, x - r0, G_TIE, tie_depth(kp, dep, pseudo));
-                        }
-                    }
-                    if (x < c) lcp[s0 + x] = group_lcp(kp, kx, dep, pseudo);
-                    kp = kx;
-                    r0 = x;
-                }
-            }
-            // the next pass counts from zero
-#pragma unroll
-            for (int q = 0; q < PER; q += 4)
-                *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
-            __syncthreads();
-            if (threadIdx.x == 0) s_nt = 0;  // pushed to again only after the next pass's barriers
-        }
-        const uint32_t nwl = s_nw;
-        for (uint32_t e = w; e < nwl; e += NW) {
-            const uint2 g = M.wl[e];
-            const uint32_t ws = group_start(g), wn = group_size(g);
-            uint64_t key = 0;
-            uint32_t id = 0;
-            if (lane < wn) {
-                id = M.id[ws + lane];
-                key = M.key[ws + lane];
-            }
-            warp_group(S.a, wn, g.y, group_kind(g), key, id, lcp + ws);
-            if (lane < wn) M.id[ws + lane] = id;
-        }
+        if (threadIdx.x == 0) M.ns = M.nw = M.nt = M.claim = 0;
+        cta_pass<CAP, NT, true>(S, M, 0, size, seg.depth, (seg.flags & F_ID) ? G_ID : G_PLAIN, o, k, lcp);
+        if (M.ns | M.nw) sort_rest<CAP, NT>(S, lcp);
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < size; i += NT) S.ord_out[start + i] = M.id[i];
         __syncthreads();  // shared memory is reused by the next segment
     }
 }
 
-template <int CAP>
-constexpr size_t seg_sort_smem() {
-    return sizeof(SegSmem<CAP>);
-}
-
 template <int CAP, int NT>
 static int launch_seg_sort(const SortState& S, const SmallSeg* segs, uint32_t n, const char* name, cudaStream_t st) {
     if (!n) return DSSS_OK;
-    constexpr size_t shm = seg_sort_smem<CAP>();
+    constexpr size_t shm = sizeof(SegSmem<CAP, NT>);
     static std::atomic<uint64_t> configured{0};
     DSSS_TRY(set_smem_once(configured, k_seg_sort<CAP, NT>, (int)shm));
     DSSS_LAUNCH(name, st, k_seg_sort<CAP, NT><<<n, NT, shm, st>>>(S, segs, n));

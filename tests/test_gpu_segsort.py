@@ -67,3 +67,24 @@ def test_long_common_parts(dsss, orc, ctx):
 def test_prefixes_and_many_segments(dsss, orc, ctx):
     check(dsss, orc, ctx, prefixes_of_each_other(4096, seed=2))
     check(dsss, orc, ctx, with_duplicates(random_strings(20000, 0, 30, b"ab", seed=5), 0.5, seed=6), p=23)
+
+
+@pytest.mark.parametrize("sizes", [(2, 3, 4, 5), (31, 32, 33), (63, 64, 65), (2, 60, 3, 62, 64, 33, 7)],
+                         ids=["small", "lanes", "elements", "mixed"])
+@pytest.mark.parametrize("reach", [20, 200, 700, 17000])
+def test_groups_of_one_warp(dsss, orc, ctx, sizes, reach):
+    """Groups with one 8-byte key, of sizes at the hand-over between warp and
+    CTA and in mixtures that share a warp: copies of up to `reach` bytes of a
+    common text, equal strings among them, a few that agree for much longer
+    than the others."""
+    rng = np.random.default_rng(reach + len(sizes))
+    strs, g = [], 0
+    while len(strs) < min(1500, 12_000_000 // reach):
+        c = sizes[g % len(sizes)]
+        head = bytes(rng.integers(65, 91, reach).astype(np.uint8))
+        for _ in range(c):
+            cut = reach if rng.random() < 0.1 else 8 + int(rng.integers(0, reach - 7))
+            strs.append(head[:cut] + bytes(rng.integers(65, 68, int(rng.integers(0, 3))).astype(np.uint8)))
+        g += 1
+    rng.shuffle(strs)
+    check(dsss, orc, ctx, strs)

@@ -183,7 +183,7 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
         StageTimer t("stage:local", st);
         DSSS_TRY(project_setup(L.proj, nsets, p, pb, factor, pinp, st));
         DSSS_TRY(project_local(L.proj, a, n, nsets, p, ord, lcp, L.stats, pe, bucket, out->local_order,
-                               out->perm_index, out->dp, st));
+                               out->perm_index, out->dp, nullptr, nullptr, st));
     }
     // 3. splitters and every PE's bounds; receiving PE (s, r) is bucket s*p + r
     {
@@ -236,15 +236,6 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
 // to 200 (avg + 5) bytes, then the receiving PEs' sequences (the global order,
 // or its multisplit by receiver when ties cross a splitter) and their strings
 // copied out whole.
-
-__global__ void k_sum_u32_to_u64(const uint32_t* v, uint64_t n, unsigned long long* total) {
-    unsigned long long s = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        s += v[i];
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0 && s) atomicAdd(total, s);
-}
 
 // Input index, source offset and length (+ 1 for the scan) of every output
 // string (the string at global position map[o], or o): the copy then reads its
@@ -306,7 +297,7 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     const uint32_t factor = 2, smax = smallmax_of(opts);  // computePartition(..., 2): misc.hpp call in :238
     const uint64_t N = n ? n : 1;
     PdLayout L;
-    uint32_t *src_tmp, *len1, *pe, *rank, *llcp;
+    uint32_t *src_tmp, *len1, *pe, *rank, *edges;
     uint64_t* srcoff;
     unsigned long long* total;
     void* scan;
@@ -316,7 +307,7 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
         len1 = c.take<uint32_t>(N);
         pe = c.take<uint32_t>(N);
         rank = c.take<uint32_t>(N);
-        llcp = c.take<uint32_t>(N);
+        edges = c.take<uint32_t>(project_edge_words(N, p));
         srcoff = c.take<uint64_t>(N);
         total = c.take<unsigned long long>(2);
         scan = c.take<unsigned char>(scan_scratch_bytes(N));
@@ -353,13 +344,11 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
         a.h = L.handles;
     }
     const uint64_t bytes = hstats->sum + n;  // the sort has synchronised on st
-    // local orders per PE and their LCP arrays (0 at each PE start)
+    // local orders per PE and the sum of their LCPs
     StageTimer t_local("stage:local", st);
     DSSS_TRY(project_setup(L.proj, 1, p, pb, factor, pinp, st));
-    DSSS_TRY(project_local(L.proj, a, n, 1, p, L.ord, out->lcp, nullptr, pe, pe, out->local_order, rank, nullptr, st));
-    DSSS_TRY(adjacent_lcp(a, out->local_order, n, llcp, L.tie[0], L.nlong, st));
-    DSSS_LAUNCH("k_zero_starts", st, k_zero_starts<<<grid_for(p, 128), 128, 0, st>>>(llcp, L.proj.pb, p));
-    DSSS_LAUNCH("k_sum_u32_to_u64", st, k_sum_u32_to_u64<<<148 * 4, 256, 0, st>>>(llcp, n, total));
+    DSSS_TRY(project_local(L.proj, a, n, 1, p, L.ord, out->lcp, nullptr, pe, pe, out->local_order, rank, nullptr, edges,
+                           total, st));
     unsigned long long* hsum = (unsigned long long*)((char*)ctx->pin + 192);
     DSSS_CUDA(cudaMemcpyAsync(hsum, total, 8, cudaMemcpyDeviceToHost, st));
     t_local.end();

@@ -88,15 +88,31 @@ __global__ void __launch_bounds__(PJ_NT) k_pe_hist(const uint32_t* ord, uint64_t
     }
 }
 
+// Where a tile leaves the local LCPs open: per PE and tile the least LCP up to
+// the PE's first string (PJ_NONE: it has none here) and from behind its last
+// one to the tile's end, both PE-major, and each tile's least LCP.
+struct LcpEdges {
+    uint32_t *head, *tail, *tmin;
+    unsigned long long* sum;
+};
+constexpr uint32_t PJ_NONE = 0xFFFFFFFFu;
+
 // Stable scatter of every position's id (and distinguishing prefix, computed
 // here from the LCPs) to its PE's local order, and its rank there.  The tile
 // is reordered by PE in shared memory, so that each PE's run is written
 // contiguously.  Bound by shared-memory latency (the stable rank), then by 24
 // bytes moved per position.  Peers by ballots instead of a match instruction:
 // 0.36 -> 0.25 ms on 32e6 strings and 64 PEs.
+//
+// Without DP it sums the PEs' local LCPs instead (the merge-sort path needs
+// their average alone): two strings that follow one another on a PE have the
+// least LCP of the global order between them, which blocks' prefix and suffix
+// minima in shared memory give; what crosses tiles is left to
+// k_local_lcp_edges.  Comparing the strings themselves again read every
+// string's first bytes in random order: 8e6 strings 0.53 ms in all, now 0.17 ms.
 template <bool DP>
 constexpr size_t pj_scatter_smem(uint32_t P) {
-    return (size_t)PJ_TILE * ((DP ? 8 : 4) + 2) + (size_t)P * 4 * (3 + PJ_NW);
+    return (size_t)PJ_TILE * (DP ? 8 + 2 : 4 * 4 + 2 * 2) + (size_t)P * 4 * (3 + PJ_NW);
 }
 
 template <bool DP>
@@ -105,12 +121,16 @@ __global__ void __launch_bounds__(PJ_NT, 5) k_local_scatter(const uint32_t* buck
                                                             const LenStats* stats, uint64_t n, uint32_t P,
                                                             uint64_t tiles, const uint32_t* off, const uint64_t* pb,
                                                             uint32_t* local_order,
-                                                            uint32_t* dp, uint32_t* rank, uint32_t* err) {
+                                                            uint32_t* dp, LcpEdges E, uint32_t* rank,
+                                                            uint32_t* err) {
     extern __shared__ __align__(16) uint32_t pj_sm[];
     uint32_t* sid = pj_sm;                                       // PJ_TILE
-    uint32_t* sdp = sid + PJ_TILE;                               // PJ_TILE (DP)
-    uint16_t* sbk = (uint16_t*)(sid + (DP ? 2 : 1) * PJ_TILE);   // PJ_TILE
-    uint32_t* base = (uint32_t*)(sbk + PJ_TILE);                 // P
+    uint32_t* sdp = sid + PJ_TILE;                               // PJ_TILE; !DP: the tile's LCPs
+    uint32_t* pmin = sdp + PJ_TILE;                              // PJ_TILE (!DP): least LCP from the block of 32's start
+    uint32_t* smin = pmin + PJ_TILE;                             // PJ_TILE (!DP): least LCP to the block's end
+    uint16_t* sbk = (uint16_t*)(sid + (DP ? 2 : 4) * PJ_TILE);   // PJ_TILE
+    uint16_t* spos = sbk + PJ_TILE;                              // PJ_TILE (!DP)
+    uint32_t* base = (uint32_t*)(sbk + (DP ? 1 : 2) * PJ_TILE);  // P
     uint32_t* first = base + P;                                  // P
     uint32_t* tloff = first + P;                                 // P
     uint32_t* wcnt = tloff + P;                                  // PJ_NW x P
@@ -143,6 +163,22 @@ __global__ void __launch_bounds__(PJ_NT, 5) k_local_scatter(const uint32_t* buck
             uint64_t d = dp_depth_above(dv[j]);
             if (d > minlen && wb + j * 32 + lane < n) d = min(d, (uint64_t)len[id[j]]);
             dv[j] = (uint32_t)d;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < PJ_IPT; ++j) {
+            const uint64_t i = wb + j * 32 + lane;
+            const uint32_t t = w * 32 * PJ_IPT + j * 32 + lane, v = i < n ? lcp[i] : PJ_NONE;
+            uint32_t up = v, down = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t x = __shfl_up_sync(PJ_FULL, up, o), y = __shfl_down_sync(PJ_FULL, down, o);
+                if (lane >= o) up = min(up, x);
+                if (lane + o < 32) down = min(down, y);
+            }
+            sdp[t] = v;
+            pmin[t] = up;
+            smin[t] = down;
         }
     }
     // the lanes with the same PE (one ballot per bit of the PE number), all
@@ -205,6 +241,7 @@ __global__ void __launch_bounds__(PJ_NT, 5) k_local_scatter(const uint32_t* buck
         }
         sid[lp] = id[j];
         if (DP) sdp[lp] = dv[j];
+        else spos[lp] = (uint16_t)(i - tb);
         sbk[lp] = (uint16_t)d;
         rank[i] = base[d] - first[d] + in_tile;
     }
@@ -218,6 +255,81 @@ __global__ void __launch_bounds__(PJ_NT, 5) k_local_scatter(const uint32_t* buck
         }
         local_order[dest] = sid[xx];
         if (DP) dp[dest] = sdp[xx];
+    }
+    if (DP) return;
+    // the least LCP over the tile's positions from .. to
+    auto least = [&](uint32_t from, uint32_t to) {
+        const uint32_t fb = from / 32, lb = to / 32;
+        uint32_t m = PJ_NONE;
+        if (fb == lb) {
+            for (uint32_t t = from; t <= to; ++t) m = min(m, sdp[t]);
+        } else {
+            m = min(smin[from], pmin[to]);
+            for (uint32_t b = fb + 1; b < lb; ++b) m = min(m, smin[b * 32]);
+        }
+        return m;
+    };
+    unsigned long long total = 0;
+    for (uint32_t xx = threadIdx.x; xx < tn; xx += PJ_NT) {
+        const uint32_t d = sbk[xx], t = spos[xx];
+        const uint64_t cell = (uint64_t)d * tiles + blockIdx.x;
+        if (xx > tloff[d]) total += least(spos[xx - 1] + 1u, t);
+        else E.head[cell] = least(0, t);
+        if (xx + 1 == tn || sbk[xx + 1] != d) E.tail[cell] = t + 1 < tn ? least(t + 1, tn - 1) : PJ_NONE;
+    }
+    for (uint32_t b = threadIdx.x; b < P; b += PJ_NT)
+        if (tloff[b] == (b + 1 < P ? tloff[b + 1] : tn)) E.head[(uint64_t)b * tiles + blockIdx.x] = PJ_NONE;
+    if (w == 0) {
+        static_assert(PJ_TILE == 64 * 32, "two blocks per lane");
+        const uint32_t m = __reduce_min_sync(PJ_FULL, min(smin[lane * 32], smin[(lane + 32) * 32]));
+        if (lane == 0) E.tmin[blockIdx.x] = m;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) total += __shfl_xor_sync(PJ_FULL, total, o);
+    if (lane == 0 && total) atomicAdd(E.sum, total);
+}
+
+// The local LCPs that cross tiles: one block per PE, a contiguous run of tiles
+// per thread, the runs combined in order.  A run holds the least LCP up to its
+// first string (all of it if it has none), the least one behind its last
+// string, and the sum between.
+struct LcpRun {
+    uint32_t has, head, tail;
+    unsigned long long sum;
+};
+__device__ __forceinline__ void lcp_run_append(LcpRun& a, const LcpRun& b) {
+    a.sum += b.sum;
+    if (a.has && b.has) a.sum += min(a.tail, b.head);
+    if (!a.has) a.head = min(a.head, b.head);
+    a.tail = b.has ? b.tail : min(a.tail, b.head);
+    a.has |= b.has;
+}
+
+__global__ void __launch_bounds__(PJ_NT) k_local_lcp_edges(LcpEdges E, uint64_t tiles) {
+    __shared__ LcpRun s_run[PJ_NW];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint64_t per = (tiles + PJ_NT - 1) / PJ_NT, t0 = threadIdx.x * per, t1 = min(tiles, t0 + per);
+    const uint32_t *head = E.head + blockIdx.x * tiles, *tail = E.tail + blockIdx.x * tiles;
+    LcpRun r{0u, PJ_NONE, PJ_NONE, 0ull};
+    for (uint64_t t = t0; t < t1; ++t) {
+        const uint32_t h = head[t];
+        const LcpRun x{h != PJ_NONE, h != PJ_NONE ? h : E.tmin[t], h != PJ_NONE ? tail[t] : PJ_NONE, 0ull};
+        lcp_run_append(r, x);
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        LcpRun x;
+        x.has = __shfl_down_sync(PJ_FULL, r.has, o);
+        x.head = __shfl_down_sync(PJ_FULL, r.head, o);
+        x.tail = __shfl_down_sync(PJ_FULL, r.tail, o);
+        x.sum = __shfl_down_sync(PJ_FULL, r.sum, o);
+        if (lane + o < 32) lcp_run_append(r, x);  // what lanes not at a multiple of 2 o hold is not read again
+    }
+    if (lane == 0) s_run[w] = r;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < PJ_NW; ++q) lcp_run_append(r, s_run[q]);
+        if (r.sum) atomicAdd(E.sum, r.sum);
     }
 }
 
@@ -515,6 +627,11 @@ void layout_project(Carve& c, ProjectLayout& L, uint64_t n, uint32_t nsets, uint
     L.flags = c.sizing ? nullptr : L.bounds + npe * (p + 1);
 }
 
+uint64_t project_edge_words(uint64_t n, uint32_t npe) {
+    const uint64_t tiles = (std::max<uint64_t>(n, 1) + PJ_TILE - 1) / PJ_TILE;
+    return tiles * (2 * (uint64_t)npe + 1);
+}
+
 uint64_t project_pin_bytes(uint32_t nsets, uint32_t p) {
     const uint64_t npe = (uint64_t)nsets * p;
     return std::max<uint64_t>((npe + 1) * 8 + nsets * sizeof(SetSplit), (npe * (p + 1) + 2) * 4) + 64;
@@ -545,7 +662,8 @@ int project_setup(const ProjectLayout& L, uint32_t nsets, uint32_t p, const uint
 
 int project_local(const ProjectLayout& L, const ArenaDev& a, uint64_t n, uint32_t nsets, uint32_t p,
                   const uint32_t* ord, const uint32_t* lcp, const LenStats* stats, uint32_t* pe, uint32_t* bucket,
-                  uint32_t* local_order, uint32_t* rank, uint32_t* dp, cudaStream_t st) {
+                  uint32_t* local_order, uint32_t* rank, uint32_t* dp, uint32_t* edges, unsigned long long* lcp_sum,
+                  cudaStream_t st) {
     const uint32_t npe = nsets * p;
     const uint64_t cells = L.tiles * npe;
     if (cells >= (1ull << 32)) return fail(DSSS_ENOTSUP, "local orders: too many tiles x PEs");
@@ -558,12 +676,16 @@ int project_local(const ProjectLayout& L, const ArenaDev& a, uint64_t n, uint32_
         DSSS_TRY(set_smem_once(c0, k_local_scatter<true>, (int)pj_scatter_smem<true>(MAX_SPLIT_BUCKETS)));
         DSSS_LAUNCH("k_ms_scatter_pay", st,  // the multisplit by PE
                     k_local_scatter<true><<<(unsigned)L.tiles, PJ_NT, pj_scatter_smem<true>(npe), st>>>(
-                        bucket, ord, lcp, a.len, stats, n, npe, L.tiles, L.off, L.pb, local_order, dp, rank, L.flags));
+                        bucket, ord, lcp, a.len, stats, n, npe, L.tiles, L.off, L.pb, local_order, dp, LcpEdges{}, rank,
+                        L.flags));
     } else {
+        const LcpEdges E{edges, edges + cells, edges + 2 * cells, lcp_sum};
         DSSS_TRY(set_smem_once(c1, k_local_scatter<false>, (int)pj_scatter_smem<false>(MAX_SPLIT_BUCKETS)));
         DSSS_LAUNCH("k_ms_scatter_pay", st,  // the multisplit by PE
                     k_local_scatter<false><<<(unsigned)L.tiles, PJ_NT, pj_scatter_smem<false>(npe), st>>>(
-                        bucket, ord, lcp, a.len, stats, n, npe, L.tiles, L.off, L.pb, local_order, dp, rank, L.flags));
+                        bucket, ord, lcp, a.len, stats, n, npe, L.tiles, L.off, L.pb, local_order, dp, E, rank,
+                        L.flags));
+        DSSS_LAUNCH("k_local_lcp_edges", st, k_local_lcp_edges<<<npe, PJ_NT, 0, st>>>(E, L.tiles));
     }
     DSSS_CUDA(cudaGetLastError());
     return DSSS_OK;

@@ -37,11 +37,14 @@ int project_setup(const ProjectLayout& L, uint32_t nsets, uint32_t p, const uint
 
 // Local orders: pe[g] (the PE of global position g inside its set) and, with
 // several sets, bucket[g] (set * p + pe), local_order, rank[g] (position in
-// the PE's local order), and, when dp is given, the distinguishing prefixes
-// in local order.  bucket may be pe itself with one set.
+// the PE's local order), and either the distinguishing prefixes in local order
+// (dp) or, dp == nullptr, *lcp_sum += the sum of the PEs' local LCPs (edges:
+// scratch of project_edge_words).  bucket may be pe itself with one set.
 int project_local(const ProjectLayout& L, const ArenaDev& a, uint64_t n, uint32_t nsets, uint32_t p,
                   const uint32_t* ord, const uint32_t* lcp, const LenStats* stats, uint32_t* pe, uint32_t* bucket,
-                  uint32_t* local_order, uint32_t* rank, uint32_t* dp, cudaStream_t st);
+                  uint32_t* local_order, uint32_t* rank, uint32_t* dp, uint32_t* edges, unsigned long long* lcp_sum,
+                  cudaStream_t st);
+uint64_t project_edge_words(uint64_t n, uint32_t npe);
 
 // Splitters and every PE's bounds against them (computePartition), from the
 // global order.  Samples are cut to their distinguishing prefixes (cut ==

@@ -92,3 +92,21 @@ def test_samples_cut_inside_a_run(dsss, orc, ctx, p, seed):
     out = dsss.ms_sort(ctx, dsss.DeviceStrings(hs), p, part_begin=pb)
     assert out["avg_lcp"] == avg
     check_ms(dsss, orc, hs, out, pb)
+
+
+@pytest.mark.parametrize("n,parts", [
+    (1, [0, 1]), (2, [0, 1, 2]), (31, [0, 31]), (2048, [0, 1024, 2048]), (2049, [0, 2, 4, 2049]),
+    (4500, [0, 2, 2, 5, 4500]), (6200, [0, 1, 3, 40, 3000, 6200]), (6200, None),
+], ids=str)
+def test_sum_of_local_lcps(dsss, orc, ctx, n, parts):
+    """The average local LCP comes from the global LCPs, tile by tile: PEs
+    with two strings many tiles apart, with none in most tiles and with all of
+    them.  LCPs are longer than n, so that one wrong pair changes the average."""
+    rng = np.random.default_rng(n)
+    head = b"h" * (n + 50)
+    strs = [head + bytes(rng.integers(65, 91, 12).astype(np.uint8)) for _ in range(n)]
+    rng.shuffle(strs)
+    pb = dsss.equal_parts(n, 37) if parts is None else np.array(parts, np.uint64)
+    hs = dsss.from_bytes_list(strs)
+    out = dsss.ms_sort(ctx, dsss.DeviceStrings(hs), len(pb) - 1, part_begin=pb)
+    assert out["avg_lcp"] == orc.ms_sort(orc.Strings.from_host(hs), pb)["avg_lcp"]

@@ -228,9 +228,16 @@ __device__ __forceinline__ void copy_words(uint8_t* dst, const uint8_t* src, uin
 
 // copy_words with dst's aligned 16-byte words stored whole, each from three
 // aligned 8-byte loads of src (reads at most 8 bytes past src + len), the at
-// most 15 bytes before and after them singly.
+// most 15 bytes before and after them singly.  The loads of up to 2 L words
+// and of the single bytes are all issued before the first store: a string
+// costs one memory latency instead of up to four (8e6 sorted strings of 200
+// bytes: 1.05 -> 0.96 ms; their reads fetch 325 bytes each and every second
+// issue slot is free, so what bounds it is reads in flight; a persistent form
+// that loads the next string ahead has fewer warps and took 1.14 ms, one that
+// loads every input byte once 1.53 ms).
 template <uint32_t L>
 __device__ __forceinline__ void copy_words16(uint8_t* dst, const uint8_t* src, uint32_t len, uint32_t lane) {
+    static_assert(L >= 8 && L <= 32, "two rounds of lanes hold 15 bytes");
     const uintptr_t d0 = (uintptr_t)dst, e = d0 + len;
     const uintptr_t a0 = (d0 + 15) & ~(uintptr_t)15, a1 = e & ~(uintptr_t)15;
     if (a0 >= a1) {
@@ -238,23 +245,42 @@ __device__ __forceinline__ void copy_words16(uint8_t* dst, const uint8_t* src, u
         return;
     }
     const uint32_t head = (uint32_t)(a0 - d0), tail = (uint32_t)(a1 - d0);
-    for (uint32_t k = lane; k < head; k += L) dst[k] = src[k];
-    for (uint32_t k = tail + lane; k < len; k += L) dst[k] = src[k];
     const uint32_t nw = (uint32_t)((a1 - a0) >> 4);
     uint4* w = reinterpret_cast<uint4*>(a0);
     const uintptr_t sa = (uintptr_t)(src + head);
     const unsigned long long* q = reinterpret_cast<const unsigned long long*>(sa & ~(uintptr_t)7);
     const unsigned sh = (unsigned)(sa & 7) * 8;
-#pragma unroll 2
-    for (uint32_t k = lane; k < nw; k += L) {
-        const uint64_t x0 = __ldg(q + 2 * k), x1 = __ldg(q + 2 * k + 1);
-        uint64_t lo = x0, hi = x1;
-        if (sh) {
-            const uint64_t x2 = __ldg(q + 2 * k + 2);
-            lo = (x0 >> sh) | (x1 << (64 - sh));
-            hi = (x1 >> sh) | (x2 << (64 - sh));
+    uint8_t hb[2], tb[2];
+#pragma unroll
+    for (uint32_t r = 0; r < 2; ++r) {
+        if (lane + r * L < head) hb[r] = __ldg(src + lane + r * L);
+        if (tail + lane + r * L < len) tb[r] = __ldg(src + tail + lane + r * L);
+    }
+    for (uint32_t k0 = 0; k0 < nw; k0 += 2 * L) {
+        uint64_t x[2][3];
+#pragma unroll
+        for (uint32_t r = 0; r < 2; ++r) {
+            const uint32_t k = k0 + r * L + lane;
+            x[r][2] = 0;
+            if (k < nw) {
+                x[r][0] = __ldg(q + 2 * (uint64_t)k);
+                x[r][1] = __ldg(q + 2 * (uint64_t)k + 1);
+                if (sh) x[r][2] = __ldg(q + 2 * (uint64_t)k + 2);
+            }
         }
-        w[k] = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+#pragma unroll
+        for (uint32_t r = 0; r < 2; ++r) {
+            const uint32_t k = k0 + r * L + lane;
+            if (k >= nw) continue;
+            const uint64_t lo = sh ? (x[r][0] >> sh) | (x[r][1] << (64 - sh)) : x[r][0];
+            const uint64_t hi = sh ? (x[r][1] >> sh) | (x[r][2] << (64 - sh)) : x[r][1];
+            w[k] = make_uint4((uint32_t)lo, (uint32_t)(lo >> 32), (uint32_t)hi, (uint32_t)(hi >> 32));
+        }
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < 2; ++r) {
+        if (lane + r * L < head) dst[lane + r * L] = hb[r];
+        if (tail + lane + r * L < len) dst[tail + lane + r * L] = tb[r];
     }
 }
 

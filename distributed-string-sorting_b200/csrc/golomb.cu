@@ -11,8 +11,9 @@
 // k - 1 bits holding r); the last word's unused bits are ones.  A destination
 // without values gets no words.
 //
-// Encoding is data-parallel: code lengths, a scan, then every code ORed into
-// its words.  A variable-length code is read sequentially; the decoder cuts
+// Encoding is data-parallel: code lengths summed per tile of values, a scan of
+// the tiles, then each thread puts the codes of its consecutive values together
+// word by word; the words it shares with its neighbours are ORed in.  A variable-length code is read sequentially; the decoder cuts
 // each block's bits into chunks of GB_CHUNK_BITS, reads every chunk from a
 // guessed code start and again from where its predecessor's last code ended,
 // until no start changes.  The first chunk of a block starts right, so the
@@ -63,6 +64,12 @@ __device__ __forceinline__ void gb_code(const GbParams& P, uint32_t r, uint64_t 
                                         uint32_t& kk) {
     const uint64_t b = P.b[r], little = P.little[r];
     const uint32_t k = P.k[r];
+    if (little == 0) {  // b = 2^k
+        q = gap >> k;   // k <= 63
+        val = gap & (b - 1);
+        kk = k;
+        return;
+    }
     q = gap / b;
     const uint64_t rem = gap - q * b;
     if (rem >= little) {
@@ -74,86 +81,176 @@ __device__ __forceinline__ void gb_code(const GbParams& P, uint32_t r, uint64_t 
     }
 }
 
-__global__ void k_gb_len(const uint64_t* v, uint64_t n, GbParams P, uint32_t* len, uint32_t* err) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t r = gb_range_of(P.rbeg, P.nranges, i);
-    if (i == P.rbeg[r]) {  // the first value of a range is not coded
-        len[i] = 0;
-        return;
-    }
-    if (v[i] < v[i - 1]) atomicOr(err, 1u);  // not ascending
+constexpr uint32_t GE_NT = 256, GE_IPT = 8, GE_TILE = GE_NT * GE_IPT;  // values of an encoder's tile
+
+// Length of value i's code in range r; the first value of a range is not
+// coded.  err bit 1: not ascending, bit 2: too long.
+__device__ __forceinline__ uint32_t gb_code_len(const uint64_t* v, uint64_t i, const GbParams& P, uint32_t r, uint32_t* err) {
+    if (i == P.rbeg[r]) return 0;
+    const uint64_t x = v[i], y = v[i - 1];
+    if (x < y && err) atomicOr(err, 1u);
     uint64_t q, val;
     uint32_t kk;
-    gb_code(P, r, v[i] - v[i - 1], q, val, kk);
+    gb_code(P, r, x - y, q, val, kk);
     if (q > GB_MAX_Q) {
-        atomicOr(err, 2u);
-        len[i] = 0;
-        return;
+        if (err) atomicOr(err, 2u);
+        return 0;
     }
-    len[i] = (uint32_t)(q + 1 + kk);
+    return (uint32_t)(q + 1 + kk);
 }
 
-// Bits and words of every range's block (0 words for an empty range).
-__global__ void k_gb_range_words(const uint64_t* pos, uint64_t n, const uint64_t* total, GbParams P, uint64_t* rbits,
-                                 uint64_t* rwords) {
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= P.nranges) return;
-    const uint64_t b0 = P.rbeg[r], b1 = P.rbeg[r + 1];
-    if (b1 == b0) {
-        rbits[r] = 0;
-        rwords[r] = 0;
-        return;
-    }
-    const uint64_t bits = (b1 < n ? pos[b1] : *total) - pos[b0];
-    rbits[r] = bits;
-    rwords[r] = 3 + (bits + 63) / 64;
+// Sum over the block; every thread gets it.
+__device__ __forceinline__ uint64_t gb_block_sum(uint64_t x) {
+    __shared__ uint64_t ws[GE_NT / 32];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = x;
+    __syncthreads();
+    uint64_t t = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < GE_NT / 32; ++q) t += ws[q];
+    return t;
 }
 
-// Ones over bits [t, t + q) of w (bit 0 = the first word's most significant).
-__device__ __forceinline__ void gb_ones(unsigned long long* w, uint64_t t, uint64_t q) {
-    if (q == 0) return;
-    const uint64_t e = t + q - 1;
-    const uint64_t w0 = t >> 6, w1 = e >> 6;
-    const uint32_t a = (uint32_t)(t & 63), z = (uint32_t)(e & 63);
-    if (w0 == w1) {
-        atomicOr(&w[w0], (~0ull >> a) & (~0ull << (63 - z)));
-        return;
+// Code bits of each tile of values.  Most tiles lie in one range, whose search
+// then is the tile's.  (Lengths and their positions of every value, 64-bit
+// divisions where b is a power of two and an OR per code: 4e6 hashes to 23 MB
+// 0.22 ms with the size query, now 0.13.)
+__global__ void __launch_bounds__(GE_NT) k_gb_len(const uint64_t* v, uint64_t n, GbParams P, uint64_t* bits, uint32_t* err) {
+    const uint64_t tb = (uint64_t)blockIdx.x * GE_TILE;
+    const uint32_t r0 = gb_range_of(P.rbeg, P.nranges, tb), r1 = gb_range_of(P.rbeg, P.nranges, min(n, tb + GE_TILE) - 1);
+    uint64_t s = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < GE_IPT; ++j) {
+        const uint64_t i = tb + j * GE_NT + threadIdx.x;
+        if (i < n) s += gb_code_len(v, i, P, r0 == r1 ? r0 : gb_range_of(P.rbeg, P.nranges, i), err);
     }
-    atomicOr(&w[w0], ~0ull >> a);
-    for (uint64_t x = w0 + 1; x < w1; ++x) w[x] = ~0ull;  // words wholly inside one code
-    atomicOr(&w[w1], ~0ull << (63 - z));
+    s = gb_block_sum(s);
+    if (threadIdx.x == 0) bits[blockIdx.x] = s;
 }
 
-// The nb (1..64) low bits of val at bits [t, t + nb), most significant first.
-__device__ __forceinline__ void gb_bits(unsigned long long* w, uint64_t t, uint64_t val, uint32_t nb) {
-    const uint32_t a = (uint32_t)(t & 63);
-    const uint64_t x = t >> 6;
-    if (a + nb <= 64) {
-        atomicOr(&w[x], (unsigned long long)(val << (64 - a - nb)));
-    } else {
-        const uint32_t second = a + nb - 64;
-        atomicOr(&w[x], (unsigned long long)(val >> second));
-        atomicOr(&w[x + 1], (unsigned long long)(val << (64 - second)));
+// One block: exclusive sums of the tiles' bits in place; the total behind them.
+__global__ void __launch_bounds__(1024) k_gb_scan(uint64_t* bits, uint64_t tiles) {
+    __shared__ uint64_t ws[32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint64_t carry = 0;
+    for (uint64_t b = 0; b < tiles; b += 1024) {
+        const uint64_t i = b + threadIdx.x, x = i < tiles ? bits[i] : 0ull;
+        uint64_t y = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t z = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= (uint32_t)o) y += z;
+        }
+        if (lane == 31) ws[w] = y;
+        __syncthreads();
+        uint64_t before = carry;
+        for (uint32_t q = 0; q < 32; ++q) {
+            if (q < w) before += ws[q];
+            carry += ws[q];
+        }
+        if (i < tiles) bits[i] = before + y - x;
+        __syncthreads();
     }
+    if (threadIdx.x == 0) bits[tiles] = carry;
 }
 
-__global__ void k_gb_write(const uint64_t* v, uint64_t n, GbParams P, const uint64_t* pos, const uint64_t* woff,
-                           unsigned long long* out) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t r = gb_range_of(P.rbeg, P.nranges, i);
-    const uint64_t b0 = P.rbeg[r];
-    if (i == b0) return;
-    unsigned long long* w = out + woff[r] + 3;
-    uint64_t t = pos[i] - pos[b0];
-    uint64_t q, val;
-    uint32_t kk;
-    gb_code(P, r, v[i] - v[i - 1], q, val, kk);
-    if (q > GB_MAX_Q) return;
-    gb_ones(w, t, q);
-    t += q + 1;  // the zero is already there
-    if (kk) gb_bits(w, t, val, kk);
+// Bits before each range (and behind the last): its tile's and those of the
+// values in the tile before it.  A block per range.
+__global__ void __launch_bounds__(GE_NT) k_gb_range_bits(const uint64_t* v, uint64_t n, GbParams P, const uint64_t* bits,
+                                                       uint64_t tiles, uint64_t* rpos) {
+    const uint32_t r = blockIdx.x;
+    const uint64_t e = P.rbeg[r];
+    uint64_t s = 0;
+    if (e < n)
+        for (uint64_t i = e / GE_TILE * GE_TILE + threadIdx.x; i < e; i += GE_NT)
+            s += gb_code_len(v, i, P, gb_range_of(P.rbeg, P.nranges, i), nullptr);
+    s = gb_block_sum(s);
+    if (threadIdx.x == 0) rpos[r] = e < n ? bits[e / GE_TILE] + s : bits[tiles];
+}
+
+// Appends bits to a zeroed stream, most significant first: a word that the
+// writer fills from its first bit is stored, the others are ORed in.
+struct GbWriter {
+    unsigned long long* w;
+    uint64_t acc;
+    uint32_t a;   // bits of the current word before the next one
+    bool shared;  // the current word's first bits are another's
+    __device__ __forceinline__ void open(unsigned long long* words, uint64_t t) {
+        w = words + (t >> 6);
+        a = (uint32_t)(t & 63);
+        acc = 0;
+        shared = a != 0;
+    }
+    __device__ __forceinline__ void next() {
+        if (shared) atomicOr(w, (unsigned long long)acc);
+        else *w = acc;
+        ++w;
+        acc = 0;
+        a = 0;
+        shared = false;
+    }
+    // the nb (1..64) low bits of x, which has no others
+    __device__ __forceinline__ void put(uint64_t x, uint32_t nb) {
+        if (a + nb < 64) {
+            acc |= x << (64 - a - nb);
+            a += nb;
+            return;
+        }
+        const uint32_t rest = a + nb - 64;  // 0..63
+        acc |= x >> rest;
+        next();
+        if (rest) acc = x << (64 - rest);
+        a = rest;
+    }
+    __device__ __forceinline__ void close() {
+        if (acc) atomicOr(w, (unsigned long long)acc);
+    }
+};
+
+__global__ void __launch_bounds__(GE_NT) k_gb_write(const uint64_t* v, uint64_t n, GbParams P, const uint64_t* bits,
+                                                    const uint64_t* rpos, const uint64_t* woff, unsigned long long* out) {
+    __shared__ uint64_t ws[GE_NT / 32];
+    const uint64_t i0 = (uint64_t)blockIdx.x * GE_TILE + threadIdx.x * GE_IPT;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t r = i0 < n ? gb_range_of(P.rbeg, P.nranges, i0) : 0u;
+    const uint32_t r0 = r;
+    uint64_t sum = 0;
+    for (uint32_t j = 0; j < GE_IPT && i0 + j < n; ++j) {
+        while (i0 + j >= P.rbeg[r + 1]) ++r;  // (ranges without values too)
+        sum += gb_code_len(v, i0 + j, P, r, nullptr);
+    }
+    uint64_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) ws[w] = x;
+    __syncthreads();
+    uint64_t t = bits[blockIdx.x] + x - sum;
+    for (uint32_t q = 0; q < w; ++q) t += ws[q];
+    if (i0 >= n) return;
+    r = r0;
+    GbWriter W;
+    W.open(out + woff[r] + 3, t - rpos[r]);
+    for (uint32_t j = 0; j < GE_IPT && i0 + j < n; ++j) {
+        const uint64_t i = i0 + j;
+        if (i >= P.rbeg[r + 1]) {
+            W.close();
+            while (i >= P.rbeg[r + 1]) ++r;
+            W.open(out + woff[r] + 3, 0);
+        }
+        if (i == P.rbeg[r]) continue;
+        uint64_t q, val;
+        uint32_t kk;
+        gb_code(P, r, v[i] - v[i - 1], q, val, kk);
+        if (q > GB_MAX_Q) continue;  // (an error by now)
+        for (; q >= 64; q -= 64) W.put(~0ull, 64);
+        W.put((2ull << q) - 2, (uint32_t)q + 1);  // q ones, a zero
+        if (kk) W.put(val, kk);
+    }
+    W.close();
 }
 
 // Header words and the ones after the last code (after k_gb_write).
@@ -212,7 +309,8 @@ struct GbBlock {
 // the same place of their chunks read different banks.
 constexpr uint32_t GB_TILE = 256;
 constexpr uint32_t GB_CUT = 1u << 31;  // in a chunk's count: its last code is cut off by the block's end
-constexpr uint32_t GB_STAGE = GB_TILE * (GB_CHUNK_BITS / 64) + 3 * GB_TILE + 2;
+constexpr uint32_t GB_WARM = 32;  // chunks before the tile that its first reading runs in over
+constexpr uint32_t GB_STAGE = (GB_TILE + GB_WARM) * (GB_CHUNK_BITS / 64 + 3) + 2;
 __device__ __forceinline__ uint32_t gb_skew(uint32_t i) { return i + (i >> 5); }
 constexpr size_t GB_SMEM = (size_t)(2 * GB_STAGE + GB_STAGE / 16 + 2) * 4;
 
@@ -283,13 +381,14 @@ __device__ __forceinline__ uint32_t gb_chunk(const GbBlock* blk, uint32_t nb, ui
 }
 
 // Stages the tile's words (the block's threads together) and sets up each
-// thread's reader; cs, ce: the thread's chunk (cs = ce: none).  Returns its
-// block's number.
+// thread's reader for its chunk c (none from nch on); cs, ce: the chunk's bits.
+// The chunks staged are [first, nch or the tile's end).  Returns its block's
+// number.
 __device__ __forceinline__ uint32_t gb_stage(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
-                                             uint32_t nb, uint32_t nch, uint32_t* sw, GbReader& R,
-                                             uint64_t& cs, uint64_t& ce) {
+                                             uint32_t nb, uint32_t nch, uint32_t* sw, GbReader& R, uint32_t c,
+                                             uint32_t first, uint64_t& cs, uint64_t& ce) {
     __shared__ unsigned long long s_range[2];
-    const uint32_t c0 = blockIdx.x * GB_TILE, c = c0 + threadIdx.x, cl = min(nch, c0 + GB_TILE) - 1;
+    const uint32_t cl = min(nch, blockIdx.x * GB_TILE + GB_TILE) - 1;
     uint32_t j = 0xFFFFFFFFu;
     cs = ce = 0;
     R.w = w;
@@ -305,13 +404,13 @@ __device__ __forceinline__ uint32_t gb_stage(const unsigned long long* w, uint64
         R.b = blk[j].b;
         R.little = blk[j].little;
         R.k = blk[j].k;
-        if (c == c0) s_range[0] = cs >> 6;
+        if (c == first) s_range[0] = cs >> 6;
         if (c == cl) s_range[1] = min((ce + 63) / 64 + 2, nwords);
     }
     __syncthreads();
     R.w0 = s_range[0];
     R.w1 = min((uint64_t)s_range[1], R.w0 + GB_STAGE);
-    for (uint32_t i = threadIdx.x; i < (uint32_t)(R.w1 - R.w0); i += GB_TILE) {
+    for (uint32_t i = threadIdx.x; i < (uint32_t)(R.w1 - R.w0); i += blockDim.x) {
         const uint64_t v = w[R.w0 + i];
         sw[gb_skew(2 * i)] = (uint32_t)(v >> 32);
         sw[gb_skew(2 * i + 1)] = (uint32_t)v;
@@ -327,21 +426,28 @@ __device__ __forceinline__ uint32_t gb_stage(const unsigned long long* w, uint64
 // holds is left as it is.  cnt, sum: the codes that start in each chunk and
 // the sum of their gaps; end_out: where each tile stopped; *changed: some
 // tile now stops elsewhere.  A wrong start falls into step after some hundred
-// codes (20 chunks of 40-bit codes), far less than a tile, so two rounds
-// settle the stream.  (Rounds over the whole stream, each re-reading every
+// codes (20 chunks of 40-bit codes), so in round 0 another warp reads the
+// GB_WARM chunks before the tile in step with it and the tile's own start is
+// right already: round 1 then finds nothing to do, and if that ever is not so
+// the rounds go on.  (Without that warp every tile was read again in round 1:
+// 0.31 ms for the four launches, now 0.26.)  (Rounds over the whole stream, each re-reading every
 // chunk, took 21 launches of 0.5 ms for 4e6 hashes, 20.5 of the 29 ms of a
 // there-and-back.)  Bound by the instructions per code and round: where b is a
 // power of two a code's length is its unary part plus a constant, so the
 // repetitions read one funnel-shifted word per code and no remainder (1.08 ->
-// 0.31 ms for the four launches); counts and gap sums are taken once, at the
+// 0.31 ms); counts and gap sums are taken once, at the
 // end.
-__global__ void __launch_bounds__(GB_TILE) k_gb_walk(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
+__global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
                                                      uint32_t nb, uint32_t nch, int round, const uint64_t* end_in,
                                                      uint64_t* end_out, uint64_t* g, uint32_t* cnt,
                                                      unsigned long long* sum, uint32_t* changed) {
     extern __shared__ __align__(16) uint32_t gb_sm[];
-    __shared__ unsigned long long e[GB_TILE];
-    const uint32_t c0 = blockIdx.x * GB_TILE, c = c0 + threadIdx.x;
+    __shared__ unsigned long long e[GB_TILE + GB_WARM];
+    // threads GB_TILE on (round 0): the chunks before the tile
+    const bool warm = threadIdx.x >= GB_TILE;
+    const uint32_t c0 = blockIdx.x * GB_TILE;
+    const uint32_t first = round == 0 && c0 ? c0 - GB_WARM : c0;
+    const uint32_t c = !warm ? c0 + threadIdx.x : c0 ? c0 - GB_WARM + (threadIdx.x - GB_TILE) : nch;
     if (round) {  // the tile's start: unchanged, or settled since the stream's (or the block's) first bit
         uint64_t cs, ce;
         const uint32_t j = gb_chunk(blk, nb, c0, cs, ce);
@@ -353,9 +459,10 @@ __global__ void __launch_bounds__(GB_TILE) k_gb_walk(const unsigned long long* w
     }
     GbReader R;
     uint64_t cs, ce;
-    const uint32_t j = gb_stage(w, nwords, blk, nb, nch, gb_sm, R, cs, ce);
+    const uint32_t j = gb_stage(w, nwords, blk, nb, nch, gb_sm, R, c, first, cs, ce);
     const bool valid = c < nch;
-    const bool chained = valid && threadIdx.x > 0 && blk[j].chunk0 != c;  // starts where the thread before stopped
+    const bool chained = valid && c != first && blk[j].chunk0 != c;  // starts where the thread with the chunk before stopped
+    const uint32_t before = threadIdx.x ? threadIdx.x - 1 : GB_TILE + GB_WARM - 1;
     uint64_t start = valid ? (round ? g[c] : cs) : 0;
     if (round && threadIdx.x == 0) start = end_in[blockIdx.x - 1];
     // the codes a repetition can step over by their unary part alone: b a
@@ -392,25 +499,23 @@ __global__ void __launch_bounds__(GB_TILE) k_gb_walk(const unsigned long long* w
             e[threadIdx.x] = t;
         }
         __syncthreads();
-        redo = chained && e[threadIdx.x - 1] != start;
-        if (redo) start = e[threadIdx.x - 1];
+        redo = chained && e[before] != start;
+        if (redo) start = e[before];
         if (!__syncthreads_or(redo)) break;
     }
+    if (!valid || warm) return;
     uint32_t m = 0;
     unsigned long long s = 0;
-    if (valid) {
-        t = start;
-        while (t < ce) {
-            uint64_t gap;
-            if (!R.read(t, gap)) {
-                t = R.bit1;
-                break;
-            }
-            ++m;
-            s += gap;
+    t = start;
+    while (t < ce) {
+        uint64_t gap;
+        if (!R.read(t, gap)) {
+            t = R.bit1;
+            break;
         }
+        ++m;
+        s += gap;
     }
-    if (!valid) return;
     g[c] = start;
     cnt[c] = m | (t > R.bit1 ? GB_CUT : 0u);
     sum[c] = s;
@@ -527,8 +632,8 @@ __global__ void __launch_bounds__(GB_TILE) k_gb_emit(const unsigned long long* w
     extern __shared__ __align__(16) uint32_t gb_sm[];
     GbReader R;
     uint64_t cs, ce;
-    const uint32_t j = gb_stage(w, nwords, blk, nb, nch, gb_sm, R, cs, ce);
     const uint32_t c = blockIdx.x * GB_TILE + threadIdx.x;
+    const uint32_t j = gb_stage(w, nwords, blk, nb, nch, gb_sm, R, c, blockIdx.x * GB_TILE, cs, ce);
     if (c >= nch) return;
     uint64_t t = g[c];
     uint64_t o = bcnt[blockIdx.x] + pcnt[c] + j + 1;
@@ -581,69 +686,64 @@ int dsss_golomb_encode(dsss_ctx* ctx, const uint64_t* values, const uint64_t* ra
     if (n && !values) return fail(DSSS_EINVAL, "values is NULL");
     DSSS_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t st = (cudaStream_t)stream;
-    const uint64_t N = n ? n : 1, R = nranges ? nranges : 1;
-    auto plan = [&](Carve& c, uint32_t*& len, uint64_t*& pos, uint64_t*& tot, void*& scan, uint64_t*& prm,
-                    uint32_t*& pk, uint64_t*& rbits, uint64_t*& rw, uint64_t*& woff, uint32_t*& err) {
-        len = c.take<uint32_t>(N);
-        pos = c.take<uint64_t>(N);
-        tot = c.take<uint64_t>(1);
-        scan = c.take<unsigned char>(scan_scratch_bytes(N));
-        prm = c.take<uint64_t>(3 * R + 1);  // rbeg, b, little
-        pk = c.take<uint32_t>(R);
-        rbits = c.take<uint64_t>(R);
-        rw = c.take<uint64_t>(R);
-        woff = c.take<uint64_t>(R);
-        err = c.take<uint32_t>(1);
+    const uint64_t R = nranges ? nranges : 1, tiles = (n + GE_TILE - 1) / GE_TILE;
+    const uint64_t prm_bytes = (3 * R + 1) * 8 + R * 4;  // rbeg, b, 2^k - b, k
+    uint64_t *prm, *bits, *rpos, *place;
+    uint32_t* err;
+    auto plan = [&](Carve& c) {
+        prm = (uint64_t*)c.take<unsigned char>(prm_bytes);
+        bits = c.take<uint64_t>(tiles + 1);
+        rpos = c.take<uint64_t>(R + 2);  // the error flags behind it
+        place = c.take<uint64_t>(3 * R);  // the blocks' bits, words and offsets
     };
-    uint32_t *len, *pk, *err;
-    uint64_t *pos, *tot, *prm, *rbits, *rw, *woff;
-    void* scan;
     Carve s0(nullptr);
-    plan(s0, len, pos, tot, scan, prm, pk, rbits, rw, woff, err);
+    plan(s0);
     DSSS_TRY(ensure_ws(ctx, s0.used));
-    DSSS_TRY(ensure_pin(ctx, 8 * (R + 4)));
+    DSSS_TRY(ensure_pin(ctx, prm_bytes + 64));
     Carve c(ctx->ws);
-    plan(c, len, pos, tot, scan, prm, pk, rbits, rw, woff, err);
-    uint64_t* pin = (uint64_t*)ctx->pin;
+    plan(c);
+    err = (uint32_t*)(rpos + R + 1);
+    uint64_t* pin = (uint64_t*)ctx->pin;  // in turn: parameters, rpos, place
     *out_words = 0;
     if (nranges == 0) return DSSS_OK;
-    DSSS_CUDA(cudaMemcpyAsync(prm, rbeg.data(), (nranges + 1) * 8, cudaMemcpyHostToDevice, st));
-    DSSS_CUDA(cudaMemcpyAsync(prm + nranges + 1, bb.data(), nranges * 8, cudaMemcpyHostToDevice, st));
-    DSSS_CUDA(cudaMemcpyAsync(prm + 2 * nranges + 1, little.data(), nranges * 8, cudaMemcpyHostToDevice, st));
-    DSSS_CUDA(cudaMemcpyAsync(pk, kk.data(), nranges * 4, cudaMemcpyHostToDevice, st));
-    DSSS_CUDA(cudaMemsetAsync(err, 0, 4, st));
-    GbParams P{prm, prm + nranges + 1, prm + 2 * nranges + 1, pk, nranges};
+    std::copy(rbeg.begin(), rbeg.end(), pin);
+    std::copy(bb.begin(), bb.end(), pin + R + 1);
+    std::copy(little.begin(), little.end(), pin + 2 * R + 1);
+    std::copy(kk.begin(), kk.end(), (uint32_t*)(pin + 3 * R + 1));
+    DSSS_CUDA(cudaMemcpyAsync(prm, pin, prm_bytes, cudaMemcpyHostToDevice, st));
+    DSSS_CUDA(cudaMemsetAsync(rpos, 0, (R + 2) * 8, st));
+    GbParams P{prm, prm + R + 1, prm + 2 * R + 1, (const uint32_t*)(prm + 3 * R + 1), nranges};
     if (n) {
-        DSSS_LAUNCH("k_gb_len", st, k_gb_len<<<grid_for(n, 256), 256, 0, st>>>(values, n, P, len, err));
-        DSSS_TRY(exclusive_scan_u32_to_u64(len, pos, n, tot, scan, st));
-    } else {
-        DSSS_CUDA(cudaMemsetAsync(tot, 0, 8, st));
+        DSSS_LAUNCH("k_gb_len", st, k_gb_len<<<(unsigned)tiles, GE_NT, 0, st>>>(values, n, P, bits, err));
+        DSSS_LAUNCH("k_gb_scan", st, k_gb_scan<<<1, 1024, 0, st>>>(bits, tiles));
+        DSSS_LAUNCH("k_gb_range_bits", st,
+                    k_gb_range_bits<<<(unsigned)R + 1, GE_NT, 0, st>>>(values, n, P, bits, tiles, rpos));
     }
-    DSSS_LAUNCH("k_gb_range_words", st,
-                k_gb_range_words<<<grid_for(nranges, 128), 128, 0, st>>>(pos, n, tot, P, rbits, rw));
-    DSSS_CUDA(cudaMemcpyAsync(pin, rw, nranges * 8, cudaMemcpyDeviceToHost, st));
-    DSSS_CUDA(cudaMemcpyAsync(pin + nranges, err, 4, cudaMemcpyDeviceToHost, st));
+    DSSS_CUDA(cudaMemcpyAsync(pin, rpos, (R + 2) * 8, cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));
-    const uint32_t e = (uint32_t)(pin[nranges] & 0xFFFFFFFFu);
+    const uint32_t e = (uint32_t)(pin[R + 1] & 0xFFFFFFFFu);
     if (e & 1u) return fail(DSSS_EINVAL, "the values of a range must be ascending");
     if (e & 2u) return fail(DSSS_EINVAL, "a gap needs more than 2^31 unary bits (b too small for the values)");
-    std::vector<uint64_t> wo(nranges);
+    std::vector<uint64_t> at(3 * R);  // a block's bits, words (0 for an empty range) and offset
     uint64_t total = 0;
     for (uint32_t r = 0; r < nranges; ++r) {
-        range_words[r] = pin[r];
-        wo[r] = total;
-        total += pin[r];
+        at[r] = pin[r + 1] - pin[r];
+        at[R + r] = range_words[r] = rbeg[r + 1] == rbeg[r] ? 0 : 3 + (at[r] + 63) / 64;
+        at[2 * R + r] = total;
+        total += range_words[r];
     }
     *out_words = total;
     if (!out) return DSSS_OK;  // size query
     if (total > out_cap) return fail(DSSS_EINVAL, "out_cap %llu below the %llu coded words",
                                      (unsigned long long)out_cap, (unsigned long long)total);
     if (total == 0) return DSSS_OK;
-    DSSS_CUDA(cudaMemcpyAsync(woff, wo.data(), nranges * 8, cudaMemcpyHostToDevice, st));
+    std::copy(at.begin(), at.end(), pin);
+    DSSS_CUDA(cudaMemcpyAsync(place, pin, 3 * R * 8, cudaMemcpyHostToDevice, st));
     DSSS_CUDA(cudaMemsetAsync(out, 0, total * 8, st));
     unsigned long long* o = (unsigned long long*)out;
-    if (n) DSSS_LAUNCH("k_gb_write", st, k_gb_write<<<grid_for(n, 256), 256, 0, st>>>(values, n, P, pos, woff, o));
-    DSSS_LAUNCH("k_gb_head", st, k_gb_head<<<grid_for(nranges, 128), 128, 0, st>>>(values, P, rbits, rw, woff, o));
+    DSSS_LAUNCH("k_gb_write", st, k_gb_write<<<(unsigned)tiles, GE_NT, 0, st>>>(values, n, P, bits, rpos, place + 2 * R, o));
+    DSSS_LAUNCH("k_gb_head", st,
+                k_gb_head<<<grid_for(nranges, 128), 128, 0, st>>>(values, P, place, place + R, place + 2 * R, o));
     DSSS_CUDA(cudaGetLastError());
     DSSS_CUDA(cudaStreamSynchronize(st));
     return DSSS_OK;
@@ -679,17 +779,20 @@ int dsss_golomb_decode(dsss_ctx* ctx, const uint64_t* words, uint64_t nwords, ui
         uint32_t* dnb = c.take<uint32_t>(2);
         DSSS_CUDA(cudaMemsetAsync(dnb, 0, 8, st));
         DSSS_LAUNCH("k_gb_blocks", st, k_gb_blocks<<<1, 1, 0, st>>>(w, nwords, max_blocks, dblk, dnb, dnb + 1));
-        uint32_t* pin = (uint32_t*)ctx->pin;
+        uint64_t* pin64 = (uint64_t*)ctx->pin;
+        uint32_t* pin = (uint32_t*)(pin64 + 4ull * max_blocks);
+        const uint32_t early = max_blocks <= 1024 ? max_blocks : 0;  // a table that small comes along at once
+        if (early) DSSS_CUDA(cudaMemcpyAsync(pin64, dblk, 32ull * early, cudaMemcpyDeviceToHost, st));
         DSSS_CUDA(cudaMemcpyAsync(pin, dnb, 8, cudaMemcpyDeviceToHost, st));
         DSSS_CUDA(cudaStreamSynchronize(st));
         nb = pin[0];
         if (pin[1] & 1u) return fail(DSSS_EINVAL, "a Golomb block runs past the buffer, is too short or has b = 0");
         if (pin[1] & 2u) return fail(DSSS_EINVAL, "more than max_blocks = %u blocks", max_blocks);
-        blk.resize(4ull * nb);
-        uint64_t* pin64 = (uint64_t*)ctx->pin;
-        DSSS_CUDA(cudaMemcpyAsync(pin64, dblk, 32ull * nb, cudaMemcpyDeviceToHost, st));
-        DSSS_CUDA(cudaStreamSynchronize(st));
-        std::copy(pin64, pin64 + 4ull * nb, blk.begin());
+        if (!early) {
+            DSSS_CUDA(cudaMemcpyAsync(pin64, dblk, 32ull * nb, cudaMemcpyDeviceToHost, st));
+            DSSS_CUDA(cudaStreamSynchronize(st));
+        }
+        blk.assign(pin64, pin64 + 4ull * nb);
     }
     // 2. the blocks with their chunks
     std::vector<GbBlock> hb(nb + 1);
@@ -739,36 +842,33 @@ int dsss_golomb_decode(dsss_ctx* ctx, const uint64_t* words, uint64_t nwords, ui
     static std::atomic<uint64_t> walk_configured{0}, emit_configured{0};
     DSSS_TRY(set_smem_once(walk_configured, k_gb_walk, (int)GB_SMEM));
     DSSS_TRY(set_smem_once(emit_configured, k_gb_emit, (int)GB_SMEM));
-    if (nch) {
-        // 3. read the tiles until no tile stops elsewhere (each round settles
-        // at least one more tile of every block)
-        bool settled = false;
-        for (uint32_t round = 0; round <= tiles + 1 && !settled; ++round) {
-            if (round > 1) DSSS_CUDA(cudaMemsetAsync(flags, 0, 4, st));
+    // 3. read the tiles until no tile stops elsewhere (each round settles at
+    // least one more tile of every block); the output places follow every
+    // round from the second on, since that one nearly always is the last:
+    // each block's first value, then its chunks' codes
+    bool settled = false;
+    for (uint32_t round = 0; round <= tiles + 1 && !settled; ++round) {
+        if (nch) {
+            if (round > 1) DSSS_CUDA(cudaMemsetAsync(flags, 0, 8, st));
             DSSS_LAUNCH("k_gb_walk", st,
-                        k_gb_walk<<<tiles, GB_TILE, GB_SMEM, st>>>(w, nwords, dblk, nb, nch, (int)round,
+                        k_gb_walk<<<tiles, GB_TILE + (round ? 0 : GB_WARM), GB_SMEM, st>>>(w, nwords, dblk, nb, nch, (int)round,
                                                                   end[(round & 1) ^ 1], end[round & 1], g, cnt, sum,
                                                                   flags));
             if (round == 0) continue;
-            DSSS_CUDA(cudaGetLastError());
-            DSSS_CUDA(cudaMemcpyAsync(pin, flags, 4, cudaMemcpyDeviceToHost, st));
-            DSSS_CUDA(cudaStreamSynchronize(st));
-            settled = pin[0] == 0;
+            DSSS_LAUNCH("k_gb_prefix", st,
+                        k_gb_prefix<<<tiles, GB_TILE, 0, st>>>(nch, cnt, sum, pcnt, psum, tcnt, tsum, flags + 1));
         }
-        if (!settled) return fail(DSSS_EDEVICE, "Golomb chunk starts did not settle");
+        DSSS_LAUNCH("k_gb_tiles", st, k_gb_tiles<<<1, GB_TILE, 0, st>>>(tiles, tcnt, tsum, bcnt, bsum));
+        DSSS_LAUNCH("k_gb_starts", st,
+                    k_gb_starts<<<grid_for(nb + 1, 128), 128, 0, st>>>(dblk, nb, nch, tiles, bcnt, bsum, pcnt, psum,
+                                                                      ocnt, osum));
+        DSSS_CUDA(cudaGetLastError());
+        DSSS_CUDA(cudaMemcpyAsync(pin64, ocnt, (nb + 1) * 8, cudaMemcpyDeviceToHost, st));
+        DSSS_CUDA(cudaMemcpyAsync(pin, flags, 8, cudaMemcpyDeviceToHost, st));
+        DSSS_CUDA(cudaStreamSynchronize(st));
+        settled = nch == 0 || pin[0] == 0;
     }
-    // 4. output places: each block's first value, then its chunks' codes
-    if (nch)
-        DSSS_LAUNCH("k_gb_prefix", st,
-                    k_gb_prefix<<<tiles, GB_TILE, 0, st>>>(nch, cnt, sum, pcnt, psum, tcnt, tsum, flags + 1));
-    DSSS_LAUNCH("k_gb_tiles", st, k_gb_tiles<<<1, GB_TILE, 0, st>>>(tiles, tcnt, tsum, bcnt, bsum));
-    DSSS_LAUNCH("k_gb_starts", st,
-                k_gb_starts<<<grid_for(nb + 1, 128), 128, 0, st>>>(dblk, nb, nch, tiles, bcnt, bsum, pcnt, psum, ocnt,
-                                                                  osum));
-    DSSS_CUDA(cudaGetLastError());
-    DSSS_CUDA(cudaMemcpyAsync(pin64, ocnt, (nb + 1) * 8, cudaMemcpyDeviceToHost, st));
-    DSSS_CUDA(cudaMemcpyAsync(pin, flags, 8, cudaMemcpyDeviceToHost, st));
-    DSSS_CUDA(cudaStreamSynchronize(st));
+    if (!settled) return fail(DSSS_EDEVICE, "Golomb chunk starts did not settle");
     if (pin[1]) return fail(DSSS_EINVAL, "a Golomb code is cut off by its block's end");
     const uint64_t total = pin64[nb] + nb;
     for (uint32_t j = 0; j < nb; ++j) block_counts[j] = pin64[j + 1] - pin64[j] + 1;

@@ -1087,7 +1087,7 @@ __global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* se
 // The first pass, which is all that most segments need, stands by itself: the
 // rest is one call behind it, whose registers would else cut into the first
 // pass's (1e8 strings in segments of about 700: 1.32 ms inlined, 1.18 ms as a
-// call, 1.03 ms with the five blocks per SM that then fit; six: 1.04).
+// call, 1.03 ms with the five blocks per SM that then fit).
 //
 // What bounds the groups that go deeper is latency, not instructions: a group
 // of the CTA takes a dozen barriers, of the warps a chain of loads per round.
@@ -1099,8 +1099,8 @@ __global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* se
 // a string costs about 60 thread instructions; the stable byte passes with
 // match instructions and bitonic networks that this replaces took 26 warp
 // instructions per string.  B200, 32e6 strings in segments of about 700:
-// 1.12 -> 0.34 ms; a 4e6-string request whose segments are chains of nested
-// prefixes: 0.61 -> 0.17 ms; 9e6 suffixes of copied text: 9.2 -> 3.8 ms.
+// 1.12 -> 0.29 ms; a 4e6-string request whose segments are chains of nested
+// prefixes: 0.61 -> 0.12 ms; 9e6 suffixes of copied text: 9.2 -> 3.8 ms.
 constexpr unsigned FULL = 0xffffffffu;
 enum GroupKind : uint32_t { G_PLAIN = 0, G_TIE = 1, G_ID = 2, G_PSEUDO = 3 };  // G_TIE: keys still to be made
 // Pivot code of a string with LCP l: l below the pivot, CODE_MID for strings
@@ -1459,7 +1459,7 @@ struct SegSmem {
     static constexpr int NW = NT / 32;
     static constexpr int NB = CAP <= 256 ? 1024 : CAP <= 1024 ? 2048 : 4096;  // buckets
     unsigned long long key[CAP];
-    uint32_t cnt[NB + 4];  // bucket counts, then starts (the last one the group's size)
+    __align__(16) uint16_t cnt[NB + 8];  // bucket counts, then starts (the last one the group's size)
     uint32_t id[CAP];
     uint2 wl[CAP / 2];         // groups for the warps
     uint32_t tl[CAP / 2];      // the pass's buckets of 2..TINY_MAX strings
@@ -1566,9 +1566,112 @@ __device__ __forceinline__ void warps_sort_groups(const SortState& S, SegSmem<CA
     }
 }
 
+// The first pass from the buckets' starts (cnt) on; br holds a string's bucket
+// and its place there.  What bounds it is the shared memory's throughput: the
+// counts, places and keys of random buckets take a wavefront for every two or
+// three strings.  So counts are 16 bits wide, a string reads its bucket's start
+// once, buckets join the list by one atomic per warp, and the LCPs are taken in
+// sorted order, from neighbouring keys to neighbouring places (at the buckets'
+// first strings, in the order of the input, they cost a random key and a
+// scattered store each).  1e8 strings: 1.03 -> 1.00 ms, and 0.89 ms with the
+// six blocks per SM that the smaller counts allow (seven or eight: 0.92).  Inside the groups still to be sorted the LCPs written
+// here are not yet right; sort_rest replaces them.
+template <int CAP, int NT>
+__device__ __forceinline__ void first_pass_rest(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bn, uint32_t dep,
+                                                uint32_t kind, const uint32_t (&o)[CAP / NT],
+                                                const uint64_t (&k)[CAP / NT], const uint32_t (&br)[CAP / NT],
+                                                uint32_t* lcp) {
+    constexpr int IPT = CAP / NT;
+    const uint32_t lane = threadIdx.x & 31;
+    const bool all = M.bits.all != 0;
+    bool bad = false;
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+        uint32_t s0 = 0, c = 0;  // its bucket's start and, for the first one there, size
+        if (threadIdx.x + j * NT < bn) {
+            const uint32_t b = br[j] & 0xFFFFu;
+            s0 = M.cnt[b];
+            const uint32_t at = s0 + (br[j] >> 16);
+            if (at < bn) {  // only the counts' sum bounds a place, always so
+                M.key[at] = k[j];
+                M.id[at] = o[j];
+                if (at == s0) c = M.cnt[b + 1] - s0;
+            } else {
+                bad = true;
+            }
+        }
+        const bool tiny = c >= 2 && c <= TINY_MAX;
+        const uint32_t peers = __ballot_sync(FULL, tiny);
+        if (peers) {
+            uint32_t at = 0;
+            if (lane == (uint32_t)__ffs(peers) - 1) at = atomicAdd(&M.nt, __popc(peers));
+            at = __shfl_sync(FULL, at, __ffs(peers) - 1);
+            if (tiny) M.tl[at + __popc(peers & ((1u << lane) - 1u))] = s0 | c << 16;
+        }
+        if (c > TINY_MAX) {
+            uint32_t gk = kind, gd = dep;
+            if (kind != G_ID && all) {  // one key in the bucket
+                const bool ended = key_ended(k[j], false);
+                gk = ended ? G_ID : G_TIE;
+                gd = ended ? dep + key_end(k[j], false) : dep + 8;
+            }
+            const uint2 g = group_pack(s0, c, gk, gd);
+            if (c <= MID_MAX) M.wl[atomicAdd(&M.nw, 1u)] = g;
+            else M.stk[atomicAdd(&M.ns, 1u)] = g;
+        }
+    }
+    if (bad) atomicExch(&S.counters[10], 1u);
+    __syncthreads();
+    // buckets of 2..TINY_MAX strings: insertion sort on (key, id), then the
+    // runs that go deeper
+    const uint32_t nt = M.nt;
+    for (uint32_t e = threadIdx.x; e < nt; e += NT) {
+        const uint32_t s0 = M.tl[e] & 0xFFFFu, c = M.tl[e] >> 16;
+        uint32_t same = 0;  // neighbours that were found equal
+        for (uint32_t x = 1; x < c; ++x) {
+            const uint64_t kx = M.key[s0 + x];
+            const uint32_t ox = M.id[s0 + x];
+            uint32_t y = x;
+            for (; y > 0; --y) {
+                const uint64_t ky = M.key[s0 + y - 1];
+                const uint32_t oy = M.id[s0 + y - 1];
+                same |= ky == kx;
+                if (ky < kx || (ky == kx && oy < ox)) break;
+                M.key[s0 + y] = ky;
+                M.id[s0 + y] = oy;
+            }
+            if (y != x) {
+                M.key[s0 + y] = kx;
+                M.id[s0 + y] = ox;
+            }
+        }
+        if (!same) continue;
+        uint64_t kp = M.key[s0];
+        uint32_t r0 = 0;  // start of the run of equal keys
+        for (uint32_t x = 1; x <= c; ++x) {
+            const uint64_t kx = x < c ? M.key[s0 + x] : ~kp;
+            if (kx == kp) continue;
+            if (x - r0 > 1 && !key_ended(kp, false))
+                M.wl[atomicAdd(&M.nw, 1u)] = group_pack(s0 + r0, x - r0, G_TIE, dep + 8);
+            kp = kx;
+            r0 = x;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+        const uint32_t i = threadIdx.x + j * NT;
+        if (i == 0 || i >= bn) continue;
+        const uint64_t kp = M.key[i - 1], kx = M.key[i];
+        if (kind == G_ID) lcp[i] = dep;
+        else if (kp != kx) lcp[i] = dep + key_lcp(kp, kx);
+        else if (key_ended(kx, false)) lcp[i] = dep + key_end(kx, false);  // equal strings
+    }
+}
+
 // One bucket pass over the CTA's group at [bs, bs + bn): thread t holds its
 // strings t, t + NT, ... (o) and their keys (k).  Every count in cnt is zero
-// before and after.  FIRST: the whole segment, not yet in shared memory, with
+// before and, unless FIRST, after.  FIRST: the whole segment, not yet in shared memory, with
 // plain keys or ids.
 template <int CAP, int NT, bool FIRST>
 __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bs, uint32_t bn, uint32_t dep,
@@ -1649,18 +1752,23 @@ __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M
     // counts; br: the bucket and, above it, the place inside it
 #pragma unroll
     for (int j = 0; j < IPT; ++j)
-        if (threadIdx.x + j * NT < bn) br[j] |= atomicAdd(&M.cnt[br[j]], 1u) << 16;
+        if (threadIdx.x + j * NT < bn) {
+            const uint32_t half = (br[j] & 1u) * 16;
+            br[j] |= atomicAdd(reinterpret_cast<uint32_t*>(M.cnt) + (br[j] >> 1), 1u << half) >> half << 16;
+        }
     __syncthreads();
     {
         uint32_t v[PER], sum = 0;
 #pragma unroll
-        for (int q = 0; q < PER; q += 4) {
+        for (int q = 0; q < PER; q += 8) {
             const uint4 c = *reinterpret_cast<const uint4*>(&M.cnt[threadIdx.x * PER + q]);
-            v[q] = c.x;
-            v[q + 1] = c.y;
-            v[q + 2] = c.z;
-            v[q + 3] = c.w;
-            sum += c.x + c.y + c.z + c.w;
+            const uint32_t p[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                v[q + 2 * h] = p[h] & 0xFFFFu;
+                v[q + 2 * h + 1] = p[h] >> 16;
+                sum += v[q + 2 * h] + v[q + 2 * h + 1];
+            }
         }
         uint32_t x = sum;
 #pragma unroll
@@ -1675,18 +1783,22 @@ __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M
         for (int q = 0; q < NW; ++q)
             if ((uint32_t)q < w) run += M.sum[q];
 #pragma unroll
-        for (int q = 0; q < PER; q += 4) {
-            uint4 c;
-            c.x = run;
-            c.y = c.x + v[q];
-            c.z = c.y + v[q + 1];
-            c.w = c.z + v[q + 2];
-            run = c.w + v[q + 3];
-            *reinterpret_cast<uint4*>(&M.cnt[threadIdx.x * PER + q]) = c;
+        for (int q = 0; q < PER; q += 8) {
+            uint32_t p[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                p[h] = run | (run + v[q + 2 * h]) << 16;
+                run += v[q + 2 * h] + v[q + 2 * h + 1];
+            }
+            *reinterpret_cast<uint4*>(&M.cnt[threadIdx.x * PER + q]) = make_uint4(p[0], p[1], p[2], p[3]);
         }
-        if (threadIdx.x == NT - 1) M.cnt[NB] = run;
+        if (threadIdx.x == NT - 1) M.cnt[NB] = (uint16_t)run;
     }
     __syncthreads();
+    if (FIRST) {
+        first_pass_rest<CAP, NT>(S, M, bn, dep, kind, o, k, br, lcp);
+        return;
+    }
     // places (a thread holds its strings, so the group is permuted in
     // place); only the counts' sum bounds a place, never taken else
     bool bad = false;
@@ -1779,8 +1891,8 @@ __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M
     }
     // the next pass counts from zero
 #pragma unroll
-    for (int q = 0; q < PER; q += 4)
-        *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
+    for (int q = 0; q < PER; q += 8)
+        *reinterpret_cast<uint4*>(&M.cnt[8 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
     __syncthreads();
     if (threadIdx.x == 0) M.nt = 0;  // pushed to again only after the next pass's barriers
 }
@@ -1789,9 +1901,14 @@ __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M
 // warps' list.
 template <int CAP, int NT>
 __device__ __noinline__ void sort_rest(const SortState& S, uint32_t* lcp) {
-    constexpr int IPT = CAP / NT;
+    constexpr int IPT = CAP / NT, PER = SegSmem<CAP, NT>::NB / NT;
     extern __shared__ __align__(16) unsigned char smem[];
     SegSmem<CAP, NT>& M = *reinterpret_cast<SegSmem<CAP, NT>*>(smem);
+#pragma unroll
+    for (int q = 0; q < PER; q += 8)
+        *reinterpret_cast<uint4*>(&M.cnt[8 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x == 0) M.nt = 0;
+    __syncthreads();
     while (M.ns) {
         const uint2 g = M.stk[M.ns - 1];
         const uint32_t bs = group_start(g), bn = group_size(g), dep = g.y;
@@ -1816,7 +1933,7 @@ __device__ __noinline__ void sort_rest(const SortState& S, uint32_t* lcp) {
 }
 
 template <int CAP, int NT>
-__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 5 : 8) k_seg_sort(const __grid_constant__ SortState S,
+__global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 6 : 8) k_seg_sort(const __grid_constant__ SortState S,
                                                                                        const SmallSeg* segs,
                                                                                        uint32_t nseg) {
     constexpr int IPT = CAP / NT, PER = SegSmem<CAP, NT>::NB / NT;
@@ -1845,8 +1962,8 @@ __global__ void __launch_bounds__(NT, CAP >= 4096 ? 2 : CAP >= 1024 ? 5 : 8) k_s
                 if (threadIdx.x + j * NT < size) k[j] = key8_of(S.a, o[j], seg.depth);
         }
 #pragma unroll
-        for (int q = 0; q < PER; q += 4)
-            *reinterpret_cast<uint4*>(&M.cnt[4 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
+        for (int q = 0; q < PER; q += 8)
+            *reinterpret_cast<uint4*>(&M.cnt[8 * threadIdx.x + q * NT]) = make_uint4(0u, 0u, 0u, 0u);
         if (threadIdx.x == 0) M.ns = M.nw = M.nt = M.claim = 0;
         cta_pass<CAP, NT, true>(S, M, 0, size, seg.depth, (seg.flags & F_ID) ? G_ID : G_PLAIN, o, k, lcp);
         if (M.ns | M.nw) sort_rest<CAP, NT>(S, lcp);

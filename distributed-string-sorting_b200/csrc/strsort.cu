@@ -1223,18 +1223,13 @@ __device__ __forceinline__ uint64_t pseudo_key(const ArenaDev& a, StrRef x, StrR
     return (uint64_t)c << 48 | bx >> 16;
 }
 
-// Pseudo key of string id against pivot hid of a group of depth d, and
+// Pseudo key of string x against pivot h of a group of depth d, and
 // whether the comparison ended at the cap; every lane of the warp calls it.
 struct PivotKey {
     uint64_t key;
     bool capped;
 };
-__device__ __forceinline__ PivotKey pivot_key(const ArenaDev& a, uint32_t id, uint32_t hid, uint32_t d, bool active) {
-    StrRef x{0, 0}, h{0, 0};
-    if (active) {
-        x = ref_of(a, id);
-        h = ref_of(a, hid);
-    }
+__device__ __forceinline__ PivotKey pivot_key(const ArenaDev& a, StrRef x, StrRef h, uint32_t d, bool active) {
     const uint32_t l = warp_lcp(a.chars, x, h, d, active);
     PivotKey r{0, false};
     if (active) {
@@ -1307,6 +1302,7 @@ __device__ __forceinline__ void warp_groups(const ArenaDev& a, uint32_t n, uint3
                                             uint32_t (&id)[I], uint32_t* lcp) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t P = n <= 2 ? 2u : 1u << (32 - __clz(n - 1));
+    static_assert(I <= 2, "places are 6 bits");
     uint32_t rs[I];  // start of the element's run
     bool unres[I];   // the run goes on
     bool sort = false;
@@ -1367,15 +1363,37 @@ __device__ __forceinline__ void warp_groups(const ArenaDev& a, uint32_t n, uint3
 #pragma unroll
         for (int q = 0; q < I; ++q) any = any || unres[q];
         if (!__any_sync(FULL, any)) return;
-        // every unresolved run goes on against its first string
-        uint32_t hid[I];
+        // every unresolved run goes on against its first string, the one with
+        // the longest string against that: where one common part is shared up
+        // to different depths, the longest string likely shares the most of it
+        // and leaves none of the others together (a chain of 64 strings: 6
+        // rounds against any of them, 1 or 2 against the longest)
+        StrRef x[I], h[I];
+        uint32_t pv[I], best = 0;
 #pragma unroll
         for (int q = 0; q < I; ++q) {
-            hid[q] = 0;
+            x[q] = StrRef{0, 0};
+            if (unres[q]) {
+                x[q] = ref_of(a, id[q]);
+                best = max(best, min(x[q].len, 0x3FFFFFFu) << 6 | (q * 32 + lane));
+            }
+        }
+        best = __reduce_max_sync(FULL, best) & 63u;
+        uint32_t best_run = __shfl_sync(FULL, rs[0], best & 31u);
+        if (I > 1) {
+            const uint32_t t = __shfl_sync(FULL, rs[I - 1], best & 31u);
+            if (best >= 32) best_run = t;
+        }
 #pragma unroll
-            for (int r = 0; r <= q; ++r) {
-                const uint32_t t = __shfl_sync(FULL, id[r], rs[q] & 31u);
-                if (rs[q] >> 5 == (uint32_t)r) hid[q] = t;
+        for (int q = 0; q < I; ++q) pv[q] = unres[q] && rs[q] == best_run ? best : rs[q];
+#pragma unroll
+        for (int q = 0; q < I; ++q) {
+            h[q] = StrRef{0, 0};
+#pragma unroll
+            for (int r = 0; r < I; ++r) {
+                const uint64_t off = __shfl_sync(FULL, x[r].off, pv[q] & 31u);
+                const uint32_t len = __shfl_sync(FULL, x[r].len, pv[q] & 31u);
+                if (pv[q] >> 5 == (uint32_t)r) h[q] = StrRef{off, len};
             }
         }
         bool capped[I];
@@ -1383,24 +1401,25 @@ __device__ __forceinline__ void warp_groups(const ArenaDev& a, uint32_t n, uint3
         for (int q = 0; q < I; ++q) capped[q] = false;
 #pragma unroll 1
         for (int q = 0; q < I; ++q) {  // one copy of the comparison's code: warps are at different places in it
-            uint32_t qi = id[0], qh = hid[0], qd = dep[0], qt = kind[0], qr = rs[0];
+            StrRef qx = x[0], qh = h[0];
+            uint32_t qd = dep[0], qt = kind[0], qr = pv[0];
             uint64_t qk = key[0];
             bool qu = unres[0];
 #pragma unroll
             for (int r = 1; r < I; ++r)
                 if (r == q) {
-                    qi = id[r];
-                    qh = hid[r];
+                    qx = x[r];
+                    qh = h[r];
                     qd = dep[r];
                     qt = kind[r];
-                    qr = rs[r];
+                    qr = pv[r];
                     qk = key[r];
                     qu = unres[r];
                 }
             if (I > 1 && !__any_sync(FULL, qu)) continue;
             if (qt != G_TIE) qd = tie_depth(qk, qd, qt == G_PSEUDO);
             const bool cmp = qu && q * 32 + lane != qr;
-            const PivotKey t = pivot_key(a, qi, qh, qd, cmp);
+            const PivotKey t = pivot_key(a, qx, qh, qd, cmp);
 #pragma unroll
             for (int r = 0; r < I; ++r)
                 if (r == q && qu) {
@@ -1410,13 +1429,13 @@ __device__ __forceinline__ void warp_groups(const ArenaDev& a, uint32_t n, uint3
                     capped[r] = cmp && t.capped;
                 }
         }
-        // a run's first string keeps to those that agree with it up to the cap
+        // a run's pivot keeps to those that agree with it up to the cap
 #pragma unroll
         for (int q = 0; q < I; ++q)
             for (uint32_t m = __ballot_sync(FULL, capped[q]); m; m &= m - 1) {
-                const uint32_t f = __shfl_sync(FULL, rs[q], __ffs(m) - 1);
+                const uint32_t f = __shfl_sync(FULL, pv[q], __ffs(m) - 1);
 #pragma unroll
-                for (int r = 0; r <= q; ++r)
+                for (int r = 0; r < I; ++r)
                     if (f == r * 32 + lane) key[r] |= 0x010101010101ull;
             }
         sort = true;
@@ -1566,6 +1585,13 @@ __device__ __forceinline__ void warps_sort_groups(const SortState& S, SegSmem<CA
     }
 }
 
+// Whether a bucket of c out of n strings goes on by a pivot although its plain
+// keys still differ: more than three in four together look like a chain of
+// nested prefixes, from which passes over plain keys peel a byte or two each,
+// a pivot pass nearly all.  (1000 strings with shared parts of random length:
+// five plain passes of 5 us before the first pivot pass of 15.)
+__device__ __forceinline__ bool chained(uint32_t c, uint32_t n) { return c > MID_MAX && 4 * c > 3 * n; }
+
 // The first pass from the buckets' starts (cnt) on; br holds a string's bucket
 // and its place there.  What bounds it is the shared memory's throughput: the
 // counts, places and keys of random buckets take a wavefront for every two or
@@ -1610,6 +1636,7 @@ __device__ __forceinline__ void first_pass_rest(const SortState& S, SegSmem<CAP,
         }
         if (c > TINY_MAX) {
             uint32_t gk = kind, gd = dep;
+            if (kind == G_PLAIN && chained(c, bn)) gk = G_TIE;
             if (kind != G_ID && all) {  // one key in the bucket
                 const bool ended = key_ended(k[j], false);
                 gk = ended ? G_ID : G_TIE;
@@ -1838,6 +1865,7 @@ __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M
             continue;
         }
         uint32_t gk = kind, gd = dep;
+        if (kind == G_PLAIN && chained(c, bn)) gk = G_TIE;
         if (kind != G_ID && all) {  // one key in the bucket
             const bool ended = key_ended(k[j], pseudo);
             gk = ended ? G_ID : G_TIE;

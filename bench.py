@@ -577,16 +577,16 @@ def run_path(args, cfg, which):
 
 # Algorithmic bytes of the kernels that carry a roofline, per step of one
 # sort (n strings, lengths L, DP lengths dp, schedule depths 8, 24, 40, 72, ...):
-#   k_prefix   the string sort's first pass over the arena: each string's
-#              first min(L + 1, 72) bytes read once, its 8-byte key and the
-#              four 8-byte prefix hashes of the dense rounds written, its id
-#              and handle read (16 + 4 B): min(L + 1, 72) + 60 per string
-#   k_dp_part  the dense hash round's partition: for every string hashed at
-#              its final depth, the stored 8-byte hash read and the 12-byte
-#              (hash, string) pair written: 20 per string
+#   k_prefix   the string sort's first pass over the arena, with the
+#              prefix hashes that it stored while the sort ran hash rounds;
+#              sort_rooflines reports it as the pass is now
+#   k_pp_scatter1  the dense hash round's partition: for every string hashed
+#              at its final depth, its 8-byte hash read and the 12-byte
+#              (hash, string) pair written: 20 per string (the hash rounds
+#              run in the stage entries only)
 #   k_dp_bucket_dups  the pairs read back: 12 per string
-#   k_dp_lens  per sorted position the 4-byte id read, the 16-byte handle
-#              gathered and 12 bytes written: 32 per string
+#   k_ms_scatter_pay  per position of the global order its PE, id and LCP
+#              read, id, prefix length and rank written: 24
 ROOFLINE_BYTES = {
     "k_prefix": "sum over strings of (min(L + 1, 72) + 36)",
     "k_pp_hist1": "8 per string hashed at its final depth",
@@ -598,9 +598,22 @@ ROOFLINE_BYTES = {
     "k_bucket_direct": "24 per string",
     "k_ms_scatter_pay": "24 per string (the multisplit by PE)",
 }
-SORT_KERNELS = ("k_init", "k_tile_counts", "k_prefix", "k_keys_diff", "k_hist", "k_chunk_sum", "k_seg_scan",
-                "k_scatter", "k_seg_sort", "k_warp_segs", "k_spec", "k_pivot", "k_seg_offsets", "k_split_sample",
-                "k_lcp_fix", "scan_")
+SORT_KERNELS = ("k_init", "k_prefix", "k_keys_diff", "k_hist", "k_seg_scan", "k_scatter", "k_seg_sort",
+                "k_warp_segs", "k_spec", "k_pivot", "k_seg_offsets", "scan_")
+PREFIX_FORMULA = "sum over strings of (min(L + 1, 64) + 20)"
+
+
+def sort_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known=True):
+    """pd_rooflines with the first pass counted as it runs: at most 64 bytes
+    of a string, its offset and length read, its 8-byte key written."""
+    roof = pd_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known)
+    algo = int(np.minimum(np.asarray(lengths, np.uint64) + 1, 64).sum()) + 20 * n
+    for r in (roof["rooflines"].get("k_prefix"), roof["roofline"]):
+        if r and r["kernel"] == "k_prefix":
+            ach = algo / (r["kernel_ms"] * 1e-3) / 1e9 if r["kernel_ms"] > 0 else float("nan")
+            r.update(algo_bytes=algo, achieved=ach, frac=ach / peak,
+                     algo_formula=PREFIX_FORMULA + " (per step: all launches)")
+    return roof
 
 
 def pd_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known=True):
@@ -694,7 +707,7 @@ def bench_config_device(d, torch, name, steps, warmup, peak, peak_kind):
     kt = ctx.kernel_times()
     ctx.set_timing(False)
     lengths = ds.lengths.cpu().numpy().view(np.uint32)
-    roof = pd_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known=False)
+    roof = sort_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known=False)
     res = {"workload": desc + " (generated on the device)", "n": n, "len": L, "p": p, "steps": steps,
            "ms_per_step": ms, "strings_per_s": n / (ms * 1e-3),
            "char_gbs": (int(lengths.astype(np.uint64).sum()) + n) / (ms * 1e-3) / 1e9,
@@ -804,7 +817,7 @@ def main():
     kt = ctx.kernel_times()
     ctx.set_timing(False)
     peak, peak_kind = read_peaks()
-    roof = pd_rooflines(out, hs.lengths, n, kt, args.steps, peak, peak_kind, traffic_known=not gk)
+    roof = sort_rooflines(out, hs.lengths, n, kt, args.steps, peak, peak_kind, traffic_known=not gk)
     char_bytes = int(hs.lengths.astype(np.uint64).sum()) + n
     value = n * world / (ms * 1e-3)
 

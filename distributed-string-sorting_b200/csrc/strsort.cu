@@ -1100,7 +1100,7 @@ __global__ void __launch_bounds__(SC_NT, 2) k_scatter(SortState S, const Seg* se
 // match instructions and bitonic networks that this replaces took 26 warp
 // instructions per string.  B200, 32e6 strings in segments of about 700:
 // 1.12 -> 0.29 ms; a 4e6-string request whose segments are chains of nested
-// prefixes: 0.61 -> 0.12 ms; 9e6 suffixes of copied text: 9.2 -> 3.8 ms.
+// prefixes: 0.61 -> 0.13 ms; 9e6 suffixes of copied text: 9.2 -> 3.8 ms.
 constexpr unsigned FULL = 0xffffffffu;
 enum GroupKind : uint32_t { G_PLAIN = 0, G_TIE = 1, G_ID = 2, G_PSEUDO = 3 };  // G_TIE: keys still to be made
 // Pivot code of a string with LCP l: l below the pivot, CODE_MID for strings

@@ -1,13 +1,9 @@
 // Autotuner: times the full path on the caller's input under every setting of
 // the tuning knobs in a small grid (small-segment cutoff of the string sort,
-// pivot passes, the MSD digit: one key byte, sampled splitters where a key
-// byte splits poorly, the keys' top differing bits in the passes over the
-// arena or inside the segment sorter) and leaves the fastest setting in
-// force.
-// Results never depend on the knobs, so tuning only changes speed.  The
-// digit's bucket count (256) and the scatter tile (2048 strings) are fixed in
-// this build: the shared-memory histograms and the 13-byte-per-string
-// staging of the scatter are sized for them.
+// pivot passes, and the digit knobs, which are accepted without effect since
+// every pass takes its digit from the keys' differing bits) and leaves the
+// fastest setting in force.
+// Results never depend on the knobs, so tuning only changes speed.
 #include <cstdio>
 #include <vector>
 

@@ -155,12 +155,8 @@ int dsss_tune_get(const char* name, int64_t* value);
 /* Autotuner (no reference counterpart): runs the full path (as
  * dsss_pd_sort_batched; nsets = 1 for one set) on the given device input
  * under each setting of a grid of the knobs above (sort_small_max 256 / 1024 /
- * 4096, sort_pivot on / off, and the MSD digit: one key byte, sampled
- * splitters where a key byte splits poorly (sort_split_min 65536), the keys'
- * top differing bits in the passes over the arena where a byte varies in at
- * most four bits (sort_bits 2), in the first pass and inside the segment
- * sorter (sort_bits 3, sort_seg_bits 1), or inside the segment sorter only
- * (sort_seg_bits 1)),
+ * 4096, sort_pivot on / off, and the digit knobs sort_split_min, sort_bits and
+ * sort_seg_bits, which no longer have an effect),
  * 1 + trials runs each, and leaves the fastest setting in force for later
  * calls.  out: the chosen setting (dp_filter_min: the value in force, not
  * searched), its time (minimum over trials) and the default setting's

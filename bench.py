@@ -65,9 +65,9 @@ CONFIGS = {
 # DRAM bytes (read + write) per unit of the kernels that carry a roofline,
 # from one ncu capture each on 8e6 strings x 200 B (D/N 0.25, p = 64); the
 # traffic of a launch grows with its units.  None: not captured.
-DRAM_PER_UNIT = {"k_prefix": 234.6, "k_pp_hist1": None, "k_pp_scatter1": 13.5, "k_pp_hist2": None,
+DRAM_PER_UNIT = {"k_prefix": 205.4, "k_pp_hist1": None, "k_pp_scatter1": 13.5, "k_pp_hist2": None,
                  "k_pp_scatter2": 18.8, "k_dp_bucket_dups": 8.1, "k_dp_lens": None, "k_bucket_direct": 18.1,
-                 "k_ms_scatter_pay": 18.2}
+                 "k_ms_scatter_pay": 19.4}
 
 
 def read_peaks():

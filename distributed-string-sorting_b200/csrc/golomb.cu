@@ -169,6 +169,44 @@ __global__ void __launch_bounds__(GE_NT) k_gb_range_bits(const uint64_t* v, uint
     if (threadIdx.x == 0) rpos[r] = e < n ? bits[e / GE_TILE] + s : bits[tiles];
 }
 
+// The same with more ranges than tiles: a block per tile scans its values once
+// and serves every range that starts there (the last tile also those at n).
+__global__ void __launch_bounds__(GE_NT) k_gb_range_bits_tiled(const uint64_t* v, uint64_t n, GbParams P,
+                                                               const uint64_t* bits, uint64_t tiles, uint64_t* rpos) {
+    __shared__ uint64_t pre[GE_TILE], ws[GE_NT / 32];
+    const uint64_t tb = (uint64_t)blockIdx.x * GE_TILE, i0 = tb + threadIdx.x * GE_IPT;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint32_t len[GE_IPT];
+    uint64_t sum = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < GE_IPT; ++j) {
+        len[j] = i0 + j < n ? gb_code_len(v, i0 + j, P, gb_range_of(P.rbeg, P.nranges, i0 + j), nullptr) : 0u;
+        sum += len[j];
+    }
+    uint64_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31) ws[w] = x;
+    __syncthreads();
+    uint64_t t = bits[blockIdx.x] + x - sum;
+    for (uint32_t q = 0; q < w; ++q) t += ws[q];
+#pragma unroll
+    for (uint32_t j = 0; j < GE_IPT; ++j) {
+        pre[threadIdx.x * GE_IPT + j] = t;
+        t += len[j];
+    }
+    __syncthreads();
+    const uint32_t lo = first_at_least(P.rbeg, P.nranges + 1, tb);
+    const uint32_t hi = blockIdx.x + 1 == tiles ? P.nranges + 1 : first_at_least(P.rbeg, P.nranges + 1, tb + GE_TILE);
+    for (uint32_t r = lo + threadIdx.x; r < hi; r += GE_NT) {
+        const uint64_t e = P.rbeg[r];
+        rpos[r] = e < n ? pre[e - tb] : bits[tiles];
+    }
+}
+
 // Appends bits to a zeroed stream, most significant first: a word that the
 // writer fills from its first bit is stored, the others are ORed in.
 struct GbWriter {
@@ -716,8 +754,12 @@ int dsss_golomb_encode(dsss_ctx* ctx, const uint64_t* values, const uint64_t* ra
     if (n) {
         DSSS_LAUNCH("k_gb_len", st, k_gb_len<<<(unsigned)tiles, GE_NT, 0, st>>>(values, n, P, bits, err));
         DSSS_LAUNCH("k_gb_scan", st, k_gb_scan<<<1, 1024, 0, st>>>(bits, tiles));
-        DSSS_LAUNCH("k_gb_range_bits", st,
-                    k_gb_range_bits<<<(unsigned)R + 1, GE_NT, 0, st>>>(values, n, P, bits, tiles, rpos));
+        if (R + 1 > tiles)
+            DSSS_LAUNCH("k_gb_range_bits", st,
+                        k_gb_range_bits_tiled<<<(unsigned)tiles, GE_NT, 0, st>>>(values, n, P, bits, tiles, rpos));
+        else
+            DSSS_LAUNCH("k_gb_range_bits", st,
+                        k_gb_range_bits<<<(unsigned)R + 1, GE_NT, 0, st>>>(values, n, P, bits, tiles, rpos));
     }
     DSSS_CUDA(cudaMemcpyAsync(pin, rpos, (R + 2) * 8, cudaMemcpyDeviceToHost, st));
     DSSS_CUDA(cudaStreamSynchronize(st));

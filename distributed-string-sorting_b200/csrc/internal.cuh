@@ -193,6 +193,17 @@ __device__ __forceinline__ uint64_t bswap64(uint64_t x) {
     return ((uint64_t)__byte_perm(lo, 0, 0x0123) << 32) | (uint64_t)__byte_perm(hi, 0, 0x0123);
 }
 
+// The first of n ascending values that is at least v (n if none is).
+__device__ __forceinline__ uint32_t first_at_least(const uint64_t* a, uint32_t n, uint64_t v) {
+    uint32_t lo = 0, hi = n;
+    while (lo < hi) {
+        const uint32_t m = lo + (hi - lo) / 2;
+        if (a[m] < v) lo = m + 1;
+        else hi = m;
+    }
+    return lo;
+}
+
 // 8 bytes at an arbitrary address as a little-endian word, from two aligned
 // 8-byte loads.  Reads up to 15 bytes past p; the arena contract pads 32.
 __device__ __forceinline__ uint64_t load_le8(const uint8_t* p) {

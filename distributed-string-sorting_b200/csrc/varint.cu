@@ -120,6 +120,32 @@ __global__ void __launch_bounds__(128) k_varint_bounds(const uint32_t* v, uint64
     if ((threadIdx.x & 31) == 0) out[r] = at[e / VI_TILE] + s;
 }
 
+// The same with more boundaries than tiles: a block per tile scans its sizes
+// once and serves every boundary in it (the last tile also those at n).
+__global__ void __launch_bounds__(VI_NT) k_varint_bounds_tiled(const uint32_t* v, uint64_t n, const uint64_t* at,
+                                                               uint64_t total, const uint64_t* bound, uint32_t nb,
+                                                               uint64_t* out) {
+    __shared__ uint32_t pre[VI_TILE];
+    const uint64_t tb = (uint64_t)blockIdx.x * VI_TILE;
+    uint32_t sz[VI_IPT], s = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < VI_IPT; ++j) {
+        const uint64_t i = tb + threadIdx.x * VI_IPT + j;
+        sz[j] = i < n ? varint_size(v[i]) : 0u;
+        s += sz[j];
+    }
+    uint32_t o = vi_scan(s, nullptr);
+#pragma unroll
+    for (uint32_t j = 0; j < VI_IPT; ++j) {
+        pre[threadIdx.x * VI_IPT + j] = o;
+        o += sz[j];
+    }
+    __syncthreads();
+    const uint32_t lo = first_at_least(bound, nb, tb);
+    const uint32_t hi = blockIdx.x + 1 == gridDim.x ? nb : first_at_least(bound, nb, tb + VI_TILE);
+    for (uint32_t r = lo + threadIdx.x; r < hi; r += VI_NT) out[r] = bound[r] < n ? at[blockIdx.x] + pre[bound[r] - tb] : total;
+}
+
 // The coded bytes are read in aligned 16-byte words from the one that holds
 // the first: 16 of them, mis + m in all from there, per thread.
 struct CodedBytes {
@@ -241,8 +267,13 @@ int dsss_varint_encode(dsss_ctx* ctx, const uint32_t* values, uint64_t n, const 
     if (n) DSSS_LAUNCH("k_varint_write", st, k_varint_write<<<(unsigned)tiles, VI_NT, 0, st>>>(values, n, at, out));
     if (nranges) {
         DSSS_CUDA(cudaMemcpyAsync(bd, range_begin, (nranges + 1) * 8, cudaMemcpyHostToDevice, st));
-        DSSS_LAUNCH("k_varint_bounds", st,
-                    k_varint_bounds<<<grid_for(nranges + 1, 4), 128, 0, st>>>(values, n, at, total, bd, nranges + 1, bo));
+        if (n && nranges >= tiles)
+            DSSS_LAUNCH("k_varint_bounds", st,
+                        k_varint_bounds_tiled<<<(unsigned)tiles, VI_NT, 0, st>>>(values, n, at, total, bd, nranges + 1, bo));
+        else
+            DSSS_LAUNCH("k_varint_bounds", st,
+                        k_varint_bounds<<<grid_for(nranges + 1, 4), 128, 0, st>>>(values, n, at, total, bd, nranges + 1,
+                                                                                 bo));
         DSSS_CUDA(cudaMemcpyAsync(pin, bo, (nranges + 1) * 8, cudaMemcpyDeviceToHost, st));
     }
     DSSS_CUDA(cudaStreamSynchronize(st));

@@ -45,3 +45,14 @@ def test_many_short_blocks(dsss, ctx):
     bs = [int(x) for x in rng.choice([1 << 20, 1 << 44, 12345678901], 3000)]
     v = np.concatenate([np.cumsum(rng.integers(0, 3 * b, c, dtype=np.uint64)) for c, b in zip(counts, bs)])
     trip(dsss, ctx, v, counts, bs)
+
+
+@pytest.mark.parametrize("n,nr", [(2048, 1), (2048, 5000), (4096, 2), (6145, 3), (6145, 4), (30000, 20000)])
+def test_many_ranges(dsss, ctx, n, nr):
+    """More ranges than the encoder's tiles of 2048 values, and fewer; range
+    starts at the tiles' edges, empty ranges at the end."""
+    rng = np.random.default_rng(n + nr)
+    cuts = np.sort(np.concatenate([rng.integers(0, n + 1, nr), np.arange(0, n, 2048)]))
+    counts = np.diff(np.concatenate([[0], cuts, [n, n, n]])).tolist()
+    v = np.cumsum(rng.integers(0, 900, n, dtype=np.uint64))
+    trip(dsss, ctx, v, counts, [256] * len(counts))

@@ -47,3 +47,17 @@ def test_malformed_values(dsss, ctx, at):
     b[at] = 0x81  # cut off
     with pytest.raises(dsss.DsssError):
         dsss.varint_decode(ctx, torch.from_numpy(b).cuda(), at)
+
+
+@pytest.mark.parametrize("n,nr", [(4096, 1), (4096, 2), (4096, 9000), (12288, 3), (12289, 4), (50021, 20000), (1, 7)])
+def test_many_ranges(dsss, orc, ctx, n, nr):
+    """More boundaries than tiles (counted per tile) and fewer (one by one),
+    boundaries at the tiles' edges and at n among them."""
+    v = values(n + nr, n)
+    rng = np.random.default_rng(nr)
+    cuts = np.sort(np.concatenate([rng.integers(0, n + 1, nr), np.minimum(np.arange(0, n, 4096), n)]))
+    ranges = np.diff(np.concatenate([[0], cuts, [n, n]])).tolist()
+    got, per = dsss.varint_encode(ctx, dev(v), ranges)
+    want, wper = orc.varint_encode(v, ranges)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert np.array_equal(per, wper)

@@ -737,11 +737,13 @@ int dsss_golomb_encode(dsss_ctx* ctx, const uint64_t* values, const uint64_t* ra
     Carve s0(nullptr);
     plan(s0);
     DSSS_TRY(ensure_ws(ctx, s0.used));
-    DSSS_TRY(ensure_pin(ctx, prm_bytes + 64));
+    const uint64_t prm_words = (prm_bytes + 7) / 8;
+    DSSS_TRY(ensure_pin(ctx, (prm_words + 3 * R) * 8 + 64));
     Carve c(ctx->ws);
     plan(c);
     err = (uint32_t*)(rpos + R + 1);
-    uint64_t* pin = (uint64_t*)ctx->pin;  // in turn: parameters, rpos, place
+    uint64_t* pin = (uint64_t*)ctx->pin;  // the parameters, then rpos
+    uint64_t* at = pin + prm_words;       // place
     *out_words = 0;
     if (nranges == 0) return DSSS_OK;
     std::copy(rbeg.begin(), rbeg.end(), pin);
@@ -766,7 +768,7 @@ int dsss_golomb_encode(dsss_ctx* ctx, const uint64_t* values, const uint64_t* ra
     const uint32_t e = (uint32_t)(pin[R + 1] & 0xFFFFFFFFu);
     if (e & 1u) return fail(DSSS_EINVAL, "the values of a range must be ascending");
     if (e & 2u) return fail(DSSS_EINVAL, "a gap needs more than 2^31 unary bits (b too small for the values)");
-    std::vector<uint64_t> at(3 * R);  // a block's bits, words (0 for an empty range) and offset
+    // a block's bits, words (0 for an empty range) and offset
     uint64_t total = 0;
     for (uint32_t r = 0; r < nranges; ++r) {
         at[r] = pin[r + 1] - pin[r];
@@ -779,8 +781,7 @@ int dsss_golomb_encode(dsss_ctx* ctx, const uint64_t* values, const uint64_t* ra
     if (total > out_cap) return fail(DSSS_EINVAL, "out_cap %llu below the %llu coded words",
                                      (unsigned long long)out_cap, (unsigned long long)total);
     if (total == 0) return DSSS_OK;
-    std::copy(at.begin(), at.end(), pin);
-    DSSS_CUDA(cudaMemcpyAsync(place, pin, 3 * R * 8, cudaMemcpyHostToDevice, st));
+    DSSS_CUDA(cudaMemcpyAsync(place, at, 3 * R * 8, cudaMemcpyHostToDevice, st));
     DSSS_CUDA(cudaMemsetAsync(out, 0, total * 8, st));
     unsigned long long* o = (unsigned long long*)out;
     DSSS_LAUNCH("k_gb_write", st, k_gb_write<<<(unsigned)tiles, GE_NT, 0, st>>>(values, n, P, bits, rpos, place + 2 * R, o));

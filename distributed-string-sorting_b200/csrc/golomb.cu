@@ -504,10 +504,12 @@ __global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned lo
     uint64_t start = valid ? (round ? g[c] : cs) : 0;
     if (round && threadIdx.x == 0) start = end_in[blockIdx.x - 1];
     // the codes a repetition can step over by their unary part alone: b a
-    // power of two, the word read and the code's end inside the block
+    // power of two, the word read and the code's end inside the block.  Places
+    // are 32 bits from the first staged word; blocks of one value have no
+    // chunk, and enough of them put a chunk of the tile further off.
     const uint64_t o = R.w0 * 64;
     uint32_t lim = 0;
-    if (valid && R.little == 0) {
+    if (valid && R.little == 0 && (ce - o) >> 32 == 0) {
         const uint64_t staged = (R.w1 - R.w0) * 64, left = R.bit1 - o;
         const uint64_t room = min(staged, left);
         if (room > 64ull + R.k + 33) lim = (uint32_t)(room - 64 - R.k - 33);
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned lo
         if (redo) {
             t = start;
             while (t < ce) {
-                const uint32_t u = (uint32_t)(t - o);  // t >= cs >= o: a chunk's codes start inside it
+                const uint32_t u = (uint32_t)(t - o);  // o <= cs <= t < ce: exact wherever lim is not 0
                 if (u < lim) {
                     const uint32_t i = u >> 5;
                     const uint32_t x = __funnelshift_l(gb_sm[gb_skew(i + 1)], gb_sm[gb_skew(i)], u & 31);

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "varint_bytes.cuh"
 
 namespace dsss {
 
@@ -146,19 +147,11 @@ __global__ void __launch_bounds__(VI_NT) k_varint_bounds_tiled(const uint32_t* v
     for (uint32_t r = lo + threadIdx.x; r < hi; r += VI_NT) out[r] = bound[r] < n ? at[blockIdx.x] + pre[bound[r] - tb] : total;
 }
 
-// The coded bytes are read in aligned 16-byte words from the one that holds
-// the first: 16 of them, mis + m in all from there, per thread.
-struct CodedBytes {
-    const uint4* words;
-    uint32_t mis;
-    uint64_t end;  // mis + m
-};
-
 // Bit b: byte b of word i (of the thread) is the last one of a value.
 __device__ __forceinline__ uint32_t value_ends(const CodedBytes& c, uint64_t i, uint4& w) {
     w = make_uint4(0, 0, 0, 0);
     if (16 * i >= c.end) return 0;
-    w = __ldg(c.words + i);
+    w = coded_word(c, i);
     const uint32_t x[4] = {w.x, w.y, w.z, w.w};
     uint32_t m = 0;
 #pragma unroll
@@ -190,7 +183,7 @@ __global__ void __launch_bounds__(VI_NT) k_varint_read(CodedBytes c, const uint3
     uint4 w;
     const uint32_t ends = value_ends(c, i, w);
     *reinterpret_cast<uint4*>(sb + 16 + 16 * threadIdx.x) = w;
-    if (threadIdx.x == 0) *reinterpret_cast<uint4*>(sb) = i ? __ldg(c.words + i - 1) : make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) *reinterpret_cast<uint4*>(sb) = i ? coded_word(c, i - 1) : make_uint4(0, 0, 0, 0);
     uint32_t cnt;
     uint32_t o = vi_scan(__popc(ends), &cnt);  // its barrier covers sb
     const uint32_t first = blockIdx.x ? 0u : c.mis + 16u;  // first byte of the stream in sb
@@ -293,8 +286,7 @@ int dsss_varint_decode(dsss_ctx* ctx, const uint8_t* in, uint64_t nbytes, uint32
         return DSSS_OK;
     }
     if (nbytes >= (1ull << 32)) return fail(DSSS_ENOTSUP, "more than 4 GiB of coded values per call");
-    const CodedBytes coded{reinterpret_cast<const uint4*>((uintptr_t)in & ~(uintptr_t)15), (uint32_t)((uintptr_t)in & 15),
-                           ((uintptr_t)in & 15) + nbytes};
+    const CodedBytes coded = coded_bytes(in, nbytes);
     const uint64_t tiles = (coded.end + VI_TILE - 1) / VI_TILE;
     auto plan = [&](Carve& c, uint32_t*& cnt, uint32_t*& at, void*& scan, uint32_t*& state) {
         cnt = c.take<uint32_t>(tiles);

@@ -168,8 +168,7 @@ int pd_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t nsets, uint32_t p, cons
     uint32_t* lcp = p > 1 && out->merged_lcp ? out->merged_lcp : p == 1 && want_local_lcp ? out->local_lcp : L.lcp;
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, ord, lcp, smax, pin, st,
-                              L.handles));
+        DSSS_TRY(sort_strings(L.sort, a, n, nsets, set_begin.data(), nullptr, ord, lcp, pin, st, L.handles));
     }
     if (p == 1) {  // prefix_doubling.hpp:236: one PE sorts locally and returns no permutation
         for (uint32_t r = 0; r < npe; ++r) out->recv_counts[r] = 0;
@@ -337,7 +336,7 @@ static int ms_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     const uint64_t set_begin[2] = {0, n};
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(L.sort, a, n, 1, set_begin, nullptr, L.ord, out->lcp, smax, pin, st, L.handles));
+        DSSS_TRY(sort_strings(L.sort, a, n, 1, set_begin, nullptr, L.ord, out->lcp, pin, st, L.handles));
     }
     if (!a.h) {  // every string is gathered below
         DSSS_TRY(make_handles(a, L.handles, st));
@@ -712,7 +711,7 @@ static int hq_sort_dev(Ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_
     const uint64_t set_begin[2] = {0, n};
     {
         StageTimer t("stage:sort", st);
-        DSSS_TRY(sort_strings(sl, a, n, 1, set_begin, nullptr, ord, lcp, smax, (uint32_t*)ctx->pin, st, handles));
+        DSSS_TRY(sort_strings(sl, a, n, 1, set_begin, nullptr, ord, lcp, (uint32_t*)ctx->pin, st, handles));
     }
     if (!a.h) {  // every string is gathered below
         DSSS_TRY(make_handles(a, handles, st));
@@ -853,7 +852,7 @@ int dsss_local_sort_lcp(dsss_ctx* ctx, const dsss_arena* in, uint32_t p, const u
     ulonglong2* h = c.take<ulonglong2>(in->n ? in->n : 1);
     layout_sort(c, L, in->n, p, smax);
     ArenaDev a = view(in);
-    return sort_strings(L, a, in->n, p, part_begin, nullptr, order, lcp, smax, (uint32_t*)ctx->pin, st, h);
+    return sort_strings(L, a, in->n, p, part_begin, nullptr, order, lcp, (uint32_t*)ctx->pin, st, h);
 }
 
 int dsss_dp_prefixes(dsss_ctx* ctx, const dsss_arena* in, uint32_t p, const uint64_t* part_begin,

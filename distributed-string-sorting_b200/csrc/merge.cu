@@ -812,7 +812,7 @@ int lcp_merge(Ctx* ctx, const uint8_t* chars, uint64_t bytes, const uint32_t* ch
         DSSS_CUDA(cudaMemcpyAsync(K.tstart + P.nt, &n, 8, cudaMemcpyHostToDevice, st));
         // samples of every run, sorted per receiving PE
         DSSS_LAUNCH("k_kw_samples", st, k_kw_samples<<<nruns, 256, 0, st>>>(L.run_begin, L.run_len, K.sbase, K.samp));
-        DSSS_TRY(sort_strings(K.SL, fa, P.ns, nrecv, P.sb.data(), K.samp, K.ssort, K.slcp, 0, (uint32_t*)ctx->pin, st));
+        DSSS_TRY(sort_strings(K.SL, fa, P.ns, nrecv, P.sb.data(), K.samp, K.ssort, K.slcp, (uint32_t*)ctx->pin, st));
         if (P.ns)
             DSSS_LAUNCH("k_kw_posof", st,
                         k_kw_posof<<<grid_for(P.ns, 256), 256, 0, st>>>(K.ssort, P.ns, L.run_of, L.run_begin, K.sbase,
@@ -830,8 +830,8 @@ int lcp_merge(Ctx* ctx, const uint8_t* chars, uint64_t bytes, const uint32_t* ch
         DSSS_CUDA(cudaMemcpyAsync(ts.data(), K.tstart, (P.nt + 1) * 8, cudaMemcpyDeviceToHost, st));
         DSSS_CUDA(cudaStreamSynchronize(st));
         // every tile sorted on its own, from its strings' shared prefix
-        DSSS_TRY(sort_strings(K.SL, fa, n, (uint32_t)P.nt, ts.data(), K.gathered, order, mlcp, 0, (uint32_t*)ctx->pin,
-                              st, nullptr, K.tdepth));
+        DSSS_TRY(sort_strings(K.SL, fa, n, (uint32_t)P.nt, ts.data(), K.gathered, order, mlcp, (uint32_t*)ctx->pin, st,
+                              nullptr, K.tdepth));
         DSSS_LAUNCH("k_kw_lcp_fix", st,
                     k_kw_lcp_fix<<<grid_for(P.nt, 256), 256, 0, st>>>(f, K.tstart, K.tb, nrecv, order, mlcp));
         DSSS_LAUNCH("k_merge_tags", st,
@@ -852,7 +852,7 @@ int lcp_merge(Ctx* ctx, const uint8_t* chars, uint64_t bytes, const uint32_t* ch
         for (uint32_t r = 0; r < nrecv; ++r) rbnd[r] = rb[(uint64_t)r * p];
         ArenaDev fa{L.full, L.foff, L.flen, n};
         uint32_t* mlcp = merged_lcp ? merged_lcp : L.l[1];
-        DSSS_TRY(sort_strings(SL, fa, n, nrecv, rbnd.data(), nullptr, order, mlcp, 0, (uint32_t*)ctx->pin, st));
+        DSSS_TRY(sort_strings(SL, fa, n, nrecv, rbnd.data(), nullptr, order, mlcp, (uint32_t*)ctx->pin, st));
         DSSS_LAUNCH("k_merge_tags", st,
                     k_merge_tags<<<grid_for(n, 256), 256, 0, st>>>(order, lcp, L.run_start, L.run_of, L.run_begin,
                                                                   L.run_offset, p, n, old_lcp, perm_index, perm_pe));

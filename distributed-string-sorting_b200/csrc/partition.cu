@@ -126,7 +126,7 @@ int partition_pes(const PartitionLayout& L, Ctx* ctx, const ArenaDev& a, uint32_
     const uint64_t sbeg[2] = {0, S};
     // sort_strings synchronises on st before reading its counts back, so the
     // sample positions copied above are consumed before hpin is reused.
-    DSSS_TRY(sort_strings(L.sort, sa, S, 1, sbeg, nullptr, L.sorted, L.slcp, 0, (uint32_t*)hpin, st));
+    DSSS_TRY(sort_strings(L.sort, sa, S, 1, sbeg, nullptr, L.sorted, L.slcp, (uint32_t*)hpin, st));
     uint32_t* hsorted = (uint32_t*)hpin;
     uint64_t* hoff = (uint64_t*)(hpin + (S + 1) / 2 + 1);
     uint32_t* hlen = (uint32_t*)(hoff + S);

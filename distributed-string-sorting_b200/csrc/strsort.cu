@@ -2054,25 +2054,30 @@ static uint32_t clamp_small_max(uint32_t m) {
     return (m == 0 || m > (uint32_t)bin_cap(NBINS - 1)) ? (uint32_t)bin_cap(NBINS - 1) : (m < 2 ? 2 : m);
 }
 
+// Tables of the passes: per possible large segment its record twice and three
+// rows of D words.  Large segments are disjoint and hold more than small_max
+// strings each, so the strings bound their number (and that of a bin's small
+// ones), whatever the number of parts.  The rows take 3 bytes per string at the
+// default cutoff, 12 at 1024 and 48 at 256; below that a segment needs no wide
+// digit.  (Digits of 8 bits at 256: 12 bytes, but 32e6 strings of D/N 0.25 took
+// 6.8 ms instead of 5.4.)
 void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small_max) {
     small_max = clamp_small_max(small_max);
     uint64_t N = n ? n : 1;
+    L.small_max = small_max;
     L.ord[0] = c.take<uint32_t>(N);
     L.ord[1] = c.take<uint32_t>(N);
     L.key[0] = c.take<unsigned long long>(N);
     L.key[1] = c.take<unsigned long long>(N);
-    L.cap_large = N / (small_max + 1) + p + 1;
+    L.cap_large = N / (small_max + 1) + 1;
     L.cap_tiles = N / LT_TILE + L.cap_large + 1;
     L.large[0] = c.take<unsigned char>(L.cap_large * sizeof(Seg));
     L.large[1] = c.take<unsigned char>(L.cap_large * sizeof(Seg));
     for (int b = 0; b < NBINS; ++b) {
-        // segments of a bin are disjoint and larger than the bin below
-        L.cap_small[b] = N / (b ? bin_cap(b - 1) + 1 : 2) + p + 1;
+        L.cap_small[b] = N / (b ? bin_cap(b - 1) + 1 : 2) + 1;
         L.small[b] = c.take<unsigned char>(L.cap_small[b] * sizeof(SmallSeg));
     }
     L.tile0 = c.take<uint32_t>(L.cap_large);
-    // a segment of a few hundred strings needs no wide digit (and such cutoffs
-    // allow many segments)
     L.dbits = small_max >= 256 ? DIGIT_BITS_MAX : 8;
     const uint64_t D = 1ull << L.dbits;
     L.hist = c.take<uint32_t>(L.cap_large * D);
@@ -2083,8 +2088,8 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
 }
 
 int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
-                 const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t small_max,
-                 uint32_t* pin, cudaStream_t st, ulonglong2* handles, const uint32_t* seg_depth) {
+                 const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t* pin, cudaStream_t st,
+                 ulonglong2* handles, const uint32_t* seg_depth) {
     if (n == 0) return DSSS_OK;
     SortState S;
     S.a = a;
@@ -2107,7 +2112,7 @@ int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const
     S.cursor = L.cursor;
     S.dbits = L.dbits;
     S.counters = L.counters;
-    S.small_max = clamp_small_max(small_max);
+    S.small_max = L.small_max;
     S.pivot = tune(TUNE_SORT_PIVOT) ? 1u : 0u;
     S.n = n;
     S.cap_large = L.cap_large;
@@ -2125,7 +2130,6 @@ int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const
     static std::atomic<uint64_t> scatter_configured{0};
     DSSS_TRY(set_smem_once(scatter_configured, k_scatter, (int)SCATTER_SMEM));
     DSSS_CUDA(cudaMemsetAsync(L.counters, 0, 16 * sizeof(uint32_t), st));
-    if (nlarge) DSSS_CUDA(cudaMemsetAsync(L.hist, 0, (L.cap_large << L.dbits) * sizeof(uint32_t), st));
     if (!S.iota) DSSS_LAUNCH("k_init_ids", st, k_init_ids<<<grid_for(n, 256), 256, 0, st>>>(S.ord[0], ids_in, n));
     const bool one = p == 1 && pb_host[0] == 0 && pb_host[1] == n;
     if (!one) DSSS_CUDA(cudaMemcpyAsync(L.pb, pb_host, (p + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
@@ -2136,8 +2140,17 @@ int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const
     // whether the list holds a segment without keys (the first pass, a pivot
     // pass, equal strings): only then the passes that make keys run
     bool keyless = true;
+    uint64_t rows = 0;  // zeroed rows of hist; a pass leaves those it uses zero again
     while (nlarge) {
         if (++guard > (1u << 24)) return fail(DSSS_EDEVICE, "string sort made no progress");
+        if (nlarge > L.cap_large) return fail(DSSS_EDEVICE, "string sort: large-segment list overflow");
+        if (nlarge > rows) {
+            // for the segments there are, with room for the next passes' (all
+            // rows of 1e8 strings are 100 MB, 1.6 GB at a cutoff of 256)
+            const uint64_t to = std::min<uint64_t>(L.cap_large, std::max<uint64_t>(4ull * nlarge, 256));
+            DSSS_CUDA(cudaMemsetAsync(L.hist + (rows << L.dbits), 0, ((to - rows) << L.dbits) * sizeof(uint32_t), st));
+            rows = to;
+        }
         Seg* segs = large[cur];
         Seg* next = large[cur ^ 1];
         // an upper bound for the grids (kernels exit past the real count)
@@ -2159,7 +2172,6 @@ int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const
         nlarge = pin[0];
         keyless = pin[11] != 0;
         if (pin[10]) return fail(DSSS_EDEVICE, "string sort: internal consistency guard tripped");
-        if (nlarge > L.cap_large) return fail(DSSS_EDEVICE, "string sort: large-segment list overflow");
         cur ^= 1;
         S.iota = 0;
         if (nlarge && keyless && handles && !a.h) {

@@ -15,7 +15,7 @@ struct SortLayout {
     uint32_t* cursor;
     uint32_t* counters;
     uint64_t* pb;
-    uint32_t dbits;
+    uint32_t dbits, small_max;
     uint64_t cap_large, cap_small[4], cap_tiles;
 };
 
@@ -34,7 +34,7 @@ void layout_sort(Carve& c, SortLayout& L, uint64_t n, uint32_t p, uint32_t small
 // the sort goes back to the strings in an order other than the arena's; a sort
 // whose first keys tell all strings apart never needs them.
 int sort_strings(const SortLayout& L, ArenaDev& a, uint64_t n, uint32_t p, const uint64_t* pb_host,
-                 const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t small_max,
-                 uint32_t* pin, cudaStream_t st, ulonglong2* handles = nullptr, const uint32_t* seg_depth = nullptr);
+                 const uint32_t* ids_in, uint32_t* ord_out, uint32_t* lcp_out, uint32_t* pin, cudaStream_t st,
+                 ulonglong2* handles = nullptr, const uint32_t* seg_depth = nullptr);
 
 }  // namespace dsss

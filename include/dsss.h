@@ -156,11 +156,12 @@ int dsss_tune_get(const char* name, int64_t* value);
  * dsss_pd_sort_batched; nsets = 1 for one set) on the given device input
  * under each setting of a grid of the knobs above (sort_small_max 256 / 1024 /
  * 4096, sort_pivot on / off, and the digit knobs sort_split_min, sort_bits and
- * sort_seg_bits, which no longer have an effect),
- * 1 + trials runs each, and leaves the fastest setting in force for later
- * calls.  out: the chosen setting (dp_filter_min: the value in force, not
- * searched), its time (minimum over trials) and the default setting's
- * time. */
+ * sort_seg_bits, which no longer have an effect), 1 + trials runs each, and
+ * leaves the fastest setting in force for later calls.  Settings that differ
+ * in the digit knobs alone share their runs and the first of equals wins, so
+ * these stay 0.  out: the chosen setting (dp_filter_min: the value in force,
+ * not searched), its time (minimum over trials), the default setting's time
+ * and the settings compared (30). */
 typedef struct {
     int64_t sort_small_max, sort_pivot, dp_filter_min;
     double best_ms, default_ms;

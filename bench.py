@@ -577,16 +577,19 @@ def run_path(args, cfg, which):
 
 # Algorithmic bytes of the kernels that carry a roofline, per step of one
 # sort (n strings, lengths L, DP lengths dp, schedule depths 8, 24, 40, 72, ...):
-#   k_prefix   the string sort's first pass over the arena, with the
-#              prefix hashes that it stored while the sort ran hash rounds;
-#              sort_rooflines reports it as the pass is now
+#   k_prefix   the string sort's first pass over the arena as it was while
+#              it stored prefix hashes; sort_rooflines counts it as it runs
 #   k_pp_scatter1  the dense hash round's partition: for every string hashed
 #              at its final depth, its 8-byte hash read and the 12-byte
 #              (hash, string) pair written: 20 per string (the hash rounds
 #              run in the stage entries only)
 #   k_dp_bucket_dups  the pairs read back: 12 per string
-#   k_ms_scatter_pay  per position of the global order its PE, id and LCP
-#              read, id, prefix length and rank written: 24
+#   k_ms_scatter_pay  the multisplit by PE (k_local_scatter): per position of
+#              the global order its PE, id and LCP read, id, prefix length and
+#              rank written: 24; the one of tied calls (bucket and two columns
+#              read, three written) the same
+# The sort of the timed path launches k_prefix and k_ms_scatter_pay of these;
+# k_bucket_direct is a label of earlier versions' records.
 ROOFLINE_BYTES = {
     "k_prefix": "sum over strings of (min(L + 1, 72) + 36)",
     "k_pp_hist1": "8 per string hashed at its final depth",
@@ -600,19 +603,51 @@ ROOFLINE_BYTES = {
 }
 SORT_KERNELS = ("k_init", "k_prefix", "k_keys_diff", "k_hist", "k_seg_scan", "k_scatter", "k_seg_sort",
                 "k_warp_segs", "k_spec", "k_pivot", "k_seg_offsets", "scan_")
-PREFIX_FORMULA = "sum over strings of (min(L + 1, 64) + 20)"
+PREFIX_FORMULA = "sum over strings of (min(L + 1, 8 ((D + 15) div 8)) + 20), D = %d bytes shared by all"
+PREFIX_FORMULA_LONG = "sum over strings of (min(L, D) + 13), D = %d bytes shared by all"
+SPEC_MAX = 56  # shared parts below this: the first pass writes the keys too
 
 
-def sort_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known=True):
-    """pd_rooflines with the first pass counted as it runs: at most 64 bytes
-    of a string, its offset and length read, its 8-byte key written."""
+def shared_prefix(out, ds, n):
+    """Bytes that all n strings share: the LCP of the smallest and the largest."""
+    pb = out["part_begin"]
+
+    def text(pos):
+        at = pos if len(pb) == 2 else int(pb[int(out["perm_pe"][pos])]) + int(out["perm_index"][pos])
+        i = int(out["local_order"][at])
+        o, ln = int(ds.offsets[i]), int(ds.lengths[i])
+        return bytes(ds.chars[o:o + ln].tolist())
+
+    return len(os.path.commonprefix([text(0), text(n - 1)])) if n else 0
+
+
+def first_pass_bytes(lengths, shared):
+    """Bytes of the sort's first pass over the arena: the words of a string up
+    to the key behind the shared part (whose last byte may be the NUL), its
+    offset and length read, its 8-byte key written; where the shared part is
+    SPEC_MAX bytes or more it only finds the first byte that differs."""
+    L = np.asarray(lengths, np.uint64)
+    if shared < SPEC_MAX:
+        return int(np.minimum(L + 1, 8 * ((shared + 15) // 8)).sum()) + 20 * len(L), PREFIX_FORMULA % shared
+    return int(np.minimum(L, shared).sum()) + 13 * len(L), PREFIX_FORMULA_LONG % shared
+
+
+def sort_rooflines(out, lengths, n, kt, steps, peak, peak_kind, shared, traffic_known=True):
+    """pd_rooflines with the first pass counted as it runs (shared: the bytes
+    that all strings share) and the multisplits once per launch (a call whose
+    equal strings cross a splitter has a second one)."""
     roof = pd_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known)
-    algo = int(np.minimum(np.asarray(lengths, np.uint64) + 1, 64).sum()) + 20 * n
-    for r in (roof["rooflines"].get("k_prefix"), roof["roofline"]):
-        if r and r["kernel"] == "k_prefix":
-            ach = algo / (r["kernel_ms"] * 1e-3) / 1e9 if r["kernel_ms"] > 0 else float("nan")
-            r.update(algo_bytes=algo, achieved=ach, frac=ach / peak,
-                     algo_formula=PREFIX_FORMULA + " (per step: all launches)")
+    algo, formula = first_pass_bytes(lengths, shared)
+
+    def recount(r, algo, formula):
+        ach = algo / (r["kernel_ms"] * 1e-3) / 1e9 if r["kernel_ms"] > 0 else float("nan")
+        r.update(algo_bytes=algo, achieved=ach, frac=ach / peak, algo_formula=formula + " (per step: all launches)")
+
+    for r in [roof["roofline"]] + list(roof["rooflines"].values()):
+        if r["kernel"] == "k_prefix":
+            recount(r, algo, formula)
+        elif r["kernel"] == "k_ms_scatter_pay":
+            recount(r, int(24 * n * r["launches"]), "24 per string and launch (the multisplits)")
     return roof
 
 
@@ -707,7 +742,7 @@ def bench_config_device(d, torch, name, steps, warmup, peak, peak_kind):
     kt = ctx.kernel_times()
     ctx.set_timing(False)
     lengths = ds.lengths.cpu().numpy().view(np.uint32)
-    roof = sort_rooflines(out, lengths, n, kt, steps, peak, peak_kind, traffic_known=False)
+    roof = sort_rooflines(out, lengths, n, kt, steps, peak, peak_kind, shared_prefix(out, ds, n), traffic_known=False)
     res = {"workload": desc + " (generated on the device)", "n": n, "len": L, "p": p, "steps": steps,
            "ms_per_step": ms, "strings_per_s": n / (ms * 1e-3),
            "char_gbs": (int(lengths.astype(np.uint64).sum()) + n) / (ms * 1e-3) / 1e9,
@@ -817,7 +852,8 @@ def main():
     kt = ctx.kernel_times()
     ctx.set_timing(False)
     peak, peak_kind = read_peaks()
-    roof = sort_rooflines(out, hs.lengths, n, kt, args.steps, peak, peak_kind, traffic_known=not gk)
+    roof = sort_rooflines(out, hs.lengths, n, kt, args.steps, peak, peak_kind, shared_prefix(out, ds, n),
+                          traffic_known=not gk)
     char_bytes = int(hs.lengths.astype(np.uint64).sum()) + n
     value = n * world / (ms * 1e-3)
 

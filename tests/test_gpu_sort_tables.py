@@ -6,7 +6,7 @@ dirty)."""
 import numpy as np
 import pytest
 
-from inputs import random_strings
+from inputs import random_strings, shared_head, with_duplicates
 from test_gpu_parity import u64
 
 pytestmark = pytest.mark.gpu
@@ -39,3 +39,18 @@ def test_rows_as_passes_use_them(dsss, orc, ctx, p, small_max):
     ds = dsss.DeviceStrings(hs)
     dsss.pd_sort(ctx, ds, 3)  # leaves its own data where the rows will be
     check(dsss, orc, ctx, hs, dsss.equal_parts(n, p), small_max)
+
+
+@pytest.mark.parametrize("pivot", [0, 1])
+@pytest.mark.parametrize("small_max", [64, 255, 256, 4096])
+@pytest.mark.parametrize("fam", ["dups", "head", "distinct"])
+def test_digits_and_pivots(dsss, orc, ctx, fam, small_max, pivot):
+    """Digits of 8 and of 10 bits with and without pivot passes; distinct
+    strings need no handles, the others go back to theirs."""
+    n = 40000
+    strs = {"dups": lambda: with_duplicates(random_strings(n, 0, 40, b"ACGT", seed=3), 0.5, seed=4),
+            "head": lambda: shared_head(n, 200, 8, seed=5),
+            "distinct": lambda: random_strings(n, 8, 9, bytes(range(33, 127)), seed=6)}[fam]()
+    hs = dsss.from_bytes_list(strs)
+    with dsss.tuned(sort_pivot=pivot):
+        check(dsss, orc, ctx, hs, dsss.equal_parts(n, 3), small_max)

@@ -380,19 +380,40 @@ struct GbReader {
     // ones up to bit1: the padding); else sets the gap and moves t past the
     // code (t > bit1: the code is cut off).
     __device__ __forceinline__ bool read(uint64_t& t, uint64_t& gap) const {
+        uint64_t v = peek(t);
+        uint32_t ones = (uint32_t)__clzll(~v);
+        if (ones + 1 + k <= 64) {  // the whole code, or the stream's end, in one word
+            if (t + ones >= bit1) return false;
+            t += ones + 1;
+            uint64_t r = 0;
+            if (k) {
+                const uint32_t lo = k - 1;
+                v <<= ones + 1;
+                if (lo) r = v >> (64 - lo);
+                t += lo;
+                if (r >= little) {
+                    r = ((r << 1) | ((v << lo) >> 63)) - little;
+                    ++t;
+                }
+            }
+            gap = ones * b + r;
+            return true;
+        }
         uint64_t q = 0;
-        for (;;) {
-            const uint32_t ones = (uint32_t)__clzll(~peek(t));
+        for (bool zero = ones < 64;;) {
             t += ones;
             q += ones;
             if (t >= bit1) return false;
-            if (ones < 64) break;
+            if (zero) break;
+            const uint32_t left = 64 - (uint32_t)(t & 63);  // to the word's end; a block ends with a word
+            ones = min((uint32_t)__clzll(~(word(t >> 6) << (64 - left))), left);
+            zero = ones < left;
         }
         ++t;  // the zero
         uint64_t r = 0;
         if (k) {
             const uint32_t lo = k - 1;
-            const uint64_t v = peek(t);
+            v = peek(t);
             if (lo) r = v >> (64 - lo);
             t += lo;
             if (r >= little) {
@@ -514,11 +535,18 @@ __global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned lo
         const uint64_t room = min(staged, left);
         if (room > 64ull + R.k + 33) lim = (uint32_t)(room - 64 - R.k - 33);
     }
+    // without such codes a reading counts as it goes; else the counts and gap
+    // sums are taken once, at the end
+    const bool counted = lim == 0;
     bool redo = valid;
     uint64_t t = start;
+    uint32_t m = 0;
+    unsigned long long s = 0;
     for (;;) {
         if (redo) {
             t = start;
+            m = 0;
+            s = 0;
             while (t < ce) {
                 const uint32_t u = (uint32_t)(t - o);  // o <= cs <= t < ce: exact wherever lim is not 0
                 if (u < lim) {
@@ -535,6 +563,8 @@ __global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned lo
                     t = R.bit1;
                     break;
                 }
+                ++m;
+                s += gap;
             }
             e[threadIdx.x] = t;
         }
@@ -544,17 +574,29 @@ __global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned lo
         if (!__syncthreads_or(redo)) break;
     }
     if (!valid || warm) return;
-    uint32_t m = 0;
-    unsigned long long s = 0;
-    t = start;
-    while (t < ce) {
-        uint64_t gap;
-        if (!R.read(t, gap)) {
-            t = R.bit1;
-            break;
+    if (!counted && R.k == 0) {  // b = 1: a zero per code, its gap the ones before it
+        m = 0;
+        uint64_t last = start;  // behind the last zero
+        for (uint64_t p = start; p < t; p += 64) {
+            uint64_t zeros = ~R.peek(p);
+            if (t - p < 64) zeros &= ~0ull << (64 - (t - p));
+            m += (uint32_t)__popcll(zeros);
+            if (zeros) last = p + 65 - (uint32_t)__ffsll((long long)zeros);
         }
-        ++m;
-        s += gap;
+        s = last - start - m;
+    } else if (!counted) {
+        m = 0;
+        s = 0;
+        t = start;
+        while (t < ce) {
+            uint64_t gap;
+            if (!R.read(t, gap)) {
+                t = R.bit1;
+                break;
+            }
+            ++m;
+            s += gap;
+        }
     }
     g[c] = start;
     cnt[c] = m | (t > R.bit1 ? GB_CUT : 0u);

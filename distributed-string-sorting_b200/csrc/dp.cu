@@ -20,14 +20,14 @@
 // The hash table is sized by the number of strings hashed in the round.
 //
 // Where one GPU holds every PE, the global sorted order and its LCPs decide
-// the rounds without a hash (k_local_scatter, project.cu): the strings that share a string's
-// d-byte prefix are its neighbours with LCPs of at least d, all of them still
-// candidates, since they share every shorter prefix too.  So a string stays in
-// the round at depth d exactly while m = max(LCP with its predecessor, LCP
-// with its successor) >= d, and its distinguishing prefix is the schedule's
-// first depth above m, or its length if that is smaller.  (The rounds differ
-// from this only if two different prefixes have the same 64-bit hash.)  The
-// hash rounds are for orders that are sorted per PE only.
+// the rounds without a hash (k_local_scatter, project.cu): the strings that
+// share a string's d-byte prefix are its neighbours with LCPs of at least d, all
+// of them still candidates, since they share every shorter prefix too.  So a
+// string stays in the round at depth d exactly while m = max(LCP with its
+// predecessor, LCP with its successor) >= d, and its distinguishing prefix is
+// the schedule's first depth above m, or its length if that is smaller.  (The
+// rounds differ from this only if two different prefixes have the same 64-bit
+// hash.)  The hash rounds are for orders that are sorted per PE only.
 #include "internal.cuh"
 #include "dp.cuh"
 #include "util.cuh"

@@ -13,16 +13,16 @@
 //
 // Encoding is data-parallel: code lengths summed per tile of values, a scan of
 // the tiles, then each thread puts the codes of its consecutive values together
-// word by word; the words it shares with its neighbours are ORed in.  A variable-length code is read sequentially; the decoder cuts
-// each block's bits into chunks of GB_CHUNK_BITS, reads every chunk from a
-// guessed code start and again from where its predecessor's last code ended,
-// until no start changes.  The first chunk of a block starts right, so the
-// starts are exact once they agree.  A reader that starts inside a code falls
-// into step with the codes after some of them (a few for short remainders,
-// some hundred for 40-bit ones), so the repetitions run inside a block of
-// threads, over 256 chunks in shared memory, and the blocks of threads then
-// agree among themselves in two rounds (in the worst case, as many as the
-// stream has such tiles).
+// word by word; the words it shares with its neighbours are ORed in.  A
+// variable-length code is read sequentially; the decoder cuts each block's bits
+// into chunks of GB_CHUNK_BITS, reads every chunk from a guessed code start and
+// again from where its predecessor's last code ended, until no start changes.
+// The first chunk of a block starts right, so the starts are exact once they
+// agree.  A reader that starts inside a code falls into step with the codes
+// after some of them (a few for short remainders, some hundred for 40-bit
+// ones), so the repetitions run inside a block of threads, over 256 chunks in
+// shared memory, and the blocks of threads then agree among themselves in two
+// rounds (in the worst case, as many as the stream has such tiles).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -489,13 +489,14 @@ __device__ __forceinline__ uint32_t gb_stage(const unsigned long long* w, uint64
 // GB_WARM chunks before the tile in step with it and the tile's own start is
 // right already: round 1 then finds nothing to do, and if that ever is not so
 // the rounds go on.  (Without that warp every tile was read again in round 1:
-// 0.31 ms for the four launches, now 0.26.)  (Rounds over the whole stream, each re-reading every
-// chunk, took 21 launches of 0.5 ms for 4e6 hashes, 20.5 of the 29 ms of a
-// there-and-back.)  Bound by the instructions per code and round: where b is a
-// power of two a code's length is its unary part plus a constant, so the
-// repetitions read one funnel-shifted word per code and no remainder (1.08 ->
-// 0.31 ms); counts and gap sums are taken once, at the
-// end.
+// 0.31 ms for the four launches, now 0.25.  Rounds over the whole stream, each
+// re-reading every chunk, took 21 launches of 0.5 ms for 4e6 hashes, 20.5 of the
+// 29 ms of a there-and-back.)  Bound by the instructions per code and round:
+// where b is a power of two a code's length is its unary part plus a constant,
+// so the repetitions read one funnel-shifted word per code and no remainder
+// (1.08 -> 0.31 ms), and counts and gap sums are taken once, at the end.  Other
+// codes are counted as they are read (b = 3, 2000 values there and back: 1.34 ->
+// 0.76 ms with one read of 64 bits per code).
 __global__ void __launch_bounds__(GB_TILE + GB_WARM) k_gb_walk(const unsigned long long* w, uint64_t nwords, const GbBlock* blk,
                                                      uint32_t nb, uint32_t nch, int round, const uint64_t* end_in,
                                                      uint64_t* end_out, uint64_t* g, uint32_t* cnt,

@@ -38,8 +38,9 @@ constexpr unsigned PJ_FULL = 0xffffffffu;
 // ------------------------------------------------------------- local orders --
 // PE of every position and the PE counts of each tile.  The PE bounds are
 // looked up in shared memory: the PE that equal parts would give, or one of
-// its neighbours; PEs of very uneven sizes fall back to a binary search.  Bound by the 4-byte id read and the 4-byte PE written per
-// position (one pass where finding the PEs and counting them were two).
+// its neighbours; PEs of very uneven sizes fall back to a binary search.
+// Bound by the 4-byte id read and the 4-byte PE written per position (one pass
+// where finding the PEs and counting them were two).
 __global__ void __launch_bounds__(PJ_NT) k_pe_hist(const uint32_t* ord, uint64_t n, const uint64_t* pb, uint32_t npe,
                                                    uint32_t p, uint64_t tiles, uint32_t* pe, uint32_t* bucket,
                                                    uint32_t* hist) {
@@ -674,14 +675,14 @@ int project_local(const ProjectLayout& L, const ArenaDev& a, uint64_t n, uint32_
     static std::atomic<uint64_t> c0{0}, c1{0};
     if (dp) {
         DSSS_TRY(set_smem_once(c0, k_local_scatter<true>, (int)pj_scatter_smem<true>(MAX_SPLIT_BUCKETS)));
-        DSSS_LAUNCH("k_ms_scatter_pay", st,  // the multisplit by PE
+        DSSS_LAUNCH("k_ms_scatter_pay", st,  // timed under the multisplits' label
                     k_local_scatter<true><<<(unsigned)L.tiles, PJ_NT, pj_scatter_smem<true>(npe), st>>>(
                         bucket, ord, lcp, a.len, stats, n, npe, L.tiles, L.off, L.pb, local_order, dp, LcpEdges{}, rank,
                         L.flags));
     } else {
         const LcpEdges E{edges, edges + cells, edges + 2 * cells, lcp_sum};
         DSSS_TRY(set_smem_once(c1, k_local_scatter<false>, (int)pj_scatter_smem<false>(MAX_SPLIT_BUCKETS)));
-        DSSS_LAUNCH("k_ms_scatter_pay", st,  // the multisplit by PE
+        DSSS_LAUNCH("k_ms_scatter_pay", st,  // timed under the multisplits' label
                     k_local_scatter<false><<<(unsigned)L.tiles, PJ_NT, pj_scatter_smem<false>(npe), st>>>(
                         bucket, ord, lcp, a.len, stats, n, npe, L.tiles, L.off, L.pb, local_order, dp, E, rank,
                         L.flags));

@@ -20,7 +20,7 @@ struct ProjectLayout {
     SetSplit* sets;
     uint32_t* bounds;    // npe x (p + 1): where PE g's strings for receiver r start
     uint32_t* start;     // global position where receiver (set, k)'s strings start
-    uint32_t* flags;     // [0] a guard tripped, [1] ties cross a splitter (project_merge_ties)
+    uint32_t* flags;     // [0] a guard tripped, [1] ties cross a splitter (project_buckets)
     uint64_t tiles;
 };
 

@@ -702,9 +702,9 @@ __device__ __forceinline__ void digits_of(const BucketBits& B, const uint64_t (&
     }
 }
 
-// Counts per segment and digit, and the bits in which the keys do differ: a tile's counts in shared memory (a row for
-// every two warps), then one global atomic per digit.  Bound by the 8-byte key
-// read.
+// Counts per segment and digit, and the bits in which the keys do differ: a
+// tile's counts in shared memory (a row for every two warps), then one global
+// atomic per digit.  Bound by the 8-byte key read.
 constexpr int HIST_ROWS = LT_NT / 64;
 __global__ void __launch_bounds__(LT_NT, 4) k_hist(SortState S, Seg* segs, uint32_t nseg) {
     __shared__ uint32_t hist[HIST_ROWS][DIGIT_MAX];
@@ -920,7 +920,8 @@ __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, Seg* n
             // their strings share
             if (big) {
                 // (the code of the pivot itself has no byte behind it)
-                push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO, d == PIVOT_CAP ? 0 : rest & ~(0xFFull << 56));
+                push_large(S, next, cs, total, depth, np | F_KEYS | F_PSEUDO,
+                           d == PIVOT_CAP ? 0 : rest & ~(0xFFull << 56));
             } else {
                 uint32_t cd = depth + pivot_l(d);
                 if (d == PIVOT_CAP) {
@@ -939,7 +940,10 @@ __global__ void __launch_bounds__(256) k_seg_scan(SortState S, Seg* segs, Seg* n
         }
     }
     __syncthreads();
-    if (threadIdx.x < NBINS) s_base[threadIdx.x] = s_small[threadIdx.x] ? atomicAdd(&S.counters[1 + threadIdx.x], s_small[threadIdx.x]) : 0u;
+    if (threadIdx.x < NBINS) {
+        const uint32_t m = s_small[threadIdx.x];
+        s_base[threadIdx.x] = m ? atomicAdd(&S.counters[1 + threadIdx.x], m) : 0u;
+    }
     __syncthreads();
     cs = cs0;
 #pragma unroll
@@ -1495,41 +1499,41 @@ template <int CAP, int NT>
 __device__ __forceinline__ void cta_pivot_keys(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bs, uint32_t bn, uint32_t dep) {
     constexpr int NW = NT / 32, IPT = CAP / NT;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-                    // the pivot: of 8 evenly spaced strings the one with the
-                    // largest sum of LCPs (256 bytes at most) with the others
-                    for (uint32_t c = w; c < 8; c += NW) {
-                        const StrRef x = ref_of(S.a, M.id[bs + c * bn / 8]);
-                        const uint64_t kx = key8(S.a.chars, x.off, x.len, dep + 8 * lane);
-                        uint32_t sum = 0;
-    #pragma unroll 4
-                        for (uint32_t q = 0; q < 8; ++q) {
-                            const StrRef y = ref_of(S.a, M.id[bs + q * bn / 8]);
-                            const uint64_t ky = key8(S.a.chars, y.off, y.len, dep + 8 * lane);
-                            const uint32_t e = kx != ky ? key_lcp(kx, ky) : 8u;
-                            const uint32_t hit = __ballot_sync(FULL, e < 8);
-                            const int f = hit ? __ffs(hit) - 1 : 0;
-                            const uint32_t ef = __shfl_sync(FULL, e, f);
-                            sum += hit ? 8 * f + ef : 256u;
-                        }
-                        if (lane == 0) M.piv[c] = sum << 3 | c;
-                    }
-                    __syncthreads();
-                    uint32_t best = 0;
-    #pragma unroll
-                    for (int c = 0; c < 8; ++c) best = max(best, M.piv[c]);
-                    const uint32_t pid = M.id[bs + (best & 7u) * bn / 8];
-                    const StrRef h = ref_of(S.a, pid);
-    #pragma unroll 1
-                    for (int j = 0; j < IPT; ++j) {
-                        const uint32_t i = threadIdx.x + j * NT;
-                        if (i - lane >= bn) break;  // the same for the whole warp
-                        const bool v = i < bn;
-                        StrRef x{0, 0};
-                        uint32_t oj = v ? M.id[bs + i] : 0u;
-                        if (v) x = ref_of(S.a, oj);
-                        const uint32_t l = warp_lcp(S.a.chars, x, h, dep, v);
-                        if (v) M.key[bs + i] = pseudo_key(S.a, x, h, l, dep);
-                    }
+    // the pivot: of 8 evenly spaced strings the one with the largest sum of LCPs
+    // (256 bytes at most) with the others
+    for (uint32_t c = w; c < 8; c += NW) {
+        const StrRef x = ref_of(S.a, M.id[bs + c * bn / 8]);
+        const uint64_t kx = key8(S.a.chars, x.off, x.len, dep + 8 * lane);
+        uint32_t sum = 0;
+#pragma unroll 4
+        for (uint32_t q = 0; q < 8; ++q) {
+            const StrRef y = ref_of(S.a, M.id[bs + q * bn / 8]);
+            const uint64_t ky = key8(S.a.chars, y.off, y.len, dep + 8 * lane);
+            const uint32_t e = kx != ky ? key_lcp(kx, ky) : 8u;
+            const uint32_t hit = __ballot_sync(FULL, e < 8);
+            const int f = hit ? __ffs(hit) - 1 : 0;
+            const uint32_t ef = __shfl_sync(FULL, e, f);
+            sum += hit ? 8 * f + ef : 256u;
+        }
+        if (lane == 0) M.piv[c] = sum << 3 | c;
+    }
+    __syncthreads();
+    uint32_t best = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) best = max(best, M.piv[c]);
+    const uint32_t pid = M.id[bs + (best & 7u) * bn / 8];
+    const StrRef h = ref_of(S.a, pid);
+#pragma unroll 1
+    for (int j = 0; j < IPT; ++j) {
+        const uint32_t i = threadIdx.x + j * NT;
+        if (i - lane >= bn) break;  // the same for the whole warp
+        const bool v = i < bn;
+        StrRef x{0, 0};
+        uint32_t oj = v ? M.id[bs + i] : 0u;
+        if (v) x = ref_of(S.a, oj);
+        const uint32_t l = warp_lcp(S.a.chars, x, h, dep, v);
+        if (v) M.key[bs + i] = pseudo_key(S.a, x, h, l, dep);
+    }
 }
 
 // The groups on the warps' list, claimed up to 8 at a time; as many of these
@@ -1600,8 +1604,9 @@ __device__ __forceinline__ bool chained(uint32_t c, uint32_t n) { return c > MID
 // sorted order, from neighbouring keys to neighbouring places (at the buckets'
 // first strings, in the order of the input, they cost a random key and a
 // scattered store each).  1e8 strings: 1.03 -> 1.00 ms, and 0.89 ms with the
-// six blocks per SM that the smaller counts allow (seven or eight: 0.92).  Inside the groups still to be sorted the LCPs written
-// here are not yet right; sort_rest replaces them.
+// six blocks per SM that the smaller counts allow (seven or eight: 0.92).
+// Inside the groups still to be sorted the LCPs written here are not yet right;
+// sort_rest replaces them.
 template <int CAP, int NT>
 __device__ __forceinline__ void first_pass_rest(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bn, uint32_t dep,
                                                 uint32_t kind, const uint32_t (&o)[CAP / NT],
@@ -1698,8 +1703,8 @@ __device__ __forceinline__ void first_pass_rest(const SortState& S, SegSmem<CAP,
 
 // One bucket pass over the CTA's group at [bs, bs + bn): thread t holds its
 // strings t, t + NT, ... (o) and their keys (k).  Every count in cnt is zero
-// before and, unless FIRST, after.  FIRST: the whole segment, not yet in shared memory, with
-// plain keys or ids.
+// before and, unless FIRST, after.  FIRST: the whole segment, not yet in shared
+// memory, with plain keys or ids.
 template <int CAP, int NT, bool FIRST>
 __device__ __forceinline__ void cta_pass(const SortState& S, SegSmem<CAP, NT>& M, uint32_t bs, uint32_t bn, uint32_t dep,
                                          uint32_t kind, const uint32_t (&o)[CAP / NT], const uint64_t (&k)[CAP / NT],
